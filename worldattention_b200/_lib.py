@@ -6,12 +6,14 @@ fails with an explicit error.  Build the library with `python -m worldattention_
 from __future__ import annotations
 
 import ctypes as C
+import importlib.util
 import os
 from typing import Optional
 
 import torch
 
 _HERE = os.path.dirname(os.path.abspath(__file__))
+HOST_PATH = os.path.join(_HERE, "_host.so")
 LIB_PATH = os.environ.get("WORLDATTENTION_B200_LIB") or os.path.join(_HERE, "libwa_b200.so")
 
 WA_F32, WA_BF16 = 0, 1
@@ -119,6 +121,26 @@ def lib() -> C.CDLL:
             raise RuntimeError("libwa_b200.so ABI mismatch (version or wa_hsa_params layout); rebuild the library")
         _lib = handle
     return _lib
+
+
+_host = None
+
+
+def host():
+    """The native host module (csrc/host), loaded once and bound to the library's entry points."""
+    global _host
+    if _host is None:
+        if not os.path.exists(HOST_PATH):
+            raise RuntimeError(f"{HOST_PATH} is missing: the host module has not been built (run `python -m worldattention_b200.build`)")
+        handle = lib()
+        spec = importlib.util.spec_from_file_location("worldattention_b200._host", HOST_PATH)
+        module = importlib.util.module_from_spec(spec)
+        spec.loader.exec_module(module)
+        module.bind({name: C.cast(getattr(handle, name), C.c_void_p).value for name in SIGNATURES},
+                    lambda index: status_word(torch.device("cuda", index)).data_ptr(),
+                    lambda index: raise_if_failed(torch.device("cuda", index)))
+        _host = module
+    return _host
 
 
 def check(rc: int) -> None:

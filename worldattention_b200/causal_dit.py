@@ -84,46 +84,15 @@ def rope_table(head_dim: int, rows: int = 1024) -> torch.Tensor:
     return torch.cat([band(d - 4 * (d // 6)), band(2 * (d // 6)), band(2 * (d // 6))], dim=1)
 
 
-def _frame_vectors(e: Optional[torch.Tensor], dim: int):
-    """`[B, F, 1, C]` modulation view -> (pointer, elements between consecutive frames); it must step uniformly over (b, f)."""
-    if e is None:
-        return None, 0
-    b, f = e.shape[:2]
-    if e.stride(-1) != 1 or e.shape[-1] != dim or (b > 1 and e.stride(0) != f * e.stride(1)):
-        e = e.contiguous()
-    return e.data_ptr(), e.stride(1)
-
-
 def ln_modulate(x: torch.Tensor, eps: float, *, weight=None, bias=None, scale=None, shift=None, tokens_per_frame: int = 1):
     """`LayerNorm(x) [* weight + bias]`, then `* (1 + scale) + shift` per frame, in one pass over bf16 `[B, L, C]`
     (causal_model.py:616-619, 642-646; model.py:89-103)."""
-    dev = _lib.require_cuda(x)
-    if x.dtype != torch.bfloat16:
-        raise NotImplementedError("the fused block glue is bf16 only")
-    x = x.contiguous()
-    out = torch.empty_like(x)
-    c = x.shape[-1]
-    sp, s_stride = _frame_vectors(scale, c)
-    hp, h_stride = _frame_vectors(shift, c)
-    if sp is not None and hp is not None and s_stride != h_stride:
-        raise ValueError("scale and shift must share a layout")
-    _lib.check(_lib.lib().wa_ln_modulate(x.data_ptr(), out.data_ptr(), x.numel() // c, c, float(eps), _lib.ptr(weight), _lib.ptr(bias),
-                                         sp, hp, s_stride or h_stride, int(tokens_per_frame), _lib.stream_ptr(dev)))
-    return out
+    return _lib.host().ln_modulate(x, eps, weight, bias, scale, shift, tokens_per_frame)
 
 
 def gated_residual(x: torch.Tensor, y: torch.Tensor, gate=None, *, tokens_per_frame: int = 1):
     """`x + y * gate` per frame (gate None: `x + y`) in one pass (causal_model.py:633, 637-638, 647-648)."""
-    dev = _lib.require_cuda(x)
-    if x.dtype != torch.bfloat16 or y.dtype != torch.bfloat16:
-        raise NotImplementedError("the fused block glue is bf16 only")
-    x, y = x.contiguous(), y.contiguous()
-    out = torch.empty_like(x)
-    c = x.shape[-1]
-    gp, g_stride = _frame_vectors(gate, c)
-    _lib.check(_lib.lib().wa_gated_residual(x.data_ptr(), y.data_ptr(), out.data_ptr(), x.numel() // c, c, gp, g_stride,
-                                            int(tokens_per_frame), _lib.stream_ptr(dev)))
-    return out
+    return _lib.host().gated_residual(x, y, gate, tokens_per_frame)
 
 
 class _RMSNorm(nn.Module):   # model.py:70-86

@@ -10,7 +10,6 @@ Inference only: the CUDA forward builds no autograd graph.
 """
 from __future__ import annotations
 
-import ctypes
 import math
 
 import torch
@@ -82,9 +81,6 @@ def _compress_blhd(k, v, *, segment_len, k_proj_mat, v_proj_mat, block_size):
     return out_k, out_v
 
 
-_append_workspaces: dict = {}
-
-
 def append_kv(k_new, v_new, k_cache, v_cache, k_coarse, v_coarse, *, position: int, segment_len: int, k_proj_mat, v_proj_mat,
               block_size: int) -> None:
     """Write `n_new` token rows into the K/V cache at `position` and compress the segments they complete, in ONE kernel.
@@ -95,41 +91,21 @@ def append_kv(k_new, v_new, k_cache, v_cache, k_coarse, v_coarse, *, position: i
     cache rows themselves (rows already in place): then the call only compresses.  Shapes the fused kernel does not cover
     go through a copy and `compress_kv`.
     """
-    dev = _lib.require_cuda(k_new, v_new, k_cache, v_cache, k_coarse, v_coarse)
-    bsz, n_new, heads, head_dim = k_new.shape
-    if position % segment_len:
-        raise ValueError(f"rows are appended at segment boundaries, got position={position}, segment_len={segment_len}")
-    if position + n_new > k_cache.shape[1]:
-        raise ValueError("the rows do not fit the cache")
-    pk = k_proj_mat.detach().to(device=dev).contiguous()
-    pv = v_proj_mat.detach().to(device=dev, dtype=pk.dtype).contiguous()
-    lib = _lib.lib()
-    need = lib.wa_kv_append_workspace_bytes(bsz, n_new, heads, head_dim, segment_len, block_size, pk.shape[0])
-    key = (dev, torch.cuda.current_stream(dev).cuda_stream)
-    ws = _append_workspaces.get(key)
-    if ws is None or ws.numel() < need:
-        ws = torch.zeros(max(need, 1 << 16), device=dev, dtype=torch.uint8)      # zeroed once; every call leaves it zeroed
-        _append_workspaces[key] = ws
-    with _lib.device_guard(dev):
-        rc = lib.wa_kv_append_compress(
-            _lib.t4_blhd(k_new), _lib.t4_blhd(v_new), _lib.t4_blhd(k_cache), _lib.t4_blhd(v_cache), _lib.t4_blhd(k_coarse),
-            _lib.t4_blhd(v_coarse), bsz, n_new, int(position), heads, head_dim, int(segment_len), int(block_size), pk.data_ptr(),
-            pv.data_ptr(), _lib.dtype_code(pk.dtype), pk.shape[0], pk.shape[1], ws.data_ptr(), ws.numel(), _lib.stream_ptr(dev))
-    if rc == _lib.WA_ERR_UNSUPPORTED:
-        rows_k, rows_v = k_cache[:, position:position + n_new], v_cache[:, position:position + n_new]
-        if rows_k.data_ptr() != k_new.data_ptr():
-            rows_k.copy_(k_new)
-            rows_v.copy_(v_new)
-        per_segment = min(pk.shape[0], math.ceil(segment_len / block_size))      # slots of a whole segment in the cache
-        for s0 in range(0, n_new, segment_len):                                 # the last segment may be short (fewer slots)
-            s1 = min(n_new, s0 + segment_len)
-            kn, vn = _compress_blhd(rows_k[:, s0:s1], rows_v[:, s0:s1], segment_len=segment_len, k_proj_mat=pk, v_proj_mat=pv,
-                                    block_size=block_size)
-            first = (position + s0) // segment_len * per_segment
-            k_coarse[:, first:first + kn.shape[1]].copy_(kn)
-            v_coarse[:, first:first + vn.shape[1]].copy_(vn)
+    if _lib.host().append_kv(k_new, v_new, k_cache, v_cache, k_coarse, v_coarse, position, segment_len, k_proj_mat, v_proj_mat, block_size):
         return
-    _lib.check(rc)
+    n_new = k_new.shape[1]
+    rows_k, rows_v = k_cache[:, position:position + n_new], v_cache[:, position:position + n_new]
+    if rows_k.data_ptr() != k_new.data_ptr():
+        rows_k.copy_(k_new)
+        rows_v.copy_(v_new)
+    per_segment = min(k_proj_mat.shape[0], math.ceil(segment_len / block_size))      # slots of a whole segment in the cache
+    for s0 in range(0, n_new, segment_len):                                 # the last segment may be short (fewer slots)
+        s1 = min(n_new, s0 + segment_len)
+        kn, vn = _compress_blhd(rows_k[:, s0:s1], rows_v[:, s0:s1], segment_len=segment_len, k_proj_mat=k_proj_mat, v_proj_mat=v_proj_mat,
+                                block_size=block_size)
+        first = (position + s0) // segment_len * per_segment
+        k_coarse[:, first:first + kn.shape[1]].copy_(kn)
+        v_coarse[:, first:first + vn.shape[1]].copy_(vn)
 
 
 def compress_kv(k, v, *, segment_len: int, k_proj_mat, v_proj_mat, block_size: int):
@@ -231,110 +207,18 @@ def hsa_attention(
     """
     if (k_coarse is None) != (v_coarse is None):
         raise ValueError("k_coarse and v_coarse must be provided together")
-    resolve_backend(backend)
-
-    bsz, q_len, heads, head_dim = q.shape
-    kv_len = k.shape[1]
-    if q_len <= 0 or kv_len <= 0:
-        raise ValueError("q_len and kv_len must be positive")
-    dev = _lib.require_cuda(q, k, v, k_coarse, v_coarse)
-    _lib.raise_if_failed(dev)
-
-    p = _lib.HsaParams()
-    p.B, p.H, p.D, p.Lq, p.Lkv = bsz, heads, head_dim, q_len, kv_len
-    p.block_size = int(block_size)
-    p.tau_min, p.tau_max = float(tau_min), float(tau_max)
-    p.flags = _lib.WA_HSA_FORCE_GENERIC if force_generic else 0
-    p.status_mirror = _lib.status_word(dev).data_ptr()
-    q, k, v = _unit_last(q), _unit_last(k), _unit_last(v.to(k.dtype))
-    keep = [q, k, v]
-    p.q, p.k, p.v = _lib.t4_blhd(q), _lib.t4_blhd(k), _lib.t4_blhd(v)
-    if k_pooled_cache is not None:
-        n_blocks = -(-kv_len // int(block_size))
-        if (k_pooled_cache.dtype != torch.float32 or tuple(k_pooled_cache.shape) != (bsz, heads, n_blocks, head_dim)
-                or not k_pooled_cache.is_contiguous() or k_pooled_cache.device != dev):
-            raise ValueError(f"expected k_pooled_cache: contiguous float32 [{bsz}, {heads}, {n_blocks}, {head_dim}] on {dev}")
-        if not 0 <= int(k_pooled_valid) <= n_blocks:
-            raise ValueError(f"k_pooled_valid must be in [0, {n_blocks}], got {k_pooled_valid}")
-        p.k_pooled, p.k_pooled_valid = k_pooled_cache.data_ptr(), int(k_pooled_valid)
-        keep.append(k_pooled_cache)
-
-    if k_coarse is not None:
-        if k_coarse.shape[0] != bsz or tuple(k_coarse.shape[2:]) != (heads, head_dim):
-            raise ValueError(
-                f"expected k_coarse shaped [B, Lc, {heads}, {head_dim}], got {tuple(k_coarse.shape)}"
-            )
-        if v_coarse.shape != k_coarse.shape:
-            raise ValueError("v_coarse must have the same shape as k_coarse")
-        k_coarse, v_coarse = _unit_last(k_coarse.to(v_coarse.dtype)), _unit_last(v_coarse)
-        p.Lc = k_coarse.shape[1]
-        p.k_coarse, p.v_coarse = _lib.t4_blhd(k_coarse), _lib.t4_blhd(v_coarse)
-        keep += [k_coarse, v_coarse]
-    else:
-        if k_proj_mat.shape != v_proj_mat.shape:
-            raise ValueError(
-                "k_proj_mat and v_proj_mat must have the same shape, got "
-                f"{tuple(k_proj_mat.shape)} and {tuple(v_proj_mat.shape)}"
-            )
-        seg = proj_segment_len if proj_segment_len > 0 else kv_len
-        if min(seg, kv_len) > k_proj_mat.shape[1]:
-            raise ValueError(
-                f"segment length {min(seg, kv_len)} exceeds projection length {k_proj_mat.shape[1]}; "
-                "increase proj_segment_len"
-            )
-        pk = k_proj_mat.detach().to(device=dev).contiguous()
-        pv = v_proj_mat.detach().to(device=dev, dtype=pk.dtype).contiguous()
-        keep += [pk, pv]
-        p.Lc = 0
-        p.proj_segment_len, p.proj_rank, p.proj_cols = int(seg), pk.shape[0], pk.shape[1]
-        p.proj_dtype = _lib.dtype_code(pk.dtype)
-        p.k_proj, p.v_proj = pk.data_ptr(), pv.data_ptr()
-
-    if gate_lin is not None:
-        gw = gate_lin.weight.detach().to(device=dev).contiguous()
-        gb = gate_lin.bias.detach().to(device=dev, dtype=gw.dtype).contiguous() if gate_lin.bias is not None else None
-        keep += [gw, gb]
-        p.gate_dtype = _lib.dtype_code(gw.dtype)
-        p.gate_w, p.gate_b = gw.data_ptr(), _lib.ptr(gb)
-
-    if topk_per_head is not None:
-        topk = topk_per_head.to(device=dev, dtype=torch.int32).contiguous()
-        if topk.numel() != heads:
-            raise ValueError(f"topk_per_head must have {heads} entries")
-        keep.append(topk)
-        p.topk_per_head = topk.data_ptr()
-
-    out = torch.empty((bsz, q_len, heads, head_dim), device=dev, dtype=q.dtype)
-    p.out = _lib.t4_blhd(out)
-
-    routing = None
-    if return_routing:
-        nq, nkv = math.ceil(q_len / block_size), math.ceil(kv_len / block_size)
-        index = torch.empty((bsz, heads, nq, nkv), device=dev, dtype=torch.int32)
-        num = torch.empty((bsz, heads, nq), device=dev, dtype=torch.int32)
-        thresholds = torch.empty((heads,), device=dev, dtype=torch.float32)
-        p.index_out, p.num_out, p.thresholds_out = index.data_ptr(), num.data_ptr(), thresholds.data_ptr()
-        routing = (index, num, thresholds)
-
-    lib = _lib.lib()
-    need = lib.wa_hsa_workspace_bytes(ctypes.byref(p))
-    ws = _workspace(dev, need)
-    p.workspace, p.workspace_bytes = ws.data_ptr(), ws.numel()
-    used = ctypes.c_int(0)
-    with _lib.device_guard(dev):
-        _lib.check(lib.wa_hsa_forward(ctypes.byref(p), ctypes.byref(used), _lib.stream_ptr(dev)))
-    if check_status and used.value:
-        status = ctypes.c_int(0)
-        _lib.check(lib.wa_hsa_status(ctypes.byref(p), ctypes.byref(status), _lib.stream_ptr(dev)))
-        if status.value:
-            _lib.status_word(dev).zero_()
-            raise RuntimeError(f"tcgen05 HSA kernel gave up at wait site {status.value}; its output is invalid")
-
+    if backend != "auto":
+        resolve_backend(backend)
+    gate_w, gate_b = (None, None) if gate_lin is None else (gate_lin.weight, gate_lin.bias)
+    res = _lib.host().hsa_forward(
+        q, k, v, k_coarse, v_coarse, k_proj_mat, v_proj_mat, gate_w, gate_b, topk_per_head, block_size, tau_min, tau_max,
+        proj_segment_len, _lib.WA_HSA_FORCE_GENERIC if force_generic else 0, k_pooled_cache, k_pooled_valid, bool(return_routing),
+        bool(check_status))
     if distill.distill_enabled() and torch.is_grad_enabled():
-        distill.record_against_dense(out, q, k, v)
+        distill.record_against_dense(res[0] if return_routing else res, q, k, v)
     if return_routing:
-        return out, (*routing, bool(used.value))
-    return out
+        return res[0], res[1:]
+    return res
 
 
 class HSAAttention(nn.Module):

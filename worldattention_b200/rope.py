@@ -21,6 +21,8 @@ def _table(freqs: torch.Tensor, dev: torch.device) -> torch.Tensor:
 
 
 def _grid(grid_sizes) -> tuple[int, int, int]:
+    if type(grid_sizes) is tuple and len(grid_sizes) == 3:
+        return grid_sizes
     rows = grid_sizes.tolist() if hasattr(grid_sizes, "tolist") else list(grid_sizes)
     if rows and isinstance(rows[0], (list, tuple)):
         if any(tuple(r) != tuple(rows[0]) for r in rows):
@@ -36,31 +38,18 @@ def qk_norm_rope(x: torch.Tensor, norm_weight: torch.Tensor | None, eps: float, 
 
     `table` is `_table(freqs)` kept by the caller (saves the conversion per call).  `start_frame` may be an int32 device
     tensor of one element: the kernel then reads the position when it runs (for launches replayed from a CUDA graph)."""
-    dev = _lib.require_cuda(x)
     if x.dim() == 3:
         if heads is None:
             raise ValueError("heads is needed to split the last axis of a [B, L, H*D] tensor")
         x = x.view(x.shape[0], x.shape[1], heads, -1)
-    bsz, length, n_heads, head_dim = x.shape
-    x = x if x.stride(-1) == 1 else x.contiguous()
-    out = torch.empty((bsz, length, n_heads, head_dim), device=dev, dtype=x.dtype)
-    f = h = w = 1
+    h = w = 1
     if freqs is not None or table is not None:
         f, h, w = _grid(grid_sizes)
-        if f * h * w != length:
-            raise NotImplementedError(f"the grid {f}x{h}x{w} must cover all {length} tokens")
-        table = _table(freqs, dev) if table is None else table
-    weight = None if norm_weight is None else norm_weight.detach().to(dev).contiguous()
-    head = (_lib.t4_blhd(x), _lib.t4_blhd(out), bsz, length, n_heads, head_dim, _lib.ptr(weight),
-            _lib.dtype_code(weight.dtype) if weight is not None else 0, float(eps), _lib.ptr(table),
-            int(table.shape[0]) if table is not None else 0)
-    if isinstance(start_frame, torch.Tensor):
-        if start_frame.dtype != torch.int32 or start_frame.numel() != 1 or start_frame.device != dev:
-            raise ValueError("a device-resident start_frame must be one int32 on the tensors' device")
-        _lib.check(_lib.lib().wa_qk_norm_rope_at(*head, start_frame.data_ptr(), h, w, _lib.stream_ptr(dev)))
-    else:
-        _lib.check(_lib.lib().wa_qk_norm_rope(*head, int(start_frame), h, w, _lib.stream_ptr(dev)))
-    return out
+        if f * h * w != x.shape[1]:
+            raise NotImplementedError(f"the grid {f}x{h}x{w} must cover all {x.shape[1]} tokens")
+        if table is None:
+            table = _table(freqs, _lib.require_cuda(x))
+    return _lib.host().qk_norm_rope(x, norm_weight, eps, table, start_frame, h, w)
 
 
 def causal_rope_apply(x: torch.Tensor, grid_sizes, freqs: torch.Tensor, start_frame: int = 0) -> torch.Tensor:
