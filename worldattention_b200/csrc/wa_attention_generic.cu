@@ -162,9 +162,335 @@ generic_attention_kernel(GenericAttnParams p) {
     }
 }
 
+// ------------------------------------------------------------------------------------------------
+// head_dim 128: the same contract on the warp-level matrix instructions, without giving up float32 anywhere.
+//
+// Two warps share 16 of the CTA's 64 query rows, each with one half of a chunk's keys and sums of its own (merged at the
+// end); chunks may span several routing blocks.  Every product is a sum of bf16 products accumulated in float32, whose
+// operands are exact:
+//   NS = 1  q, k and v are bf16 values (bf16 tensors, or `round_in`): one product for the scores; the float32
+//           probabilities are three bf16 parts (8 + 8 + 8 bits of the significand), so P V takes three.
+//   NS = 3  float32 operands, three parts each: the six products of order up to 2^-16 of the leading one; the
+//           dropped ones are below 2^-23.
+// Parts are cut off, not rounded, so they keep the sign of their value, and a part that would be zero is a tiny
+// number instead: infinities in V or K then give what a float32 product gives and not 0 * inf.
+// The SIMT kernel above is bound by shared-memory reads (one per four multiply-adds).  float32 layer, 12 heads, 1560 queries
+// over 4680 keys in 64-token blocks: both branches 2094 -> 255 us (sparse 200, linear 54).
+// ------------------------------------------------------------------------------------------------
+constexpr int SA_ROWS = 64;                  // query rows of a CTA
+constexpr int SA_THREADS = 256;
+constexpr int SA_D = 128;
+constexpr int SA_LD = SA_D + 8;              // bf16 elements of a shared-memory row: ldmatrix without bank conflicts
+constexpr int sa_keys(int ns) { return ns == 1 ? 64 : 32; }
+constexpr size_t sa_smem(int ns) { return (size_t)ns * (SA_ROWS + 2 * sa_keys(ns)) * SA_LD * 2 + 32; }
+
+__device__ __forceinline__ uint32_t sa_u32(const void *p) { return (uint32_t)__cvta_generic_to_shared(p); }
+__device__ __forceinline__ void ldsm4(uint32_t (&r)[4], uint32_t addr) {
+    asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0, %1, %2, %3}, [%4];"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(addr) : "memory");
+}
+__device__ __forceinline__ void ldsm4_t(uint32_t (&r)[4], uint32_t addr) {
+    asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0, %1, %2, %3}, [%4];"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(addr) : "memory");
+}
+__device__ __forceinline__ void mma16816(float (&c)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
+    asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
+                 : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3]) : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
+}
+
+constexpr float SA_TINY = 2.3509887e-38f;    // 2^-125, a bf16 number
+__device__ __forceinline__ float top_part(float x) { return __uint_as_float(__float_as_uint(x) & 0xffff0000u); }
+__device__ __forceinline__ float rest_of(float x, float hi) {
+    const float r = x - hi;
+    return isinf(hi) || (r == 0.f && x != 0.f) ? copysignf(SA_TINY, x) : r;
+}
+// the upper halves of two floats as a bf16 pair (x in the low half)
+__device__ __forceinline__ uint32_t top_pair(float x, float y) { return __byte_perm(__float_as_uint(x), __float_as_uint(y), 0x7632); }
+
+template <int NS>
+__device__ __forceinline__ void stage4(__nv_bfloat16 *dst, size_t part_stride, float4 x) {   // four elements of a row, NS parts
+    if constexpr (NS == 1) {
+        __nv_bfloat162 a = __floats2bfloat162_rn(x.x, x.y), b = __floats2bfloat162_rn(x.z, x.w);
+        *reinterpret_cast<uint2 *>(dst) = make_uint2(*reinterpret_cast<uint32_t *>(&a), *reinterpret_cast<uint32_t *>(&b));
+    } else {
+#pragma unroll
+        for (int i = 0; i < NS; ++i) {
+            *reinterpret_cast<uint2 *>(dst + i * part_stride) = make_uint2(top_pair(x.x, x.y), top_pair(x.z, x.w));
+            x = make_float4(rest_of(x.x, top_part(x.x)), rest_of(x.y, top_part(x.y)), rest_of(x.z, top_part(x.z)), rest_of(x.w, top_part(x.w)));
+        }
+    }
+}
+__device__ __forceinline__ float4 fetch4(const void *base, int dtype, long long off) {
+    if (dtype == WA_F32) return *reinterpret_cast<const float4 *>((const float *)base + off);
+    const uint2 raw = *reinterpret_cast<const uint2 *>((const __nv_bfloat16 *)base + off);
+    const float2 a = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162 *>(&raw.x));
+    const float2 b = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162 *>(&raw.y));
+    return make_float4(a.x, a.y, b.x, b.y);
+}
+
+template <int NS>
+__global__ void __launch_bounds__(SA_THREADS, NS == 1 ? 2 : 1)
+split_attention_kernel(GenericAttnParams p) {
+    constexpr int KC = sa_keys(NS), KW = KC / 2, NT = KW / 8, RW = KC / 8;   // keys of a chunk and of a warp; 8-key tiles; rows a warp stages
+    extern __shared__ __align__(16) uint8_t sa_raw[];
+    __nv_bfloat16 *qs = reinterpret_cast<__nv_bfloat16 *>(sa_raw);   // [NS][SA_ROWS][SA_LD]
+    __nv_bfloat16 *ks = qs + NS * SA_ROWS * SA_LD;                    // [NS][KC][SA_LD]
+    __nv_bfloat16 *vs = ks + NS * KC * SA_LD;                         // [NS][KC][SA_LD]
+    unsigned *real = reinterpret_cast<unsigned *>(vs + NS * KC * SA_LD);   // per warp: which of the rows it staged are real keys
+
+    const int qb = blockIdx.x / p.tiles_per_block, tile = blockIdx.x % p.tiles_per_block;
+    const int h = blockIdx.y, b = blockIdx.z;
+    const int row0 = qb * p.q_block + tile * p.q_tile;
+    const int rows_here = max(0, min(min(p.q_tile, p.q_block - tile * p.q_tile), p.Lq - row0));
+    if (rows_here <= 0) return;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int g = lane >> 2, c2 = 2 * (lane & 3);
+    const int rg = warp & 3, half_keys = warp >> 2;   // row group; which half of every chunk's keys
+
+    const long long qbase = (long long)b * p.q.sb + (long long)h * p.q.sh;
+    for (int r = warp; r < SA_ROWS; r += SA_THREADS / 32) {
+        const float4 x = r < rows_here ? fetch4(p.q.ptr, p.q.dtype, qbase + (long long)(row0 + r) * p.q.sl + 4 * lane)
+                                       : make_float4(0.f, 0.f, 0.f, 0.f);
+        stage4<NS>(qs + r * SA_LD + 4 * lane, (size_t)SA_ROWS * SA_LD, x);
+    }
+
+    float o[SA_D / 8][4];
+#pragma unroll
+    for (int j = 0; j < SA_D / 8; ++j) o[j][0] = o[j][1] = o[j][2] = o[j][3] = 0.f;
+    float mA = -INFINITY, mB = -INFINITY, lA = 0.f, lB = 0.f;   // rows g and g + 8 of the warp; l: this thread's columns only
+
+    const long long meta = ((long long)b * p.H + h) * (long long)((p.Lq + p.q_block - 1) / p.q_block) + qb;
+    const int n_sel = p.dense ? p.n_kv_blocks : max(0, min(p.num[meta], p.index_stride));
+    const int32_t *ids = p.dense ? nullptr : p.index + meta * (long long)p.index_stride;
+    const long long kbase = (long long)b * p.k.sb + (long long)h * p.k.sh, vbase = (long long)b * p.v.sb + (long long)h * p.v.sh;
+    const long long total = (long long)n_sel * p.kv_block;
+    const bool rows_mine = 16 * rg < rows_here;
+
+    // ldmatrix addresses of this lane (A operand; B operand of the scores; B operand of P V, transposed)
+    const uint32_t qa = sa_u32(qs + (16 * rg + (lane & 15)) * SA_LD + (lane >> 4) * 8);
+    const uint32_t ka = sa_u32(ks + (half_keys * KW + (lane & 7) + (lane >> 4) * 8) * SA_LD + ((lane >> 3) & 1) * 8);
+    const uint32_t va = sa_u32(vs + (half_keys * KW + (lane & 15)) * SA_LD + (lane >> 4) * 8);
+    constexpr uint32_t Q_PART = SA_ROWS * SA_LD * 2, K_PART = KC * SA_LD * 2;   // bytes between the parts of an operand
+
+    for (long long c0 = 0; c0 < total; c0 += KC) {
+        __syncthreads();   // the chunk before this one has been read
+        // this warp stages rows warp * RW ... of the chunk; lane i looks up the i-th of them
+        int token = -1;
+        if (lane < RW) {
+            const long long j = c0 + warp * RW + lane;
+            if (j < total) {
+                const int s = (int)(j / p.kv_block), off = (int)(j - (long long)s * p.kv_block);
+                const int id = max(0, min(p.dense ? s : ids[s], p.n_kv_blocks - 1));
+                int size = p.block_sizes ? p.block_sizes[id] : p.Lkv - id * p.kv_block;
+                size = max(0, min(size, min(p.kv_block, p.Lkv - id * p.kv_block)));
+                if (off < size) token = id * p.kv_block + off;
+            }
+        }
+        const unsigned found = __ballot_sync(0xffffffffu, token >= 0);
+        if (lane == 0) real[warp] = found;
+#pragma unroll
+        for (int r0 = 0; r0 < RW; r0 += 4) {
+            float4 kx[4], vx[4];
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                const int t = __shfl_sync(0xffffffffu, token, r0 + i);
+                kx[i] = vx[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+                if (t >= 0) {
+                    kx[i] = fetch4(p.k.ptr, p.k.dtype, kbase + (long long)t * p.k.sl + 4 * lane);
+                    vx[i] = fetch4(p.v.ptr, p.v.dtype, vbase + (long long)t * p.v.sl + 4 * lane);
+                }
+            }
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                const int r = warp * RW + r0 + i;
+                stage4<NS>(ks + r * SA_LD + 4 * lane, (size_t)KC * SA_LD, kx[i]);
+                stage4<NS>(vs + r * SA_LD + 4 * lane, (size_t)KC * SA_LD, vx[i]);
+            }
+        }
+        __syncthreads();
+        if (!rows_mine) continue;
+        unsigned keep = 0;   // this warp's keys that are real
+#pragma unroll
+        for (int w = 0; w < 4; ++w) keep |= real[4 * half_keys + w] << (w * RW);
+        if (keep == 0) continue;
+        const bool full = keep == (KW == 32 ? ~0u : (1u << (KW & 31)) - 1);
+
+        float sc[NT][4];
+#pragma unroll
+        for (int j = 0; j < NT; ++j) sc[j][0] = sc[j][1] = sc[j][2] = sc[j][3] = 0.f;
+#pragma unroll
+        for (int kk = 0; kk < SA_D / 16; ++kk) {
+            uint32_t a[NS][4];
+#pragma unroll
+            for (int i = 0; i < NS; ++i) ldsm4(a[i], qa + i * Q_PART + kk * 32);
+#pragma unroll
+            for (int j = 0; j < NT; j += 2) {
+                // smallest products first
+#pragma unroll
+                for (int i = NS - 1; i >= 0; --i) {
+                    uint32_t kb[4];
+                    ldsm4(kb, ka + i * K_PART + (uint32_t)(j * 8 * SA_LD + kk * 16) * 2);
+#pragma unroll
+                    for (int u = NS - 1 - i; u >= 0; --u) {
+                        mma16816(sc[j], a[u], kb[0], kb[1]);
+                        mma16816(sc[j + 1], a[u], kb[2], kb[3]);
+                    }
+                }
+            }
+        }
+        // scale, mask, running maximum
+        float xA = -INFINITY, xB = -INFINITY;
+#pragma unroll
+        for (int j = 0; j < NT; ++j) {
+#pragma unroll
+            for (int u = 0; u < 4; ++u) sc[j][u] *= p.scale;
+            if (!full) {
+                if (!((keep >> (8 * j + c2)) & 1)) sc[j][0] = sc[j][2] = -INFINITY;
+                if (!((keep >> (8 * j + c2 + 1)) & 1)) sc[j][1] = sc[j][3] = -INFINITY;
+            }
+            xA = fmaxf(xA, fmaxf(sc[j][0], sc[j][1]));
+            xB = fmaxf(xB, fmaxf(sc[j][2], sc[j][3]));
+        }
+#pragma unroll
+        for (int w = 1; w < 4; w <<= 1) {
+            xA = fmaxf(xA, __shfl_xor_sync(0xffffffffu, xA, w));
+            xB = fmaxf(xB, __shfl_xor_sync(0xffffffffu, xB, w));
+        }
+        const float nA = fmaxf(mA, xA), nB = fmaxf(mB, xB);
+        const float fA = mA == -INFINITY ? 0.f : expf(mA - nA), fB = mB == -INFINITY ? 0.f : expf(mB - nB);
+        mA = nA; mB = nB;
+        lA *= fA; lB *= fB;
+#pragma unroll
+        for (int j = 0; j < SA_D / 8; ++j) { o[j][0] *= fA; o[j][1] *= fA; o[j][2] *= fB; o[j][3] *= fB; }
+#pragma unroll
+        for (int j = 0; j < NT; ++j) {
+            sc[j][0] = expf(sc[j][0] - nA); sc[j][1] = expf(sc[j][1] - nA);
+            sc[j][2] = expf(sc[j][2] - nB); sc[j][3] = expf(sc[j][3] - nB);
+            if (!full) {
+                if (!((keep >> (8 * j + c2)) & 1)) sc[j][0] = sc[j][2] = 0.f;
+                if (!((keep >> (8 * j + c2 + 1)) & 1)) sc[j][1] = sc[j][3] = 0.f;
+            }
+            lA += sc[j][0] + sc[j][1];
+            lB += sc[j][2] + sc[j][3];
+        }
+        // O += P V, 16 keys at a time
+#pragma unroll
+        for (int kk = 0; kk < KW / 16; ++kk) {
+            uint32_t a[3][4];
+#pragma unroll
+            for (int u = 0; u < 4; ++u) {   // a0: row g, first 8 keys; a1: row g + 8; a2, a3: the same of the last 8 keys
+                float x = sc[2 * kk + (u >> 1)][2 * (u & 1)], y = sc[2 * kk + (u >> 1)][2 * (u & 1) + 1];
+                const float tx = x > 0.f ? SA_TINY : 0.f, ty = y > 0.f ? SA_TINY : 0.f;
+#pragma unroll
+                for (int i = 0; i < 3; ++i) {
+                    a[i][u] = top_pair(x, y);
+                    x = fmaxf(x - top_part(x), tx);
+                    y = fmaxf(y - top_part(y), ty);
+                }
+            }
+#pragma unroll
+            for (int j = 0; j < SA_D / 8; j += 2) {
+#pragma unroll
+                for (int i = NS - 1; i >= 0; --i) {
+                    uint32_t vb[4];
+                    ldsm4_t(vb, va + i * K_PART + (uint32_t)(kk * 16 * SA_LD + j * 8) * 2);
+#pragma unroll
+                    for (int u = 2 - i; u >= 0; --u) {
+                        mma16816(o[j], a[u], vb[0], vb[1]);
+                        mma16816(o[j + 1], a[u], vb[2], vb[3]);
+                    }
+                }
+            }
+        }
+    }
+#pragma unroll
+    for (int w = 1; w < 4; w <<= 1) {
+        lA += __shfl_xor_sync(0xffffffffu, lA, w);
+        lB += __shfl_xor_sync(0xffffffffu, lB, w);
+    }
+    // merge the halves: the second one leaves maximum, sum and accumulator of its rows where the keys and values were
+    __syncthreads();
+    float4 *left = reinterpret_cast<float4 *>(ks) + (size_t)rg * (SA_D / 8 + 1) * 32 + lane;   // [SA_D / 8 + 1][32 lanes]
+    static_assert(4 * (SA_D / 8 + 1) * 32 * 16 <= NS * 2 * KC * SA_LD * 2, "the accumulators fit where the keys and values were");
+    if (half_keys && rows_mine) {
+#pragma unroll
+        for (int j = 0; j < SA_D / 8; ++j) left[j * 32] = make_float4(o[j][0], o[j][1], o[j][2], o[j][3]);
+        left[SA_D / 8 * 32] = make_float4(mA, mB, lA, lB);
+    }
+    __syncthreads();
+    if (half_keys || !rows_mine) return;
+    {
+        const float4 other = left[SA_D / 8 * 32];
+        const float nA = fmaxf(mA, other.x), nB = fmaxf(mB, other.y);
+        const float fA = mA == -INFINITY ? 0.f : expf(mA - nA), fB = mB == -INFINITY ? 0.f : expf(mB - nB);
+        const float hA = other.x == -INFINITY ? 0.f : expf(other.x - nA), hB = other.y == -INFINITY ? 0.f : expf(other.y - nB);
+        mA = nA; mB = nB;
+        lA = lA * fA + other.z * hA;
+        lB = lB * fB + other.w * hB;
+#pragma unroll
+        for (int j = 0; j < SA_D / 8; ++j) {
+            const float4 x = left[j * 32];
+            o[j][0] = o[j][0] * fA + x.x * hA; o[j][1] = o[j][1] * fA + x.y * hA;
+            o[j][2] = o[j][2] * fB + x.z * hB; o[j][3] = o[j][3] * fB + x.w * hB;
+        }
+    }
+#pragma unroll
+    for (int half = 0; half < 2; ++half) {
+        const int lr = 16 * rg + g + 8 * half, row = row0 + lr;
+        if (lr >= rows_here) continue;
+        const float l = half ? lB : lA, m = half ? mB : mA, inv = l > 0.f ? 1.0f / l : 0.f;
+        const long long at = (long long)b * p.osb + (long long)row * p.osl + (long long)h * p.osh + c2;
+#pragma unroll
+        for (int j = 0; j < SA_D / 8; ++j) {
+            float x = o[j][2 * half] * inv, y = o[j][2 * half + 1] * inv;
+            __nv_bfloat162 xy = __floats2bfloat162_rn(x, y);
+            if (p.out_dtype == WA_BF16) {
+                *reinterpret_cast<__nv_bfloat162 *>((__nv_bfloat16 *)p.out + at + 8 * j) = xy;
+            } else {
+                if (p.round_out) {
+                    x = __low2float(xy);
+                    y = __high2float(xy);
+                }
+                *reinterpret_cast<float2 *>((float *)p.out + at + 8 * j) = make_float2(x, y);
+            }
+        }
+        if (p.lse && c2 == 0) p.lse[((long long)b * p.H + h) * p.Lq + row] = l > 0.f ? m + logf(l) : -INFINITY;
+    }
+}
+
+template <int NS>
+int launch_split_attention(GenericAttnParams &p, int B, int n_q_blocks, cudaStream_t stream, const char *what) {
+    p.q_tile = p.q_block < SA_ROWS ? p.q_block : SA_ROWS;
+    p.tiles_per_block = ceil_div(p.q_block, p.q_tile);
+    const long long gx = (long long)n_q_blocks * p.tiles_per_block;
+    WA_REQUIRE(gx < (1ll << 31) && p.H <= 65535 && B <= 65535, WA_ERR_UNSUPPORTED, "%s: grid too large", what);
+    static PerDeviceOnce attr_set;
+    if (!attr_set.done()) {
+        const cudaError_t e = cudaFuncSetAttribute(split_attention_kernel<NS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sa_smem(NS));
+        if (e != cudaSuccess) return fail((int)e, "%s: %s", what, cudaGetErrorString(e));
+        attr_set.mark();
+    }
+    split_attention_kernel<NS><<<dim3((unsigned)gx, p.H, B), SA_THREADS, sa_smem(NS), stream>>>(p);
+    return check_launch(what);
+}
+
+// four consecutive elements of every row as one load or store
+static bool rows_of_four(const void *ptr, int dtype, long long sb, long long sl, long long sh) {
+    return (uintptr_t)ptr % (4 * dtype_size(dtype)) == 0 && sb % 4 == 0 && sl % 4 == 0 && sh % 4 == 0;
+}
+
 int launch_generic_attention(GenericAttnParams &p, int B, int n_q_blocks, cudaStream_t stream,
                              const char *what) {
     WA_REQUIRE(p.D <= GA_MAXD, WA_ERR_UNSUPPORTED, "%s: head_dim %d > %d", what, p.D, GA_MAXD);
+    if (p.D == SA_D && rows_of_four(p.q.ptr, p.q.dtype, p.q.sb, p.q.sl, p.q.sh) && rows_of_four(p.k.ptr, p.k.dtype, p.k.sb, p.k.sl, p.k.sh) &&
+        rows_of_four(p.v.ptr, p.v.dtype, p.v.sb, p.v.sl, p.v.sh) && rows_of_four(p.out, p.out_dtype, p.osb, p.osl, p.osh)) {
+        if (p.dense) {   // every block, any grouping of the rows
+            n_q_blocks = ceil_div(p.Lq, SA_ROWS);
+            p.q_block = SA_ROWS;
+        }
+        const bool exact = p.round_in || (p.q.dtype == WA_BF16 && p.k.dtype == WA_BF16 && p.v.dtype == WA_BF16);
+        return exact ? launch_split_attention<1>(p, B, n_q_blocks, stream, what) : launch_split_attention<3>(p, B, n_q_blocks, stream, what);
+    }
     p.q_tile = p.q_block < GA_QT ? p.q_block : GA_QT;
     p.tiles_per_block = ceil_div(p.q_block, p.q_tile);
     const long long gx = (long long)n_q_blocks * p.tiles_per_block;
@@ -223,43 +549,102 @@ gate_combine_kernel(View4 q, View4 sp, View4 li, void *out, int out_dtype, long 
     }
 }
 
-// Same operation with the gate weight staged in shared memory (head_dim <= 128): a persistent grid, each
-// warp walks over (batch, token, head) vectors, a lane produces outputs lane, lane + 32, ...
+// Same operation with the gate weight staged in shared memory (head_dim <= 128): a persistent grid, each warp takes eight
+// (batch, token, head) vectors at a time and a lane produces outputs lane, lane + 32, ... of all of them, so that a weight
+// read from shared memory serves eight multiply-adds (the dot products add up in the order of the channels, as before).
+// Bound by shared-memory reads and the latency of its loads, which are therefore issued together: 18 720 vectors
+// of 128 float32 channels 100 -> 47 us (one vector per warp took a read per multiply-add).
 constexpr int GS_WARPS = 8;
+constexpr int GS_VECS = 8;
+constexpr int GS_MAXD = 128;
+inline int gs_ld(int D) { return (D + 3) / 4 * 4 + 4; }   // floats of a staged row: 16-byte reads of neighbouring rows do not collide
+inline size_t gs_smem(int D) { return ((size_t)(D + GS_WARPS * GS_VECS) * gs_ld(D) + D) * sizeof(float); }
 
 __global__ void __launch_bounds__(GS_WARPS * 32)
 gate_combine_smem_kernel(View4 q, View4 sp, View4 li, void *out, int out_dtype, long long osb, long long osl,
-                         long long osh, long long n_vec, int L, int H, int D, const void *gw, const void *gb, int gdt,
+                         long long osh, long long n_vec, int L, int H, int D, int ld, const void *gw, const void *gb, int gdt,
                          int round_gate) {
-    extern __shared__ float gs_smem[];
-    const int ldw = D + 1;
-    float *ws = gs_smem;                       // [D][D + 1]
-    float *bs = ws + D * ldw;                  // [D]
-    float *qv = bs + D + (threadIdx.x >> 5) * D;   // [GS_WARPS][D]
-    for (int e = threadIdx.x; e < D * D; e += GS_WARPS * 32) ws[(e / D) * ldw + (e % D)] = load_elem(gw, gdt, e);
+    extern __shared__ __align__(16) float gs_smem_raw[];
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    float *ws = gs_smem_raw;                                   // [D][ld], zero beyond column D
+    float *qv = ws + D * ld + warp * GS_VECS * ld;             // [GS_WARPS][GS_VECS][ld]
+    float *bs = ws + (D + GS_WARPS * GS_VECS) * ld;            // [D]
+    for (int r = warp; r < D; r += GS_WARPS)
+        for (int d = lane; d < ld; d += 32) ws[r * ld + d] = d < D ? load_elem(gw, gdt, (long long)r * D + d) : 0.f;
     for (int e = threadIdx.x; e < D; e += GS_WARPS * 32) bs[e] = gb ? load_elem(gb, gdt, e) : 0.f;
+    for (int e = lane; e < GS_VECS * ld; e += 32) qv[e] = 0.f;
     __syncthreads();
-    const int lane = threadIdx.x & 31;
-    const long long stride = (long long)gridDim.x * GS_WARPS;
-    for (long long vec = (long long)blockIdx.x * GS_WARPS + (threadIdx.x >> 5); vec < n_vec; vec += stride) {
-        const int h = (int)(vec % H);
-        const int l = (int)((vec / H) % L);
-        const int b = (int)(vec / ((long long)H * L));
-        const long long qoff = (long long)b * q.sb + (long long)l * q.sl + (long long)h * q.sh;
+    const long long stride = (long long)gridDim.x * GS_WARPS * GS_VECS;
+    for (long long v0 = ((long long)blockIdx.x * GS_WARPS + warp) * GS_VECS; v0 < n_vec; v0 += stride) {
+        const int n = (int)min((long long)GS_VECS, n_vec - v0);
+        // lane i places vector i; the others ask it
+        const long long vec = min(v0 + (lane & (GS_VECS - 1)), n_vec - 1), row = vec / H;
+        const int h_of = (int)(vec - row * H), b_of = (int)(row / L), l_of = (int)(row - (long long)b_of * L);
+        auto place = [&](int i, int &b, int &l, int &h) {
+            b = __shfl_sync(0xffffffffu, b_of, i);
+            l = __shfl_sync(0xffffffffu, l_of, i);
+            h = __shfl_sync(0xffffffffu, h_of, i);
+        };
         __syncwarp();
-        for (int d = lane; d < D; d += 32) qv[d] = load_elem(q.ptr, q.dtype, qoff + d);
+        float x0[GS_VECS][GS_MAXD / 32];
+#pragma unroll
+        for (int i = 0; i < GS_VECS; ++i) {
+            int b, l, h;
+            place(i, b, l, h);
+            const long long qoff = (long long)b * q.sb + (long long)l * q.sl + (long long)h * q.sh;
+#pragma unroll
+            for (int c = 0; c < GS_MAXD / 32; ++c) x0[i][c] = lane + 32 * c < D ? load_elem(q.ptr, q.dtype, qoff + lane + 32 * c) : 0.f;
+        }
+#pragma unroll
+        for (int i = 0; i < GS_VECS; ++i)
+#pragma unroll
+            for (int c = 0; c < GS_MAXD / 32; ++c)
+                if (lane + 32 * c < D) qv[i * ld + lane + 32 * c] = x0[i][c];
         __syncwarp();
-        const long long soff = (long long)b * sp.sb + (long long)l * sp.sl + (long long)h * sp.sh;
-        const long long loff = (long long)b * li.sb + (long long)l * li.sl + (long long)h * li.sh;
-        const long long ooff = (long long)b * osb + (long long)l * osl + (long long)h * osh;
-        for (int e = lane; e < D; e += 32) {
-            float z = bs[e];
-            const float *w = ws + e * ldw;
-            for (int d = 0; d < D; ++d) z = fmaf(qv[d], w[d], z);
-            float g = 1.0f / (1.0f + expf(-z));
-            if (round_gate) g = bf16_round_f(g);
-            store_elem(out, out_dtype, ooff + e,
-                       fmaf(load_elem(li.ptr, li.dtype, loff + e), g, load_elem(sp.ptr, sp.dtype, soff + e)));
+        float z[GS_MAXD / 32][GS_VECS];
+#pragma unroll
+        for (int c = 0; c < GS_MAXD / 32; ++c)
+#pragma unroll
+            for (int i = 0; i < GS_VECS; ++i) z[c][i] = lane + 32 * c < D ? bs[lane + 32 * c] : 0.f;
+        for (int d = 0; d < D; d += 4) {
+            float4 w[GS_MAXD / 32];
+#pragma unroll
+            for (int c = 0; c < GS_MAXD / 32; ++c)
+                w[c] = lane + 32 * c < D ? *reinterpret_cast<const float4 *>(ws + (lane + 32 * c) * ld + d) : make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+            for (int i = 0; i < GS_VECS; ++i) {
+                const float4 x = *reinterpret_cast<const float4 *>(qv + i * ld + d);
+#pragma unroll
+                for (int c = 0; c < GS_MAXD / 32; ++c)
+                    z[c][i] = fmaf(x.w, w[c].w, fmaf(x.z, w[c].z, fmaf(x.y, w[c].y, fmaf(x.x, w[c].x, z[c][i]))));
+            }
+        }
+        float branch[2][GS_VECS][GS_MAXD / 32];
+#pragma unroll
+        for (int i = 0; i < GS_VECS; ++i) {
+            int b, l, h;
+            place(i, b, l, h);
+            const long long soff = (long long)b * sp.sb + (long long)l * sp.sl + (long long)h * sp.sh;
+            const long long loff = (long long)b * li.sb + (long long)l * li.sl + (long long)h * li.sh;
+#pragma unroll
+            for (int c = 0; c < GS_MAXD / 32; ++c) {
+                const int e = lane + 32 * c;
+                branch[0][i][c] = e < D ? load_elem(sp.ptr, sp.dtype, soff + e) : 0.f;
+                branch[1][i][c] = e < D ? load_elem(li.ptr, li.dtype, loff + e) : 0.f;
+            }
+        }
+#pragma unroll
+        for (int i = 0; i < GS_VECS; ++i) {
+            int b, l, h;
+            place(i, b, l, h);
+            const long long ooff = (long long)b * osb + (long long)l * osl + (long long)h * osh;
+#pragma unroll
+            for (int c = 0; c < GS_MAXD / 32; ++c) {
+                const int e = lane + 32 * c;
+                float gate = 1.0f / (1.0f + expf(-z[c][i]));
+                if (round_gate) gate = bf16_round_f(gate);
+                if (e < D && i < n) store_elem(out, out_dtype, ooff + e, fmaf(branch[1][i][c], gate, branch[0][i][c]));
+            }
         }
     }
 }
@@ -394,23 +779,21 @@ extern "C" int wa_gate_combine(const wa_tensor4 *q, const wa_tensor4 *sparse, co
     const long long n_vec = (long long)B * L * H;
     const long long blocks = (n_vec + GC_WARPS - 1) / GC_WARPS;
     WA_REQUIRE(blocks < (1ll << 31), WA_ERR_UNSUPPORTED, "%s: too many tokens", what);
-    if (gate_w && D <= 128) {
-        const size_t smem2 = ((size_t)D * (D + 1) + D + (size_t)GS_WARPS * D) * sizeof(float);
+    if (gate_w && D <= GS_MAXD) {
         static PerDeviceOnce attr_set;
-        if (smem2 > 48 * 1024 && !attr_set.done()) {
-            cudaError_t e = cudaFuncSetAttribute(gate_combine_smem_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                                 (int)(((size_t)128 * 129 + 128 + GS_WARPS * 128) * sizeof(float)));
+        if (gs_smem(D) > 48 * 1024 && !attr_set.done()) {
+            cudaError_t e = cudaFuncSetAttribute(gate_combine_smem_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)gs_smem(GS_MAXD));
             if (e != cudaSuccess) return fail((int)e, "%s: %s", what, cudaGetErrorString(e));
             attr_set.mark();
         }
         int dev = 0, sms = 148;
         cudaGetDevice(&dev);
         cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-        const long long want = (n_vec + GS_WARPS - 1) / GS_WARPS;
+        const long long want = (n_vec + GS_WARPS * GS_VECS - 1) / (GS_WARPS * GS_VECS);
         const unsigned grid = (unsigned)(want < 2ll * sms ? want : 2ll * sms);
-        gate_combine_smem_kernel<<<grid, GS_WARPS * 32, smem2, (cudaStream_t)stream>>>(
+        gate_combine_smem_kernel<<<grid, GS_WARPS * 32, gs_smem(D), (cudaStream_t)stream>>>(
             make_view(q), make_view(sparse), make_view(linear), out->ptr, out->dtype, out->stride_b, out->stride_l,
-            out->stride_h, n_vec, L, H, D, gate_w, gate_b, gate_dtype, round_gate_bf16);
+            out->stride_h, n_vec, L, H, D, gs_ld(D), gate_w, gate_b, gate_dtype, round_gate_bf16);
         return check_launch(what);
     }
     const size_t smem = (size_t)GC_WARPS * D * sizeof(float);
