@@ -213,6 +213,7 @@ extern "C" int wa_hsa_forward(const wa_hsa_params *p, int *used_tuned, void *str
             return rc;
         SchedJob job{};
         if (tuned) job = hsa_sm100_sched_job(p, ws + w.tuned);
+        job.release_at_start = compress_inline;
         if ((rc = route_fused_launch(q_pooled, k_pooled, p->B, p->H, w.Nq, w.Nkv, p->D, p->tau_min, p->tau_max,
                                      p->topk_per_head, block_attn, index, num, thresholds, gini, counters, job, stream,
                                      /*whole_order=*/p->index_out != nullptr || p->thresholds_out != nullptr)))
@@ -221,9 +222,8 @@ extern "C" int wa_hsa_forward(const wa_hsa_params *p, int *used_tuned, void *str
     }
 
     if (compress_inline) {
-        if ((rc = wa_compress_kv(&p->k, &p->v, &kc, &vc, p->B, p->Lkv, p->H, p->D, p->proj_segment_len,
-                                 p->block_size, p->k_proj, p->v_proj, p->proj_dtype, p->proj_rank, p->proj_cols,
-                                 stream)))
+        if ((rc = compress_kv_launch(&p->k, &p->v, &kc, &vc, p->B, p->Lkv, p->H, p->D, p->proj_segment_len, p->block_size, p->k_proj,
+                                     p->v_proj, p->proj_dtype, p->proj_rank, p->proj_cols, /*beside_routing=*/!p->index_in, stream)))
             return rc;
     }
 

@@ -4,6 +4,8 @@
 // tokens, out[r, :] = sum_t E[r, t] * x[t, :], r < min(proj_rank, ceil(seg_tokens / block_size)).
 // SIMT kernel: one thread per (head, channel) column, the projection tile broadcast from shared
 // memory, float32 accumulation.
+#include <cooperative_groups.h>
+
 #include "wa_common.cuh"
 #include "wa_internal.cuh"
 
@@ -65,96 +67,175 @@ compress_kernel(View4 k, View4 v, void *ok, void *ov, int out_dtype, long long o
 
 
 // ------------------------------------------------------------------------------------------------
-// Fast path: bf16, heads contiguous (stride_h == D), rank <= 32.  One CTA per (128 columns, segment,
-// K|V, batch); the eight warps take every eighth token, a lane owns four adjacent columns (8-byte
-// loads), the projection tile is staged in shared memory as float32 [token][rank] so that four
-// ranks come from one 16-byte broadcast load.  Partial sums of the warps are added in warp order.
+// Fast path: bf16 or float32 rows with contiguous heads (stride_h == D), rank <= 32, any projection type: what the
+// tensor-core stream (bf16 throughout, wa_compress_sm100.cu) does not take.  A group = (128 columns, segment, K|V,
+// batch).  Bound by the latency of its loads where a call has few segments, so the tokens of a group are split over a
+// thread-block cluster: each CTA sums its share (the eight warps take every eighth token, a lane owns four adjacent
+// columns, the projection tile is staged in shared memory as float32 [token][rank] so that four ranks come from one
+// 16-byte broadcast load), leaves one partial sum in its shared memory, and the CTAs then add the partials of all of
+// them, each for its share of the output, over distributed shared memory: a fixed order, no workspace, no counters.
+// 12 heads of 128: three bf16 segments of 390 tokens 32 -> 16 us, three float32 segments of 1560 tokens 550 -> 51 us.
 // ------------------------------------------------------------------------------------------------
 constexpr int CF_WARPS = 8;
 constexpr int CF_TT = 128;      // tokens per staged projection tile (16 per warp)
 constexpr int CF_PF = 8;        // token rows a warp keeps in flight
+constexpr int CF_MAX_SPLIT = 8; // CTAs of a cluster (the portable limit)
 
-template <int R>                // padded rank: 16 or 32
+__device__ __forceinline__ float4 load4(const __nv_bfloat16 *p) {
+    const uint2 raw = *reinterpret_cast<const uint2 *>(p);
+    const float2 a = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162 *>(&raw.x));
+    const float2 b = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162 *>(&raw.y));
+    return make_float4(a.x, a.y, b.x, b.y);
+}
+__device__ __forceinline__ float4 load4(const float *p) { return *reinterpret_cast<const float4 *>(p); }
+__device__ __forceinline__ void store1(__nv_bfloat16 *p, float x) { *p = __float2bfloat16_rn(x); }
+__device__ __forceinline__ void store1(float *p, float x) { *p = x; }
+
+template <int R, typename T>    // R: padded rank, 16 or 32
+constexpr size_t compress_cluster_smem() {
+    // the staged projection tile (rows padded by 16 bytes), reused for the warps' sums; then the CTA's partial sum
+    const size_t tile = (size_t)CF_TT * (R + 4) * sizeof(float), sums = (size_t)CF_WARPS / 2 * R * 128 * sizeof(float);
+    return (tile > sums ? tile : sums) + (size_t)R * 128 * sizeof(float);
+}
+
+template <int R, typename T>
 __global__ void __launch_bounds__(CF_WARPS * 32)
-compress_fast_kernel(const __nv_bfloat16 *__restrict__ k, const __nv_bfloat16 *__restrict__ v, long long xsb, long long xsl,
-                     __nv_bfloat16 *__restrict__ ok, __nv_bfloat16 *__restrict__ ov, long long osb, long long osl, int L,
-                     int segment_len, int block_size, const void *pk, const void *pv, int pdt, int proj_rank,
-                     int proj_cols, int rank_full) {
-    __shared__ __align__(16) float es[CF_TT][R];
-    __shared__ float red[R][128];
+compress_cluster_kernel(const T *__restrict__ k, const T *__restrict__ v, long long xsb, long long xsl, T *__restrict__ ok,
+                        T *__restrict__ ov, long long osb, long long osl, int L, int segment_len, int block_size, const void *pk,
+                        const void *pv, int pdt, int proj_rank, int proj_cols, int rank_full, int split, int tokens_per_split) {
+    extern __shared__ __align__(16) float cc_smem[];
+    constexpr int LD = R + 4;
+    constexpr size_t HEAD = compress_cluster_smem<R, T>() / sizeof(float) - (size_t)R * 128;
+    float *es = cc_smem, *part_sum = cc_smem + HEAD;          // [CF_TT][LD]; [R][128]
     const int col0 = blockIdx.x * 128;
-    const int seg = blockIdx.y;
+    const int seg = blockIdx.y / split, part = blockIdx.y % split;   // a cluster is the `split` CTAs of one segment
     const int b = blockIdx.z >> 1, which = blockIdx.z & 1;
-    const __nv_bfloat16 *x = (which ? v : k) + (long long)b * xsb + col0;
+    const T *x = (which ? v : k) + (long long)b * xsb + col0;
     const void *proj = which ? pv : pk;
-    __nv_bfloat16 *out = (which ? ov : ok) + (long long)b * osb + col0;
+    T *out = (which ? ov : ok) + (long long)b * osb + col0;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
 
     const int t0 = seg * segment_len;
     const int n_tok = min(segment_len, L - t0);
     const int rank = min(proj_rank, (n_tok + block_size - 1) / block_size);
+    const int p0 = part * tokens_per_split, p1 = min(n_tok, p0 + tokens_per_split);   // may be empty
 
     float acc[R][4];
 #pragma unroll
     for (int r = 0; r < R; ++r) acc[r][0] = acc[r][1] = acc[r][2] = acc[r][3] = 0.f;
 
-    for (int tt0 = 0; tt0 < n_tok; tt0 += CF_TT) {
-        const int nt = min(CF_TT, n_tok - tt0);
+    for (int tt0 = p0; tt0 < p1; tt0 += CF_TT) {
+        const int nt = min(CF_TT, p1 - tt0);
         __syncthreads();
         for (int e = threadIdx.x; e < CF_TT * R; e += CF_WARPS * 32) {
             const int r = e / CF_TT, t = e % CF_TT;     // consecutive threads read consecutive tokens of one row
-            es[t][r] = (r < rank && t < nt) ? load_elem(proj, pdt, (long long)r * proj_cols + tt0 + t) : 0.f;
+            es[t * LD + r] = (r < rank && t < nt) ? load_elem(proj, pdt, (long long)r * proj_cols + tt0 + t) : 0.f;
         }
         __syncthreads();
         // this warp's tokens of the tile: warp, warp + 8, ...; CF_PF rows are loaded before any is used
         for (int g0 = 0; g0 < CF_TT / CF_WARPS; g0 += CF_PF) {
-            uint2 raw[CF_PF];
+            if (warp + g0 * CF_WARPS >= nt) break;
+            float4 xv[CF_PF];
 #pragma unroll
             for (int i = 0; i < CF_PF; ++i) {
                 const int t = warp + (g0 + i) * CF_WARPS;
-                raw[i] = t < nt ? *reinterpret_cast<const uint2 *>(x + (long long)(t0 + tt0 + t) * xsl + lane * 4)
-                                : make_uint2(0u, 0u);
+                xv[i] = t < nt ? load4(x + (long long)(t0 + tt0 + t) * xsl + lane * 4) : make_float4(0.f, 0.f, 0.f, 0.f);
             }
 #pragma unroll
             for (int i = 0; i < CF_PF; ++i) {
                 const int t = warp + (g0 + i) * CF_WARPS;
                 if (t >= nt) break;
-                const float2 x01 = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162 *>(&raw[i].x));
-                const float2 x23 = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162 *>(&raw[i].y));
 #pragma unroll
                 for (int r4 = 0; r4 < R; r4 += 4) {
-                    const float4 e4 = *reinterpret_cast<const float4 *>(&es[t][r4]);
+                    const float4 e4 = *reinterpret_cast<const float4 *>(&es[t * LD + r4]);
                     const float ev[4] = {e4.x, e4.y, e4.z, e4.w};
 #pragma unroll
                     for (int u = 0; u < 4; ++u) {
-                        acc[r4 + u][0] = fmaf(ev[u], x01.x, acc[r4 + u][0]);
-                        acc[r4 + u][1] = fmaf(ev[u], x01.y, acc[r4 + u][1]);
-                        acc[r4 + u][2] = fmaf(ev[u], x23.x, acc[r4 + u][2]);
-                        acc[r4 + u][3] = fmaf(ev[u], x23.y, acc[r4 + u][3]);
+                        acc[r4 + u][0] = fmaf(ev[u], xv[i].x, acc[r4 + u][0]);
+                        acc[r4 + u][1] = fmaf(ev[u], xv[i].y, acc[r4 + u][1]);
+                        acc[r4 + u][2] = fmaf(ev[u], xv[i].z, acc[r4 + u][2]);
+                        acc[r4 + u][3] = fmaf(ev[u], xv[i].w, acc[r4 + u][3]);
                     }
                 }
             }
         }
     }
-    // ordered reduction over the warps
-    for (int w = 0; w < CF_WARPS; ++w) {
+    // sum over the warps by halves: the upper half leaves its sums in shared memory, the lower half adds them to its own
+#pragma unroll
+    for (int half = CF_WARPS / 2; half >= 1; half >>= 1) {
         __syncthreads();
-        if (warp == w) {
+        if (warp >= half && warp < 2 * half) {
+#pragma unroll
+            for (int r = 0; r < R; ++r)
+                *reinterpret_cast<float4 *>(&es[((warp - half) * R + r) * 128 + lane * 4]) = make_float4(acc[r][0], acc[r][1], acc[r][2], acc[r][3]);
+        }
+        __syncthreads();
+        if (warp < half) {
 #pragma unroll
             for (int r = 0; r < R; ++r) {
-#pragma unroll
-                for (int u = 0; u < 4; ++u) {
-                    if (w == 0) red[r][lane * 4 + u] = acc[r][u];
-                    else red[r][lane * 4 + u] += acc[r][u];
-                }
+                const float4 o = *reinterpret_cast<const float4 *>(&es[(warp * R + r) * 128 + lane * 4]);
+                acc[r][0] += o.x; acc[r][1] += o.y; acc[r][2] += o.z; acc[r][3] += o.w;
             }
         }
     }
-    __syncthreads();
-    for (int e = threadIdx.x; e < rank * 128; e += CF_WARPS * 32) {
-        const int r = e / 128, c = e % 128;
-        out[(long long)(seg * rank_full + r) * osl + c] = __float2bfloat16_rn(red[r][c]);
+    if (warp == 0) {
+#pragma unroll
+        for (int r = 0; r < R; ++r)
+            *reinterpret_cast<float4 *>(&part_sum[r * 128 + lane * 4]) = make_float4(acc[r][0], acc[r][1], acc[r][2], acc[r][3]);
     }
+    auto cluster = cooperative_groups::this_cluster();
+    cluster.sync();
+    for (int e = part * (CF_WARPS * 32) + threadIdx.x; e < rank * 128; e += split * (CF_WARPS * 32)) {
+        float sum = 0.f;
+        for (int s = 0; s < split; ++s) sum += cluster.map_shared_rank(part_sum, s)[e];
+        store1(&out[(long long)(seg * rank_full + e / 128) * osl + e % 128], sum);
+    }
+    cluster.sync();   // a CTA's sums are read by the others until here
+    pdl_wait();       // beside the routing (see compress_kv_launch): done only when that is
+}
+
+// CTAs per group: as many as are resident at once (`ctas`: one or two per SM) where the call has few groups, no share
+// shorter than 64 tokens
+inline int compress_split(long long groups, int longest, int ctas) {
+    int split = groups >= ctas ? 1 : (int)(ctas / groups);
+    if (split > ceil_div(longest, 64)) split = ceil_div(longest, 64);
+    return split > CF_MAX_SPLIT ? CF_MAX_SPLIT : split;
+}
+
+template <int R, typename T>
+int compress_cluster_launch(const wa_tensor4 *k, const wa_tensor4 *v, const wa_tensor4 *ok, const wa_tensor4 *ov, int B, int L, int HD,
+                            int segment_len, int block_size, const void *k_proj, const void *v_proj, int proj_dtype, int proj_rank,
+                            int proj_cols, int rank_full, bool beside, cudaStream_t stream, const char *what) {
+    const auto kernel = compress_cluster_kernel<R, T>;
+    constexpr size_t smem = compress_cluster_smem<R, T>();
+    static PerDeviceOnce attr_set;
+    if (smem > 48 * 1024 && !attr_set.done()) {
+        const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        if (e != cudaSuccess) return fail((int)e, "%s: %s", what, cudaGetErrorString(e));
+        attr_set.mark();
+    }
+    const int n_seg = ceil_div(L, segment_len), longest = L < segment_len ? L : segment_len;
+    const int split = compress_split((long long)(HD / 128) * n_seg * 2 * B, longest, R == 32 ? 148 : 296);
+    const int tokens = ceil_div(ceil_div(longest, split), CF_WARPS) * CF_WARPS;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(HD / 128, n_seg * split, 2 * B);
+    cfg.blockDim = dim3(CF_WARPS * 32);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = stream;
+    cudaLaunchAttribute attr[2];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = 1;
+    attr[0].val.clusterDim.y = split;
+    attr[0].val.clusterDim.z = 1;
+    attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[1].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = beside && pdl_enabled() ? 2 : 1;
+    const cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, (const T *)k->ptr, (const T *)v->ptr, (long long)k->stride_b, (long long)k->stride_l,
+                                             (T *)ok->ptr, (T *)ov->ptr, (long long)ok->stride_b, (long long)ok->stride_l, L, segment_len,
+                                             block_size, k_proj, v_proj, proj_dtype, proj_rank, proj_cols, rank_full, split, tokens);
+    if (e != cudaSuccess) return fail((int)e, "%s: %s", what, cudaGetErrorString(e));
+    return check_launch(what);
 }
 
 // ------------------------------------------------------------------------------------------------
@@ -274,6 +355,13 @@ extern "C" int wa_compress_kv(const wa_tensor4 *k, const wa_tensor4 *v, const wa
                               const wa_tensor4 *out_v, int B, int L, int H, int D, int segment_len, int block_size,
                               const void *k_proj, const void *v_proj, int proj_dtype, int proj_rank, int proj_cols,
                               void *stream) {
+    return wa::compress_kv_launch(k, v, out_k, out_v, B, L, H, D, segment_len, block_size, k_proj, v_proj, proj_dtype, proj_rank,
+                                  proj_cols, /*beside_routing=*/false, (cudaStream_t)stream);
+}
+
+int wa::compress_kv_launch(const wa_tensor4 *k, const wa_tensor4 *v, const wa_tensor4 *out_k, const wa_tensor4 *out_v, int B, int L, int H,
+                           int D, int segment_len, int block_size, const void *k_proj, const void *v_proj, int proj_dtype, int proj_rank,
+                           int proj_cols, bool beside_routing, cudaStream_t stream) {
     const char *what = "wa_compress_kv";
     WA_REQUIRE(k && v && out_k && out_v && k->ptr && v->ptr && out_k->ptr && out_v->ptr && k_proj && v_proj,
                WA_ERR_ARG, "%s: null pointer", what);
@@ -295,27 +383,20 @@ extern "C" int wa_compress_kv(const wa_tensor4 *k, const wa_tensor4 *v, const wa
     // bf16 with contiguous heads on an sm_100 device: the TMA + tcgen05 stream (reads K and V once at HBM speed)
     if (compress_sm100_supported(k, v, out_k, out_v, nullptr, nullptr, H, D, proj_dtype, proj_cols, rank_full, k_proj, v_proj))
         return compress_sm100_launch(k, v, out_k, out_v, nullptr, nullptr, 0, B, L, H, D, segment_len, block_size, k_proj, v_proj,
-                                     proj_rank, proj_cols, 0, rank_full, (cudaStream_t)stream);
-    const bool fast = k->dtype == WA_BF16 && out_k->dtype == WA_BF16 && k->stride_h == D && v->stride_h == D &&
-                      out_k->stride_h == D && (H * D) % 128 == 0 && rank_full <= 32 && k->stride_b == v->stride_b &&
-                      k->stride_l == v->stride_l && k->stride_l % 4 == 0 && k->stride_b % 4 == 0 &&
-                      ((uintptr_t)k->ptr % 8 == 0) && ((uintptr_t)v->ptr % 8 == 0);
+                                     proj_rank, proj_cols, 0, rank_full, stream, beside_routing);
+    const size_t row4 = 4 * dtype_size(k->dtype);   // bytes of the four columns a lane loads
+    const bool fast = k->dtype == out_k->dtype && k->stride_h == D && v->stride_h == D && out_k->stride_h == D && (H * D) % 128 == 0 &&
+                      rank_full <= 32 && k->stride_b == v->stride_b && k->stride_l == v->stride_l && k->stride_l % 4 == 0 &&
+                      k->stride_b % 4 == 0 && (uintptr_t)k->ptr % row4 == 0 && (uintptr_t)v->ptr % row4 == 0 &&
+                      (long long)n_seg * CF_MAX_SPLIT <= 65535;
     if (fast) {
-        dim3 fgrid(H * D / 128, n_seg, 2 * B);
-        if (rank_full <= 16)
-            compress_fast_kernel<16><<<fgrid, CF_WARPS * 32, 0, (cudaStream_t)stream>>>(
-                (const __nv_bfloat16 *)k->ptr, (const __nv_bfloat16 *)v->ptr, k->stride_b, k->stride_l,
-                (__nv_bfloat16 *)out_k->ptr, (__nv_bfloat16 *)out_v->ptr, out_k->stride_b, out_k->stride_l, L,
-                segment_len, block_size, k_proj, v_proj, proj_dtype, proj_rank, proj_cols, rank_full);
-        else
-            compress_fast_kernel<32><<<fgrid, CF_WARPS * 32, 0, (cudaStream_t)stream>>>(
-                (const __nv_bfloat16 *)k->ptr, (const __nv_bfloat16 *)v->ptr, k->stride_b, k->stride_l,
-                (__nv_bfloat16 *)out_k->ptr, (__nv_bfloat16 *)out_v->ptr, out_k->stride_b, out_k->stride_l, L,
-                segment_len, block_size, k_proj, v_proj, proj_dtype, proj_rank, proj_cols, rank_full);
-        return check_launch(what);
+        const auto launch = k->dtype == WA_BF16 ? (rank_full <= 16 ? compress_cluster_launch<16, __nv_bfloat16> : compress_cluster_launch<32, __nv_bfloat16>)
+                                                : (rank_full <= 16 ? compress_cluster_launch<16, float> : compress_cluster_launch<32, float>);
+        return launch(k, v, out_k, out_v, B, L, H * D, segment_len, block_size, k_proj, v_proj, proj_dtype, proj_rank, proj_cols, rank_full,
+                      beside_routing, stream, what);
     }
     dim3 grid(ceil_div(H * D, CK_THREADS), n_seg, 2 * B);
-    compress_kernel<<<grid, CK_THREADS, 0, (cudaStream_t)stream>>>(
+    compress_kernel<<<grid, CK_THREADS, 0, stream>>>(
         make_view(k), make_view(v), out_k->ptr, out_v->ptr, out_k->dtype, out_k->stride_b, out_k->stride_l,
         out_k->stride_h, L, H, D, segment_len, block_size, k_proj, v_proj, proj_dtype, proj_rank, proj_cols,
         rank_full);

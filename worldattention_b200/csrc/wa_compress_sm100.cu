@@ -3,15 +3,20 @@
 // compress_kv (wan/modules/hsa/attention.py:64-110) is, per segment, the product of the [rank x tokens]
 // projection with the [tokens x H*D] token rows: 13..25 output rows for 1560 x 1536 inputs, so the
 // kernel's job is to read K and V once at HBM speed; the contraction itself rides along on the tensor
-// cores.  Work item = (128 columns, segment, K|V, batch).  A persistent CTA of four warps streams the
-// item's tokens in 128-token tiles through a three-stage shared-memory ring:
-//   warp 1  TMA loads: the token tile [128 tokens x 128 columns] and the matching [128 rows x 128 tokens]
-//           tile of the projection (rows past the rank and tokens past the segment come back as zeros);
+// cores.  Work item = (128 or 64 columns, segment, K|V, batch).  A persistent CTA of four warps streams the
+// item's tokens in 128-token tiles through a five-stage shared-memory ring:
+//   warp 1  TMA loads: the token tile [128 tokens x columns] and the matching [32 rows x 128 tokens] tile of the
+//           projection (rows past the rank and tokens past the segment come back as zeros).  The copy engine works by
+//           128-byte row pieces, so only the rows that a rank can have are loaded: the product has M = 128 rows, and
+//           what lies in shared memory behind the 32 enters accumulator lanes that nobody reads;
 //   warp 2  tcgen05.mma, D[rank rows x 128 columns] (+)= E_tile . X_tile, float32 in tensor memory,
 //           two accumulators so that the next item starts while the last one is read out;
 //   warp 3  (append only) TMA store of the same shared-memory tile into the KV cache -- the rows are
 //           read from HBM once and leave twice;
 //   warp 0  reads the accumulator's first `rank` lanes and writes the bf16 slots.
+// 64 columns per item where items of 128 would leave SMs without one (a chunk of a few segments).
+// 12 heads of 128, segments of 1560 tokens: twelve segments 32.7 -> 23 us (115 MB: 5.0 TB/s), three appended ones 17.4 -> 13.3 us
+// against three stages and projection tiles of 128 rows.
 // Every mbarrier wait is bounded; a wait that runs out raises a flag that wa_compress_status reads.
 #include "wa_internal.cuh"
 #include "wa_sm100_ptx.cuh"
@@ -21,9 +26,11 @@ namespace sm100 {
 namespace compress {
 
 constexpr int THREADS = 128;
-constexpr int STAGES = 3;
-constexpr int STAGE_BYTES = 2 * TILE_BYTES;                // token tile + projection tile
-constexpr int SMEM_BYTES = STAGES * STAGE_BYTES + 1024;
+constexpr int STAGES = 5;
+constexpr int E_ROWS = 32, E_HALF_BYTES = E_ROWS * 128;    // projection tile: two halves of 64 tokens, 32 rows of 128 bytes each
+constexpr int STAGE_BYTES = TILE_BYTES + 2 * E_HALF_BYTES; // token tile + projection tile
+// the A operand of the last stage's products reaches 128 rows past the start of its second half
+constexpr int SMEM_BYTES = STAGES * STAGE_BYTES - E_HALF_BYTES + HALF_BYTES + 1024;
 constexpr int TMEM_COLS = 256;                             // two [128 x 128] float32 accumulators
 
 struct Barriers {
@@ -32,9 +39,11 @@ struct Barriers {
     uint32_t tmem_base;
     int abort_flag;
 };
+static_assert(STAGES * STAGE_BYTES + sizeof(Barriers) <= SMEM_BYTES && SMEM_BYTES <= 227 * 1024, "shared memory budget");
 
 struct Job {
     int n_seg, tiles_cols, B;          // items = B * 2 * n_seg * tiles_cols
+    int cols;                          // columns of an item: 128 or 64
     int L, segment_len, block_size, proj_rank;
     int slot0, slot_stride;            // first compressed slot of segment 0; slots between consecutive segments
     int copy;                          // also store the token tiles through the destination maps
@@ -106,18 +115,18 @@ compress_stream_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_co
                     ok = mbar_wait(&bar->empty[s], ((count / STAGES) & 1u) ^ 1u, abort_flag, sink, 1);
                     if (!ok) break;
                     uint8_t *xs = smem + s * STAGE_BYTES, *es = xs + TILE_BYTES;
-                    mbar_expect_tx(&bar->full[s], STAGE_BYTES);
-                    tma_load_3d(xs, tx, &bar->full[s], ct * TILE, tok0 + t * TILE, b);
-                    tma_load_3d(xs + HALF_BYTES, tx, &bar->full[s], ct * TILE + 64, tok0 + t * TILE, b);
+                    mbar_expect_tx(&bar->full[s], (job.cols == TILE ? TILE_BYTES : HALF_BYTES) + 2 * E_HALF_BYTES);
+                    tma_load_3d(xs, tx, &bar->full[s], ct * job.cols, tok0 + t * TILE, b);
+                    if (job.cols == TILE) tma_load_3d(xs + HALF_BYTES, tx, &bar->full[s], ct * job.cols + 64, tok0 + t * TILE, b);
                     tma_load_2d(es, te, &bar->full[s], t * TILE, 0);
-                    tma_load_2d(es + HALF_BYTES, te, &bar->full[s], t * TILE + 64, 0);
+                    tma_load_2d(es + E_HALF_BYTES, te, &bar->full[s], t * TILE + 64, 0);
                 }
             }
         }
     } else if (warp == 2) {
         // ================= issuer =================
         const bool leader = elect_one();
-        constexpr uint32_t IDESC = instr_desc(true, TILE);   // A = projection tile (K-major), B = token tile (columns contiguous)
+        const uint32_t idesc = job.cols == TILE ? instr_desc(true, TILE) : instr_desc(true, 64);   // A = projection tile (K-major), B = token tile (columns contiguous)
         uint32_t count = 0, n_done = 0;
         bool ok = true;
         for (int item = blockIdx.x; item < n_items && ok; item += gridDim.x, ++n_done) {
@@ -138,8 +147,8 @@ compress_stream_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_co
                     const uint64_t bd = smem_desc(xs, HALF_BYTES, 1024), ad = smem_desc(xs + TILE_BYTES, 16, 1024);
 #pragma unroll
                     for (int kk = 0; kk < 8; ++kk)
-                        mma_ss(tmem + buf * TILE, ad + (uint64_t)(((kk >> 2) * HALF_BYTES + (kk & 3) * 32) >> 4),
-                               bd + (uint64_t)((kk * 2048) >> 4), IDESC, !(t == 0 && kk == 0));
+                        mma_ss(tmem + buf * TILE, ad + (uint64_t)(((kk >> 2) * E_HALF_BYTES + (kk & 3) * 32) >> 4),
+                               bd + (uint64_t)((kk * 2048) >> 4), idesc, !(t == 0 && kk == 0));
                     tc_commit(&bar->empty[s]);
                     if (t == n_tiles - 1) tc_commit(&bar->acc_full[buf]);
                 }
@@ -162,8 +171,8 @@ compress_stream_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_co
                     if (!ok) break;
                     uint8_t *xs = smem + s * STAGE_BYTES;
                     // rows past the appended range are clipped by the destination map
-                    tma_store_3d(td, xs, ct * TILE, tok0 + t * TILE, b);
-                    tma_store_3d(td, xs + HALF_BYTES, ct * TILE + 64, tok0 + t * TILE, b);
+                    tma_store_3d(td, xs, ct * job.cols, tok0 + t * TILE, b);
+                    if (job.cols == TILE) tma_store_3d(td, xs + HALF_BYTES, ct * job.cols + 64, tok0 + t * TILE, b);
                     asm volatile("cp.async.bulk.commit_group;" ::: "memory");
                     asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
                     mbar_arrive(&bar->empty[s]);
@@ -185,10 +194,11 @@ compress_stream_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_co
             const int n_tok = min(job.segment_len, job.L - seg * job.segment_len);
             const int rank = min(job.proj_rank, (n_tok + job.block_size - 1) / job.block_size);
             __nv_bfloat16 *out = (which ? job.out_v : job.out_k) + (long long)b * job.osb +
-                                 (long long)(job.slot0 + seg * job.slot_stride + lane) * job.osl + ct * TILE;
+                                 (long long)(job.slot0 + seg * job.slot_stride + lane) * job.osl + ct * job.cols;
             {   // this warp reads tensor-memory lanes 0..31: rank <= 32 is a condition of this path
 #pragma unroll
                 for (int c = 0; c < 4; ++c) {
+                    if (c * 32 >= job.cols) break;
                     uint32_t v[32];
                     TMEM_LD32(tmem + buf * TILE + c * 32, v);
                     tmem_wait_ld();
@@ -212,6 +222,7 @@ compress_stream_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_co
         }
     }
 
+    pdl_wait();       // beside the routing (see compress_kv_launch): done only when that is
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
@@ -247,11 +258,11 @@ static bool map_rows(CUtensorMap *map, void *base, int cols, int rows, int B, lo
                        CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
-// projection `[rank, proj_cols]` bf16 -> 2-D map (token, rank) restricted to the first `tokens` columns, box 64 x 128
+// projection `[rank, proj_cols]` bf16 -> 2-D map (token, rank) restricted to the first `tokens` columns, box 64 x 32
 static bool map_projection(CUtensorMap *map, const void *base, int tokens, int rank, int proj_cols) {
     cuuint64_t dims[2] = {(cuuint64_t)tokens, (cuuint64_t)rank};
     cuuint64_t strides[1] = {(cuuint64_t)proj_cols * 2};
-    cuuint32_t box[2] = {64, (cuuint32_t)TILE}, elem[2] = {1, 1};
+    cuuint32_t box[2] = {64, (cuuint32_t)E_ROWS}, elem[2] = {1, 1};
     return encode_fn()(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void *>(base), dims, strides, box, elem,
                        CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
                        CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
@@ -286,7 +297,7 @@ bool compress_sm100_supported(const wa_tensor4 *k, const wa_tensor4 *v, const wa
 int compress_sm100_launch(const wa_tensor4 *k, const wa_tensor4 *v, const wa_tensor4 *ok, const wa_tensor4 *ov,
                           const wa_tensor4 *dst_k, const wa_tensor4 *dst_v, int dst_row0, int B, int L, int H, int D,
                           int segment_len, int block_size, const void *k_proj, const void *v_proj, int proj_rank, int proj_cols,
-                          int slot0, int slot_stride, cudaStream_t stream) {
+                          int slot0, int slot_stride, cudaStream_t stream, bool beside_routing) {
     using namespace sm100::compress;
     const char *what = "wa_compress_kv(tcgen05)";
     const int cols = H * D;
@@ -321,7 +332,6 @@ int compress_sm100_launch(const wa_tensor4 *k, const wa_tensor4 *v, const wa_ten
     int *status = status_of[dev_now];
     Job job{};
     job.n_seg = ceil_div(L, segment_len);
-    job.tiles_cols = cols / sm100::TILE;
     job.B = B;
     job.L = L; job.segment_len = segment_len; job.block_size = block_size; job.proj_rank = proj_rank;
     job.slot0 = slot0; job.slot_stride = slot_stride;
@@ -329,13 +339,20 @@ int compress_sm100_launch(const wa_tensor4 *k, const wa_tensor4 *v, const wa_ten
     job.out_k = (__nv_bfloat16 *)ok->ptr; job.out_v = (__nv_bfloat16 *)ov->ptr;
     job.osb = ok->stride_b; job.osl = ok->stride_l;
     job.status = status;
-    const long long items = (long long)B * 2 * job.n_seg * job.tiles_cols;
-    WA_REQUIRE(items < (1ll << 30), WA_ERR_UNSUPPORTED, "%s: too many work items", what);
     int dev = 0, sms = 0;
     if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || sms <= 0)
         sms = 148;
+    job.cols = (long long)B * 2 * job.n_seg * (cols / sm100::TILE) < sms ? 64 : sm100::TILE;
+    job.tiles_cols = cols / job.cols;
+    const long long items = (long long)B * 2 * job.n_seg * job.tiles_cols;
+    WA_REQUIRE(items < (1ll << 30), WA_ERR_UNSUPPORTED, "%s: too many work items", what);
     const int grid = items < sms ? (int)items : sms;
-    compress_stream_kernel<<<grid, THREADS, SMEM_BYTES, stream>>>(tk, tv, tek, tev, tdk, tdv, job);
+    if (beside_routing) {
+        const cudaError_t e = launch_dependent(compress_stream_kernel, dim3(grid), dim3(THREADS), SMEM_BYTES, stream, tk, tv, tek, tev, tdk, tdv, job);
+        if (e != cudaSuccess) return fail((int)e, "%s: %s", what, cudaGetErrorString(e));
+    } else {
+        compress_stream_kernel<<<grid, THREADS, SMEM_BYTES, stream>>>(tk, tv, tek, tev, tdk, tdv, job);
+    }
     return check_launch(what);
 }
 

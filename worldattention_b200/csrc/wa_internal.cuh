@@ -15,6 +15,7 @@ struct SchedJob {
     int gate_dt;
     __nv_bfloat16 *w_out;   // [128 x 128] bf16
     float *b_out;           // [128] float32
+    bool release_at_start;  // the next launch does not wait for the routing (it compresses K and V meanwhile)
     int release_dependents_after_rows;   // timing experiment (WA_B200_PDL=2), see route_row
 };
 
@@ -137,6 +138,14 @@ bool compress_sm100_supported(const wa_tensor4 *k, const wa_tensor4 *v, const wa
 int compress_sm100_launch(const wa_tensor4 *k, const wa_tensor4 *v, const wa_tensor4 *ok, const wa_tensor4 *ov,
                           const wa_tensor4 *dst_k, const wa_tensor4 *dst_v, int dst_row0, int B, int L, int H, int D,
                           int segment_len, int block_size, const void *k_proj, const void *v_proj, int proj_rank, int proj_cols,
-                          int slot0, int slot_stride, cudaStream_t stream);
+                          int slot0, int slot_stride, cudaStream_t stream, bool beside_routing = false);
+
+// compress_kv by whichever kernel covers the call (wa_compress.cu).  `beside_routing`: the launch before this one on the
+// stream is a routing kernel that released its dependents at its start (SchedJob::release_at_start).  The two share nothing, so
+// the compression runs on what the routing leaves free of the chip; it completes only after the routing has, so that
+// whatever waits for it may read both.  (One latent frame of 390 tokens over three: the call 49.5 -> 43.1 us.)
+int compress_kv_launch(const wa_tensor4 *k, const wa_tensor4 *v, const wa_tensor4 *out_k, const wa_tensor4 *out_v, int B, int L, int H, int D,
+                       int segment_len, int block_size, const void *k_proj, const void *v_proj, int proj_dtype, int proj_rank, int proj_cols,
+                       bool beside_routing, cudaStream_t stream);
 
 }  // namespace wa

@@ -975,6 +975,7 @@ route_fused_kernel(const float *__restrict__ qp, const float *__restrict__ kp, i
     // No early release of the attention kernel here: its CTAs, once resident and waiting, slowed the tail of this
     // kernel (the per-head count and the work order are a few CTAs' work) by about 5 us.
     pdl_wait();                 // pooled means and zeroed counters come from the launch before
+    if (job.release_at_start) pdl_release_dependents();
     if (group >= (long long)B * H * groups_per_bh) return;
     const long long bh = group / groups_per_bh;
     const int i0 = (int)(group % groups_per_bh) * rows_per_cta, nrows = min(rows_per_cta, Nq - i0);
