@@ -229,7 +229,8 @@ extern "C" int wa_hsa_forward(const wa_hsa_params *p, int *used_tuned, void *str
 
     // ---- tuned tcgen05 path -------------------------------------------------------------------
     if (tuned) {
-        rc = hsa_sm100_launch(p, Lc, &kc, &vc, index, num, w.Nq, w.Nkv, ws + w.tuned, prepared, stream);
+        rc = hsa_sm100_launch(p, Lc, &kc, &vc, index, num, w.Nq, w.Nkv, ws + w.tuned, prepared,
+                              reinterpret_cast<int32_t *>(block_attn), reinterpret_cast<int32_t *>(gini), stream);   // both done with by now
         if (rc) return rc;
         if (used_tuned) *used_tuned = 1;
         return 0;

@@ -21,6 +21,7 @@
 // global memory, all roles leave their loops, tensor memory is released and the kernel returns.
 #include <climits>
 #include <cstdlib>
+#include <type_traits>
 
 #include "wa_internal.cuh"
 #include "wa_sm100_ptx.cuh"
@@ -110,12 +111,26 @@ static_assert(SMEM_BYTES <= 227 * 1024, "shared memory budget exceeded");
 // The three roles run their own loops over work items and meet only at mbarriers, so the producer
 // prefetches the next item's Q/K/V and the MMA warp starts its first products while the softmax
 // warps are still in the previous item's epilogue.
-template <int BLK>   // routing block size: 128, or 64 (see Params::blk)
+//
+// PAIR (64-token blocks, more items than SMs): a work item is TWO neighbouring query blocks of a head, so all 128 rows of
+// its tile are real.  Blocks that both query blocks selected (pair_lists_kernel puts them first in both lists) are taken
+// two per tile, for all rows: a key block is then loaded once for the two, and the loads are what sparse tiles are bound by
+// (64 KB of keys and values per tile from L2).  A tile of the others holds one block of each: keys 0..63 for rows 0..63,
+// keys 64..127 for rows 64..127.  There the score product covers all four quadrants, the softmax only reads the two that
+// count, and the P V product is two K = 64 products, each of which writes the accumulator rows of its query block only
+// (the instruction's lane mask): a block that a row did not select never enters its sums, whatever it holds (a zero
+// probability would turn its infinities into NaN).  The linear branch and the gate run on full tiles, half as many as
+// with an item per 64-row block.
+// 12 heads, 4680 queries, the whole call: 877 -> 708 us over 21 frames with counts from the mass (895 -> 762 us by the shared
+// tiles alone), 1815 -> 1561 us over 480 frames with 32 blocks a row and 12 000 compressed slots.
+template <int BLK, bool PAIR>   // routing block size: 128, or 64 (see Params::blk)
 __global__ void __launch_bounds__(THREADS, 1)
 hsa_fwd_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
                      const __grid_constant__ CUtensorMap tm_v, const __grid_constant__ CUtensorMap tm_kc,
                      const __grid_constant__ CUtensorMap tm_vc, const __grid_constant__ CUtensorMap tm_w,
                      const __grid_constant__ CUtensorMap tm_out, const Params p) {
+    static_assert(!PAIR || BLK == HALF, "query blocks are paired where a block is half a tile");
+    constexpr int Q_ROWS = PAIR ? TILE : BLK;    // query rows of a work item
     extern __shared__ __align__(1024) uint8_t smem[];   // swizzled TMA tiles need 1024-byte alignment (checked below)
     uint8_t *q_s = smem, *k_s = smem + Q_STAGES * TILE_BYTES, *v_s = smem + (Q_STAGES + KV_STAGES) * TILE_BYTES;
     Barriers *bar = reinterpret_cast<Barriers *>(smem + (Q_STAGES + KV_STAGES + V_STAGES) * TILE_BYTES);
@@ -187,20 +202,31 @@ hsa_fwd_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
                 const uint32_t slot = jcount & 1u;
                 ok = mbar_wait(&bar->item_empty[slot], ((jcount >> 1) & 1u) ^ 1u, abort_flag, sink, 11);
                 if (!ok) break;
-                int item = -1, n_sel = 0;
+                int item = -1, n_sel = 0, n_sel2 = 0, n_both = 0;   // PAIR: of the item's first and second query block; tiles for both
+                long long row0 = 0;                                 // routing row of the item's (first) query block
                 if (at < p.n_items) {
                     item = p.order[at];
-                    n_sel = max(0, min(p.num[item], p.Nkv));
+                    row0 = PAIR ? (long long)(item / p.q_items) * p.Nq + 2 * (item % p.q_items) : item;
+                    n_sel = max(0, min(p.num[row0], p.Nkv));
+                    if (PAIR && 2 * (item % p.q_items) + 1 < p.Nq) n_sel2 = max(0, min(p.num[row0 + 1], p.Nkv));
+                    if (PAIR) n_both = p.both[item] >> 1;
                 }
                 // the other roles count sparse TILES: with 64-token blocks a tile holds two selected blocks
-                const int n_st = BLK == TILE ? n_sel : (n_sel + 1) >> 1;
+                const int n_st = BLK == TILE ? n_sel : PAIR ? max(n_sel, n_sel2) - n_both : (n_sel + 1) >> 1;
                 bar->items[slot].item = item;
                 bar->items[slot].n_sel = n_st;
+                bar->items[slot].n_both = n_both;
                 mbar_arrive(&bar->item_full[slot]);
                 if (item < 0) break;
                 at = (int)gridDim.x + atomicAdd(p.work_counter, 1);   // consumed at the top of the next round
-                const int qb = item % p.Nq, h = (item / p.Nq) % p.H, b = item / (p.Nq * p.H);
-                const int32_t *ids = p.index + (long long)item * p.Nkv;
+                const int qb = item % p.q_items, h = (item / p.q_items) % p.H, b = item / (p.q_items * p.H);
+                const int32_t *ids = p.index + row0 * p.Nkv;
+                // PAIR: the blocks of tile t; one past the end of the shorter list lies beyond the keys and loads as zeros
+                auto block_of = [&](const int32_t *list, int at, int n) { return at < n ? max(0, min(list[at], p.Nkv - 1)) : p.Nkv; };
+                auto pair_first = [&](int t) { return block_of(ids, t < n_both ? 2 * t : t + n_both, n_sel); };
+                auto pair_second = [&](int t) {
+                    return t < n_both ? block_of(ids, 2 * t + 1, n_sel) : block_of(ids + p.Nkv, t + n_both, n_sel2);
+                };
                 const int n_kv = n_st + lin_tiles;
                 WA_STATS_ITEM(n_kv + 1);
 
@@ -209,8 +235,8 @@ hsa_fwd_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
                 if (!ok) break;
                 uint8_t *qdst = q_s + qs * TILE_BYTES;
                 mbar_expect_tx(&bar->q_full[qs], TILE_BYTES);
-                tma_load_4d(qdst, &tm_q, &bar->q_full[qs], 0, h, qb * BLK, b);
-                tma_load_4d(qdst + HALF_BYTES, &tm_q, &bar->q_full[qs], 64, h, qb * BLK, b);
+                tma_load_4d(qdst, &tm_q, &bar->q_full[qs], 0, h, qb * Q_ROWS, b);
+                tma_load_4d(qdst + HALF_BYTES, &tm_q, &bar->q_full[qs], 64, h, qb * Q_ROWS, b);
 
                 // K tiles and V tiles advance on cursors of their own: the V ring is shallower and its stages come back
                 // later (after the PV product), and a K load that queued behind a V wait would reach the QK warp late.
@@ -226,8 +252,8 @@ hsa_fwd_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
                             tma_load_4d(vdst, &tm_v, &bar->v_full[vs], 0, h, id * TILE, b);
                             tma_load_4d(vdst + HALF_BYTES, &tm_v, &bar->v_full[vs], 64, h, id * TILE, b);
                         } else {
-                            const int id = max(0, min(ids[2 * tv], p.Nkv - 1));
-                            const int id2 = 2 * tv + 1 < n_sel ? max(0, min(ids[2 * tv + 1], p.Nkv - 1)) : id;
+                            const int id = PAIR ? pair_first(tv) : max(0, min(ids[2 * tv], p.Nkv - 1));
+                            const int id2 = PAIR ? pair_second(tv) : 2 * tv + 1 < n_sel ? max(0, min(ids[2 * tv + 1], p.Nkv - 1)) : id;
                             tma_load_4d(vdst, &tm_v, &bar->v_full[vs], 0, h, id * HALF, b);
                             tma_load_4d(vdst + HALF_BYTES / 2, &tm_v, &bar->v_full[vs], 0, h, id2 * HALF, b);
                             tma_load_4d(vdst + HALF_BYTES, &tm_v, &bar->v_full[vs], 64, h, id * HALF, b);
@@ -271,6 +297,10 @@ hsa_fwd_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
                             id = max(0, min(ids[t], p.Nkv - 1));
                             const int n = min(TILE, p.Lkv - id * TILE);
                             valid = min(n, HALF) | (max(0, n - HALF) << 8);
+                        } else if (PAIR) {
+                            id = pair_first(t);
+                            id2 = pair_second(t);
+                            valid = max(0, min(HALF, p.Lkv - id * HALF)) | (max(0, min(HALF, p.Lkv - id2 * HALF)) << 8);
                         } else {   // two 64-token blocks; a missing second block repeats the first and is masked out
                             id = max(0, min(ids[2 * t], p.Nkv - 1));
                             const bool two = 2 * t + 1 < n_sel;
@@ -391,7 +421,7 @@ hsa_fwd_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
             const uint32_t slot = jcount & 1u;
             ok = __all_sync(0xffffffffu, mbar_wait(&bar->item_full[slot], (jcount >> 1) & 1u, abort_flag, sink, 20));
             if (!ok) break;
-            const int item = bar->items[slot].item, n_sel = bar->items[slot].n_sel;
+            const int item = bar->items[slot].item, n_sel = bar->items[slot].n_sel, n_both = bar->items[slot].n_both;
             __syncwarp();
             if (leader) mbar_arrive(&bar->item_empty[slot]);
             if (item < 0) break;
@@ -416,10 +446,22 @@ hsa_fwd_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
                 tc_fence_after();
                 if (leader) {
                     const uint64_t vd = smem_desc(smem_u32(v_s + vs * TILE_BYTES), HALF_BYTES, 1024);
+                    if (PAIR && t >= n_both && t < n_sel) {
+                        // both halves of the rows left their probabilities in the same 32 columns
 #pragma unroll
-                    for (int kk = 0; kk < 8; ++kk)
-                        mma_ts(tmem_o, tmem_s + buf * TILE + kk * 8, vd + (uint64_t)((kk * 2048) >> 4), IDESC_PV,
-                               !(first && kk == 0));
+                        for (int kk = 0; kk < 4; ++kk)
+                            mma_ts_half<false>(tmem_o, tmem_s + buf * TILE + kk * 8, vd + (uint64_t)((kk * 2048) >> 4), IDESC_PV,
+                                               !(first && kk == 0));
+#pragma unroll
+                        for (int kk = 0; kk < 4; ++kk)
+                            mma_ts_half<true>(tmem_o, tmem_s + buf * TILE + kk * 8, vd + (uint64_t)(((kk + 4) * 2048) >> 4), IDESC_PV,
+                                              !(first && kk == 0));
+                    } else {
+#pragma unroll
+                        for (int kk = 0; kk < 8; ++kk)
+                            mma_ts(tmem_o, tmem_s + buf * TILE + kk * 8, vd + (uint64_t)((kk * 2048) >> 4), IDESC_PV,
+                                   !(first && kk == 0));
+                    }
                     tc_commit(&bar->s_free[buf]);   // first: the next score product waits for it
                     tc_commit(&bar->v_empty[vs]);   // frees the V stage; the rescale path reads it as "this product has landed"
                     if (t == n_sel - 1 || t == n_kv - 1) tc_commit(&bar->o_done);
@@ -442,15 +484,15 @@ hsa_fwd_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
                 const int item = bar->items[slot].item;
                 mbar_arrive(&bar->item_empty[slot]);
                 if (item < 0) break;
-                const int qb = item % p.Nq, h = (item / p.Nq) % p.H, b = item / (p.Nq * p.H);
+                const int qb = item % p.q_items, h = (item / p.q_items) % p.H, b = item / (p.q_items * p.H);
                 const uint32_t qs = jcount % Q_STAGES;
                 ok = mbar_wait(&bar->out_ready[qs], (jcount / Q_STAGES) & 1u, abort_flag, sink, 17);
                 if (!ok) break;
                 if (!p.part_linear) {
                     // rows beyond q_len are clipped by the tensor map
                     // (with 64-token blocks the map's box is 64 rows: the tile's upper rows belong to the next item)
-                    tma_store_4d(&tm_out, q_s + qs * TILE_BYTES, 0, h, qb * BLK, b);
-                    tma_store_4d(&tm_out, q_s + qs * TILE_BYTES + HALF_BYTES, 64, h, qb * BLK, b);
+                    tma_store_4d(&tm_out, q_s + qs * TILE_BYTES, 0, h, qb * Q_ROWS, b);
+                    tma_store_4d(&tm_out, q_s + qs * TILE_BYTES + HALF_BYTES, 64, h, qb * Q_ROWS, b);
                     asm volatile("cp.async.bulk.commit_group;" ::: "memory");
                     asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");   // the Q stage is reusable afterwards
                 }
@@ -473,6 +515,7 @@ hsa_fwd_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
         const int g = lane >> 2, c2 = lane & 3;
         const int rowA = rg * 32 + hb * 16 + g, rowB = rowA + 8;
         const uint32_t lane_addr = ((uint32_t)(rg * 32 + hb * 16)) << 16;
+        const int second_block = PAIR ? rg >> 1 : 0;        // which of the item's two query blocks the rows belong to
         uint32_t jcount = 0, sg = 0;       // items and K-type tiles seen so far
         uint32_t ph_od = 0;
         uint32_t pv_count = 0;             // PV products requested so far
@@ -483,15 +526,15 @@ hsa_fwd_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
             const uint32_t slot = jcount & 1u;
             ok = __all_sync(0xffffffffu, mbar_wait(&bar->item_full[slot], (jcount >> 1) & 1u, abort_flag, sink, 15));
             if (!ok) break;
-            const int item = bar->items[slot].item, n_sel = bar->items[slot].n_sel;
+            const int item = bar->items[slot].item, n_sel = bar->items[slot].n_sel, n_both = bar->items[slot].n_both;
             warp_arrive(&bar->item_empty[slot]);
             if (item < 0) break;
-            const int qb = item % p.Nq, h = (item / p.Nq) % p.H, b = item / (p.Nq * p.H);
+            const int qb = item % p.q_items, h = (item / p.q_items) % p.H, b = item / (p.q_items * p.H);
             const int n_kv = n_sel + lin_tiles;
             const uint32_t qs = jcount % Q_STAGES;
             uint8_t *q_stage = q_s + qs * TILE_BYTES;
-            const int tokenA = qb * BLK + rowA, tokenB = tokenA + 8;
-            const bool okA = rowA < BLK && tokenA < p.Lq, okB = rowB < BLK && tokenB < p.Lq;
+            const int tokenA = qb * Q_ROWS + rowA, tokenB = tokenA + 8;
+            const bool okA = rowA < Q_ROWS && tokenA < p.Lq, okB = rowB < Q_ROWS && tokenB < p.Lq;
             // float32 offsets of the rows' normalisers
             long long lseA = (long long)b * p.lse_sb + (long long)h * p.lse_sh + (long long)tokenA * p.lse_st, lseB = lseA + 8 * p.lse_st;
             if (p.peer_rows > 0) {
@@ -511,29 +554,22 @@ hsa_fwd_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
             uint32_t park[32], gpk[32];
             float ls_spA = 0.f, ls_spB = 0.f;   // the sparse branch's log-sum-exp (packed records write both in one store)
 
+#pragma unroll 1   // one copy of each kind of tile: the loops stay in the instruction cache
             for (int phase = 0; phase < 2 && ok; ++phase) {
                 const int t0 = phase == 0 ? 0 : n_sel, t1 = phase == 0 ? n_sel : n_kv;
                 float mA = -INFINITY, mB = -INFINITY, lA = 0.f, lB = 0.f;   // l: this thread's columns only
-                for (int t = t0; t < t1 && ok; ++t) {
-                    const int buf = (sg + t) % S_BUFS;
-                    const uint32_t s_addr = tmem_s + buf * TILE + lane_addr;
-                    ok = __all_sync(0xffffffffu, mbar_wait(&bar->s_full[buf], ((sg + t) / S_BUFS) & 1u, abort_flag, sink, 8));
-                    if (!ok) break;
-                    WA_TRACE(2);
-                    tc_fence_after();
-                    // real tokens of the tile's first and last 64 keys (the producer wrote the counts); key column c is real
-                    // when c < v0 (c < 64) or c - 64 < v1: per 8-column step j that is c < lim(j)
-                    const int vword = bar->valid[(sg + t) & 7];
-                    const int v0 = vword & 0xff, v1 = (vword >> 8) & 0xff;
-                    const bool full = vword == (HALF | (HALF << 8));
-                    const int lim_lo = v0, lim_hi = HALF + v1;
-                    uint32_t r[64];
-                    TMEM_LDQ64(s_addr, r);
+                // One tile of 8 * STEPS key columns: scores at s_addr -> probabilities at p_addr, the accumulator rescaled
+                // where a running maximum outgrew it.  Columns of the first 64 keys are real below lim_lo, the others below lim_hi.
+                auto softmax_tile = [&](auto steps, uint32_t s_addr, uint32_t p_addr, bool full, int lim_lo, int lim_hi, bool later) {
+                    constexpr int STEPS = decltype(steps)::value;
+                    uint32_t r[4 * STEPS];
+                    if constexpr (STEPS == 16) TMEM_LDQ64(s_addr, r);
+                    else TMEM_LDQ32(s_addr, r);
                     tmem_wait_ld();
                     float xa0 = -INFINITY, xa1 = -INFINITY, xb0 = -INFINITY, xb1 = -INFINITY;
                     if (full) {
 #pragma unroll
-                        for (int j = 0; j < 16; ++j) {
+                        for (int j = 0; j < STEPS; ++j) {
                             xa0 = fmaxf(xa0, __uint_as_float(r[4 * j]));
                             xa1 = fmaxf(xa1, __uint_as_float(r[4 * j + 1]));
                             xb0 = fmaxf(xb0, __uint_as_float(r[4 * j + 2]));
@@ -541,7 +577,7 @@ hsa_fwd_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
                         }
                     } else {
 #pragma unroll
-                        for (int j = 0; j < 16; ++j) {
+                        for (int j = 0; j < STEPS; ++j) {
                             const int col = 8 * j + 2 * c2, lim = j < 8 ? lim_lo : lim_hi;
                             if (col < lim) {
                                 xa0 = fmaxf(xa0, __uint_as_float(r[4 * j]));
@@ -560,13 +596,13 @@ hsa_fwd_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
                     const bool growA = mxA > mA + 8.0f, growB = mxB > mB + 8.0f;
                     if (growA) mA_new = mxA;
                     if (growB) mB_new = mxB;
-                    if (__any_sync(0xffffffffu, (growA || growB) && t > t0)) {
+                    if (__any_sync(0xffffffffu, (growA || growB) && later)) {
                         // every PV requested so far must have landed before the accumulator is touched
                         ok = __all_sync(0xffffffffu, mbar_wait(&bar->v_empty[(pv_count - 1u) % V_STAGES],
                                                                ((pv_count - 1u) / V_STAGES) & 1u, abort_flag, sink, 9));
-                        if (!ok) break;
+                        if (!ok) return;
                         tc_fence_after();
-                        const float fA = (growA && t > t0) ? ex2(mA - mA_new) : 1.0f, fB = (growB && t > t0) ? ex2(mB - mB_new) : 1.0f;
+                        const float fA = (growA && later) ? ex2(mA - mA_new) : 1.0f, fB = (growB && later) ? ex2(mB - mB_new) : 1.0f;
                         lA *= fA;
                         lB *= fB;
 #pragma unroll
@@ -588,12 +624,12 @@ hsa_fwd_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
                     mA = mA_new;
                     mB = mB_new;
                     // p = 2^(s*c - m), row sums, pack to bf16, write P over the consumed S columns
-                    uint32_t pk[32];
+                    uint32_t pk[2 * STEPS];
                     const float2 nmA = make_float2(-mA, -mA), nmB = make_float2(-mB, -mB);
                     float2 accA = make_float2(0.f, 0.f), accB = make_float2(0.f, 0.f);
                     if (full) {
 #pragma unroll
-                        for (int j = 0; j < 16; ++j) {
+                        for (int j = 0; j < STEPS; ++j) {
                             if (j % POLY_EVERY == 0)
                                 exp_step<true, false>(r[4 * j], r[4 * j + 1], r[4 * j + 2], r[4 * j + 3], sc, nmA, nmB, accA, accB,
                                                       pk[2 * j], pk[2 * j + 1], 0, 0);
@@ -604,7 +640,7 @@ hsa_fwd_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
                     } else {
                         // ragged tile (the last one of a branch): 8-column steps without a real token cost nothing
 #pragma unroll
-                        for (int j = 0; j < 16; ++j) {
+                        for (int j = 0; j < STEPS; ++j) {
                             const int lim = j < 8 ? lim_lo : lim_hi;
                             if (8 * j < lim)
                                 exp_step<false, true>(r[4 * j], r[4 * j + 1], r[4 * j + 2], r[4 * j + 3], sc, nmA, nmB, accA, accB,
@@ -614,10 +650,30 @@ hsa_fwd_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
                         }
                     }
                     WA_TRACE(20);
-                    TMEM_STP32(s_addr, pk);
+                    if constexpr (STEPS == 16) TMEM_STP32(p_addr, pk);
+                    else TMEM_STP16(p_addr, pk);
                     lA += accA.x + accA.y;
                     lB += accB.x + accB.y;
                     tmem_wait_st();
+                };
+                for (int t = t0; t < t1 && ok; ++t) {
+                    const int buf = (sg + t) % S_BUFS;
+                    const uint32_t s_addr = tmem_s + buf * TILE + lane_addr;
+                    ok = __all_sync(0xffffffffu, mbar_wait(&bar->s_full[buf], ((sg + t) / S_BUFS) & 1u, abort_flag, sink, 8));
+                    if (!ok) break;
+                    WA_TRACE(2);
+                    tc_fence_after();
+                    // real tokens of the tile's first and last 64 keys (the producer wrote the counts); key column c is real
+                    // when c < v0 (c < 64) or c - 64 < v1: per 8-column step j that is c < lim(j)
+                    const int vword = bar->valid[(sg + t) & 7];
+                    const int v0 = vword & 0xff, v1 = (vword >> 8) & 0xff;
+                    if (PAIR && phase == 0 && t >= n_both) {
+                        const int v = second_block ? v1 : v0;
+                        softmax_tile(std::integral_constant<int, 8>(), s_addr + second_block * HALF, s_addr, v == HALF, v, 0, t > t0);
+                    } else {
+                        softmax_tile(std::integral_constant<int, 16>(), s_addr, s_addr, vword == (HALF | (HALF << 8)), v0, HALF + v1, t > t0);
+                    }
+                    if (!ok) break;
                     WA_TRACE(21);
                     tc_fence_before();
                     warp_arrive(&bar->p_full[buf]);
@@ -761,10 +817,10 @@ hsa_fwd_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
                 // XOR-swizzled by row) and writes 512 contiguous bytes of two rows per instruction.
                 uint8_t *scr = q_stage + warp * 4096;
                 const int lr = lane & 15, row_l = rg * 32 + hb * 16 + lr;
-                const int token_l = qb * BLK + row_l;
+                const int token_l = qb * Q_ROWS + row_l;
                 constexpr long long NO_ROW = LLONG_MIN;   // (a peer's buffer may lie below this rank's: offsets can be negative)
                 long long rec = NO_ROW;      // float offset of this lane's row (rows 0..15 of the warp) in the records
-                if (row_l < BLK && token_l < p.Lq) {
+                if (row_l < Q_ROWS && token_l < p.Lq) {
                     if (p.peer_rows > 0) {
                         const int d = min(token_l / p.peer_rows, 7);
                         rec = (((long long)p.peer_self * p.peer_rows + (token_l - d * p.peer_rows)) * p.H + h) * p.part_stride
@@ -866,14 +922,87 @@ hsa_fwd_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
     }
 }
 
+// ---- the lists of a pair: [blocks of both | the row's others], each part in ascending order ------------------------
+// A warp per item.  Ascending, so that the CTAs that work on a head sweep its keys side by side and find in L2 what the
+// first of them fetched.  A list that names a block twice (only a caller's own routing can) stays as it is.
+constexpr int PL_WARPS = 4;
+__global__ void __launch_bounds__(PL_WARPS * 32)
+pair_lists_kernel(const int32_t *__restrict__ index, const int32_t *__restrict__ num, int Nq, int Nkv, int q_items, int n_items,
+                  int32_t *__restrict__ lists, int32_t *__restrict__ both) {
+    extern __shared__ uint32_t pl_smem[];
+    const int words = (Nkv + 31) >> 5, lane = threadIdx.x & 31;
+    uint32_t *bits[2] = {pl_smem + (threadIdx.x >> 5) * 2 * words, pl_smem + ((threadIdx.x >> 5) * 2 + 1) * words};
+    pdl_wait();                 // the routing comes from the launch before
+    const int item = blockIdx.x * PL_WARPS + (threadIdx.x >> 5);
+    if (item >= n_items) return;
+    const long long row0 = (long long)(item / q_items) * Nq + 2 * (item % q_items);
+    const bool two = 2 * (item % q_items) + 1 < Nq;
+    int n[2], distinct[2] = {0, 0}, shared = 0;
+    for (int w = lane; w < words; w += 32) bits[0][w] = bits[1][w] = 0u;
+    __syncwarp();
+    auto id_of = [&](int side, int i) { return max(0, min(index[(row0 + side) * Nkv + i], Nkv - 1)); };
+#pragma unroll
+    for (int side = 0; side < 2; ++side) {
+        n[side] = side == 0 || two ? max(0, min(num[row0 + side], Nkv)) : 0;
+        for (int i = lane; i < n[side]; i += 32) {
+            const int id = id_of(side, i);
+            atomicOr(&bits[side][id >> 5], 1u << (id & 31));
+        }
+    }
+    __syncwarp();
+    for (int w = lane; w < words; w += 32) {
+        distinct[0] += __popc(bits[0][w]);
+        distinct[1] += __popc(bits[1][w]);
+        shared += __popc(bits[0][w] & bits[1][w]);
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+        distinct[0] += __shfl_xor_sync(0xffffffffu, distinct[0], o);
+        distinct[1] += __shfl_xor_sync(0xffffffffu, distinct[1], o);
+        shared += __shfl_xor_sync(0xffffffffu, shared, o);
+    }
+    const bool plain = distinct[0] != n[0] || distinct[1] != n[1];
+    const int n_both = plain ? 0 : shared;
+    int32_t *own = lists + row0 * Nkv;
+    if (plain) {
+#pragma unroll
+        for (int side = 0; side < 2; ++side)
+            for (int i = lane; i < n[side]; i += 32) own[(long long)side * Nkv + i] = id_of(side, i);
+    } else {
+        int at[3] = {0, n_both, n_both};            // next place of a block of both, of the first row's others, of the second's
+        for (int w0 = 0; w0 < words; w0 += 32) {
+            const uint32_t a = w0 + lane < words ? bits[0][w0 + lane] : 0u, b = w0 + lane < words ? bits[1][w0 + lane] : 0u;
+            const uint32_t part[3] = {a & b, a & ~b, b & ~a};
+#pragma unroll
+            for (int k = 0; k < 3; ++k) {
+                const int mine = __popc(part[k]);
+                int incl = mine;
+#pragma unroll
+                for (int o = 1; o < 32; o <<= 1) {
+                    const int v = __shfl_up_sync(0xffffffffu, incl, o);
+                    if (lane >= o) incl += v;
+                }
+                int pos = at[k] + incl - mine;
+                at[k] += __shfl_sync(0xffffffffu, incl, 31);
+                for (uint32_t m = part[k]; m; m &= m - 1, ++pos) {
+                    const int id = (w0 + lane) * 32 + __ffs(m) - 1;
+                    if (k != 2) own[pos] = id;
+                    if (k != 1 && two) own[Nkv + pos] = id;
+                }
+            }
+        }
+    }
+    if (lane == 0) both[item] = n_both;
+}
+
 // ---- launch preparation as a kernel of its own (used when the routing kernel has not done it) --------
 __global__ void __launch_bounds__(1024)
-schedule_kernel(const int32_t *__restrict__ num, int n_items, int Nkv, SchedJob job) {
+schedule_kernel(const int32_t *__restrict__ num, int rows, int Nq, int Nkv, SchedJob job) {
     if (blockIdx.x > 0) {
         if (job.gate_w) convert_gate_slice(job, (blockIdx.x - 1) * 1024, 1024);
         return;
     }
-    schedule_items(num, n_items, Nkv, job.order, job.work_counter, job.error_flag);
+    schedule_items(num, rows, Nq, Nkv, job.paired, job.by_head, job.order, job.work_counter, job.error_flag);
 }
 
 // ---- host side -----------------------------------------------------------------------------------
@@ -993,6 +1122,14 @@ SchedJob hsa_sm100_sched_job(const wa_hsa_params *p, void *workspace) {
     job.gate_w = p->gate_w; job.gate_b = p->gate_b; job.gate_dt = p->gate_dtype;
     job.w_out = (__nv_bfloat16 *)(ws + w.w_bf16);
     job.b_out = (float *)(ws + w.bias);
+    // Two 64-token query blocks share a work item as soon as one block per item would give some SM a second item.  With
+    // fewer, the chip has room for every block at once and an item of its own is done sooner: it takes two selected
+    // blocks per tile, a pair one of each query block.  (16384 key blocks: the pairs' bitmaps in shared memory.)
+    job.paired = p->block_size == sm100::HALF && (long long)p->Lkv <= 16384ll * sm100::HALF &&
+                 (long long)p->B * p->H * ceil_div(p->Lq, p->block_size) > sm100::max_grid();
+    // Head by head where the keys and values are more than L2 keeps at a time; below that nothing is gained and the lighter
+    // items of the last head are a worse end than the lightest of all (three frames, 28 MB: 107.5 against 104.9 us)
+    job.by_head = 4ll * p->B * p->H * p->Lkv * p->D > (64ll << 20);
     return job;
 }
 
@@ -1022,13 +1159,14 @@ bool hsa_sm100_supported(const wa_hsa_params *p, int Lc, const wa_tensor4 *kc, c
 }
 
 int hsa_sm100_launch(const wa_hsa_params *p, int Lc, const wa_tensor4 *kc, const wa_tensor4 *vc, const int32_t *index,
-                     const int32_t *num, int Nq, int Nkv, void *workspace, bool prepared, cudaStream_t stream) {
+                     const int32_t *num, int Nq, int Nkv, void *workspace, bool prepared, int32_t *lists, int32_t *both, cudaStream_t stream) {
     using namespace sm100;
     const SchedJob job = hsa_sm100_sched_job(p, workspace);
     int32_t *order = job.order;
     int *counter = job.work_counter;
     __nv_bfloat16 *w_bf16 = job.w_out;
     float *bias = job.b_out;
+    const bool pair = job.paired;
 
     CUtensorMap tq, tk, tv, tkc, tvc, tw, tout;
     int rc;
@@ -1039,17 +1177,27 @@ int hsa_sm100_launch(const wa_hsa_params *p, int Lc, const wa_tensor4 *kc, const
     if ((rc = make_map_4d(&tkc, kc, p->B, Lc, p->H, "k_coarse"))) return rc;
     if ((rc = make_map_4d(&tvc, vc, p->B, Lc, p->H, "v_coarse"))) return rc;
     if ((rc = make_map_w(&tw, w_bf16))) return rc;
-    if ((rc = make_map_4d(&tout, p->part_sparse ? &p->q : &p->out, p->B, p->Lq, p->H, "out", blk))) return rc;   // unused in partial mode
+    if ((rc = make_map_4d(&tout, p->part_sparse ? &p->q : &p->out, p->B, p->Lq, p->H, "out", pair ? TILE : blk))) return rc;   // unused in partial mode
 
-    const int n_items = p->B * p->H * Nq;
+    const int rows = p->B * p->H * Nq, q_items = pair ? (Nq + 1) / 2 : Nq, n_items = p->B * p->H * q_items;
     if (!prepared) {
-        schedule_kernel<<<p->gate_w ? 1 + TILE * TILE / 1024 : 1, 1024, 0, stream>>>(num, n_items, Nkv, job);
+        schedule_kernel<<<p->gate_w ? 1 + TILE * TILE / 1024 : 1, 1024, 0, stream>>>(num, rows, Nq, Nkv, job);
         if ((rc = check_launch("wa_hsa_forward(schedule)"))) return rc;
     }
 
+    if (pair) {
+        const size_t smem = (size_t)PL_WARPS * 2 * ((Nkv + 31) / 32) * sizeof(uint32_t);   // at most 16 KB
+        const cudaError_t e = launch_dependent(pair_lists_kernel, dim3(ceil_div(n_items, PL_WARPS)), dim3(PL_WARPS * 32), smem, stream, index, num, Nq,
+                                               Nkv, q_items, n_items, lists, both);
+        if (e != cudaSuccess) return fail((int)e, "wa_hsa_forward(pairs): %s", cudaGetErrorString(e));
+        if ((rc = check_launch("wa_hsa_forward(pairs)"))) return rc;
+        index = lists;
+    }
     Params kp{};
     kp.B = p->B; kp.H = p->H; kp.Lq = p->Lq; kp.Lkv = p->Lkv; kp.Lc = Lc; kp.Nq = Nq; kp.Nkv = Nkv;
     kp.n_items = n_items;
+    kp.q_items = q_items;
+    kp.both = both;
     kp.blk = blk;
     kp.index = index; kp.num = num; kp.order = order; kp.work_counter = counter; kp.error_flag = counter + 1;
     kp.status_mirror = p->status_mirror;
@@ -1077,9 +1225,9 @@ int hsa_sm100_launch(const wa_hsa_params *p, int Lc, const wa_tensor4 *kc, const
 
     static PerDeviceOnce attr_set;
     if (!attr_set.done()) {
-        cudaError_t e = cudaFuncSetAttribute(hsa_fwd_sm100_kernel<TILE>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES);
-        if (e == cudaSuccess)
-            e = cudaFuncSetAttribute(hsa_fwd_sm100_kernel<HALF>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES);
+        cudaError_t e = cudaSuccess;
+        for (auto kernel : {hsa_fwd_sm100_kernel<TILE, false>, hsa_fwd_sm100_kernel<HALF, false>, hsa_fwd_sm100_kernel<HALF, true>})
+            if (e == cudaSuccess) e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES);
         if (e != cudaSuccess) return fail((int)e, "wa_hsa_forward(tcgen05): %s", cudaGetErrorString(e));
         attr_set.mark();
     }
@@ -1088,10 +1236,8 @@ int hsa_sm100_launch(const wa_hsa_params *p, int Lc, const wa_tensor4 *kc, const
     if (getenv("WA_SM100_ONE_CTA") && grid > max_grid() / 2) grid = max_grid() / 2;   // tuning aid: one CTA per SM
 #endif
     profile_mark(true, stream);
-    cudaError_t le = blk == TILE ? launch_dependent(hsa_fwd_sm100_kernel<TILE>, dim3(grid), dim3(THREADS), SMEM_BYTES, stream, tq, tk,
-                                                    tv, tkc, tvc, tw, tout, kp)
-                                 : launch_dependent(hsa_fwd_sm100_kernel<HALF>, dim3(grid), dim3(THREADS), SMEM_BYTES, stream, tq, tk,
-                                                    tv, tkc, tvc, tw, tout, kp);
+    const auto kernel = blk == TILE ? hsa_fwd_sm100_kernel<TILE, false> : pair ? hsa_fwd_sm100_kernel<HALF, true> : hsa_fwd_sm100_kernel<HALF, false>;
+    cudaError_t le = launch_dependent(kernel, dim3(grid), dim3(THREADS), SMEM_BYTES, stream, tq, tk, tv, tkc, tvc, tw, tout, kp);
     profile_mark(false, stream);
     if (le != cudaSuccess) return fail((int)le, "wa_hsa_forward(tcgen05): %s", cudaGetErrorString(le));
     return check_launch("wa_hsa_forward(tcgen05)");
@@ -1124,7 +1270,7 @@ int hsa_sm100_launch_linear(const wa_hsa_params *p, int Lc, const wa_tensor4 *kc
     pl.part_linear = linear_out;
     profile_pause(true);   // the timing bracket of this forward belongs to the sparse-branch kernel
     const int rc = hsa_sm100_launch(&pl, Lc, kc, vc, zeros /*never read: no item selects a block*/, zeros, nq, 1, workspace, false,
-                                    stream);
+                                    nullptr, nullptr, stream);
     profile_pause(false);
     return rc;
 }

@@ -15,19 +15,64 @@ struct SchedJob {
     int gate_dt;
     __nv_bfloat16 *w_out;   // [128 x 128] bf16
     float *b_out;           // [128] float32
+    bool paired;            // a work item is two neighbouring query blocks (rows of `num`) of one head
+    bool by_head;           // work order: head by head (see schedule_items)
     bool release_at_start;  // the next launch does not wait for the routing (it compresses K and V meanwhile)
     int release_dependents_after_rows;   // timing experiment (WA_B200_PDL=2), see route_row
 };
 
 constexpr int SCHED_BINS = 4096;
+constexpr int SCHED_HEADS = 256;
 
-// Counting sort of the items by selected-block count, heaviest first.  Called by every thread of ONE
-// CTA whose size is a power of two between 32 and 1024.
-__device__ inline void schedule_items(const int32_t *num, int n_items, int Nkv, int32_t *__restrict__ order,
-                                      int *work_counter, int *error_flag) {
+// Work order of the items, heavy first (weight: selected blocks; of a pair of rows the larger count).  Called by every
+// thread of ONE CTA whose size is a power of two between 32 and 1024.
+//
+// `by_head` (the keys are more than L2 holds): head by head, the head with the most work first and a head's items heaviest
+// first, so that the CTAs at work at a time read the keys of a few heads (counts from the mass over a window of 21 frames:
+// 797 against 716 us a call).  Taken back: only the heavier 60 % of a head's items so and the rest by weight over all heads,
+// which evens out the end but mixes the heads again (764 us).
+// Calls with so many items that ranking them against one another would take too long here are counting-sorted by weight.
+static __device__ __noinline__ void schedule_items(const int32_t *num, int rows, int Nq, int Nkv, bool paired, bool by_head,
+                                                   int32_t *__restrict__ order, int *work_counter, int *error_flag) {
     __shared__ int hist[SCHED_BINS];
     __shared__ int warp_tot[32];
     const int T = blockDim.x, tid = threadIdx.x;
+    const int each = paired ? (Nq + 1) >> 1 : Nq, heads = rows / Nq, n_items = heads * each;   // items of a head, ...
+    auto count_of = [&](int i) {
+        if (!paired) return __ldcg(num + i);
+        const int head = i / each, q = 2 * (i - head * each);
+        const int32_t *at = num + (long long)head * Nq + q;
+        const int first = __ldcg(at);
+        return q + 1 < Nq ? max(first, __ldcg(at + 1)) : first;
+    };
+    if (by_head && heads <= SCHED_HEADS && n_items <= SCHED_BINS && (long long)n_items * each <= 2048ll * T) {
+        __shared__ int head_sum[SCHED_HEADS], head_rank[SCHED_HEADS];
+        for (int i = tid; i < heads; i += T) head_sum[i] = 0;
+        if (tid == 0) {
+            *work_counter = 0;
+            *error_flag = 0;
+        }
+        __syncthreads();
+        for (int i = tid; i < n_items; i += T) {
+            const int w = max(0, min(count_of(i), Nkv));
+            hist[i] = w;
+            atomicAdd(&head_sum[i / each], w);
+        }
+        __syncthreads();
+        for (int i = tid; i < heads; i += T) {
+            int rank = 0;
+            for (int j = 0; j < heads; ++j) rank += head_sum[j] > head_sum[i] || (head_sum[j] == head_sum[i] && j < i);
+            head_rank[i] = rank;
+        }
+        __syncthreads();
+        for (int i = tid; i < n_items; i += T) {
+            const int head = i / each, first = head * each, w = hist[i];
+            int rank = 0;
+            for (int j = first; j < first + each; ++j) rank += hist[j] > w || (hist[j] == w && j < i);
+            order[head_rank[head] * each + rank] = i;
+        }
+        return;
+    }
     // bins 0..top hold counts top..0 (bin 0 = heaviest); `per` bins per thread, a power of two >= 1
     const int top = min(Nkv, SCHED_BINS - 1);
     int per = 1;
@@ -44,12 +89,12 @@ __device__ inline void schedule_items(const int32_t *num, int n_items, int Nkv, 
 #pragma unroll
     for (int u = 0; u < KEEP; ++u) {
         const int i = tid + u * T;
-        bin_of[u] = i < n_items ? top - max(0, min(__ldcg(num + i), top)) : -1;
+        bin_of[u] = i < n_items ? top - max(0, min(count_of(i), top)) : -1;
     }
 #pragma unroll
     for (int u = 0; u < KEEP; ++u)
         if (bin_of[u] >= 0) atomicAdd(&hist[bin_of[u]], 1);
-    for (int i = tid + KEEP * T; i < n_items; i += T) atomicAdd(&hist[top - max(0, min(__ldcg(num + i), top))], 1);
+    for (int i = tid + KEEP * T; i < n_items; i += T) atomicAdd(&hist[top - max(0, min(count_of(i), top))], 1);
     __syncthreads();
     // exclusive prefix over the bins: a contiguous run of bins per thread, then a block scan of the run totals
     const int b0 = tid * per;
@@ -83,7 +128,7 @@ __device__ inline void schedule_items(const int32_t *num, int n_items, int Nkv, 
 #pragma unroll
     for (int u = 0; u < KEEP; ++u)
         if (bin_of[u] >= 0) order[atomicAdd(&hist[bin_of[u]], 1)] = tid + u * T;
-    for (int i = tid + KEEP * T; i < n_items; i += T) order[atomicAdd(&hist[top - max(0, min(__ldcg(num + i), top))], 1)] = i;
+    for (int i = tid + KEEP * T; i < n_items; i += T) order[atomicAdd(&hist[top - max(0, min(count_of(i), top))], 1)] = i;
 }
 
 // Elements [first, first + count) of the gate weight -> bf16 (it is an MMA operand) and of the bias -> float32.
@@ -119,7 +164,7 @@ SchedJob hsa_sm100_sched_job(const wa_hsa_params *p, void *workspace);
 // `prepared`: the SchedJob of this call has already run on the stream (as part of the routing kernel)
 int hsa_sm100_launch(const wa_hsa_params *p, int Lc, const wa_tensor4 *kc, const wa_tensor4 *vc,
                      const int32_t *index, const int32_t *num, int Nq, int Nkv, void *workspace,
-                     bool prepared, cudaStream_t stream);
+                     bool prepared, int32_t *lists, int32_t *both, cudaStream_t stream);   // scratch: as large as index, as num
 
 // the linear branch alone on the tcgen05 kernel (bf16, head_dim 128; any routing block size): float32 [B, Lq, H, 128]
 bool hsa_sm100_linear_supported(const wa_hsa_params *p, int Lc, const wa_tensor4 *kc, const wa_tensor4 *vc);

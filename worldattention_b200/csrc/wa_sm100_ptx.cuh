@@ -138,6 +138,16 @@ __device__ __forceinline__ void mma_ts(uint32_t d_tmem, uint32_t a_tmem, uint64_
         ::"r"(d_tmem), "r"(a_tmem), "l"(b_desc), "r"(idesc), "r"(acc) : "memory");
 }
 
+// The same for half of D's rows: lanes 64..127 (UPPER) or 0..63 are written, the others keep what they hold.
+template <bool UPPER>
+__device__ __forceinline__ void mma_ts_half(uint32_t d_tmem, uint32_t a_tmem, uint64_t b_desc, uint32_t idesc, uint32_t acc) {
+    const uint32_t lo = UPPER ? 0xffffffffu : 0u, hi = ~lo;   // set bits: lanes that are not written
+    asm volatile(
+        "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
+        "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, {%5, %5, %6, %6}, p;\n\t}"
+        ::"r"(d_tmem), "r"(a_tmem), "l"(b_desc), "r"(idesc), "r"(acc), "r"(lo), "r"(hi) : "memory");
+}
+
 #define TMEM_LD32(taddr, r)                                                                                          \
     asm volatile(                                                                                                    \
         "tcgen05.ld.sync.aligned.32x32b.x32.b32 "                                                                    \
@@ -180,6 +190,10 @@ __device__ __forceinline__ void mma_ts(uint32_t d_tmem, uint32_t a_tmem, uint64_
 #define TMEM_LDQ64(taddr, r) \
     asm volatile("tcgen05.ld.sync.aligned.16x256b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31, %32, %33, %34, %35, %36, %37, %38, %39, %40, %41, %42, %43, %44, %45, %46, %47, %48, %49, %50, %51, %52, %53, %54, %55, %56, %57, %58, %59, %60, %61, %62, %63}, [%64];" \
         : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15]), "=r"(r[16]), "=r"(r[17]), "=r"(r[18]), "=r"(r[19]), "=r"(r[20]), "=r"(r[21]), "=r"(r[22]), "=r"(r[23]), "=r"(r[24]), "=r"(r[25]), "=r"(r[26]), "=r"(r[27]), "=r"(r[28]), "=r"(r[29]), "=r"(r[30]), "=r"(r[31]), "=r"(r[32]), "=r"(r[33]), "=r"(r[34]), "=r"(r[35]), "=r"(r[36]), "=r"(r[37]), "=r"(r[38]), "=r"(r[39]), "=r"(r[40]), "=r"(r[41]), "=r"(r[42]), "=r"(r[43]), "=r"(r[44]), "=r"(r[45]), "=r"(r[46]), "=r"(r[47]), "=r"(r[48]), "=r"(r[49]), "=r"(r[50]), "=r"(r[51]), "=r"(r[52]), "=r"(r[53]), "=r"(r[54]), "=r"(r[55]), "=r"(r[56]), "=r"(r[57]), "=r"(r[58]), "=r"(r[59]), "=r"(r[60]), "=r"(r[61]), "=r"(r[62]), "=r"(r[63]) \
+        : "r"(taddr) : "memory")
+#define TMEM_LDQ32(taddr, r) \
+    asm volatile("tcgen05.ld.sync.aligned.16x256b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31}, [%32];" \
+        : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15]), "=r"(r[16]), "=r"(r[17]), "=r"(r[18]), "=r"(r[19]), "=r"(r[20]), "=r"(r[21]), "=r"(r[22]), "=r"(r[23]), "=r"(r[24]), "=r"(r[25]), "=r"(r[26]), "=r"(r[27]), "=r"(r[28]), "=r"(r[29]), "=r"(r[30]), "=r"(r[31]) \
         : "r"(taddr) : "memory")
 #define TMEM_LDQ16(taddr, r) \
     asm volatile("tcgen05.ld.sync.aligned.16x256b.x4.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];" \
@@ -298,12 +312,14 @@ __device__ __forceinline__ float quad_sum(float x) {
 
 struct Params {
     int B, H, Lq, Lkv, Lc, Nq, Nkv;
-    int blk;       // routing block size: 128, or 64 (a work item is then a 64-row query block in a 128-row tile whose
-                   // upper rows are computed and dropped, and a key tile holds two selected 64-token blocks)
+    int blk;       // routing block size: 128, or 64 (a key tile then holds two selected 64-token blocks; a work item is two
+                   // neighbouring query blocks, or one in a 128-row tile whose upper rows are computed and dropped)
     int n_items;
+    int q_items;   // work items per (batch, head): Nq, or (Nq + 1) / 2 where two query blocks share one
     const int32_t *index;   // [B,H,Nq,Nkv]
     const int32_t *num;     // [B,H,Nq]
     const int32_t *order;   // [n_items] work order (heaviest first)
+    const int32_t *both;    // PAIR [n_items]: blocks that both query blocks selected; they come first in both lists of `index`
     int *work_counter;
     int *error_flag;
     int *status_mirror;     // optional host-visible copy of the failure code (see wa_hsa_params::status_mirror)
@@ -325,8 +341,9 @@ struct Params {
 };
 
 struct ItemDesc {
-    int item;    // (b*H + h)*Nq + qb, or -1: no more work
-    int n_sel;   // selected key blocks of this item
+    int item;    // (b*H + h)*q_items + qb, or -1: no more work
+    int n_sel;   // sparse tiles of this item
+    int n_both;  // PAIR: the first of them hold two key blocks that both query blocks selected
 };
 
 }  // namespace sm100
