@@ -334,7 +334,8 @@ int wa_hkv_score_topk_layers(const float *page_index, const float *query, int la
 /* One page copy of the install step (cache.py:229-246).  `row_elems` contiguous elements per
  * token (H*D for whole-token pages, D for one head), token rows `src_stride` / `dst_stride`
  * elements apart.  `rot` >= 0 selects `rotations[rot]` (shift_temporal_rope, rope.py:50-67) and
- * applies it to the first 2*n_temporal elements of every head_dim-sized group; rot < 0 copies. */
+ * applies it to the first 2*n_temporal elements of every head_dim-sized group; rot < 0 copies.  A null `src` clears the
+ * rows of `dst`. */
 typedef struct wa_page_copy {
     const void *src;
     void *dst;

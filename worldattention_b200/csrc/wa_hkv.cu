@@ -3,6 +3,8 @@
 // Stand-ins for pipeline/hkv/retrieval.py:50-126, pipeline/hkv/rope.py:33-82 and the copy loop of
 // pipeline/hkv/cache.py:229-246.  All three are byte-moving, HBM-bound kernels: 128-bit coalesced
 // accesses, warp-shuffle reductions, no tensor cores.
+#include <cooperative_groups.h>
+
 #include "wa_common.cuh"
 
 namespace wa {
@@ -75,20 +77,25 @@ page_centroid_kernel(View4 keys, int B, int H, int D, const int32_t *__restrict_
 }
 
 // The same for bf16 keys whose heads lie side by side (stride D, D a multiple of 8, 16-byte aligned rows): a thread owns
-// FOUR neighbouring pairs (one 16-byte load per token) and keeps four tokens' loads in flight, so that the kernel streams
-// instead of waiting for one 4-byte load per thread at a time (1.4 TB/s).  Same arithmetic per value; the float64 sums
-// of a pair are taken token by token within a row group and the row groups are added in order, as above.
-constexpr int CV_TX = 64, CV_TY = 4, CV_U = 4;
+// FOUR neighbouring pairs (one 16-byte load per token) and keeps four tokens' loads in flight.  Same arithmetic per value;
+// float64 sums, row groups added in order.  Bound by the loads in flight, and a stored window has few pages (seven of
+// three frames: 21 CTAs streamed its 100 MB in 525 us), so the tokens of a page are split over a thread-block cluster,
+// whose first CTA adds the shares up over distributed shared memory: 88 us.
+constexpr int CV_TX = 32, CV_TY = 8, CV_U = 4;
+constexpr int CV_MAX_SPLIT = 8;   // CTAs of a cluster (the portable limit)
 
 __global__ void __launch_bounds__(CV_TX *CV_TY)
 page_centroid_vec_kernel(const __nv_bfloat16 *__restrict__ keys, long long sb, long long sl, int B, int H, int D,
                          const int32_t *__restrict__ spans, const float2 *__restrict__ derope, int n_frames, int nt,
                          int frame_seq_length, float *__restrict__ page_index) {
+    auto cluster = cooperative_groups::this_cluster();             // the CTAs that share a page and its columns (grid.z)
+    const int split = (int)cluster.num_blocks(), part = (int)cluster.block_rank();
     __shared__ double sre[CV_TY][CV_TX][4], sim[CV_TY][CV_TX][4];
     const int page = blockIdx.y, ty = threadIdx.y;
     const int pair0 = (blockIdx.x * CV_TX + threadIdx.x) * 4;      // first of this thread's four pairs within the H*D row
-    const int start = spans[2 * page], end = spans[2 * page + 1];
-    const int n_tok = max(0, end - start);
+    const int page_start = spans[2 * page], page_end = spans[2 * page + 1];
+    const int n_tok = max(0, page_end - page_start), share = (n_tok + split - 1) / split;
+    const int start = page_start + min(part * share, n_tok), end = page_start + min((part + 1) * share, n_tok);   // this CTA's tokens
     const bool active = pair0 < (H * D) / 2;
     const int dpair0 = active ? ((2 * pair0) % D) / 2 : 0;          // pair index inside the head (the four share a head)
 
@@ -142,21 +149,33 @@ page_centroid_vec_kernel(const __nv_bfloat16 *__restrict__ keys, long long sb, l
             sim[ty][threadIdx.x][e] = acc_im[e];
         }
         __syncthreads();
-        if (ty == 0 && active) {
+        double r[4] = {0.0, 0.0, 0.0, 0.0}, i[4] = {0.0, 0.0, 0.0, 0.0};
+        if (ty == 0) {
 #pragma unroll
             for (int e = 0; e < 4; ++e) {
-                double r = 0.0, i = 0.0;
                 for (int y = 0; y < CV_TY; ++y) {
-                    r += sre[y][threadIdx.x][e];
-                    i += sim[y][threadIdx.x][e];
+                    r[e] += sre[y][threadIdx.x][e];
+                    i[e] += sim[y][threadIdx.x][e];
                 }
-                out_re[e] += (double)(float)(r / (double)max(n_tok, 1));
-                out_im[e] += (double)(float)(i / (double)max(n_tok, 1));
+                sre[0][threadIdx.x][e] = r[e];     // the CTA's share, for the cluster's first CTA
+                sim[0][threadIdx.x][e] = i[e];
             }
         }
-        __syncthreads();
+        cluster.sync();
+        if (part == 0 && ty == 0 && active) {
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+                for (int c = 1; c < split; ++c) {
+                    r[e] += *cluster.map_shared_rank(&sre[0][threadIdx.x][e], c);
+                    i[e] += *cluster.map_shared_rank(&sim[0][threadIdx.x][e], c);
+                }
+                out_re[e] += (double)(float)(r[e] / (double)max(n_tok, 1));
+                out_im[e] += (double)(float)(i[e] / (double)max(n_tok, 1));
+            }
+        }
+        cluster.sync();   // the shares are read until here
     }
-    if (ty == 0 && active) {
+    if (part == 0 && ty == 0 && active) {
         float *dst = page_index + (long long)page * H * D + 2 * pair0;
         float o[8];
 #pragma unroll
@@ -258,7 +277,8 @@ score_topk_kernel(const float *__restrict__ page_index, const float *__restrict_
 }
 
 // ------------------------------------------------------------------------------------------------
-// Page install: strided row copy with an optional per-page temporal rotation of the keys.
+// Page install: strided row copy with an optional per-page temporal rotation of the keys; a record without a source clears
+// its rows (the unused tails of all layers' caches go in one launch).
 // grid (token tiles, records).  16-byte vectors when every address allows it.
 // ------------------------------------------------------------------------------------------------
 constexpr int GP_THREADS = 256;
@@ -301,7 +321,7 @@ gather_pages_kernel(const wa_page_copy *__restrict__ copies, int row_elems, int 
     const wa_page_copy rec = copies[blockIdx.y];
     const T *src = reinterpret_cast<const T *>(rec.src);
     T *dst = reinterpret_cast<T *>(rec.dst);
-    const float2 *rot = (rec.rot >= 0 && rotations) ? rotations + (long long)rec.rot * nt : nullptr;
+    const float2 *rot = (rec.rot >= 0 && rotations && src) ? rotations + (long long)rec.rot * nt : nullptr;
     const bool vec_ok = (row_elems % VE == 0) && (rec.src_stride % VE == 0) && (rec.dst_stride % VE == 0) &&
                         (reinterpret_cast<uintptr_t>(src) % 16 == 0) && (reinterpret_cast<uintptr_t>(dst) % 16 == 0) &&
                         (head_dim % VE == 0 || rot == nullptr);
@@ -318,7 +338,7 @@ gather_pages_kernel(const wa_page_copy *__restrict__ copies, int row_elems, int 
             if (e < total) {
                 tok[u] = e / vpr;
                 c[u] = (int)(e % vpr) * VE;
-                buf[u] = *reinterpret_cast<const uint4 *>(src + tok[u] * rec.src_stride + c[u]);
+                buf[u] = src ? *reinterpret_cast<const uint4 *>(src + tok[u] * rec.src_stride + c[u]) : make_uint4(0u, 0u, 0u, 0u);
             }
         }
 #pragma unroll
@@ -338,8 +358,8 @@ gather_pages_kernel(const wa_page_copy *__restrict__ copies, int row_elems, int 
             if (e >= total) break;
             const long long t = e / ppr;
             const int col = (int)(e % ppr) * 2;
-            float a = load_elem(src, sizeof(T) == 2 ? WA_BF16 : WA_F32, t * rec.src_stride + col);
-            float b = load_elem(src, sizeof(T) == 2 ? WA_BF16 : WA_F32, t * rec.src_stride + col + 1);
+            float a = src ? load_elem(src, sizeof(T) == 2 ? WA_BF16 : WA_F32, t * rec.src_stride + col) : 0.f;
+            float b = src ? load_elem(src, sizeof(T) == 2 ? WA_BF16 : WA_F32, t * rec.src_stride + col + 1) : 0.f;
             const int dpair = (col % head_dim) >> 1;
             if (rot && dpair < nt) {
                 const float2 w = rot[dpair];
@@ -371,10 +391,24 @@ extern "C" int wa_hkv_page_centroids(const wa_tensor4 *keys, int B, int T, int H
     WA_REQUIRE(P <= 65535, WA_ERR_UNSUPPORTED, "%s: at most 65535 pages per call", what);
     if (keys->dtype == WA_BF16 && keys->stride_h == D && D % 8 == 0 && (uintptr_t)keys->ptr % 16 == 0 && keys->stride_l % 8 == 0 &&
         keys->stride_b % 8 == 0 && (uintptr_t)page_index % 16 == 0) {
-        dim3 vgrid(ceil_div(H * D / 2, CV_TX * 4), P), vblock(CV_TX, CV_TY);
-        page_centroid_vec_kernel<<<vgrid, vblock, 0, (cudaStream_t)stream>>>(
-            (const __nv_bfloat16 *)keys->ptr, keys->stride_b, keys->stride_l, B, H, D, spans, reinterpret_cast<const float2 *>(derope),
-            n_frames, n_temporal, frame_seq_length, page_index);
+        // shares per page: as many CTAs as are resident at once (two per SM) where a call has few pages
+        const long long groups = (long long)ceil_div(H * D / 2, CV_TX * 4) * P;
+        const int split = groups >= 296 ? 1 : (int)(296 / groups < CV_MAX_SPLIT ? 296 / groups : CV_MAX_SPLIT);
+        cudaLaunchConfig_t cfg{};
+        cfg.gridDim = dim3(ceil_div(H * D / 2, CV_TX * 4), P, split);
+        cfg.blockDim = dim3(CV_TX, CV_TY);
+        cfg.stream = (cudaStream_t)stream;
+        cudaLaunchAttribute attr[1];
+        attr[0].id = cudaLaunchAttributeClusterDimension;
+        attr[0].val.clusterDim.x = 1;
+        attr[0].val.clusterDim.y = 1;
+        attr[0].val.clusterDim.z = split;
+        cfg.attrs = attr;
+        cfg.numAttrs = 1;
+        const cudaError_t e = cudaLaunchKernelEx(&cfg, page_centroid_vec_kernel, (const __nv_bfloat16 *)keys->ptr, (long long)keys->stride_b,
+                                                 (long long)keys->stride_l, B, H, D, spans, reinterpret_cast<const float2 *>(derope), n_frames,
+                                                 n_temporal, frame_seq_length, page_index);
+        if (e != cudaSuccess) return fail((int)e, "%s: %s", what, cudaGetErrorString(e));
         return check_launch(what);
     }
     dim3 grid(ceil_div(H * D / 2, CT_TX), P), block(CT_TX, CT_TY);

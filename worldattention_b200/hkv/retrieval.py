@@ -14,7 +14,7 @@ import torch
 import torch.nn.functional as F
 
 from .. import _lib
-from .rope import rotation_table, temporal_complex_dims
+from .rope import rotation_table, temporal_complex_dims, to_device
 
 __all__ = ["prompt_index", "query_index", "page_key_index", "score_pages", "select_top_chunks",
            "select_topk_pages", "score_and_topk"]
@@ -45,8 +45,8 @@ def page_key_index(keys: torch.Tensor, page_spans: Sequence[Tuple[int, int]], *,
     nt = temporal_complex_dims(head_dim)
     n_frames = (tokens + frame_seq_length - 1) // frame_seq_length
     frames = start_frame + np.arange(n_frames)
-    rot = torch.from_numpy(rotation_table(temporal_freqs, np.zeros_like(frames), frames, nt)).to(dev)
-    spans = torch.tensor([[int(s), int(e)] for s, e in page_spans], dtype=torch.int32).to(dev)
+    rot = to_device(rotation_table(temporal_freqs, np.zeros_like(frames), frames, nt), dev)
+    spans = to_device(np.array([[int(s), int(e)] for s, e in page_spans], dtype=np.int32), dev)
     out = torch.empty((len(page_spans), heads * head_dim), device=dev, dtype=torch.float32)
     keys = keys if keys.stride(-1) == 1 else keys.contiguous()
     _lib.check(_lib.lib().wa_hkv_page_centroids(

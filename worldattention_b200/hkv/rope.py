@@ -29,10 +29,16 @@ def temporal_band(freqs: torch.Tensor, head_dim: int) -> torch.Tensor:
     return freqs[:, : temporal_complex_dims(head_dim)]
 
 
-def _freqs_numpy(temporal_freqs) -> np.ndarray:
+def host_table(temporal_freqs) -> np.ndarray:
+    """The frequency table on the host (a table on the device is fetched, which waits for the device)."""
     if isinstance(temporal_freqs, torch.Tensor):
         return temporal_freqs.detach().to("cpu").numpy()
     return np.asarray(temporal_freqs)
+
+
+def to_device(array: np.ndarray, dev) -> torch.Tensor:
+    """A small host array on the device, in the order of the current stream; nothing waits on the host."""
+    return torch.from_numpy(np.ascontiguousarray(array)).pin_memory().to(dev, non_blocking=True)
 
 
 def rotation_table(temporal_freqs, new_ids, orig_ids, num_temporal: int) -> np.ndarray:
@@ -40,7 +46,7 @@ def rotation_table(temporal_freqs, new_ids, orig_ids, num_temporal: int) -> np.n
 
     Returns float32 `[rows, num_temporal, 2]` (complex64 as re/im pairs), computed in complex128.
     """
-    table = _freqs_numpy(temporal_freqs)
+    table = host_table(temporal_freqs)
     n = table.shape[0]
     new = np.clip(np.asarray(new_ids, dtype=np.int64).reshape(-1), 0, n - 1)
     orig = np.clip(np.asarray(orig_ids, dtype=np.int64).reshape(-1), 0, n - 1)
