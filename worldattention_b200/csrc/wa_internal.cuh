@@ -32,18 +32,17 @@ constexpr int SCHED_HEADS = 256;
 // 797 against 716 us a call).  Taken back: only the heavier 60 % of a head's items so and the rest by weight over all heads,
 // which evens out the end but mixes the heads again (764 us).
 // Calls with so many items that ranking them against one another would take too long here are counting-sorted by weight.
-static __device__ __noinline__ void schedule_items(const int32_t *num, int rows, int Nq, int Nkv, bool paired, bool by_head,
-                                                   int32_t *__restrict__ order, int *work_counter, int *error_flag) {
+__device__ inline void schedule_items(const int32_t *num, int rows, int Nq, int Nkv, bool paired, bool by_head,
+                                      int32_t *__restrict__ order, int *work_counter, int *error_flag) {
     __shared__ int hist[SCHED_BINS];
     __shared__ int warp_tot[32];
     const int T = blockDim.x, tid = threadIdx.x;
     const int each = paired ? (Nq + 1) >> 1 : Nq, heads = rows / Nq, n_items = heads * each;   // items of a head, ...
+    // without branches, so that a thread's look-ups are all on their way at once (one after the other they cost the call 3 us)
     auto count_of = [&](int i) {
-        if (!paired) return __ldcg(num + i);
         const int head = i / each, q = 2 * (i - head * each);
-        const int32_t *at = num + (long long)head * Nq + q;
-        const int first = __ldcg(at);
-        return q + 1 < Nq ? max(first, __ldcg(at + 1)) : first;
+        const int32_t *at = num + (paired ? (long long)head * Nq + q : i);
+        return max(__ldcg(at), __ldcg(at + (paired && q + 1 < Nq ? 1 : 0)));
     };
     if (by_head && heads <= SCHED_HEADS && n_items <= SCHED_BINS && (long long)n_items * each <= 2048ll * T) {
         __shared__ int head_sum[SCHED_HEADS], head_rank[SCHED_HEADS];
