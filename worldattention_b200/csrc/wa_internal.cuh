@@ -85,10 +85,17 @@ __device__ inline void schedule_items(const int32_t *num, int rows, int Nq, int 
     // the counts were written by other CTAs of this launch: read them past L1, and only once when they fit in registers
     constexpr int KEEP = 4;
     int bin_of[KEEP];
+    if (!paired) {
+#pragma unroll
+        for (int u = 0; u < KEEP; ++u) bin_of[u] = tid + u * T < n_items ? __ldcg(num + tid + u * T) : -1;
+    } else {
+#pragma unroll
+        for (int u = 0; u < KEEP; ++u) bin_of[u] = tid + u * T < n_items ? count_of(tid + u * T) : -1;
+    }
 #pragma unroll
     for (int u = 0; u < KEEP; ++u) {
         const int i = tid + u * T;
-        bin_of[u] = i < n_items ? top - max(0, min(count_of(i), top)) : -1;
+        bin_of[u] = i < n_items ? top - max(0, min(bin_of[u], top)) : -1;
     }
 #pragma unroll
     for (int u = 0; u < KEEP; ++u)
