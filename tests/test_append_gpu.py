@@ -87,3 +87,24 @@ def test_append_rejects_unaligned_positions_and_falls_back_for_other_dtypes():
                            segment_len=seg, k_proj_mat=ek, v_proj_mat=ev, block_size=bs, dtype="fp32")
     first = position // seg * slots_per
     np.testing.assert_allclose(to_np(kc)[:, first:first + slots_per], okc.transpose(0, 2, 1, 3), rtol=1e-5, atol=1e-5)
+
+
+@pytest.mark.parametrize("proj_dtype", [torch.bfloat16, torch.float32])
+def test_appends_of_different_sizes_share_a_workspace(proj_dtype):
+    """Segments that the tensor-core stream does not take (an odd row length of the projection, or a float32 one) go through
+    the kept workspace: calls of three, one and three segments on one stream all write every slot."""
+    import worldattention_b200 as wa
+    from worldattention_b200.hsa.attention import append_kv
+    heads, d, seg, bs = 12, 128, 1558, 128
+    hsa, rng, mk, ek, ev, _, _, k_cache, v_cache, kc, vc, _, slots_per = _setup(wa, heads, d, seg, bs, 0, 3)
+    pk, pv = to_gpu(ek).to(proj_dtype), to_gpu(ev).to(proj_dtype)
+    rows_k, rows_v = to_gpu(mk(3 * seg), "bf16"), to_gpu(mk(3 * seg), "bf16")
+    for n_seg in (3, 1, 3):
+        n = n_seg * seg
+        kc.fill_(7.0); vc.fill_(-7.0)
+        append_kv(rows_k[:, :n], rows_v[:, :n], k_cache, v_cache, kc, vc, position=0, segment_len=seg, k_proj_mat=pk, v_proj_mat=pv,
+                         block_size=bs)
+        for got, rows, proj in ((kc, rows_k, pk), (vc, rows_v, pv)):
+            want = torch.einsum("rt,bsthd->bsrhd", proj.double(), rows[:, :n].view(1, n_seg, seg, heads, d).double())
+            np.testing.assert_allclose(to_np(got)[:, :n_seg * slots_per], to_np(want.reshape(1, n_seg * slots_per, heads, d).float()),
+                                       rtol=2 ** -7, atol=1e-5)

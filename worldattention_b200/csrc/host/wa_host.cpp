@@ -359,7 +359,7 @@ PyObject *append_kv(PyObject *const *a, Py_ssize_t n) {
     };
     int rc = call(nullptr, 0);                                     // the tensor-core stream needs no workspace
     if (rc == WA_ERR_WORKSPACE) {
-        const Tensor ws = workspace(1, dev, stream, f_append_bytes(B, N, H, D, (int)seg, (int)block, rank), true);   // zeroed once; every call leaves it zeroed
+        const Tensor ws = workspace(1, dev, stream, f_append_bytes(B, N, H, D, (int)seg, (int)block, rank), true);   // zeroed once; every call leaves the counters zeroed
         rc = call(ws.data_ptr(), (size_t)ws.numel());
     }
     if (rc == WA_ERR_UNSUPPORTED) Py_RETURN_FALSE;

@@ -333,7 +333,7 @@ append_compress_kernel(const __nv_bfloat16 *__restrict__ k_new, const __nv_bfloa
     for (int e = threadIdx.x; e < rank * 128; e += CF_WARPS * 32) mine[e] = red[e / 128][e % 128];
     __threadfence();
     __syncthreads();
-    if (threadIdx.x == 0) last_flag = atomicAdd(&counters[group], 1) == split - 1;
+    if (threadIdx.x == 0) last_flag = split == 1 || atomicAdd(&counters[group], 1) == split - 1;
     __syncthreads();
     if (!last_flag) return;
     __threadfence();
@@ -344,7 +344,7 @@ append_compress_kernel(const __nv_bfloat16 *__restrict__ k_new, const __nv_bfloa
         for (int s = 0; s < split; ++s) sum += __ldcg(all + (long long)s * (R * 128) + e);
         out[(long long)(slot0 + seg * slot_stride + e / 128) * osl + e % 128] = __float2bfloat16_rn(sum);
     }
-    if (threadIdx.x == 0) counters[group] = 0;   // ready for the next call on this workspace
+    if (threadIdx.x == 0 && split > 1) counters[group] = 0;   // ready for the next call on this workspace
 }
 
 }  // namespace wa
@@ -404,11 +404,14 @@ int wa::compress_kv_launch(const wa_tensor4 *k, const wa_tensor4 *v, const wa_te
 }
 
 // Workspace of wa_kv_append_compress: counters first (they must be zero before the FIRST call and are left zero by every
-// call), then the float32 partial sums.
+// call), then the float32 partial sums, which no call clears.  The counters' part is as large for every call: with a size
+// of its own per call, the partial sums of one call would lie where the counters of a later, larger one are.
 namespace {
+constexpr int AP_SPLIT_BELOW = 296;   // groups; with as many (two CTAs per SM) a group is one CTA and needs no counter
+constexpr size_t AP_COUNTER_BYTES = (AP_SPLIT_BELOW * sizeof(int) + 255) / 256 * 256;
 struct AppendPlan {
     int n_seg, split, tokens_per_split, rank_full, slot_stride, tiles;
-    size_t counters_bytes, total_bytes;
+    size_t total_bytes;
 };
 AppendPlan append_plan(int B, int n_new, int H, int D, int segment_len, int block_size, int proj_rank) {
     AppendPlan a{};
@@ -420,14 +423,13 @@ AppendPlan append_plan(int B, int n_new, int H, int D, int segment_len, int bloc
     a.tiles = H * D / 128;
     // enough CTAs for two per SM of a large GPU, but no split shorter than one staged projection tile
     const int groups = a.tiles * a.n_seg * 2 * B;
-    int split = groups >= 296 ? 1 : ceil_div(296, groups);
+    int split = groups >= AP_SPLIT_BELOW ? 1 : ceil_div(AP_SPLIT_BELOW, groups);
     const int max_split = longest / CF_TT > 0 ? longest / CF_TT : 1;
     if (split > max_split) split = max_split;
     if (split > 16) split = 16;
     a.split = split;
     a.tokens_per_split = ceil_div(ceil_div(longest, split), CF_WARPS) * CF_WARPS;
-    a.counters_bytes = align_up((size_t)groups * sizeof(int), 256);
-    a.total_bytes = a.counters_bytes + (size_t)groups * split * 32 * 128 * sizeof(float);
+    a.total_bytes = AP_COUNTER_BYTES + (size_t)groups * split * 32 * 128 * sizeof(float);
     return a;
 }
 }  // namespace
@@ -480,7 +482,7 @@ extern "C" int wa_kv_append_compress(const wa_tensor4 *k_new, const wa_tensor4 *
     WA_REQUIRE(workspace && workspace_bytes >= a.total_bytes && (uintptr_t)workspace % 256 == 0, WA_ERR_WORKSPACE,
                "%s: a 256-byte aligned workspace of %zu bytes is required (zeroed before its first use)", what, a.total_bytes);
     int *counters = (int *)workspace;
-    float *partials = (float *)((char *)workspace + a.counters_bytes);
+    float *partials = (float *)((char *)workspace + AP_COUNTER_BYTES);
     const int slot0 = position / segment_len * a.slot_stride;
     dim3 grid(a.tiles, a.n_seg * a.split, 2 * B);
 #define WA_APPEND_LAUNCH(R)                                                                                                      \
