@@ -1,8 +1,9 @@
 """The float32-exact attention on matrix instructions (head_dim 128) against float64 softmax attention.
 
 Every product is a sum of exact bf16 products accumulated in float32, so a result is off by the float32 accumulation of the
-scores (128 terms, |s| up to a few units) and of P V: a few 1e-6 relative to the values.  The bound below is 2e-5 of the
-largest value of the result, which a probability or an operand kept in 16 bits (2^-9) would miss by two orders."""
+scores (128 terms, |s| up to a few units) and of P V: a few 1e-6 of the largest value.  The bound of the first tests is 2e-5 of
+that, which a probability or an operand kept in 16 bits (2^-9) would miss by two orders; the last ones look for products left
+out and for sums that lose the same way at every step."""
 import numpy as np
 import pytest
 import torch
@@ -38,11 +39,11 @@ def _sparse(q, k, v, index, num, block):
     return out
 
 
-def _linear(q, kc, vc):
+def _linear(q, kc, vc, lse=None):
     from worldattention_b200 import _lib
     out = torch.empty(q.shape, device=q.device, dtype=torch.float32)
     _lib.check(_lib.lib().wa_linear_branch(_lib.t4_blhd(q), _lib.t4_blhd(kc), _lib.t4_blhd(vc), _lib.t4_blhd(out), 1, q.shape[2], q.shape[1],
-                                           kc.shape[1], D, 0, None, _lib.stream_ptr(q.device)))
+                                           kc.shape[1], D, 0, _lib.ptr(lse), _lib.stream_ptr(q.device)))
     return out
 
 
@@ -87,3 +88,32 @@ def test_strided_rows_and_infinities():
     assert bool((got[0, :, 1, 9] == -float("inf")).all())
     got[0, :, 1, 9] = 0
     assert bool(torch.isfinite(got).all())
+
+
+def test_every_partial_product_of_a_score_counts():
+    # parts 1, 2^-7 - 2^-15 and 2^-15 - 2^-23: the products of the second and third ones are 2^-21 of the whole
+    q = torch.full((1, 64, 1, D), 1 + 2.0 ** -7 - 2.0 ** -23, device=dev())
+    lse = torch.empty((1, 1, 64), device=dev())
+    _linear(q, q[:, :1].contiguous(), q[:, :1].contiguous(), lse)          # one slot: the score itself
+    want = float(q[0, 0, 0, 0].double()) ** 2 * np.sqrt(D)
+    # eight 16-term sums, each cut by 2^-23 at most, added up with 4.5 roundings of the whole (n / 8 at the n-th), one for the scale
+    assert float((lse.double() / want - 1).abs().max()) <= 2.0 ** -23 + 5.5 * 2.0 ** -24
+
+
+@pytest.mark.parametrize("keys,rounded", [(4680, True), (2000, False)])
+def test_long_rows_of_one_sign_lose_nothing(keys, rounded):
+    g = torch.Generator(device=dev()).manual_seed(keys)
+    q, k, v = (torch.randn((1, 2, n, D), generator=g, device=dev()) for n in (128, keys, keys))
+    v = v.abs()
+    if rounded:
+        block = 64
+        nkv = -(-keys // block)
+        index = torch.arange(nkv, device=dev(), dtype=torch.int32).expand(1, 2, 2, nkv).contiguous()
+        got = _sparse(q, k, v, index, torch.full((1, 2, 2), nkv, device=dev(), dtype=torch.int32), block)
+        q, k, v = (t.to(torch.bfloat16) for t in (q, k, v))
+    else:
+        got = _linear(*(t.transpose(1, 2).contiguous() for t in (q, k, v))).transpose(1, 2)
+    s = q[0].double() @ k[0].double().transpose(1, 2) / np.sqrt(D)
+    want = torch.softmax(s, -1) @ v[0].double()
+    # a step of 16 keys is cut by 2^-23 per leading product, always downward; everything else rounds either way
+    assert abs(float((got[0].double() / want - 1).mean())) <= 3 * 2.0 ** -23

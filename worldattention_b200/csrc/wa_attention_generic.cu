@@ -163,19 +163,24 @@ generic_attention_kernel(GenericAttnParams p) {
 }
 
 // ------------------------------------------------------------------------------------------------
-// head_dim 128: the same contract on the warp-level matrix instructions, without giving up float32 anywhere.
+// head_dim 128: the same contract on the warp-level matrix instructions, with the accuracy of the float32 kernel above.
 //
 // Two warps share 16 of the CTA's 64 query rows, each with one half of a chunk's keys and sums of its own (merged at the
-// end); chunks may span several routing blocks.  Every product is a sum of bf16 products accumulated in float32, whose
-// operands are exact:
+// end); chunks may span several routing blocks.  Operands are sums of bf16 parts without a remainder, and every product of
+// parts is taken:
 //   NS = 1  q, k and v are bf16 values (bf16 tensors, or `round_in`): one product for the scores; the float32
 //           probabilities are three bf16 parts (8 + 8 + 8 bits of the significand), so P V takes three.
-//   NS = 3  float32 operands, three parts each: the six products of order up to 2^-16 of the leading one; the
-//           dropped ones are below 2^-23.
+//   NS = 3  float32 operands, three parts each: nine products, of which the smallest still matter: a part is cut off, so
+//           the second is up to 2^-7 and the third up to 2^-15 of its value and a product of both 2^-22.
 // Parts are cut off, not rounded, so they keep the sign of their value, and a part that would be zero is a tiny
 // number instead: infinities in V or K then give what a float32 product gives and not 0 * inf.
-// The SIMT kernel above is bound by shared-memory reads (one per four multiply-adds).  float32 layer, 12 heads, 1560 queries
-// over 4680 keys in 64-token blocks: both branches 2094 -> 255 us (sparse 200, linear 54).
+// The instruction's own accumulator cuts what does not fit its 24 bits, always toward zero: a sum carried in it through all
+// products and keys was up to 2.6e-5 too small.  So each accumulation starts at zero and takes only the products of one
+// 16-term step, smallest first; the steps are added with rounding in registers.
+// Error against float64 (2-norm of the result), SIMT kernel -> this one: 75 float32 slots 3.8e-7 -> 1.8e-7, 2000 slots
+// 9.2e-7 -> 2.6e-7, 4680 rounded keys 1.25e-6 -> 2.9e-7; the log-sum-exp has the same error within 6 % or less.
+// The SIMT kernel above is bound by shared-memory reads (one per four multiply-adds).  12 heads, 1560 queries: a third of
+// 4680 keys in 64-token blocks 1480 -> 238 us, 75 float32 slots 92 -> 57 us.
 // ------------------------------------------------------------------------------------------------
 constexpr int SA_ROWS = 64;                  // query rows of a CTA
 constexpr int SA_THREADS = 256;
@@ -193,9 +198,28 @@ __device__ __forceinline__ void ldsm4_t(uint32_t (&r)[4], uint32_t addr) {
     asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0, %1, %2, %3}, [%4];"
                  : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(addr) : "memory");
 }
+__device__ __forceinline__ void mma16816_new(float (&c)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {   // from zero
+    asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%10, %10, %10, %10};"
+                 : "=f"(c[0]), "=f"(c[1]), "=f"(c[2]), "=f"(c[3]) : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1), "f"(0.f));
+}
 __device__ __forceinline__ void mma16816(float (&c)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
     asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
                  : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3]) : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
+}
+
+// two 8-column products of one step, from zero or onto what the step has summed up
+__device__ __forceinline__ void mma_step(bool first, float (&x0)[4], float (&x1)[4], const uint32_t (&a)[4], const uint32_t (&b)[4]) {
+    if (first) {
+        mma16816_new(x0, a, b[0], b[1]);
+        mma16816_new(x1, a, b[2], b[3]);
+    } else {
+        mma16816(x0, a, b[0], b[1]);
+        mma16816(x1, a, b[2], b[3]);
+    }
+}
+__device__ __forceinline__ void add4(float (&c)[4], const float (&x)[4]) {
+#pragma unroll
+    for (int i = 0; i < 4; ++i) c[i] += x[i];
 }
 
 constexpr float SA_TINY = 2.3509887e-38f;    // 2^-125, a bf16 number
@@ -325,17 +349,16 @@ split_attention_kernel(GenericAttnParams p) {
             for (int i = 0; i < NS; ++i) ldsm4(a[i], qa + i * Q_PART + kk * 32);
 #pragma unroll
             for (int j = 0; j < NT; j += 2) {
-                // smallest products first
+                float x0[4], x1[4];   // this step's 16 channels
 #pragma unroll
                 for (int i = NS - 1; i >= 0; --i) {
                     uint32_t kb[4];
                     ldsm4(kb, ka + i * K_PART + (uint32_t)(j * 8 * SA_LD + kk * 16) * 2);
 #pragma unroll
-                    for (int u = NS - 1 - i; u >= 0; --u) {
-                        mma16816(sc[j], a[u], kb[0], kb[1]);
-                        mma16816(sc[j + 1], a[u], kb[2], kb[3]);
-                    }
+                    for (int u = NS - 1; u >= 0; --u) mma_step(i == NS - 1 && u == NS - 1, x0, x1, a[u], kb);
                 }
+                add4(sc[j], x0);
+                add4(sc[j + 1], x1);
             }
         }
         // scale, mask, running maximum
@@ -390,16 +413,16 @@ split_attention_kernel(GenericAttnParams p) {
             }
 #pragma unroll
             for (int j = 0; j < SA_D / 8; j += 2) {
+                float x0[4], x1[4];   // this step's 16 keys
 #pragma unroll
                 for (int i = NS - 1; i >= 0; --i) {
                     uint32_t vb[4];
                     ldsm4_t(vb, va + i * K_PART + (uint32_t)(kk * 16 * SA_LD + j * 8) * 2);
 #pragma unroll
-                    for (int u = 2 - i; u >= 0; --u) {
-                        mma16816(o[j], a[u], vb[0], vb[1]);
-                        mma16816(o[j + 1], a[u], vb[2], vb[3]);
-                    }
+                    for (int u = 2; u >= 0; --u) mma_step(i == NS - 1 && u == 2, x0, x1, a[u], vb);
                 }
+                add4(o[j], x0);
+                add4(o[j + 1], x1);
             }
         }
     }
