@@ -117,3 +117,16 @@ def test_long_rows_of_one_sign_lose_nothing(keys, rounded):
     want = torch.softmax(s, -1) @ v[0].double()
     # a step of 16 keys is cut by 2^-23 per leading product, always downward; everything else rounds either way
     assert abs(float((got[0].double() / want - 1).mean())) <= 3 * 2.0 ** -23
+
+
+@pytest.mark.parametrize("hidden", [8, 16, 32, 40])
+def test_leading_keys_without_weight(hidden):
+    # the first `hidden` keys score -inf: they have no weight, whatever chunk of keys they fill; a row of nothing else is NaN
+    g = torch.Generator(device=dev()).manual_seed(hidden)
+    q, kc, vc = (torch.randn((1, n, 2, D), generator=g, device=dev()) for n in (20, 70, 70))
+    q[..., 5] = 1.0
+    kc[:, :hidden, :, 5] = -float("inf")
+    want = _exact(q[0], kc[0, hidden:], vc[0, hidden:], lambda h, r: list(range(70 - hidden)))
+    got = _linear(q, kc, vc)[0].double().cpu().numpy()
+    assert np.abs(got - want).max() <= 2e-5 * np.abs(want).max()
+    assert bool(torch.isnan(_linear(q, kc[:, :hidden], vc[:, :hidden])).all())

@@ -289,6 +289,7 @@ split_attention_kernel(GenericAttnParams p) {
     const long long kbase = (long long)b * p.k.sb + (long long)h * p.k.sh, vbase = (long long)b * p.v.sb + (long long)h * p.v.sh;
     const long long total = (long long)n_sel * p.kv_block;
     const bool rows_mine = 16 * rg < rows_here;
+    unsigned any_key = 0;   // this warp's half had a real key
 
     // ldmatrix addresses of this lane (A operand; B operand of the scores; B operand of P V, transposed)
     const uint32_t qa = sa_u32(qs + (16 * rg + (lane & 15)) * SA_LD + (lane >> 4) * 8);
@@ -337,6 +338,7 @@ split_attention_kernel(GenericAttnParams p) {
 #pragma unroll
         for (int w = 0; w < 4; ++w) keep |= real[4 * half_keys + w] << (w * RW);
         if (keep == 0) continue;
+        any_key = 1;
         const bool full = keep == (KW == 32 ? ~0u : (1u << (KW & 31)) - 1);
 
         float sc[NT][4];
@@ -383,12 +385,13 @@ split_attention_kernel(GenericAttnParams p) {
         const float fA = mA == -INFINITY ? 0.f : expf(mA - nA), fB = mB == -INFINITY ? 0.f : expf(mB - nB);
         mA = nA; mB = nB;
         lA *= fA; lB *= fB;
+        const float eA = nA == -INFINITY ? 0.f : nA, eB = nB == -INFINITY ? 0.f : nB;   // only scores of -inf so far: weights of zero
 #pragma unroll
         for (int j = 0; j < SA_D / 8; ++j) { o[j][0] *= fA; o[j][1] *= fA; o[j][2] *= fB; o[j][3] *= fB; }
 #pragma unroll
         for (int j = 0; j < NT; ++j) {
-            sc[j][0] = expf(sc[j][0] - nA); sc[j][1] = expf(sc[j][1] - nA);
-            sc[j][2] = expf(sc[j][2] - nB); sc[j][3] = expf(sc[j][3] - nB);
+            sc[j][0] = expf(sc[j][0] - eA); sc[j][1] = expf(sc[j][1] - eA);
+            sc[j][2] = expf(sc[j][2] - eB); sc[j][3] = expf(sc[j][3] - eB);
             if (!full) {
                 if (!((keep >> (8 * j + c2)) & 1)) sc[j][0] = sc[j][2] = 0.f;
                 if (!((keep >> (8 * j + c2 + 1)) & 1)) sc[j][1] = sc[j][3] = 0.f;
@@ -435,6 +438,7 @@ split_attention_kernel(GenericAttnParams p) {
     __syncthreads();
     float4 *left = reinterpret_cast<float4 *>(ks) + (size_t)rg * (SA_D / 8 + 1) * 32 + lane;   // [SA_D / 8 + 1][32 lanes]
     static_assert(4 * (SA_D / 8 + 1) * 32 * 16 <= NS * 2 * KC * SA_LD * 2, "the accumulators fit where the keys and values were");
+    if (lane == 0) real[warp] = any_key;
     if (half_keys && rows_mine) {
 #pragma unroll
         for (int j = 0; j < SA_D / 8; ++j) left[j * 32] = make_float4(o[j][0], o[j][1], o[j][2], o[j][3]);
@@ -442,6 +446,7 @@ split_attention_kernel(GenericAttnParams p) {
     }
     __syncthreads();
     if (half_keys || !rows_mine) return;
+    any_key |= real[warp + 4];
     {
         const float4 other = left[SA_D / 8 * 32];
         const float nA = fmaxf(mA, other.x), nB = fmaxf(mB, other.y);
@@ -461,7 +466,9 @@ split_attention_kernel(GenericAttnParams p) {
     for (int half = 0; half < 2; ++half) {
         const int lr = 16 * rg + g + 8 * half, row = row0 + lr;
         if (lr >= rows_here) continue;
-        const float l = half ? lB : lA, m = half ? mB : mA, inv = l > 0.f ? 1.0f / l : 0.f;
+        const float l = half ? lB : lA, m = half ? mB : mA;
+        // no key: zeros; keys, but every score -inf: not a number, as a softmax of them is
+        const float inv = l > 0.f ? 1.0f / l : any_key && m == -INFINITY ? NAN : 0.f;
         const long long at = (long long)b * p.osb + (long long)row * p.osl + (long long)h * p.osh + c2;
 #pragma unroll
         for (int j = 0; j < SA_D / 8; ++j) {
