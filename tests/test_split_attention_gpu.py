@@ -130,3 +130,15 @@ def test_leading_keys_without_weight(hidden):
     got = _linear(q, kc, vc)[0].double().cpu().numpy()
     assert np.abs(got - want).max() <= 2e-5 * np.abs(want).max()
     assert bool(torch.isnan(_linear(q, kc[:, :hidden], vc[:, :hidden])).all())
+
+
+@pytest.mark.parametrize("bits", [0x7f800001, 0x7fc00000, -0x7fffff])    # the first and last (0xff800001) are infinities in their upper halves
+def test_every_nan_stays_one(bits):
+    g = torch.Generator(device=dev()).manual_seed(1)
+    q, kc, vc = (torch.randn((1, n, 2, D), generator=g, device=dev()) for n in (20, 40, 40))
+    q.view(torch.int32)[0, 3, 1, 7] = bits
+    vc.view(torch.int32)[0, 9, 0, 5] = bits
+    nan = torch.isnan(_linear(q, kc, vc))
+    want = torch.zeros_like(nan)
+    want[0, 3, 1], want[0, :, 0, 5] = True, True
+    assert torch.equal(nan, want)

@@ -223,6 +223,7 @@ __device__ __forceinline__ void add4(float (&c)[4], const float (&x)[4]) {
 }
 
 constexpr float SA_TINY = 2.3509887e-38f;    // 2^-125, a bf16 number
+__device__ __forceinline__ float plain_nan(float x) { return x == x ? x : NAN; }   // one whose upper half is a NaN by itself
 __device__ __forceinline__ float top_part(float x) { return __uint_as_float(__float_as_uint(x) & 0xffff0000u); }
 __device__ __forceinline__ float rest_of(float x, float hi) {
     const float r = x - hi;
@@ -237,6 +238,7 @@ __device__ __forceinline__ void stage4(__nv_bfloat16 *dst, size_t part_stride, f
         __nv_bfloat162 a = __floats2bfloat162_rn(x.x, x.y), b = __floats2bfloat162_rn(x.z, x.w);
         *reinterpret_cast<uint2 *>(dst) = make_uint2(*reinterpret_cast<uint32_t *>(&a), *reinterpret_cast<uint32_t *>(&b));
     } else {
+        x = make_float4(plain_nan(x.x), plain_nan(x.y), plain_nan(x.z), plain_nan(x.w));
 #pragma unroll
         for (int i = 0; i < NS; ++i) {
             *reinterpret_cast<uint2 *>(dst + i * part_stride) = make_uint2(top_pair(x.x, x.y), top_pair(x.z, x.w));
