@@ -268,3 +268,22 @@ def test_sharded_forward_rejects_unknown_options_before_touching_tensors():
     for bad in (dict(exchange="ring"), dict(routing="everything"), dict(routing="candidates")):   # the last: no fixed top-k given
         with pytest.raises(ValueError):
             sharded.hsa_attention_kv_sharded(hsa, q, q, q, q, q, kv_len=64, shards=[(0, 64)], **bad)
+
+
+def _cpu_cache(rows, layers=3, heads=2, d=8, filled=0):
+    return [{"k": torch.zeros(1, rows, heads, d), "v": torch.zeros(1, rows, heads, d), "local_end_index": torch.tensor([filled]),
+             "global_end_index": torch.tensor([filled])} for _ in range(layers)]
+
+
+@pytest.mark.parametrize("short", ["all", "one"])
+def test_store_refuses_more_tokens_than_the_cache_holds(monkeypatch, short):
+    """The copy kernel takes addresses, so the check stands before it: nothing is launched and nothing is banked."""
+    from worldattention_b200.hkv import cache as C
+    monkeypatch.setattr(C._lib, "require_cuda", lambda *tensors: torch.device("cpu"))
+    monkeypatch.setattr(C, "gather_records_device", lambda *a, **k: pytest.fail("launched"))
+    kv = _cpu_cache(100 if short == "all" else 160, filled=160)
+    kv[1]["v"] = torch.zeros(1, 100, 2, 8)
+    bank = wa.hkv.HKVCache(frame_seq_length=16, page_size_frames=2)
+    with pytest.raises(RuntimeError, match="160 tokens"):
+        bank.store(kv, prompt_embeds=torch.zeros(1, 4, 8), current_start_frame=10, temporal_freqs=None)
+    assert len(bank) == 0

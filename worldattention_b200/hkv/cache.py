@@ -84,6 +84,9 @@ class HKVCache:
         if valid_tokens <= 0:
             return -1
         _lib.require_cuda(kv_cache[0]["k"])
+        short = next((block[name] for block in kv_cache for name in ("k", "v") if block[name].shape[1] < valid_tokens), None)
+        if short is not None:          # the copy kernel takes addresses: nothing behind it would stop at the end of a cache
+            raise RuntimeError(f"local_end_index says {valid_tokens} tokens, but an online cache tensor holds {short.shape[1]} rows")
         temporal_freqs = host_table(temporal_freqs)     # before the copies: it waits for the device
 
         chunk_id = len(self.chunks)
