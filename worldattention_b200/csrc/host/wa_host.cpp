@@ -13,6 +13,7 @@
 #include <torch/csrc/autograd/python_variable.h>
 
 #include <algorithm>
+#include <climits>
 #include <cmath>
 #include <list>
 #include <string>
@@ -199,6 +200,7 @@ PyObject *hsa_forward(PyObject *const *a, Py_ssize_t n) {
     Tensor keep[12];
     wa_hsa_params p{};
     const long long block = integer(a[10]);
+    if (block <= 0 || block > INT_MAX) fail(PyExc_ValueError, "block_size must be positive, got " + std::to_string(block));   // divided by below
     p.B = (int)B; p.H = (int)H; p.D = (int)D; p.Lq = (int)Lq; p.Lkv = (int)Lkv;
     p.block_size = (int)block;
     p.tau_min = real(a[11]);
@@ -214,7 +216,7 @@ PyObject *hsa_forward(PyObject *const *a, Py_ssize_t n) {
     p.k = view4(k, keep[2]);
     p.v = view4(*v, keep[3]);
     if (pooled) {
-        const int64_t blocks = block > 0 ? (Lkv + block - 1) / block : 0;
+        const int64_t blocks = (Lkv + block - 1) / block;
         if (pooled->scalar_type() != at::kFloat || pooled->sizes() != at::IntArrayRef({B, H, blocks, D}) || !pooled->is_contiguous() ||
             pooled->device() != dev)
             fail(PyExc_ValueError, "expected k_pooled_cache: contiguous float32 [" + std::to_string(B) + ", " + std::to_string(H) + ", " +
