@@ -287,3 +287,17 @@ def test_store_refuses_more_tokens_than_the_cache_holds(monkeypatch, short):
     with pytest.raises(RuntimeError, match="160 tokens"):
         bank.store(kv, prompt_embeds=torch.zeros(1, 4, 8), current_start_frame=10, temporal_freqs=None)
     assert len(bank) == 0
+
+
+@pytest.mark.parametrize("grid", [(2, 3, 4), [2, 3, 4], (2.0, np.int64(3), 4), np.array([2, 3, 4]), torch.tensor([[2, 3, 4]] * 3),
+                                  ((2, 3, 4),), ((2, 3, 4),) * 2, ((2, 3, 4),) * 3, ([2, 3, 4], (2, 3, 4), [2, 3, 4]), [(2, 3, 4)] * 3])
+def test_grid_of_one_sample_or_of_a_batch(grid):
+    from worldattention_b200.rope import _grid
+    f, h, w = _grid(grid)
+    assert (f, h, w) == (2, 3, 4) and all(type(v) is int for v in (f, h, w))
+
+
+def test_grids_that_differ_within_a_batch_are_refused():
+    from worldattention_b200.rope import _grid
+    with pytest.raises(NotImplementedError):
+        _grid(((2, 3, 4), (2, 3, 4), (4, 3, 2)))

@@ -21,7 +21,7 @@ def _table(freqs: torch.Tensor, dev: torch.device) -> torch.Tensor:
 
 
 def _grid(grid_sizes) -> tuple[int, int, int]:
-    if type(grid_sizes) is tuple and len(grid_sizes) == 3:
+    if type(grid_sizes) is tuple and len(grid_sizes) == 3 and all(type(v) is int for v in grid_sizes):
         return grid_sizes
     rows = grid_sizes.tolist() if hasattr(grid_sizes, "tolist") else list(grid_sizes)
     if rows and isinstance(rows[0], (list, tuple)):
