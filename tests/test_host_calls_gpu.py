@@ -1,4 +1,7 @@
 """The native host module's own work: what it refuses, how it reads its arguments, and the workspaces it keeps."""
+import sys
+
+import numpy as np
 import pytest
 import torch
 
@@ -26,3 +29,22 @@ def _attend(q, k, v, **options):
 def test_block_sizes_that_are_none(block, routing):
     with pytest.raises(ValueError):
         _attend(**{**_inputs(), "block_size": block}, return_routing=routing)
+
+
+def test_integers_of_other_types():
+    options = _inputs()
+
+    class Size:
+        def __int__(self):
+            return token
+
+    token = int("1000064")          # an object of its own, so that references to it can be counted
+    want = _attend(**options)
+    for as_given in (np.int64(64), 64.0, torch.tensor(64)):
+        assert torch.equal(_attend(**{**options, "block_size": as_given}), want)
+    before = sys.getrefcount(token)
+    for _ in range(5):
+        _attend(**{**options, "proj_segment_len": Size(), "k_pooled_valid": Size()})      # both larger than what they bound
+    assert sys.getrefcount(token) == before
+    with pytest.raises(TypeError):
+        _attend(**{**options, "block_size": "sixty-four".encode})

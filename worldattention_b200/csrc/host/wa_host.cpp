@@ -69,7 +69,15 @@ const Tensor &tensor(PyObject *o, const char *name) {
     return *t;
 }
 long long integer(PyObject *o) {
-    const long long v = PyLong_Check(o) ? PyLong_AsLongLong(o) : PyLong_AsLongLong(PyNumber_Long(o));
+    if (!PyLong_Check(o)) {
+        PyObject *as_int = PyNumber_Long(o);
+        if (!as_int) throw PyFailure();
+        const long long v = PyLong_AsLongLong(as_int);
+        Py_DECREF(as_int);
+        if (v == -1 && PyErr_Occurred()) throw PyFailure();
+        return v;
+    }
+    const long long v = PyLong_AsLongLong(o);
     if (v == -1 && PyErr_Occurred()) throw PyFailure();
     return v;
 }
