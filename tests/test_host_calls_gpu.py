@@ -48,3 +48,19 @@ def test_integers_of_other_types():
     assert sys.getrefcount(token) == before
     with pytest.raises(TypeError):
         _attend(**{**options, "block_size": "sixty-four".encode})
+
+
+def test_modulation_with_and_without_the_token_axis():
+    from worldattention_b200.causal_dit import gated_residual, ln_modulate
+    g = torch.Generator(device=dev()).manual_seed(0)
+    make = lambda *shape: torch.randn(shape, generator=g, device=dev()).to(torch.bfloat16)
+    b, f, n, c = 2, 3, 5, 256
+    x, y, e = make(b, f * n, c), make(b, f * n, c), make(b, f, 6, c)
+    for chunk in (e.chunk(6, dim=2), make(b, 2 * f, 6, c)[:, :f].chunk(6, dim=2)):     # frames of a longer tensor too
+        scale, shift = chunk[1], chunk[2]
+        want = ln_modulate(x, 1e-6, scale=scale, shift=shift, tokens_per_frame=n), gated_residual(x, y, scale, tokens_per_frame=n)
+        scale, shift = scale.squeeze(2), shift.squeeze(2)
+        assert torch.equal(ln_modulate(x, 1e-6, scale=scale, shift=shift, tokens_per_frame=n), want[0])
+        assert torch.equal(gated_residual(x, y, scale, tokens_per_frame=n), want[1])
+        strided = torch.stack([scale, shift], dim=-1)[..., 0]
+        assert torch.equal(gated_residual(x, y, strided, tokens_per_frame=n), want[1])

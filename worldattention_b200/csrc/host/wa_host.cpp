@@ -378,13 +378,14 @@ PyObject *append_kv(PyObject *const *a, Py_ssize_t n) {
 }
 
 // ---- the element-wise steps of a block (causal_dit.py) ------------------------------------------
-// `[B, F, 1, C]` modulation view -> (pointer, elements between consecutive frames); it must step uniformly over (b, f)
+// `[B, F, 1, C]` or `[B, F, C]` modulation view -> (pointer, elements between consecutive frames); it must step uniformly
+// over (b, f)
 const void *frame_vectors(const Tensor *e, int64_t dim, Tensor &keep, long long &stride) {
     if (!e) return nullptr;
     const Tensor *t = e;
-    if (e->dim() != 4) fail(PyExc_ValueError, "expected a [B, F, 1, C] modulation");
+    if (e->dim() < 2) fail(PyExc_ValueError, "expected a [B, F, 1, C] or [B, F, C] modulation, got shape " + shape_of(*e));
     const int64_t b = e->size(0), f = e->size(1);
-    if (e->stride(3) != 1 || e->size(3) != dim || (b > 1 && e->stride(0) != f * e->stride(1))) {
+    if (e->stride(-1) != 1 || e->size(-1) != dim || (b > 1 && e->stride(0) != f * e->stride(1))) {
         keep = e->contiguous();
         t = &keep;
     }
