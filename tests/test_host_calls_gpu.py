@@ -1,5 +1,7 @@
 """The native host module's own work: what it refuses, how it reads its arguments, and the workspaces it keeps."""
 import sys
+import threading
+import time
 
 import numpy as np
 import pytest
@@ -64,3 +66,26 @@ def test_modulation_with_and_without_the_token_axis():
         assert torch.equal(gated_residual(x, y, scale, tokens_per_frame=n), want[1])
         strided = torch.stack([scale, shift], dim=-1)[..., 0]
         assert torch.equal(gated_residual(x, y, strided, tokens_per_frame=n), want[1])
+
+
+def test_waiting_for_the_status_lets_other_threads_run():
+    options = _inputs()
+    want = _attend(**options, check_status=True)
+    ticks, stop = [0], threading.Event()
+
+    def tick():
+        while not stop.wait(0.002):
+            ticks[0] += 1
+
+    torch.cuda.synchronize()
+    thread = threading.Thread(target=tick)
+    thread.start()
+    try:
+        torch.cuda._sleep(10 ** 9)          # about half a second of work in front of the call
+        before, start = ticks[0], time.monotonic()
+        got = _attend(**options, check_status=True)
+        seen, waited = ticks[0] - before, time.monotonic() - start
+    finally:
+        stop.set()
+        thread.join()
+    assert waited > 0.2 and seen > 20 and torch.equal(got, want)

@@ -287,14 +287,20 @@ PyObject *hsa_forward(PyObject *const *a, Py_ssize_t n) {
         p.num_out = num.data_ptr<int32_t>();
         p.thresholds_out = thresholds.data_ptr<float>();
     }
-    const Tensor ws = workspace(0, dev, stream, f_workspace_bytes(&p), false);
+    // A call that waits for its own status lets other threads run meanwhile, so its workspace is nobody else's.
+    const size_t ws_bytes = f_workspace_bytes(&p);
+    const Tensor ws = check_status ? at::empty({(int64_t)ws_bytes}, at::TensorOptions().dtype(at::kByte).device(dev))
+                                   : workspace(0, dev, stream, ws_bytes, false);
     p.workspace = ws.data_ptr();
     p.workspace_bytes = (size_t)ws.numel();
     int used = 0;
     check(f_forward(&p, &used, stream));
     if (check_status && used) {
-        int status = 0;
-        check(f_status(&p, &status, stream));
+        int status = 0, rc = 0;
+        Py_BEGIN_ALLOW_THREADS          // waits for the stream: other threads may be what it waits for
+        rc = f_status(&p, &status, stream);
+        Py_END_ALLOW_THREADS
+        check(rc);
         if (status) {
             *status_word(dev.index()) = 0;
             fail(PyExc_RuntimeError, "tcgen05 HSA kernel gave up at wait site " + std::to_string(status) + "; its output is invalid");
