@@ -89,3 +89,26 @@ def test_waiting_for_the_status_lets_other_threads_run():
         stop.set()
         thread.join()
     assert waited > 0.2 and seen > 20 and torch.equal(got, want)
+
+
+def _append_inputs(heads=2, seg=200, block=64, capacity=3):
+    g = torch.Generator(device=dev()).manual_seed(0)
+    slots = -(-seg // block)
+    make = lambda n: torch.randn((1, n, heads, D), generator=g, device=dev()).to(torch.bfloat16)
+    empty = lambda n: torch.zeros((1, n, heads, D), device=dev(), dtype=torch.bfloat16)
+    proj = torch.randn((slots, seg), generator=g, device=dev()).to(torch.bfloat16)
+    caches = [empty(capacity * seg), empty(capacity * seg), empty(capacity * slots), empty(capacity * slots)]
+    return make(2 * seg), make(2 * seg), caches, dict(position=seg, segment_len=seg, k_proj_mat=proj, v_proj_mat=proj, block_size=block)
+
+
+@pytest.mark.parametrize("which", [0, 1, 2, 3])
+def test_append_into_caches_of_any_layout(which):
+    from worldattention_b200.hsa.attention import append_kv
+    k, v, caches, options = _append_inputs()
+    append_kv(k, v, *caches, **options)
+    _, _, others, _ = _append_inputs()
+    others[which] = torch.zeros_like(others[which]).transpose(2, 3).contiguous().transpose(2, 3)       # channels are not side by side
+    append_kv(k, v, *others, **options)
+    for got, want in zip(others, caches):
+        # the compressed slots may come from another kernel: one bf16 step of the largest value
+        assert float((got.float() - want.float()).abs().max()) <= 2.0 ** -7 * float(want.float().abs().max())

@@ -348,7 +348,7 @@ PyObject *qk_norm_rope(PyObject *const *a, Py_ssize_t n) {
 }
 
 // ---- append_kv: k_new, v_new, k_cache, v_cache, k_coarse, v_coarse, position, segment, k_proj, v_proj, block -> bool ----
-// False: the fused kernel does not cover the shape (nothing was launched).
+// False: the fused kernel does not cover the shape or the layout (nothing was launched).
 PyObject *append_kv(PyObject *const *a, Py_ssize_t n) {
     expect_args(n, 11);
     static const char *names[6] = {"k_new", "v_new", "k_cache", "v_cache", "k_coarse", "v_coarse"};
@@ -363,6 +363,10 @@ PyObject *append_kv(PyObject *const *a, Py_ssize_t n) {
     if (seg <= 0 || position % seg)
         fail(PyExc_ValueError, "rows are appended at segment boundaries, got position=" + std::to_string(position) + ", segment_len=" + std::to_string(seg));
     if (position + k_new.size(1) > THPVariable_Unpack(a[2]).size(1)) fail(PyExc_ValueError, "the rows do not fit the cache");
+    for (int i = 2; i < 6; ++i) {      // written in place: a re-laid-out copy would take the rows
+        const Tensor &dst = THPVariable_Unpack(a[i]);
+        if (dst.dim() == 4 && dst.stride(3) != 1 && dst.size(3) != 1) Py_RETURN_FALSE;
+    }
     for (int i = 0; i < 6; ++i) t[i] = view4(THPVariable_Unpack(a[i]), keep[i]);
     c10::cuda::CUDAGuard guard(dev);
     cudaStream_t stream = at::cuda::getCurrentCUDAStream(dev.index()).stream();
