@@ -112,3 +112,22 @@ def test_append_into_caches_of_any_layout(which):
     for got, want in zip(others, caches):
         # the compressed slots may come from another kernel: one bf16 step of the largest value
         assert float((got.float() - want.float()).abs().max()) <= 2.0 ** -7 * float(want.float().abs().max())
+
+
+@pytest.mark.parametrize("which", [1, 2, 3, 4, 5])
+def test_append_needs_room_in_every_tensor(which):
+    """v_new, the caches and the compressed tiers are addressed by the kernel: a row short of the need is an error on the host."""
+    from worldattention_b200.hsa.attention import append_kv
+    k, v, caches, options = _append_inputs()
+    tensors = [k, v, *caches]
+    append_kv(*tensors, **options)                        # two of three segments, up to the end
+    before = [t.clone() for t in tensors]
+    for short in (tensors[which][:, :-1], tensors[which][:, :, :1], tensors[which][..., :64], tensors[which][0]):
+        with pytest.raises(ValueError):
+            append_kv(*(short if i == which else t for i, t in enumerate(tensors)), **options)
+    assert all(torch.equal(a, b) for a, b in zip(tensors, before))
+    # a short last segment needs the slots of its own blocks only
+    _, _, fresh, _ = _append_inputs()
+    n = 200 + 70
+    append_kv(k[:, :n], v[:, :n], *fresh[:2], *(t[:, :4 + 4 + 2] for t in fresh[2:]), **options)
+    assert bool((fresh[2][:, 9] != 0).any()) and not bool((fresh[2][:, 10:] != 0).any())

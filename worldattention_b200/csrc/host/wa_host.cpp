@@ -363,6 +363,19 @@ PyObject *append_kv(PyObject *const *a, Py_ssize_t n) {
     if (seg <= 0 || position % seg)
         fail(PyExc_ValueError, "rows are appended at segment boundaries, got position=" + std::to_string(position) + ", segment_len=" + std::to_string(seg));
     if (position + k_new.size(1) > THPVariable_Unpack(a[2]).size(1)) fail(PyExc_ValueError, "the rows do not fit the cache");
+    if (seg > INT_MAX || block <= 0 || block > INT_MAX) fail(PyExc_ValueError, "segment_len and block_size must be positive");
+    // what the kernels write, addressed from here on: rows in both caches, `rank` slots per whole segment in both tiers
+    const int64_t rank_rows = tensor(a[8], "k_proj_mat").dim() == 2 ? THPVariable_Unpack(a[8]).size(0) : 0;
+    const int64_t n_new = k_new.size(1), whole = n_new / seg, tail = n_new % seg;
+    const int64_t stride = std::min<int64_t>(rank_rows, (seg + block - 1) / block);
+    const int64_t slots = (position / seg + whole) * stride + std::min<int64_t>(rank_rows, (tail + block - 1) / block);
+    for (int i = 1; i < 6; ++i) {
+        const Tensor &x = THPVariable_Unpack(a[i]);
+        const int64_t rows = i == 1 ? n_new : i < 4 ? position + n_new : slots;
+        if (x.dim() != 4 || x.size(0) < k_new.size(0) || x.size(1) < rows || x.size(2) < k_new.size(2) || x.size(3) < k_new.size(3))
+            fail(PyExc_ValueError, std::string(names[i]) + " of shape " + shape_of(x) + " does not hold the rows of k_new " + shape_of(k_new) +
+                                       " (" + std::to_string(rows) + " of them are needed)");
+    }
     for (int i = 2; i < 6; ++i) {      // written in place: a re-laid-out copy would take the rows
         const Tensor &dst = THPVariable_Unpack(a[i]);
         if (dst.dim() == 4 && dst.stride(3) != 1 && dst.size(3) != 1) Py_RETURN_FALSE;
