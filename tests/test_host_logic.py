@@ -301,3 +301,20 @@ def test_grids_that_differ_within_a_batch_are_refused():
     from worldattention_b200.rope import _grid
     with pytest.raises(NotImplementedError):
         _grid(((2, 3, 4), (2, 3, 4), (4, 3, 2)))
+
+
+@pytest.mark.parametrize("rerope,capacity,fetched", [(True, 40, 1), (False, 40, 0), (True, 0, 0)])
+def test_apply_fetches_the_frequency_table_only_to_rotate(monkeypatch, rerope, capacity, fetched):
+    """Fetching a table that lies on the device waits for everything enqueued there."""
+    from worldattention_b200.hkv import cache as C
+    calls = []
+    monkeypatch.setattr(C._lib, "require_cuda", lambda *tensors: torch.device("cpu"))
+    monkeypatch.setattr(C, "host_table", lambda table: calls.append(table))
+    for step in ("_install", "_install_sources", "_clear_tails"):
+        monkeypatch.setattr(C.HKVCache, step, lambda self, *a, **k: None)
+    bank = wa.hkv.HKVCache(frame_seq_length=8, page_size_frames=2, rerope=rerope)
+    bank.chunks.append({"chunk_id": 0, "valid_tokens": 32, "page_spans": [(0, 16), (16, 32)], "start_frame": 0, "page_index": None, "heads": 2})
+    bank.tier.put(0, {"k": [torch.zeros(1, 32, 2, 8)] * 3, "v": [torch.zeros(1, 32, 2, 8)] * 3})
+    kv = _cpu_cache(capacity)
+    assert bank.apply(kv, [(0, 0), (0, 1)], current_start_frame=9, temporal_freqs="table") == min(capacity, 32)
+    assert calls == ["table"] * fetched

@@ -183,7 +183,8 @@ class HKVCache:
             return 0
         dev = _lib.require_cuda(k0)
         tokens = int(plan["count"].sum())
-        temporal_freqs = host_table(temporal_freqs)     # before anything is launched: it waits for the device
+        if self.rerope and tokens > 0:
+            temporal_freqs = host_table(temporal_freqs)     # before anything is launched: it waits for the device
 
         compressed = all(name in kv_cache[0] for name in ("k_coarse", "v_coarse"))
         if compressed and hsa_modules is None:
