@@ -334,8 +334,7 @@ int wa_hkv_score_topk_layers(const float *page_index, const float *query, int la
 /* One page copy of the install step (cache.py:229-246).  `row_elems` contiguous elements per
  * token (H*D for whole-token pages, D for one head), token rows `src_stride` / `dst_stride`
  * elements apart.  `rot` >= 0 selects `rotations[rot]` (shift_temporal_rope, rope.py:50-67) and
- * applies it to the first 2*n_temporal elements of every head_dim-sized group; rot < 0 copies.  A null `src` clears the
- * rows of `dst`. */
+ * applies it to the first 2*n_temporal elements of every head_dim-sized group; rot < 0 copies. */
 typedef struct wa_page_copy {
     const void *src;
     void *dst;
@@ -356,6 +355,10 @@ int wa_hkv_build_records(const int32_t *top_ids, int layers, int heads, int topk
                          long long src_layer_stride, long long src_token_stride, void *dst_base,
                          long long dst_layer_stride, long long dst_token_stride, int page_tokens, int head_dim,
                          int elem_size, int rotate, wa_page_copy *records, int32_t *missing, void *stream);
+
+/* Clears the `dst` rows of `n` records in device memory (src, src_stride and rot are ignored): what lies behind
+ * the installed rows of all layers, in one launch.  max_tokens: the largest n_tokens of the records; elem_size 2 or 4. */
+int wa_hkv_clear_rows(const wa_page_copy *rows, int n, int max_tokens, int row_elems, int elem_size, void *stream);
 
 /* Promotion of cold pages (the `.to(device)` of cache.py:229-231 for chunks that live in host memory): one
  * asynchronous host-to-device copy per record of the HOST array `host_records` (src = page-locked host memory,

@@ -41,3 +41,13 @@ def test_argument_errors_are_reported_without_a_device():
     params = _lib.HsaParams()
     assert handle.wa_hsa_workspace_bytes(ctypes.byref(params)) == 0
     assert handle.wa_hsa_forward(ctypes.byref(params), None, None) == _lib.WA_ERR_ARG
+
+
+def test_a_library_of_another_version_is_refused(monkeypatch):
+    import pytest
+    import torch
+    from worldattention_b200 import _lib
+    monkeypatch.setattr(_lib, "_lib", None)
+    monkeypatch.setattr(_lib, "LIB_PATH", os.path.join(os.path.dirname(torch.__file__), "lib", "libc10.so"))     # none of the entry points
+    with pytest.raises(RuntimeError, match="rebuild"):
+        _lib.lib()

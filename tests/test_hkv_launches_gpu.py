@@ -66,3 +66,22 @@ def test_apply_installs_pages_and_clears_the_rest(hot, dtype, coarse_dtype):
         kc, vc = hsa[layer].compress_kv_cache(block["k"][:, :tokens], block["v"][:, :tokens])
         assert torch.equal(block["k_coarse"][:, :filled], kc.to(coarse_dtype)) and torch.equal(block["v_coarse"][:, :filled], vc.to(coarse_dtype))
         assert int(block["local_end_index"]) == tokens and int(block["global_end_index"]) == 40 * frame
+
+
+@pytest.mark.parametrize("dtype,row,pad,first,counts", [(torch.bfloat16, 1536, 0, 0, (40, 1, 0, 700)), (torch.bfloat16, 6, 2, 1, (5, 3000)),
+                                                        (torch.bfloat16, 16, 8, 3, (9,)), (torch.float32, 8, 0, 0, (300, 2)),
+                                                        (torch.float32, 6, 1, 1, (2000, 7)), (torch.float32, 4, 0, 0, (1,) * 65537)])
+def test_clear_rows_clears_its_rows_and_nothing_else(dtype, row, pad, first, counts):
+    # 16-byte pieces, rows and addresses that are not multiples of them, gaps between rows, records without rows, more than a launch takes
+    from worldattention_b200.hkv.install import RECORD_DTYPE, clear_rows_device
+    stride, size = row + pad, torch.empty((), dtype=dtype).element_size()
+    starts = np.cumsum([0] + [n + 2 for n in counts])            # two rows of others between the records
+    x = torch.full((first + int(starts[-1]) * stride,), 3.0, dtype=dtype, device=dev())
+    records = np.zeros(len(counts), dtype=RECORD_DTYPE)
+    records["dst"] = [x.data_ptr() + (first + int(s) * stride) * size for s in starts[:-1]]
+    records["dst_stride"], records["n_tokens"], records["src"] = stride, counts, 0
+    clear_rows_device(torch.from_numpy(records.view(np.uint8)).to(dev()), max_tokens=max(counts), row_elems=row, elem_size=size)
+    want = torch.full((int(starts[-1]), stride), 3.0)
+    for s, n in zip(starts, counts):
+        want[int(s): int(s) + n, :row] = 0
+    assert bool((x[:first] == 3.0).all()) and torch.equal(x[first:].view(-1, stride).float().cpu(), want)

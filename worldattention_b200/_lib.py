@@ -95,6 +95,7 @@ SIGNATURES = {
     "wa_hkv_build_records": [_vp, _i, _i, _i, _vp, _i, C.c_longlong, C.c_longlong, _vp, C.c_longlong, C.c_longlong,
                              _i, _i, _i, _i, _vp, _vp, _vp],
     "wa_hkv_promote_pages": [_vp, _i, _i, _i, _vp],
+    "wa_hkv_clear_rows": [_vp, _i, _i, _i, _i, _vp],
     "wa_hkv_gather_pages": [_vp, _i, _i, _i, _i, _i, _vp, _i, _vp],
 }
 _RESTYPES = {"wa_last_error": C.c_char_p, "wa_hsa_workspace_bytes": C.c_size_t, "wa_hsa_params_size": C.c_size_t, "wa_kv_append_workspace_bytes": C.c_size_t,
@@ -114,7 +115,9 @@ def lib() -> C.CDLL:
             )
         handle = C.CDLL(LIB_PATH)
         for name, argtypes in SIGNATURES.items():
-            fn = getattr(handle, name)
+            fn = getattr(handle, name, None)
+            if fn is None:
+                raise RuntimeError(f"{LIB_PATH} has no {name}: it was built from another version of the sources; rebuild the library")
             fn.argtypes = argtypes
             fn.restype = _RESTYPES.get(name, C.c_int)
         if handle.wa_abi_version() != 3 or handle.wa_hsa_params_size() != C.sizeof(HsaParams):

@@ -277,8 +277,7 @@ score_topk_kernel(const float *__restrict__ page_index, const float *__restrict_
 }
 
 // ------------------------------------------------------------------------------------------------
-// Page install: strided row copy with an optional per-page temporal rotation of the keys; a record without a source clears
-// its rows (the unused tails of all layers' caches go in one launch).
+// Page install: strided row copy with an optional per-page temporal rotation of the keys.
 // grid (token tiles, records).  16-byte vectors when every address allows it.
 // ------------------------------------------------------------------------------------------------
 constexpr int GP_THREADS = 256;
@@ -321,7 +320,7 @@ gather_pages_kernel(const wa_page_copy *__restrict__ copies, int row_elems, int 
     const wa_page_copy rec = copies[blockIdx.y];
     const T *src = reinterpret_cast<const T *>(rec.src);
     T *dst = reinterpret_cast<T *>(rec.dst);
-    const float2 *rot = (rec.rot >= 0 && rotations && src) ? rotations + (long long)rec.rot * nt : nullptr;
+    const float2 *rot = (rec.rot >= 0 && rotations) ? rotations + (long long)rec.rot * nt : nullptr;
     const bool vec_ok = (row_elems % VE == 0) && (rec.src_stride % VE == 0) && (rec.dst_stride % VE == 0) &&
                         (reinterpret_cast<uintptr_t>(src) % 16 == 0) && (reinterpret_cast<uintptr_t>(dst) % 16 == 0) &&
                         (head_dim % VE == 0 || rot == nullptr);
@@ -338,7 +337,7 @@ gather_pages_kernel(const wa_page_copy *__restrict__ copies, int row_elems, int 
             if (e < total) {
                 tok[u] = e / vpr;
                 c[u] = (int)(e % vpr) * VE;
-                buf[u] = src ? *reinterpret_cast<const uint4 *>(src + tok[u] * rec.src_stride + c[u]) : make_uint4(0u, 0u, 0u, 0u);
+                buf[u] = *reinterpret_cast<const uint4 *>(src + tok[u] * rec.src_stride + c[u]);
             }
         }
 #pragma unroll
@@ -358,8 +357,8 @@ gather_pages_kernel(const wa_page_copy *__restrict__ copies, int row_elems, int 
             if (e >= total) break;
             const long long t = e / ppr;
             const int col = (int)(e % ppr) * 2;
-            float a = src ? load_elem(src, sizeof(T) == 2 ? WA_BF16 : WA_F32, t * rec.src_stride + col) : 0.f;
-            float b = src ? load_elem(src, sizeof(T) == 2 ? WA_BF16 : WA_F32, t * rec.src_stride + col + 1) : 0.f;
+            float a = load_elem(src, sizeof(T) == 2 ? WA_BF16 : WA_F32, t * rec.src_stride + col);
+            float b = load_elem(src, sizeof(T) == 2 ? WA_BF16 : WA_F32, t * rec.src_stride + col + 1);
             const int dpair = (col % head_dim) >> 1;
             if (rot && dpair < nt) {
                 const float2 w = rot[dpair];
@@ -370,6 +369,38 @@ gather_pages_kernel(const wa_page_copy *__restrict__ copies, int row_elems, int 
             }
             store_elem(dst, sizeof(T) == 2 ? WA_BF16 : WA_F32, t * rec.dst_stride + col, a);
             store_elem(dst, sizeof(T) == 2 ? WA_BF16 : WA_F32, t * rec.dst_stride + col + 1, b);
+        }
+    }
+}
+
+// ------------------------------------------------------------------------------------------------
+// Clearing of token rows (the unused tails of all layers' caches in one launch): the same grid, stores only.  A kernel of
+// its own: a test for a missing source in the copy above costs every copy (per-head gather 1887 -> 1910 us).
+// ------------------------------------------------------------------------------------------------
+__global__ void __launch_bounds__(GP_THREADS)
+clear_rows_kernel(const wa_page_copy *__restrict__ rows, int row_elems, int elem_size) {
+    const wa_page_copy rec = rows[blockIdx.y];
+    char *dst = reinterpret_cast<char *>(rec.dst);
+    const long long row_bytes = (long long)row_elems * elem_size, stride = rec.dst_stride * elem_size;
+    const bool vec_ok = row_bytes % 16 == 0 && stride % 16 == 0 && reinterpret_cast<uintptr_t>(dst) % 16 == 0;
+    if (vec_ok) {
+        const int vpr = (int)(row_bytes / 16);
+        const long long total = (long long)rec.n_tokens * vpr, base = (long long)blockIdx.x * GP_THREADS * GP_UNROLL + threadIdx.x;
+#pragma unroll
+        for (int u = 0; u < GP_UNROLL; ++u) {
+            const long long e = base + (long long)u * GP_THREADS;
+            if (e < total) *reinterpret_cast<uint4 *>(dst + e / vpr * stride + e % vpr * 16) = make_uint4(0u, 0u, 0u, 0u);
+        }
+    } else {
+        // a tile is as many elements as 16-byte pieces would hold
+        const int per = 16 / elem_size;
+        const long long total = (long long)rec.n_tokens * row_elems;
+        for (int u = 0; u < GP_UNROLL * per; ++u) {
+            const long long e = ((long long)blockIdx.x * GP_UNROLL * per + u) * GP_THREADS + threadIdx.x;
+            if (e >= total) break;
+            char *at = dst + e / row_elems * stride + e % row_elems * elem_size;
+            if (elem_size == 2) *reinterpret_cast<uint16_t *>(at) = 0;
+            else *reinterpret_cast<uint32_t *>(at) = 0;
         }
     }
 }
@@ -543,6 +574,18 @@ extern "C" int wa_hkv_gather_pages(const wa_page_copy *copies, int n, int max_to
     else
         gather_pages_kernel<float><<<grid, GP_THREADS, 0, (cudaStream_t)stream>>>(
             copies, row_elems, head_dim, reinterpret_cast<const float2 *>(rotations), n_temporal);
+    return check_launch(what);
+}
+
+extern "C" int wa_hkv_clear_rows(const wa_page_copy *rows, int n, int max_tokens, int row_elems, int elem_size, void *stream) {
+    const char *what = "wa_hkv_clear_rows";
+    WA_REQUIRE(rows, WA_ERR_ARG, "%s: null record array", what);
+    WA_REQUIRE(n > 0 && max_tokens > 0 && row_elems > 0 && (elem_size == 2 || elem_size == 4), WA_ERR_ARG, "%s: bad sizes", what);
+    WA_REQUIRE(n <= 65535, WA_ERR_UNSUPPORTED, "%s: at most 65535 records per call", what);
+    const long long vecs = (long long)max_tokens * ceil_div(row_elems, 16 / elem_size);
+    const long long tiles = (vecs + GP_THREADS * GP_UNROLL - 1) / (GP_THREADS * GP_UNROLL);
+    WA_REQUIRE(tiles < (1ll << 31), WA_ERR_UNSUPPORTED, "%s: too many rows", what);
+    clear_rows_kernel<<<dim3((unsigned)tiles, n), GP_THREADS, 0, (cudaStream_t)stream>>>(rows, row_elems, elem_size);
     return check_launch(what);
 }
 

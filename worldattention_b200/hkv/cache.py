@@ -26,7 +26,7 @@ import numpy as np
 import torch
 
 from .. import _lib
-from .install import RECORD_DTYPE, gather_records_device
+from .install import RECORD_DTYPE, clear_rows_device, gather_records_device
 from .retrieval import page_key_index, prompt_index, score_and_topk, select_top_chunks
 from .rope import host_table, rotation_table, temporal_complex_dims, to_device
 from .tiering import HKVTierManager
@@ -288,7 +288,7 @@ class HKVCache:
     @classmethod
     def _clear_tails(cls, kv_cache, tokens: int, hsa_modules, dev) -> None:
         """Zero everything behind the installed tokens (and, with `hsa_modules`, behind their compressed slots) in all
-        layers: one launch of the page-copy kernel with records that have no source."""
+        layers in one launch."""
         k0 = kv_cache[0]["k"]
         row_elems = k0.shape[2] * k0.shape[3]
         direct = cls._copied_by_kernel(k0)
@@ -313,10 +313,8 @@ class HKVCache:
             return
         records = np.zeros(len(dst), dtype=RECORD_DTYPE)
         records["dst"], records["n_tokens"] = dst, count
-        records["src_stride"] = records["dst_stride"] = row_elems
-        records["rot"] = -1
-        gather_records_device(to_device(records.view(np.uint8), dev), max_tokens=max(count), row_elems=row_elems, head_dim=k0.shape[3],
-                              dtype=k0.dtype)
+        records["dst_stride"] = row_elems
+        clear_rows_device(to_device(records.view(np.uint8), dev), max_tokens=max(count), row_elems=row_elems, elem_size=k0.element_size())
 
     def _install_sources(self, kv_cache, plan, blobs, dtype):
         """Where the pages come from: `(whole, single, staged_elems)`.

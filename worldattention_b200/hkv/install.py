@@ -84,6 +84,14 @@ def gather_records_device(records_dev: torch.Tensor, *, max_tokens: int, row_ele
                                            _lib.stream_ptr(records_dev.device)))
 
 
+def clear_rows_device(records_dev: torch.Tensor, *, max_tokens: int, row_elems: int, elem_size: int) -> None:
+    """Clear the destination rows of records that already live on the device; their sources are ignored."""
+    n = records_dev.numel() // RECORD_DTYPE.itemsize
+    for start in range(0, n, 65535):
+        _lib.check(_lib.lib().wa_hkv_clear_rows(records_dev.data_ptr() + start * RECORD_DTYPE.itemsize, min(65535, n - start), max_tokens,
+                                                row_elems, elem_size, _lib.stream_ptr(records_dev.device)))
+
+
 def gather_pages(records: np.ndarray, *, max_tokens: int, row_elems: int, head_dim: int, dtype: torch.dtype,
                  device: torch.device, rotations: torch.Tensor | None = None, n_temporal: int = 0,
                  records_dev: torch.Tensor | None = None) -> torch.Tensor:
