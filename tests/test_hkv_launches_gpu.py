@@ -85,3 +85,9 @@ def test_clear_rows_clears_its_rows_and_nothing_else(dtype, row, pad, first, cou
     for s, n in zip(starts, counts):
         want[int(s): int(s) + n, :row] = 0
     assert bool((x[:first] == 3.0).all()) and torch.equal(x[first:].view(-1, stride).float().cpu(), want)
+
+
+@pytest.mark.parametrize("heads,pages,page", [(12, 14, 50), (12, 21, 33), (12, 30, 7), (1, 460, 384), (1, 2100, 40)])
+def test_page_centroids_by_four_three_two_and_one(heads, pages, page):
+    # CTAs per page: four, three and two resident ones, two over several waves, one
+    test_page_centroids(1, heads, pages * page - page // 3, page, 11)

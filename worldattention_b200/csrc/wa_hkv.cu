@@ -78,18 +78,20 @@ page_centroid_kernel(View4 keys, int B, int H, int D, const int32_t *__restrict_
 
 // The same for bf16 keys whose heads lie side by side (stride D, D a multiple of 8, 16-byte aligned rows): a thread owns
 // FOUR neighbouring pairs (one 16-byte load per token) and keeps four tokens' loads in flight.  Same arithmetic per value;
-// float64 sums, row groups added in order.  Bound by the loads in flight, and a stored window has few pages (seven of
-// three frames: 21 CTAs streamed its 100 MB in 525 us), so the tokens of a page are split over a thread-block cluster,
-// whose first CTA adds the shares up over distributed shared memory: 88 us.
-constexpr int CV_TX = 32, CV_TY = 8, CV_U = 4;
+// float64 sums, row groups added in order.  Bound by the loads in flight, hence three CTAs per SM (98 registers, two of
+// them: 480 pages of 1560 tokens 1000 us, three 806: 2.85 TB/s), and a stored window has few pages (seven of three frames:
+// 21 CTAs streamed its 100 MB in 525 us), so the tokens of a page are split over a thread-block cluster, whose first CTA adds
+// the shares up over distributed shared memory: 60 us.
+constexpr int CV_U = 4;
 constexpr int CV_MAX_SPLIT = 8;   // CTAs of a cluster (the portable limit)
 
-__global__ void __launch_bounds__(CV_TX *CV_TY)
+template <int CV_TX, int CV_TY, bool SPLIT>
+__global__ void __launch_bounds__(CV_TX *CV_TY, 3)
 page_centroid_vec_kernel(const __nv_bfloat16 *__restrict__ keys, long long sb, long long sl, int B, int H, int D,
                          const int32_t *__restrict__ spans, const float2 *__restrict__ derope, int n_frames, int nt,
                          int frame_seq_length, float *__restrict__ page_index) {
-    auto cluster = cooperative_groups::this_cluster();             // the CTAs that share a page and its columns (grid.z)
-    const int split = (int)cluster.num_blocks(), part = (int)cluster.block_rank();
+    auto cluster = cooperative_groups::this_cluster();             // SPLIT: the CTAs that share a page and its columns (grid.z)
+    const int split = SPLIT ? (int)cluster.num_blocks() : 1, part = SPLIT ? (int)cluster.block_rank() : 0;
     __shared__ double sre[CV_TY][CV_TX][4], sim[CV_TY][CV_TX][4];
     const int page = blockIdx.y, ty = threadIdx.y;
     const int pair0 = (blockIdx.x * CV_TX + threadIdx.x) * 4;      // first of this thread's four pairs within the H*D row
@@ -149,31 +151,47 @@ page_centroid_vec_kernel(const __nv_bfloat16 *__restrict__ keys, long long sb, l
             sim[ty][threadIdx.x][e] = acc_im[e];
         }
         __syncthreads();
-        double r[4] = {0.0, 0.0, 0.0, 0.0}, i[4] = {0.0, 0.0, 0.0, 0.0};
-        if (ty == 0) {
+        if constexpr (!SPLIT) {
+            if (ty == 0 && active) {
 #pragma unroll
-            for (int e = 0; e < 4; ++e) {
-                for (int y = 0; y < CV_TY; ++y) {
-                    r[e] += sre[y][threadIdx.x][e];
-                    i[e] += sim[y][threadIdx.x][e];
+                for (int e = 0; e < 4; ++e) {
+                    double r = 0.0, i = 0.0;
+                    for (int y = 0; y < CV_TY; ++y) {
+                        r += sre[y][threadIdx.x][e];
+                        i += sim[y][threadIdx.x][e];
+                    }
+                    out_re[e] += (double)(float)(r / (double)max(n_tok, 1));
+                    out_im[e] += (double)(float)(i / (double)max(n_tok, 1));
                 }
-                sre[0][threadIdx.x][e] = r[e];     // the CTA's share, for the cluster's first CTA
-                sim[0][threadIdx.x][e] = i[e];
             }
-        }
-        cluster.sync();
-        if (part == 0 && ty == 0 && active) {
+            __syncthreads();
+        } else {
+            double r[4] = {0.0, 0.0, 0.0, 0.0}, i[4] = {0.0, 0.0, 0.0, 0.0};
+            if (ty == 0) {
 #pragma unroll
-            for (int e = 0; e < 4; ++e) {
-                for (int c = 1; c < split; ++c) {
-                    r[e] += *cluster.map_shared_rank(&sre[0][threadIdx.x][e], c);
-                    i[e] += *cluster.map_shared_rank(&sim[0][threadIdx.x][e], c);
+                for (int e = 0; e < 4; ++e) {
+                    for (int y = 0; y < CV_TY; ++y) {
+                        r[e] += sre[y][threadIdx.x][e];
+                        i[e] += sim[y][threadIdx.x][e];
+                    }
+                    sre[0][threadIdx.x][e] = r[e];     // the CTA's share, for the cluster's first CTA
+                    sim[0][threadIdx.x][e] = i[e];
                 }
-                out_re[e] += (double)(float)(r[e] / (double)max(n_tok, 1));
-                out_im[e] += (double)(float)(i[e] / (double)max(n_tok, 1));
             }
+            cluster.sync();
+            if (part == 0 && ty == 0 && active) {
+#pragma unroll
+                for (int e = 0; e < 4; ++e) {
+                    for (int c = 1; c < split; ++c) {
+                        r[e] += *cluster.map_shared_rank(&sre[0][threadIdx.x][e], c);
+                        i[e] += *cluster.map_shared_rank(&sim[0][threadIdx.x][e], c);
+                    }
+                    out_re[e] += (double)(float)(r[e] / (double)max(n_tok, 1));
+                    out_im[e] += (double)(float)(i[e] / (double)max(n_tok, 1));
+                }
+            }
+            cluster.sync();   // the shares are read until here
         }
-        cluster.sync();   // the shares are read until here
     }
     if (part == 0 && ty == 0 && active) {
         float *dst = page_index + (long long)page * H * D + 2 * pair0;
@@ -409,6 +427,20 @@ clear_rows_kernel(const wa_page_copy *__restrict__ rows, int row_elems, int elem
 
 using namespace wa;
 
+// CTAs that share a page's tokens (`groups`: pages times column tiles; `page_tokens`: a page's average).  Three fit an SM: as
+// many as are resident at once, eight, four, three or two (14 pages of 1560 tokens take 44 us with four, 56 with five); two also
+// for up to some waves of them, which evens out the last one (60 pages: 126 us, one CTA per page 205; 300: 530 and 593; 480: 814
+// and 806), unless a page is too short to be shared (100 pages of 200 tokens: 46 and 39 us).
+static int centroid_split(long long groups, long long page_tokens) {
+    int dev = 0, sms = 148;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    const long long fit = 3ll * sms / groups;
+    if (fit >= CV_MAX_SPLIT) return CV_MAX_SPLIT;
+    if (fit >= 2) return fit < 4 ? (int)fit : 4;
+    return groups <= 14ll * sms && page_tokens >= 384 ? 2 : 1;
+}
+
 extern "C" int wa_hkv_page_centroids(const wa_tensor4 *keys, int B, int T, int H, int D, const int32_t *spans,
                                      int P, const float *derope, int n_frames, int n_temporal,
                                      int frame_seq_length, float *page_index, void *stream) {
@@ -422,23 +454,23 @@ extern "C" int wa_hkv_page_centroids(const wa_tensor4 *keys, int B, int T, int H
     WA_REQUIRE(P <= 65535, WA_ERR_UNSUPPORTED, "%s: at most 65535 pages per call", what);
     if (keys->dtype == WA_BF16 && keys->stride_h == D && D % 8 == 0 && (uintptr_t)keys->ptr % 16 == 0 && keys->stride_l % 8 == 0 &&
         keys->stride_b % 8 == 0 && (uintptr_t)page_index % 16 == 0) {
-        // shares per page: as many CTAs as are resident at once (two per SM) where a call has few pages
-        const long long groups = (long long)ceil_div(H * D / 2, CV_TX * 4) * P;
-        const int split = groups >= 296 ? 1 : (int)(296 / groups < CV_MAX_SPLIT ? 296 / groups : CV_MAX_SPLIT);
-        cudaLaunchConfig_t cfg{};
-        cfg.gridDim = dim3(ceil_div(H * D / 2, CV_TX * 4), P, split);
-        cfg.blockDim = dim3(CV_TX, CV_TY);
-        cfg.stream = (cudaStream_t)stream;
-        cudaLaunchAttribute attr[1];
-        attr[0].id = cudaLaunchAttributeClusterDimension;
-        attr[0].val.clusterDim.x = 1;
-        attr[0].val.clusterDim.y = 1;
-        attr[0].val.clusterDim.z = split;
-        cfg.attrs = attr;
-        cfg.numAttrs = 1;
-        const cudaError_t e = cudaLaunchKernelEx(&cfg, page_centroid_vec_kernel, (const __nv_bfloat16 *)keys->ptr, (long long)keys->stride_b,
-                                                 (long long)keys->stride_l, B, H, D, spans, reinterpret_cast<const float2 *>(derope), n_frames,
-                                                 n_temporal, frame_seq_length, page_index);
+        const int split = centroid_split((long long)ceil_div(H * D / 2, 32 * 4) * P, T / P);
+        const auto launch = [&](auto kernel, int tx, int ty) {
+            cudaLaunchConfig_t cfg{};
+            cfg.gridDim = dim3(ceil_div(H * D / 2, tx * 4), P, split);
+            cfg.blockDim = dim3(tx, ty);
+            cfg.stream = (cudaStream_t)stream;
+            cudaLaunchAttribute attr[1];
+            attr[0].id = cudaLaunchAttributeClusterDimension;
+            attr[0].val.clusterDim.x = 1;
+            attr[0].val.clusterDim.y = 1;
+            attr[0].val.clusterDim.z = split;
+            cfg.attrs = attr;
+            cfg.numAttrs = split > 1;
+            return cudaLaunchKernelEx(&cfg, kernel, (const __nv_bfloat16 *)keys->ptr, (long long)keys->stride_b, (long long)keys->stride_l, B, H, D,
+                                      spans, reinterpret_cast<const float2 *>(derope), n_frames, n_temporal, frame_seq_length, page_index);
+        };
+        cudaError_t e = split > 1 ? launch(page_centroid_vec_kernel<32, 8, true>, 32, 8) : launch(page_centroid_vec_kernel<64, 4, false>, 64, 4);
         if (e != cudaSuccess) return fail((int)e, "%s: %s", what, cudaGetErrorString(e));
         return check_launch(what);
     }
