@@ -215,7 +215,7 @@ hsa_fwd_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
                 const int n_st = BLK == TILE ? n_sel : PAIR ? max(n_sel, n_sel2) - n_both : (n_sel + 1) >> 1;
                 bar->items[slot].item = item;
                 bar->items[slot].n_sel = n_st;
-                bar->items[slot].n_both = n_both;
+                if (PAIR) bar->items[slot].n_both = n_both;
                 mbar_arrive(&bar->item_full[slot]);
                 if (item < 0) break;
                 at = (int)gridDim.x + atomicAdd(p.work_counter, 1);   // consumed at the top of the next round
@@ -421,7 +421,7 @@ hsa_fwd_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
             const uint32_t slot = jcount & 1u;
             ok = __all_sync(0xffffffffu, mbar_wait(&bar->item_full[slot], (jcount >> 1) & 1u, abort_flag, sink, 20));
             if (!ok) break;
-            const int item = bar->items[slot].item, n_sel = bar->items[slot].n_sel, n_both = bar->items[slot].n_both;
+            const int item = bar->items[slot].item, n_sel = bar->items[slot].n_sel, n_both = PAIR ? bar->items[slot].n_both : 0;
             __syncwarp();
             if (leader) mbar_arrive(&bar->item_empty[slot]);
             if (item < 0) break;
@@ -526,7 +526,7 @@ hsa_fwd_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
             const uint32_t slot = jcount & 1u;
             ok = __all_sync(0xffffffffu, mbar_wait(&bar->item_full[slot], (jcount >> 1) & 1u, abort_flag, sink, 15));
             if (!ok) break;
-            const int item = bar->items[slot].item, n_sel = bar->items[slot].n_sel, n_both = bar->items[slot].n_both;
+            const int item = bar->items[slot].item, n_sel = bar->items[slot].n_sel, n_both = PAIR ? bar->items[slot].n_both : 0;
             warp_arrive(&bar->item_empty[slot]);
             if (item < 0) break;
             const int qb = item % p.q_items, h = (item / p.q_items) % p.H, b = item / (p.q_items * p.H);
@@ -1002,7 +1002,7 @@ schedule_kernel(const int32_t *__restrict__ num, int rows, int Nq, int Nkv, Sche
         if (job.gate_w) convert_gate_slice(job, (blockIdx.x - 1) * 1024, 1024);
         return;
     }
-    schedule_items(num, rows, Nq, Nkv, job.paired, job.by_head, job.order, job.work_counter, job.error_flag);
+    schedule_items(num, rows, Nq, Nkv, job);
 }
 
 // ---- host side -----------------------------------------------------------------------------------
@@ -1128,8 +1128,9 @@ SchedJob hsa_sm100_sched_job(const wa_hsa_params *p, void *workspace) {
     job.paired = p->block_size == sm100::HALF && (long long)p->Lkv <= 16384ll * sm100::HALF &&
                  (long long)p->B * p->H * ceil_div(p->Lq, p->block_size) > sm100::max_grid();
     // Head by head where the keys and values are more than L2 keeps at a time; below that nothing is gained and the lighter
-    // items of the last head are a worse end than the lightest of all (three frames, 28 MB: 107.5 against 104.9 us)
-    job.by_head = 4ll * p->B * p->H * p->Lkv * p->D > (64ll << 20);
+    // items of the last head are a worse end than the lightest of all (three frames, 28 MB: 107.5 against 104.9 us).  128-token
+    // calls over the same window gain nothing by it (126 us either way) and their routing loses 1 us.
+    job.by_head = job.paired && 4ll * p->B * p->H * p->Lkv * p->D > (64ll << 20);
     return job;
 }
 

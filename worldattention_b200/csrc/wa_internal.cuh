@@ -16,7 +16,7 @@ struct SchedJob {
     __nv_bfloat16 *w_out;   // [128 x 128] bf16
     float *b_out;           // [128] float32
     bool paired;            // a work item is two neighbouring query blocks (rows of `num`) of one head
-    bool by_head;           // work order: head by head (see schedule_items)
+    bool by_head;           // paired: work order head by head (see sort_items_by_head)
     bool release_at_start;  // the next launch does not wait for the routing (it compresses K and V meanwhile)
     int release_dependents_after_rows;   // timing experiment (WA_B200_PDL=2), see route_row
 };
@@ -24,54 +24,14 @@ struct SchedJob {
 constexpr int SCHED_BINS = 4096;
 constexpr int SCHED_HEADS = 256;
 
-// Work order of the items, heavy first (weight: selected blocks; of a pair of rows the larger count).  Called by every
-// thread of ONE CTA whose size is a power of two between 32 and 1024.
-//
-// `by_head` (the keys are more than L2 holds): head by head, the head with the most work first and a head's items heaviest
-// first, so that the CTAs at work at a time read the keys of a few heads (counts from the mass over a window of 21 frames:
-// 797 against 716 us a call).  Taken back: only the heavier 60 % of a head's items so and the rest by weight over all heads,
-// which evens out the end but mixes the heads again (764 us).
-// Calls with so many items that ranking them against one another would take too long here are counting-sorted by weight.
-__device__ inline void schedule_items(const int32_t *num, int rows, int Nq, int Nkv, bool paired, bool by_head,
-                                      int32_t *__restrict__ order, int *work_counter, int *error_flag) {
-    __shared__ int hist[SCHED_BINS];
-    __shared__ int warp_tot[32];
+// Counting sort of the items by weight, heaviest first.  The last CTA of the routing runs it alone and the attention waits:
+// what is not needed for single rows (the pairs' look-ups, the order by heads) has code of its own, because instructions that
+// are fetched for the first time cost as much here as the sort (with one code for all, 16.5 -> 18.7 us of routing on
+// changing inputs).
+template <typename Count>
+__device__ __forceinline__ void sort_items(Count count_of, int n_items, int Nkv, int *hist, int *warp_tot, int32_t *__restrict__ order,
+                                           int *work_counter, int *error_flag) {
     const int T = blockDim.x, tid = threadIdx.x;
-    const int each = paired ? (Nq + 1) >> 1 : Nq, heads = rows / Nq, n_items = heads * each;   // items of a head, ...
-    // without branches, so that a thread's look-ups are all on their way at once (one after the other they cost the call 3 us)
-    auto count_of = [&](int i) {
-        const int head = i / each, q = 2 * (i - head * each);
-        const int32_t *at = num + (paired ? (long long)head * Nq + q : i);
-        return max(__ldcg(at), __ldcg(at + (paired && q + 1 < Nq ? 1 : 0)));
-    };
-    if (by_head && heads <= SCHED_HEADS && n_items <= SCHED_BINS && (long long)n_items * each <= 2048ll * T) {
-        __shared__ int head_sum[SCHED_HEADS], head_rank[SCHED_HEADS];
-        for (int i = tid; i < heads; i += T) head_sum[i] = 0;
-        if (tid == 0) {
-            *work_counter = 0;
-            *error_flag = 0;
-        }
-        __syncthreads();
-        for (int i = tid; i < n_items; i += T) {
-            const int w = max(0, min(count_of(i), Nkv));
-            hist[i] = w;
-            atomicAdd(&head_sum[i / each], w);
-        }
-        __syncthreads();
-        for (int i = tid; i < heads; i += T) {
-            int rank = 0;
-            for (int j = 0; j < heads; ++j) rank += head_sum[j] > head_sum[i] || (head_sum[j] == head_sum[i] && j < i);
-            head_rank[i] = rank;
-        }
-        __syncthreads();
-        for (int i = tid; i < n_items; i += T) {
-            const int head = i / each, first = head * each, w = hist[i];
-            int rank = 0;
-            for (int j = first; j < first + each; ++j) rank += hist[j] > w || (hist[j] == w && j < i);
-            order[head_rank[head] * each + rank] = i;
-        }
-        return;
-    }
     // bins 0..top hold counts top..0 (bin 0 = heaviest); `per` bins per thread, a power of two >= 1
     const int top = min(Nkv, SCHED_BINS - 1);
     int per = 1;
@@ -82,20 +42,13 @@ __device__ inline void schedule_items(const int32_t *num, int rows, int Nq, int 
         *error_flag = 0;
     }
     __syncthreads();
-    // the counts were written by other CTAs of this launch: read them past L1, and only once when they fit in registers
+    // the counts are read only once when they fit in registers
     constexpr int KEEP = 4;
     int bin_of[KEEP];
-    if (!paired) {
-#pragma unroll
-        for (int u = 0; u < KEEP; ++u) bin_of[u] = tid + u * T < n_items ? __ldcg(num + tid + u * T) : -1;
-    } else {
-#pragma unroll
-        for (int u = 0; u < KEEP; ++u) bin_of[u] = tid + u * T < n_items ? count_of(tid + u * T) : -1;
-    }
 #pragma unroll
     for (int u = 0; u < KEEP; ++u) {
         const int i = tid + u * T;
-        bin_of[u] = i < n_items ? top - max(0, min(bin_of[u], top)) : -1;
+        bin_of[u] = i < n_items ? top - max(0, min(count_of(i), top)) : -1;
     }
 #pragma unroll
     for (int u = 0; u < KEEP; ++u)
@@ -135,6 +88,65 @@ __device__ inline void schedule_items(const int32_t *num, int rows, int Nq, int 
     for (int u = 0; u < KEEP; ++u)
         if (bin_of[u] >= 0) order[atomicAdd(&hist[bin_of[u]], 1)] = tid + u * T;
     for (int i = tid + KEEP * T; i < n_items; i += T) order[atomicAdd(&hist[top - max(0, min(count_of(i), top))], 1)] = i;
+}
+
+// Head by head, the head with the most work first and a head's items heaviest first, so that the CTAs at work at a time read
+// the keys of a few heads (counts from the mass over a window of 21 frames: 797 against 716 us a call).  Taken back: only the
+// heavier 60 % of a head's items so and the rest by weight over all heads, which evens out the end but mixes the heads again
+// (764 us).
+template <typename Count>
+__device__ __forceinline__ void sort_items_by_head(Count count_of, int n_items, int each, int Nkv, int *hist, int32_t *__restrict__ order,
+                                                   int *work_counter, int *error_flag) {
+    const int T = blockDim.x, tid = threadIdx.x, heads = n_items / each;
+    int *head_sum = hist + SCHED_BINS - 2 * SCHED_HEADS, *head_rank = head_sum + SCHED_HEADS;   // behind the items' weights
+    for (int i = tid; i < heads; i += T) head_sum[i] = 0;
+    if (tid == 0) {
+        *work_counter = 0;
+        *error_flag = 0;
+    }
+    __syncthreads();
+    for (int i = tid; i < n_items; i += T) {
+        const int w = max(0, min(count_of(i), Nkv));
+        hist[i] = w;
+        atomicAdd(&head_sum[i / each], w);
+    }
+    __syncthreads();
+    for (int i = tid; i < heads; i += T) {
+        int rank = 0;
+        for (int j = 0; j < heads; ++j) rank += head_sum[j] > head_sum[i] || (head_sum[j] == head_sum[i] && j < i);
+        head_rank[i] = rank;
+    }
+    __syncthreads();
+    for (int i = tid; i < n_items; i += T) {
+        const int head = i / each, first = head * each, w = hist[i];
+        int rank = 0;
+        for (int j = first; j < first + each; ++j) rank += hist[j] > w || (hist[j] == w && j < i);
+        order[head_rank[head] * each + rank] = i;
+    }
+}
+
+// Work order of the items (a row of `num`, or two neighbouring ones of a head), heavy first (weight: selected blocks; of a
+// pair of rows the larger count).  Called by every thread of ONE CTA whose size is a power of two between 32 and 1024.
+// The counts were written by other CTAs of this launch: they are read past L1.
+__device__ inline void schedule_items(const int32_t *num, int rows, int Nq, int Nkv, const SchedJob &job) {
+    __shared__ int hist[SCHED_BINS];
+    __shared__ int warp_tot[32];
+    if (!job.paired) {
+        sort_items([&](int i) { return __ldcg(num + i); }, rows, Nkv, hist, warp_tot, job.order, job.work_counter, job.error_flag);
+        return;
+    }
+    const int each = (Nq + 1) >> 1, heads = rows / Nq, n_items = heads * each;
+    // without branches, so that a thread's look-ups are all on their way at once (one after the other they cost the call 3 us)
+    auto count_of = [&](int i) {
+        const int head = i / each, q = 2 * (i - head * each);
+        const int32_t *at = num + (long long)head * Nq + q;
+        return max(__ldcg(at), __ldcg(at + (q + 1 < Nq ? 1 : 0)));
+    };
+    // calls with so many items that ranking them against one another would take too long are sorted over all heads
+    if (job.by_head && heads <= SCHED_HEADS && n_items <= SCHED_BINS - 2 * SCHED_HEADS && (long long)n_items * each <= 2048ll * blockDim.x)
+        sort_items_by_head(count_of, n_items, each, Nkv, hist, job.order, job.work_counter, job.error_flag);
+    else
+        sort_items(count_of, n_items, Nkv, hist, warp_tot, job.order, job.work_counter, job.error_flag);
 }
 
 // Elements [first, first + count) of the gate weight -> bf16 (it is an MMA operand) and of the bias -> float32.

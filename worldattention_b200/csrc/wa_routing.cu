@@ -945,7 +945,7 @@ __device__ __forceinline__ void route_row(const long long row, const bool logits
     __syncthreads();
     if (!last_flag || !job.order) return;
     __threadfence();
-    schedule_items(num, B * H * Nq, Nq, Nkv, job.paired, job.by_head, job.order, job.work_counter, job.error_flag);
+    schedule_items(num, B * H * Nq, Nq, Nkv, job);
     ROUTE_STAMP(7);
 }
 
