@@ -131,3 +131,83 @@ def test_append_needs_room_in_every_tensor(which):
     n = 200 + 70
     append_kv(k[:, :n], v[:, :n], *fresh[:2], *(t[:, :4 + 4 + 2] for t in fresh[2:]), **options)
     assert bool((fresh[2][:, 9] != 0).any()) and not bool((fresh[2][:, 10:] != 0).any())
+
+
+def test_a_streams_workspace_grows_and_is_kept():
+    sizes = [(70, 130), (700, 6000), (130, 200), (1500, 9000), (70, 130)]
+    options = [_inputs(lq, lkv, seed=i) for i, (lq, lkv) in enumerate(sizes)]
+    want = []
+    for o in options:                                   # a stream of its own each
+        stream = torch.cuda.Stream()
+        stream.wait_stream(torch.cuda.current_stream())
+        with torch.cuda.stream(stream):
+            want.append(_attend(**o))
+        torch.cuda.current_stream().wait_stream(stream)
+    got = [_attend(**o) for o in options]               # one after the other on one stream, nothing waits
+    assert all(torch.equal(a, b) for a, b in zip(got, want))
+
+
+def test_workspaces_of_many_streams_are_bounded():
+    options = _inputs()
+    want = _attend(**options)
+    torch.cuda.synchronize()
+    streams = [torch.cuda.Stream() for _ in range(64)]
+    streams = list({s.cuda_stream: s for s in streams}.values())          # the pool hands streams out again
+    extra = [torch.cuda.ExternalStream(_new_stream()) for _ in range(48)]
+    before, outs = torch.cuda.memory_allocated(), []
+    for stream in streams + extra:
+        with torch.cuda.stream(stream):
+            outs.append(_attend(**options))
+    torch.cuda.synchronize()
+    assert len(streams) + len(extra) >= 48 and all(torch.equal(o, want) for o in outs)
+    results = sum(o.untyped_storage().nbytes() for o in outs)
+    assert torch.cuda.memory_allocated() - before <= 32 * (1 << 20) + results + len(outs) * 512       # 32 of the least size
+
+
+def _new_stream():
+    """A CUDA stream outside the framework's pool, never destroyed."""
+    import ctypes
+    rt = ctypes.CDLL("libcudart.so.12")
+    handle = ctypes.c_void_p()
+    assert rt.cudaStreamCreateWithFlags(ctypes.byref(handle), 1) == 0
+    return handle.value
+
+
+def test_a_captured_call_keeps_its_workspace_to_itself():
+    small, large = _inputs(130, 200, seed=1), _inputs(700, 6000, seed=2)
+    want = _attend(**small), _attend(**large)
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        got = _attend(**small), _attend(**large)
+    for _ in range(2):
+        for o in got:
+            o.zero_()
+        graph.replay()
+        eager = [_attend(**_inputs(900, 7000, seed=3)) for _ in range(3)]          # grows and uses the kept one behind the replay
+        graph.replay()
+        torch.cuda.synchronize()
+        assert torch.equal(got[0], want[0]) and torch.equal(got[1], want[1]) and torch.equal(eager[0], eager[2])
+
+
+@pytest.mark.parametrize("generic", [False, True])
+def test_partials_of_a_shard_use_the_same_workspace(generic):
+    from worldattention_b200.hsa.branches import hsa_partials, hsa_partials_packed, merge_partials, record_floats
+    options = _inputs(130, 512, block=64)
+    kc, vc = options["k"][:, ::64].contiguous(), options["v"][:, ::64].contiguous()
+    out, (index, num, _, _) = _attend(**options, k_coarse=kc, v_coarse=vc, return_routing=True)
+    torch.cuda.synchronize()
+    before = torch.cuda.memory_allocated()
+    shard = (options["q"], options["k"], options["v"], kc, vc, index, num, 64)
+    sparse, lse, linear, _, used = hsa_partials(*shard, force_generic=generic)
+    assert used is not generic
+    want = sparse + torch.sigmoid(options["q"].float()) * linear              # a call without gate weights
+    assert float((out.float() - want).abs().max()) <= 2.0 ** -6 * float(want.abs().max())
+    records = torch.zeros((1, 130, 2, record_floats(D)), device=dev())
+    assert hsa_partials_packed(*shard, records)
+    assert float((records[..., :D] - sparse).abs().max()) <= 2.0 ** -6 * float(sparse.abs().max())
+    del sparse, lse, linear, records, want
+    assert torch.cuda.memory_allocated() - before <= 1 << 16          # no second workspace
+    wide = torch.zeros((1, 130, 2, 64), device=dev(), dtype=torch.bfloat16)
+    assert not hsa_partials_packed(wide, wide, wide, wide, wide, index[..., :3].contiguous(), num, 64,
+                                   torch.zeros((1, 130, 2, record_floats(64)), device=dev()))

@@ -311,6 +311,27 @@ PyObject *hsa_forward(PyObject *const *a, Py_ssize_t n) {
                          used ? Py_True : Py_False);
 }
 
+// ---- run_forward: address of a wa_hsa_params (workspace unset), device index -> used_tuned, or None ----------------
+// For callers that fill the parameters themselves (partial outputs of a key shard): the stream's kept workspace and the
+// launches, under the interpreter lock as above.  None: the call asked for the tcgen05 kernel, which does not cover it.
+PyObject *run_forward(PyObject *const *a, Py_ssize_t n) {
+    expect_args(n, 2);
+    wa_hsa_params *p = reinterpret_cast<wa_hsa_params *>(PyLong_AsVoidPtr(a[0]));
+    if (PyErr_Occurred()) throw PyFailure();
+    if (!p) fail(PyExc_ValueError, "null parameters");
+    const c10::Device dev(c10::kCUDA, (c10::DeviceIndex)integer(a[1]));
+    c10::cuda::CUDAGuard guard(dev);
+    cudaStream_t stream = at::cuda::getCurrentCUDAStream(dev.index()).stream();
+    const Tensor ws = workspace(0, dev, stream, f_workspace_bytes(p), false);
+    p->workspace = ws.data_ptr();
+    p->workspace_bytes = (size_t)ws.numel();
+    int used = 0;
+    const int rc = f_forward(p, &used, stream);
+    if (rc == WA_ERR_UNSUPPORTED && (p->flags & WA_HSA_REQUIRE_TUNED)) Py_RETURN_NONE;
+    check(rc);
+    return PyBool_FromLong(used);
+}
+
 // ---- qk_norm_rope: x [B, L, H, D], weight|None, eps, table|None, start_frame (int or int32 device tensor), grid_h, grid_w -> out ----
 PyObject *qk_norm_rope(PyObject *const *a, Py_ssize_t n) {
     expect_args(n, 7);
@@ -512,7 +533,7 @@ PyObject *entry(PyObject *, PyObject *const *args, Py_ssize_t n) {
 }
 
 #define WA_ENTRY(name) {#name, (PyCFunction)(void (*)(void))entry<name>, METH_FASTCALL, nullptr}
-PyMethodDef methods[] = {WA_ENTRY(bind), WA_ENTRY(hsa_forward), WA_ENTRY(qk_norm_rope), WA_ENTRY(append_kv), WA_ENTRY(ln_modulate),
+PyMethodDef methods[] = {WA_ENTRY(bind), WA_ENTRY(hsa_forward), WA_ENTRY(run_forward), WA_ENTRY(qk_norm_rope), WA_ENTRY(append_kv), WA_ENTRY(ln_modulate),
                          WA_ENTRY(gated_residual), {nullptr, nullptr, 0, nullptr}};
 PyModuleDef module = {PyModuleDef_HEAD_INIT, "_host", nullptr, -1, methods, nullptr, nullptr, nullptr, nullptr};
 

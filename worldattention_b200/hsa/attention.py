@@ -155,19 +155,6 @@ def _unit_last(t: torch.Tensor) -> torch.Tensor:
     return t if t.stride(-1) == 1 else t.contiguous()
 
 
-_workspaces: dict = {}
-
-
-def _workspace(dev: torch.device, nbytes: int) -> torch.Tensor:
-    """One growing scratch buffer per (device, stream); kernels of one stream are ordered."""
-    key = (dev, torch.cuda.current_stream(dev).cuda_stream)
-    buf = _workspaces.get(key)
-    if buf is None or buf.numel() < nbytes:
-        buf = torch.empty(max(nbytes, 1 << 20), device=dev, dtype=torch.uint8)
-        _workspaces[key] = buf
-    return buf
-
-
 def hsa_attention(
     q: torch.Tensor,
     k: torch.Tensor,

@@ -87,7 +87,7 @@ def hsa_partials(q, k, v, k_coarse, v_coarse, index, num, block_size: int, *, fo
     runs when the shape qualifies (bf16, head_dim 128, 128-token blocks), the SIMT kernels otherwise.
     """
     import ctypes
-    from .attention import _unit_last, _workspace
+    from .attention import _unit_last
     dev = _lib.require_cuda(q, k, v, k_coarse, v_coarse, index, num)
     _lib.raise_if_failed(dev)
     bsz, q_len, heads, head_dim = q.shape
@@ -111,13 +111,8 @@ def hsa_partials(q, k, v, k_coarse, v_coarse, index, num, block_size: int, *, fo
     lse_l = torch.empty_like(lse_s)
     p.part_sparse, p.part_linear = sparse.data_ptr(), linear.data_ptr()
     p.lse_sparse, p.lse_linear = lse_s.data_ptr(), lse_l.data_ptr()
-    lib = _lib.lib()
-    ws = _workspace(dev, lib.wa_hsa_workspace_bytes(ctypes.byref(p)))
-    p.workspace, p.workspace_bytes = ws.data_ptr(), ws.numel()
-    used = ctypes.c_int(0)
-    with _lib.device_guard(dev):
-        _lib.check(lib.wa_hsa_forward(ctypes.byref(p), ctypes.byref(used), _lib.stream_ptr(dev)))
-    return sparse, lse_s, linear, lse_l, bool(used.value)
+    used = _lib.host().run_forward(ctypes.addressof(p), dev.index)
+    return sparse, lse_s, linear, lse_l, used
 
 
 def record_floats(head_dim: int) -> int:
@@ -140,7 +135,7 @@ def hsa_partials_packed(q, k, v, k_coarse, v_coarse, index, num, block_size: int
     `this_rank * rows_per_rank + t % rows_per_rank` of rank `t // rows_per_rank`.
     """
     import ctypes
-    from .attention import _unit_last, _workspace
+    from .attention import _unit_last
     dev = _lib.require_cuda(q, k, v, k_coarse, v_coarse, index, num, records)
     _lib.raise_if_failed(dev)
     bsz, q_len, heads, head_dim = q.shape
@@ -173,16 +168,7 @@ def hsa_partials_packed(q, k, v, k_coarse, v_coarse, index, num, block_size: int
         p.peer_rows, p.peer_self = int(rows_per_rank), int(this_rank)
         for r, delta in enumerate(deltas):
             p.peer_delta[r] = int(delta)
-    lib = _lib.lib()
-    ws = _workspace(dev, lib.wa_hsa_workspace_bytes(ctypes.byref(p)))
-    p.workspace, p.workspace_bytes = ws.data_ptr(), ws.numel()
-    used = ctypes.c_int(0)
-    with _lib.device_guard(dev):
-        rc = lib.wa_hsa_forward(ctypes.byref(p), ctypes.byref(used), _lib.stream_ptr(dev))
-    if rc == _lib.WA_ERR_UNSUPPORTED:
-        return False
-    _lib.check(rc)
-    return True
+    return _lib.host().run_forward(ctypes.addressof(p), dev.index) is not None
 
 
 def merge_packed(recv: torch.Tensor, head_dim: int):
