@@ -98,6 +98,11 @@ inline bool valid_dtype(int dt) { return dt == WA_F32 || dt == WA_BF16; }
 inline size_t dtype_size(int dt) { return dt == WA_BF16 ? 2 : 4; }
 inline int ceil_div(int a, int b) { return (a + b - 1) / b; }
 inline size_t align_up(size_t x, size_t a) { return (x + a - 1) / a * a; }
+inline int sm_count() {   // of the current device
+    int dev = 0, sms = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || sms <= 0) return 148;
+    return sms;
+}
 
 // ---- device-side view --------------------------------------------------------------------------
 struct View4 {  // [B, L, H, D], D contiguous, strides in elements

@@ -215,7 +215,7 @@ int compress_cluster_launch(const wa_tensor4 *k, const wa_tensor4 *v, const wa_t
         attr_set.mark();
     }
     const int n_seg = ceil_div(L, segment_len), longest = L < segment_len ? L : segment_len;
-    const int split = compress_split((long long)(HD / 128) * n_seg * 2 * B, longest, R == 32 ? 148 : 296);
+    const int split = compress_split((long long)(HD / 128) * n_seg * 2 * B, longest, R == 32 ? sm_count() : 2 * sm_count());
     const int tokens = ceil_div(ceil_div(longest, split), CF_WARPS) * CF_WARPS;
     cudaLaunchConfig_t cfg{};
     cfg.gridDim = dim3(HD / 128, n_seg * split, 2 * B);

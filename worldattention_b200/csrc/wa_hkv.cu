@@ -432,9 +432,7 @@ using namespace wa;
 // for up to some waves of them, which evens out the last one (60 pages: 126 us, one CTA per page 205; 300: 530 and 593; 480: 814
 // and 806), unless a page is too short to be shared (100 pages of 200 tokens: 46 and 39 us).
 static int centroid_split(long long groups, long long page_tokens) {
-    int dev = 0, sms = 148;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    const int sms = sm_count();
     const long long fit = 3ll * sms / groups;
     if (fit >= CV_MAX_SPLIT) return CV_MAX_SPLIT;
     if (fit >= 2) return fit < 4 ? (int)fit : 4;
