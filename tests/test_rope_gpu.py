@@ -37,3 +37,38 @@ def test_norm_and_rope_match_oracle_and_reference(golden):
     assert torch.equal(a, b)
     with pytest.raises(NotImplementedError):
         rope.causal_rope_apply(x.view(1, -1, 2, 128), torch.tensor([[1, 3, 4]]), freqs)
+
+
+def _awkward(x):
+    """Rows of zeros, subnormals, the largest and smallest values, infinities and NaN among the ordinary ones."""
+    rows = x.view(-1, x.shape[-1])
+    for i, value in enumerate((0.0, 1e-39, 3e38, 1e-30, 1e25, float("inf"), float("nan"))):
+        if 2 * i + 1 < rows.shape[0]:
+            rows[2 * i] = value
+            rows[2 * i + 1, i::7] = value
+    return x
+
+
+@pytest.mark.parametrize("batch,grid,heads,d", [(1, (1, 1, 1), 1, 8), (2, (1, 3, 5), 2, 128), (1, (3, 7, 11), 12, 128), (1, (2, 9, 13), 16, 128),
+                                                (1, (2, 5, 4), 12, 64), (3, (1, 4, 4), 5, 256), (1, (1, 2, 17), 24, 32)])
+def test_bf16_rows_match_the_float64_rotation_bit_for_bit(batch, grid, heads, d):
+    """bf16 weights take the kernel that rotates in float32 where that settles the result; the same weights in float32, and
+    heads that do not lie side by side, take the float64 ones."""
+    from worldattention_b200 import rope
+    from worldattention_b200.causal_dit import rope_table
+    n = grid[0] * grid[1] * grid[2]
+    g = torch.Generator(device=dev()).manual_seed(d + heads)
+    freqs = rope_table(d) if d >= 32 else torch.polar(torch.ones(64, d // 2, dtype=torch.float64), torch.randn(64, d // 2, dtype=torch.float64))
+    w = (1 + 0.3 * torch.randn(heads * d, generator=g, device=dev())).bfloat16()
+    start = torch.full((1,), 11, dtype=torch.int32, device=dev())
+    for awkward in (False, True):
+        x = torch.randn(batch, n, heads * d, generator=g, device=dev()).bfloat16()
+        x = _awkward(x) if awkward else x
+        same = lambda a, b: torch.equal(a.contiguous().view(torch.int16), b.contiguous().view(torch.int16))
+        for frame in (0, start):
+            got = rope.qk_norm_rope(x, w, 1e-6, grid, freqs, frame, heads=heads)
+            assert same(got, rope.qk_norm_rope(x, w.float(), 1e-6, grid, freqs, frame, heads=heads))
+        assert same(rope.qk_norm_rope(x, w, 1e-6, None, None, heads=heads), rope.qk_norm_rope(x, w.float(), 1e-6, None, None, heads=heads))
+        x4 = x.view(batch, n, heads, d)
+        spread = torch.empty(batch, n, heads, d + 2, dtype=x.dtype, device=dev())[..., :d].copy_(x4)
+        assert same(rope.causal_rope_apply(x4, grid, freqs, 5), rope.causal_rope_apply(spread, grid, freqs, 5))
