@@ -58,6 +58,8 @@ struct PerDeviceOnce {
 // still draining, runs its set-up (barriers, tensor memory, descriptor prefetch) and then blocks in
 // `pdl_wait()` until that kernel has completed and its writes are visible.  A kernel launched this way must reach
 // `pdl_wait()` in every thread block before it touches anything the stream's earlier work reads or writes.
+// A layer's calls are a dozen launches of 3..20 us; with the attribute on all of them a chunk's q, k and append take 31.8 us
+// instead of 38.9, and the smallest attention call 40.3 instead of 43.0.
 // WA_B200_PDL=0 in the environment turns the attribute off (plain stream order), for timing comparisons.
 inline int pdl_mode() {      // 0: plain stream order; 1: dependent launch (default); 2: and the routing kernel releases its dependents once a CTA's rows are done
     static const int mode = [] {

@@ -46,6 +46,7 @@ struct Job {
     int cols;                          // columns of an item: 128 or 64
     int L, segment_len, block_size, proj_rank;
     int slot0, slot_stride;            // first compressed slot of segment 0; slots between consecutive segments
+    int beside;                        // runs beside the launch before it, whose results it neither reads nor overwrites
     int copy;                          // also store the token tiles through the destination maps
     __nv_bfloat16 *out_k, *out_v;
     long long osb, osl;
@@ -82,6 +83,7 @@ compress_stream_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_co
                      "r"(TMEM_COLS) : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
     }
+    if (!job.beside) pdl_wait();
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
@@ -347,12 +349,9 @@ int compress_sm100_launch(const wa_tensor4 *k, const wa_tensor4 *v, const wa_ten
     const long long items = (long long)B * 2 * job.n_seg * job.tiles_cols;
     WA_REQUIRE(items < (1ll << 30), WA_ERR_UNSUPPORTED, "%s: too many work items", what);
     const int grid = items < sms ? (int)items : sms;
-    if (beside_routing) {
-        const cudaError_t e = launch_dependent(compress_stream_kernel, dim3(grid), dim3(THREADS), SMEM_BYTES, stream, tk, tv, tek, tev, tdk, tdv, job);
-        if (e != cudaSuccess) return fail((int)e, "%s: %s", what, cudaGetErrorString(e));
-    } else {
-        compress_stream_kernel<<<grid, THREADS, SMEM_BYTES, stream>>>(tk, tv, tek, tev, tdk, tdv, job);
-    }
+    job.beside = beside_routing ? 1 : 0;
+    const cudaError_t e = launch_dependent(compress_stream_kernel, dim3(grid), dim3(THREADS), SMEM_BYTES, stream, tk, tv, tek, tev, tdk, tdv, job);
+    if (e != cudaSuccess) return fail((int)e, "%s: %s", what, cudaGetErrorString(e));
     return check_launch(what);
 }
 

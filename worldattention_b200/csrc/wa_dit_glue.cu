@@ -36,6 +36,7 @@ ln_modulate_kernel(const __nv_bfloat16 *__restrict__ x, __nv_bfloat16 *__restric
                    const __nv_bfloat16 *__restrict__ weight, const __nv_bfloat16 *__restrict__ bias,
                    const __nv_bfloat16 *__restrict__ scale, const __nv_bfloat16 *__restrict__ shift, long long mod_stride,
                    int tokens_per_frame) {
+    pdl_wait();
     const long long row = (long long)blockIdx.x * GLUE_WARPS + (threadIdx.x >> 5);
     if (row >= rows) return;
     const int lane = threadIdx.x & 31, nvec = C >> 3;
@@ -121,6 +122,7 @@ template <int NV>
 __global__ void __launch_bounds__(GLUE_WARPS * 32, NV > 6 ? 3 : 4)
 gated_residual_kernel(const __nv_bfloat16 *__restrict__ x, const __nv_bfloat16 *__restrict__ y, __nv_bfloat16 *__restrict__ out,
                       long long rows, int C, const __nv_bfloat16 *__restrict__ gate, long long mod_stride, int tokens_per_frame) {
+    pdl_wait();
     const long long row = (long long)blockIdx.x * GLUE_WARPS + (threadIdx.x >> 5);
     if (row >= rows) return;
     const int lane = threadIdx.x & 31, nvec = C >> 3;
@@ -186,11 +188,13 @@ extern "C" int wa_ln_modulate(const void *x, void *out, long long rows, int C, f
     if (rows == 0) return 0;
     const long long ctas = (rows + GLUE_WARPS - 1) / GLUE_WARPS;
     WA_REQUIRE(ctas < (1ll << 31), WA_ERR_UNSUPPORTED, "%s: too many rows", what);
+    cudaError_t le = cudaSuccess;
     with_width(C, [&](auto nv) {
-        ln_modulate_kernel<decltype(nv)::value><<<(unsigned)ctas, GLUE_WARPS * 32, 0, (cudaStream_t)stream>>>(
+        le = launch_dependent(ln_modulate_kernel<decltype(nv)::value>, dim3((unsigned)ctas), dim3(GLUE_WARPS * 32), 0, (cudaStream_t)stream,
             (const __nv_bfloat16 *)x, (__nv_bfloat16 *)out, rows, C, eps, (const __nv_bfloat16 *)weight, (const __nv_bfloat16 *)bias,
             (const __nv_bfloat16 *)scale, (const __nv_bfloat16 *)shift, mod_stride, tokens_per_frame);
     });
+    if (le != cudaSuccess) return fail((int)le, "%s: %s", what, cudaGetErrorString(le));
     return check_launch(what);
 }
 
@@ -205,11 +209,13 @@ extern "C" int wa_gated_residual(const void *x, const void *y, void *out, long l
     if (rows == 0) return 0;
     const long long ctas = (rows + GLUE_WARPS - 1) / GLUE_WARPS;
     WA_REQUIRE(ctas < (1ll << 31), WA_ERR_UNSUPPORTED, "%s: too many rows", what);
+    cudaError_t le = cudaSuccess;
     with_width(C, [&](auto nv) {
         constexpr int NV = decltype(nv)::value < 8 ? decltype(nv)::value : 8;
-        gated_residual_kernel<NV><<<(unsigned)ctas, GLUE_WARPS * 32, 0, (cudaStream_t)stream>>>(
+        le = launch_dependent(gated_residual_kernel<NV>, dim3((unsigned)ctas), dim3(GLUE_WARPS * 32), 0, (cudaStream_t)stream,
             (const __nv_bfloat16 *)x, (const __nv_bfloat16 *)y, (__nv_bfloat16 *)out, rows, C, (const __nv_bfloat16 *)gate, mod_stride,
             tokens_per_frame);
     });
+    if (le != cudaSuccess) return fail((int)le, "%s: %s", what, cudaGetErrorString(le));
     return check_launch(what);
 }

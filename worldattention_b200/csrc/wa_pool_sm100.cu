@@ -63,6 +63,7 @@ pool_stream_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_consta
         }
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
+    pdl_wait();
     if (job.n_zero && blockIdx.x == 0)   // counters of the kernel that follows on the stream
         for (int i = threadIdx.x; i < job.n_zero; i += THREADS) job.zero[i] = 0;
     __syncthreads();
@@ -217,7 +218,8 @@ int pool_sm100_launch(const wa_tensor4 *x, int Lx, float *px, const wa_tensor4 *
     const long long items = (long long)B * (job.nbx + job.nby) * job.tiles;
     WA_REQUIRE(items < (1ll << 40), WA_ERR_UNSUPPORTED, "%s: too many blocks", what);
     const int grid = items < sms ? (int)items : sms;
-    pool_stream_kernel<<<grid, THREADS, SMEM_BYTES, stream>>>(tx, ty, job);
+    const cudaError_t le = launch_dependent(pool_stream_kernel, dim3(grid), dim3(THREADS), SMEM_BYTES, stream, tx, ty, job);
+    if (le != cudaSuccess) return fail((int)le, "%s: %s", what, cudaGetErrorString(le));
     return check_launch(what);
 }
 

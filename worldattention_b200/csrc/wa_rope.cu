@@ -180,6 +180,7 @@ qk_norm_rope_bits_kernel(const __nv_bfloat16 *__restrict__ x, long long xsb, lon
                          long long osb, long long osl, long long tokens, int L, int H, int D, const __nv_bfloat16 *__restrict__ weight,
                          float eps, const double2 *__restrict__ freqs, int freq_rows, int start_frame,
                          const int *__restrict__ start_frame_dev, int grid_h, int grid_w) {
+    pdl_wait();
     const long long tok = (long long)blockIdx.x * RN_WARPS + (threadIdx.x >> 5);
     if (tok >= tokens) return;
     const int lane = threadIdx.x & 31;
@@ -330,8 +331,9 @@ static int qk_norm_rope_launch(const wa_tensor4 *x, const wa_tensor4 *out, int B
     // D a power of two: the lanes' vectors lie alike in every head; float32 weights and a plain copy stay with the general form
     const bool by_bits = rows_in_registers && D <= 256 && (D & (D - 1)) == 0 && (norm_weight ? weight_dtype == WA_BF16 && (uintptr_t)norm_weight % 16 == 0 : freqs != nullptr);
     if (by_bits) {
+        cudaError_t le = cudaSuccess;
         const auto launch = [&](auto kernel) {
-            kernel<<<(unsigned)blocks, RN_WARPS * 32, 0, (cudaStream_t)stream>>>(
+            le = launch_dependent(kernel, dim3((unsigned)blocks), dim3(RN_WARPS * 32), 0, (cudaStream_t)stream,
                 (const __nv_bfloat16 *)x->ptr, x->stride_b, x->stride_l, (__nv_bfloat16 *)out->ptr, out->stride_b, out->stride_l, tokens, L, H,
                 D, (const __nv_bfloat16 *)norm_weight, eps, (const double2 *)freqs, freq_rows, start_frame, start_frame_dev, grid_h, grid_w);
         };
@@ -345,6 +347,7 @@ static int qk_norm_rope_launch(const wa_tensor4 *x, const wa_tensor4 *out, int B
         if (vectors <= 4) pick(std::integral_constant<int, 4>());
         else if (vectors <= 6) pick(std::integral_constant<int, 6>());
         else pick(std::integral_constant<int, 8>());
+        if (le != cudaSuccess) return fail((int)le, "%s: %s", what, cudaGetErrorString(le));
     } else if (rows_in_registers)
         qk_norm_rope_rows_kernel<<<(unsigned)blocks, RN_WARPS * 32, 0, (cudaStream_t)stream>>>(
             (const __nv_bfloat16 *)x->ptr, x->stride_b, x->stride_l, (__nv_bfloat16 *)out->ptr, out->stride_b, out->stride_l, tokens, L, H,
