@@ -1,0 +1,43 @@
+"""The forward's routing against the stand-alone routing functions at the sizes where its kernels change: logits of 16-row and
+128-key tiles and their remainders, and the best blocks of long rows picked in one or several pieces."""
+import pytest
+import torch
+
+from tests.helpers import dev
+
+pytestmark = pytest.mark.gpu
+BLOCK, D = 8, 128
+
+
+def _inputs(b, h, lq, lkv, seed, spread=1.0):
+    g = torch.Generator(device=dev()).manual_seed(seed)
+    draw = lambda n, s: (torch.randn(b, n, h, D, generator=g, device=dev()) * s).bfloat16()
+    kc = draw(16, 1.0)
+    proj = torch.zeros(1, 8, device=dev(), dtype=torch.bfloat16)      # not used: the compressed cache is given
+    return (draw(lq, spread), draw(lkv, spread), draw(lkv, 1.0)), dict(k_coarse=kc, v_coarse=kc, k_proj_mat=proj, v_proj_mat=proj, block_size=BLOCK)
+
+
+@pytest.mark.parametrize("b,h,nq,nkv", [(1, 16, 16, 256), (1, 32, 17, 129), (2, 4, 80, 127), (1, 3, 81, 300), (1, 1, 33, 2049),
+                                        (1, 40, 1, 1700), (1, 2, 97, 513), (1, 1, 15, 4096), (1, 1, 2, 128)])
+@pytest.mark.parametrize("ragged", [0, 3])
+def test_forward_routing_equals_the_separate_functions(b, h, nq, nkv, ragged):
+    from worldattention_b200.hsa import routing as R
+    from worldattention_b200.hsa import hsa_attention
+    lq, lkv = nq * BLOCK - ragged, nkv * BLOCK - ragged
+    qkv, kwargs = _inputs(b, h, lq, lkv, nq + nkv)
+    _, (index, num, thresholds, _) = hsa_attention(*qkv, return_routing=True, **kwargs)
+    pooled = [R.block_mean_pool(R.pad_to_len(t, n * BLOCK).transpose(1, 2).contiguous(), length, n, BLOCK).float()
+              for t, n, length in ((qkv[0], nq, lq), (qkv[1], nkv, lkv))]
+    want = R.build_block_routing(R.block_attention_map(*pooled), 0.35, 1.0)
+    assert torch.equal(index, want.index) and torch.equal(num, want.num) and torch.equal(thresholds, want.thresholds)
+
+
+@pytest.mark.parametrize("topk", [(4500, 2049), (2048, 1), (1025, 512), (5000, 0), (4097, 33)])
+@pytest.mark.parametrize("spread", [1.0, 0.0])      # 0: every probability is the same, the order is the ids'
+def test_best_blocks_of_long_rows(topk, spread):
+    from worldattention_b200.hsa import hsa_attention
+    qkv, kwargs = _inputs(1, 2, 3 * BLOCK, 5000 * BLOCK, 5, spread)
+    counts = torch.tensor(topk, dtype=torch.int32)
+    picked = hsa_attention(*qkv, topk_per_head=counts, **kwargs)
+    whole, (_, num, _, _) = hsa_attention(*qkv, topk_per_head=counts, return_routing=True, **kwargs)
+    assert num.unique().tolist() == sorted(set(topk)) and torch.equal(picked, whole)

@@ -4,6 +4,8 @@
 // of Q and K, then a few hundred short rows), so the kernels are plain coalesced / warp-shuffle
 // code; every reduction that feeds the discrete selection accumulates in float64 and rounds once,
 // which makes the chosen block ids independent of the summation order.
+#include <type_traits>
+
 #include "wa_internal.cuh"
 
 namespace wa {
@@ -336,86 +338,93 @@ __device__ __forceinline__ void row_block_attention(const float *__restrict__ q,
     row_softmax(Nkv, out, red, bcast);
 }
 
-// Logits of R neighbouring rows of one head against ONE pass over the head's pooled keys (D = 128 only): with thousands
-// of key blocks a row's CTA otherwise re-reads megabytes of pooled keys that its neighbours read too and converts each to
-// float64 again.  A lane owns a key: the keys are staged through `stage` (shared memory, 2 tiles of `tile_keys` rows)
-// TRANSPOSED in 16-byte pieces ([piece][key] with an odd pitch, filled one tile ahead through registers: coalesced reads,
-// conflict-free writes), so that a warp reads the same piece of 32 keys without bank conflicts, converts it once and uses
-// it for all R rows, whose float64 queries come from
-// shared memory as broadcasts.  No sum crosses a lane; a dot is accumulated dimension by dimension in float64 and rounded
-// once, like every other sum on the routing path.  Measured at 11 700 key blocks (one group = its rows x 11 700 keys):
-// see the numbers in the design notes.  Other forms that were built and measured: each key split over all 32 lanes with the queries
-// in registers (no transposition, but most instructions go into the transposed float64 reduction: 284 us for four rows);
-// a key per 4 lanes with a quarter of the dimensions each, so that all 16 warps compute (the query reads are then four
-// different addresses per load instead of one broadcast: 220 us + 56 us per row); the rows spread over four warp groups
-// so that all 16 warps compute whole keys (each key converted four times: 25-40 us slower).  What is left of the fixed
-// part is the keys' way from L2: every group streams its head's 6 MB, 720 MB for the 120 groups of config 5.  `q` holds the
-// rows 128 apart, `out` holds them `Nkv` apart; rows >= nrows repeat row 0's query and are not stored.
-template <int R>
-__device__ __forceinline__ void row_logits_keys(const float *__restrict__ q, int nrows, const float *__restrict__ k, int Nkv,
-                                                float scale, float *out, double *qsh, float4 *stage, int tile_keys) {
-    constexpr int D = 128, VPK = D / 4;   // 16-byte pieces per key
-    const int T = blockDim.x, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    for (int i = threadIdx.x; i < R * D; i += T) qsh[i] = (double)q[((i / D) < nrows ? (i / D) : 0) * D + (i % D)];
-    const float4 *kvec = reinterpret_cast<const float4 *>(k);
-    const int pitch = tile_keys + 1;                  // 16-byte slots per piece row: the odd pitch spreads a key's 32 pieces over the banks
-    const int tile_vecs = tile_keys * VPK, tile_slots = pitch * VPK;
-    const int n_tiles = (Nkv + tile_keys - 1) / tile_keys;
-    // a warp loads one key's 512 bytes per instruction (coalesced) into registers while the previous tile is computed on,
-    // and stores them transposed afterwards (16-byte asynchronous copies were measured at about 16 bytes per clock per SM,
-    // which made the staging, not the arithmetic, the larger part of this routine)
-    constexpr int PER_THREAD = 8;      // 16-byte loads per thread and tile: tile_keys * 32 <= 8 * 512
-    float4 pre[PER_THREAD];
-    auto fetch = [&](int tile) {
-#pragma unroll
-        for (int i = 0; i < PER_THREAD; ++i) {
-            const int v = i * T + threadIdx.x, key = v / VPK, piece = v % VPK;
-            const long long gkey = (long long)tile * tile_keys + key;
-            pre[i] = (v < tile_vecs && gkey < Nkv) ? __ldg(kvec + gkey * VPK + piece) : make_float4(0.f, 0.f, 0.f, 0.f);
+// ------------------------------------------------------------------------------------------------
+// Logits of all rows on the float64 matrix instruction (head_dim 128): out[row][key] = fl32(q . k) * scale, float64 products
+// and sums, rounded once, like row_logits.  With a row per CTA every row streams its head's pooled keys from L2 and converts
+// them to float64 for itself (a quarter of a product's rate); here a CTA holds up to 80 query rows of a head as float64
+// operands in shared memory, in the instruction's own order (16-byte loads without conflicts), and a warp reads 16 keys from
+// L2 once for all of them.  A lane's four dimensions of a step of 16 are neighbours in memory (its k indices of both operands
+// are permuted alike).  Bound by the float64 pipe: 65 multiply-adds per clock and SM measured for this instruction, 55 for scalar
+// ones.  One CTA of eight warps per SM: two warps per scheduler keep the pipe busy.
+// 12 heads, 74 rows, 11 700 keys: 103 us (12.9 T multiply-adds/s of the 18.4 measured); with eight rows per CTA on scalar float64 and
+// the row steps in the same kernel the routing took 655 us, now 103 + 119.
+// ------------------------------------------------------------------------------------------------
+constexpr int RL_WARPS = 8, RL_KEYS = 16, RL_TILE = RL_WARPS * RL_KEYS, RL_MAX_MT = 5;   // keys per warp and per tile; 16-row tiles per CTA
+
+__device__ __forceinline__ void mma_f64(double (&c)[4], const double (&a)[8], const double (&b)[4]) {
+    asm("mma.sync.aligned.m16n8k16.row.col.f64.f64.f64.f64 {%0,%1,%2,%3}, {%4,%5,%6,%7,%8,%9,%10,%11}, {%12,%13,%14,%15}, {%0,%1,%2,%3};"
+        : "+d"(c[0]), "+d"(c[1]), "+d"(c[2]), "+d"(c[3])
+        : "d"(a[0]), "d"(a[1]), "d"(a[2]), "d"(a[3]), "d"(a[4]), "d"(a[5]), "d"(a[6]), "d"(a[7]), "d"(b[0]), "d"(b[1]), "d"(b[2]), "d"(b[3]));
+}
+
+template <int MT>
+__global__ void __launch_bounds__(RL_WARPS * 32, 1)
+route_logits_kernel(const float *__restrict__ qp, const float *__restrict__ kp, int Nq, int Nkv, float scale, float *__restrict__ out,
+                    int groups, int tiles, long long units) {
+    extern __shared__ __align__(16) unsigned char logits_smem[];
+    double2 *qfrag = reinterpret_cast<double2 *>(logits_smem);        // [MT][8 steps][4 dimensions][32 lanes] of (row g, row g + 8)
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
+    pdl_wait();
+    // unit = (batch and head, group of MT * 16 rows, tile of keys), tile fastest; a CTA takes a run of them
+    const long long first = units * blockIdx.x / gridDim.x, last = units * (blockIdx.x + 1) / gridDim.x;
+    long long staged = -1;
+    for (long long u = first; u < last; ++u) {
+        const long long rows = u / tiles, bh = rows / groups;
+        const int key0 = (int)(u - rows * tiles) * RL_TILE + warp * RL_KEYS, i0 = (int)(rows - bh * groups) * MT * 16;
+        if (rows != staged) {
+            __syncthreads();
+            for (int i = threadIdx.x; i < MT * 8 * 32; i += RL_WARPS * 32) {
+                const int l = i & 31, row = i0 + (i >> 8) * 16 + (l >> 2), dim = ((i >> 5) & 7) * 16 + (l & 3) * 4;
+                const float *q = qp + (bh * Nq + row) * 128 + dim;
+                const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
+                const float4 lo = row < Nq ? *reinterpret_cast<const float4 *>(q) : zero;
+                const float4 hi = row + 8 < Nq ? *reinterpret_cast<const float4 *>(q + 8 * 128) : zero;
+                double2 *dst = qfrag + (i >> 5) * 128 + l;
+                dst[0] = make_double2(lo.x, hi.x);
+                dst[32] = make_double2(lo.y, hi.y);
+                dst[64] = make_double2(lo.z, hi.z);
+                dst[96] = make_double2(lo.w, hi.w);
+            }
+            __syncthreads();
+            staged = rows;
         }
-    };
-    auto park = [&](int tile) {
-        float4 *dst = stage + (tile & 1) * tile_slots;
+        if (key0 >= Nkv) continue;
+        const float4 *ka = reinterpret_cast<const float4 *>(kp + (bh * Nkv + min(key0 + g, Nkv - 1)) * 128) + t;
+        const float4 *kb = reinterpret_cast<const float4 *>(kp + (bh * Nkv + min(key0 + 8 + g, Nkv - 1)) * 128) + t;
+        float4 na = __ldg(ka), nb = __ldg(kb);
+        double acc[MT][2][4];
 #pragma unroll
-        for (int i = 0; i < PER_THREAD; ++i) {
-            const int v = i * T + threadIdx.x, key = v / VPK, piece = v % VPK;
-            if (v < tile_vecs) dst[piece * pitch + key] = pre[i];
-        }
-    };
-    fetch(0);
-    park(0);
-    __syncthreads();
-    for (int tile = 0; tile < n_tiles; ++tile) {
-        if (tile + 1 < n_tiles) fetch(tile + 1);
-        const int key = warp * 32 + lane;      // a lane owns a key of the tile: the first tile_keys / 32 warps compute, all warps fetch
-        const long long gkey = (long long)tile * tile_keys + key;
-        if (key < tile_keys && (long long)tile * tile_keys + warp * 32 < Nkv) {
-            const float4 *kt = stage + (tile & 1) * tile_slots + key;
-            double acc[R];
+        for (int m = 0; m < MT; ++m)
 #pragma unroll
-            for (int r = 0; r < R; ++r) acc[r] = 0.0;
-#pragma unroll 4
-            for (int piece = 0; piece < VPK; ++piece) {
-                const float4 kv = kt[piece * pitch];
-                const double k0 = (double)kv.x, k1 = (double)kv.y, k2 = (double)kv.z, k3 = (double)kv.w;
+            for (int i = 0; i < 4; ++i) acc[m][0][i] = acc[m][1][i] = 0.0;
+#pragma unroll 2
+        for (int step = 0; step < 8; ++step) {
+            const double ba[4] = {na.x, na.y, na.z, na.w}, bb[4] = {nb.x, nb.y, nb.z, nb.w};
+            const int next = min(step + 1, 7) * 4;
+            na = __ldg(ka + next);
+            nb = __ldg(kb + next);
 #pragma unroll
-                for (int r = 0; r < R; ++r) {
-                    const double2 qa = *reinterpret_cast<const double2 *>(qsh + r * D + piece * 4);      // broadcast reads
-                    const double2 qb = *reinterpret_cast<const double2 *>(qsh + r * D + piece * 4 + 2);
-                    double a = fma(qa.x, k0, acc[r]);
-                    a = fma(qa.y, k1, a);
-                    a = fma(qb.x, k2, a);
-                    acc[r] = fma(qb.y, k3, a);
+            for (int m = 0; m < MT; ++m) {
+                double a[8];
+#pragma unroll
+                for (int e = 0; e < 4; ++e) {
+                    const double2 q2 = qfrag[((m * 8 + step) * 4 + e) * 32 + lane];
+                    a[2 * e] = q2.x;
+                    a[2 * e + 1] = q2.y;
                 }
-            }
-            if (gkey < Nkv) {
-#pragma unroll
-                for (int r = 0; r < R; ++r)
-                    if (r < nrows) out[(long long)r * Nkv + gkey] = __fmul_rn((float)acc[r], scale);
+                mma_f64(acc[m][0], a, ba);
+                mma_f64(acc[m][1], a, bb);
             }
         }
-        if (tile + 1 < n_tiles) park(tile + 1);      // that buffer was last read while tile - 1 was computed, before the last barrier
-        __syncthreads();      // (after the last tile: the logits are complete and visible to the whole CTA, the staging memory is free)
+#pragma unroll
+        for (int m = 0; m < MT; ++m)
+#pragma unroll
+            for (int half = 0; half < 2; ++half)
+#pragma unroll
+                for (int i = 0; i < 4; ++i) {
+                    const int row = i0 + m * 16 + g + 8 * (i >> 1), key = key0 + half * 8 + 2 * t + (i & 1);
+                    if (row < Nq && key < Nkv) out[(bh * Nq + row) * Nkv + key] = __fmul_rn((float)acc[m][half][i], scale);
+                }
     }
 }
 
@@ -578,7 +587,46 @@ route_count_kernel(const float *__restrict__ attn, const int32_t *__restrict__ i
 // last head prepares the attention kernel's launch (work order, counters).  Same arithmetic as the
 // three separate kernels above; no CTA ever waits for another.
 // ------------------------------------------------------------------------------------------------
-__device__ __forceinline__ void sort_keys_smem(unsigned long long *keys, int n_pow2);
+// one key per thread, bitonic: exchange distances below 32 go through shuffles, the rest through `keys` (one entry per thread)
+__device__ __forceinline__ unsigned long long sort_key_per_thread(unsigned long long key, unsigned long long *keys, int n_pow2) {
+    const int tid = threadIdx.x;
+    for (int k = 2; k <= n_pow2; k <<= 1) {
+        for (int j = k >> 1; j > 0; j >>= 1) {
+            unsigned long long other;
+            if (j >= 32) {
+                keys[tid] = key;
+                __syncthreads();
+                other = keys[tid ^ j];
+                __syncthreads();
+            } else {
+                other = __shfl_xor_sync(0xffffffffu, key, j);
+            }
+            const bool keep_min = ((tid & j) == 0) == ((tid & k) == 0);
+            key = (other < key) == keep_min ? other : key;
+        }
+    }
+    return key;
+}
+
+__device__ __forceinline__ void sort_keys_smem(unsigned long long *keys, int n_pow2) {   // ascending bitonic sort, whole CTA
+    const int T = blockDim.x;
+    for (int k = 2; k <= n_pow2; k <<= 1) {
+        for (int j = k >> 1; j > 0; j >>= 1) {
+            for (int i = threadIdx.x; i < n_pow2; i += T) {
+                const int ixj = i ^ j;
+                if (ixj > i) {
+                    const unsigned long long a = keys[i], b = keys[ixj];
+                    const bool up = (i & k) == 0;
+                    if ((a > b) == up) {
+                        keys[i] = b;
+                        keys[ixj] = a;
+                    }
+                }
+            }
+            __syncthreads();
+        }
+    }
+}
 
 // The k best blocks of a row, in order, WITHOUT sorting the row: for a fixed per-head count over thousands of key blocks
 // the full bitonic sort (105 passes over 16384 keys) was two thirds of the routing kernel.  Keys are the sort's own
@@ -587,14 +635,17 @@ __device__ __forceinline__ void sort_keys_smem(unsigned long long *keys, int n_p
 // keys still needed, or the keys at or below the bin are at most 1024), the keys at or below it are collected and only
 // they are sorted.  `idx[0..k)` receive the same ids in the same order as the full sort; slots past k are not written.
 // `keys` is shared memory for `key_slots` >= max(1024, pow2(k)) entries.  Called by every thread of the CTA (>= 256 threads).
-__device__ __forceinline__ void select_top_blocks(const float *probs, int Nkv, int k, unsigned long long *keys, int key_slots,
-                                                  int32_t *idx, int id_offset = 0, unsigned long long *keys_out = nullptr) {
+// A larger k is selected in pieces: `from` is the smallest key still to be had and `n_left` how many there are of those; returns
+// the largest key taken.
+__device__ __forceinline__ unsigned long long select_top_blocks(const float *probs, int Nkv, int k, unsigned long long *keys, int key_slots,
+                                                                int32_t *idx, int id_offset, unsigned long long *keys_out,
+                                                                unsigned long long from, int n_left) {
     __shared__ unsigned int hist[256];
     __shared__ unsigned long long prefix_s, mask_s;
     __shared__ int need_s, done_s;
     __shared__ unsigned int taken_s;
     const int T = blockDim.x, tid = threadIdx.x;
-    if (k <= 0) return;
+    if (k <= 0) return 0ull;
     auto key_of = [&](int j) { return ((unsigned long long)descending_key(probs[j]) << 32) | (unsigned)(id_offset + j); };
     // the keys of a row usually agree in their leading bytes (probabilities of one softmax share sign and most of the
     // exponent; near-uniform attention agrees much further): find the common prefix with one min/max pass and start the
@@ -603,6 +654,7 @@ __device__ __forceinline__ void select_top_blocks(const float *probs, int Nkv, i
     unsigned long long lo = 0xFFFFFFFFFFFFFFFFull, hi = 0ull;
     for (int j = tid; j < Nkv; j += T) {
         const unsigned long long key = key_of(j);
+        if (key < from) continue;
         lo = key < lo ? key : lo;
         hi = key > hi ? key : hi;
     }
@@ -629,7 +681,7 @@ __device__ __forceinline__ void select_top_blocks(const float *probs, int Nkv, i
         prefix_s = lo & mask;
         mask_s = mask;
         need_s = k;
-        done_s = k >= Nkv;     // every block is kept: nothing to select
+        done_s = k >= n_left;     // every block is kept: nothing to select
         taken_s = 0u;
         lo_s[0] = (unsigned long long)top;
     }
@@ -646,7 +698,7 @@ __device__ __forceinline__ void select_top_blocks(const float *probs, int Nkv, i
         for (int j0 = 0; j0 < Nkv; j0 += T) {      // whole warps iterate together: the votes below need every lane
             const int j = j0 + tid;
             const unsigned long long key = j < Nkv ? key_of(j) : 0ull;
-            const bool cand = j < Nkv && (key & mask) == prefix;
+            const bool cand = j < Nkv && key >= from && (key & mask) == prefix;
             const unsigned int voters = __ballot_sync(0xffffffffu, cand);
             if (voters) {
                 // the probabilities of a row share their leading bits: the digit of the warp's first candidate is usually
@@ -698,8 +750,8 @@ __device__ __forceinline__ void select_top_blocks(const float *probs, int Nkv, i
                 mask_s = mask | (0xFFull << (8 * byte));
                 need_s = (int)(need - run);
                 // stop refining when the whole bin is wanted, or when the keys at or below this bin are few enough to sort
-                // directly (every further digit would cost another pass over the whole row)
-                if (in_bin == need - run || (unsigned)k - (need - run) + in_bin <= 1024u) done_s = 1;
+                // with a key per thread (every further digit would cost another pass over the whole row)
+                if (in_bin == need - run || (unsigned)k - (need - run) + in_bin <= (unsigned)min(T, 1024)) done_s = 1;
             }
         }
         __syncthreads();
@@ -709,7 +761,7 @@ __device__ __forceinline__ void select_top_blocks(const float *probs, int Nkv, i
     const unsigned long long prefix = prefix_s, mask = mask_s;
     for (int j = tid; j < Nkv; j += T) {
         const unsigned long long key = key_of(j);
-        if ((key & mask) <= prefix) keys[atomicAdd(&taken_s, 1u)] = key;
+        if (key >= from && (key & mask) <= prefix) keys[atomicAdd(&taken_s, 1u)] = key;
     }
     __syncthreads();
     const int kept = (int)taken_s;      // >= min(k, Nkv): the k best and, when the selection stopped early, the rest of the last bin
@@ -717,22 +769,31 @@ __device__ __forceinline__ void select_top_blocks(const float *probs, int Nkv, i
     while (k_pow2 < kept) k_pow2 <<= 1;
     for (int j = kept + tid; j < k_pow2; j += T) keys[j] = 0xFFFFFFFFFFFFFFFFull;
     __syncthreads();
-    sort_keys_smem(keys, k_pow2);
+    if (k_pow2 <= T && T <= key_slots) {
+        const unsigned long long key = sort_key_per_thread(tid < k_pow2 ? keys[tid] : 0xFFFFFFFFFFFFFFFFull, keys, k_pow2);
+        __syncthreads();
+        keys[tid] = key;
+        __syncthreads();
+    } else {
+        sort_keys_smem(keys, k_pow2);
+    }
     for (int m = tid; m < min(k, kept); m += T) {
         if (idx) idx[m] = (int32_t)(keys[m] & 0xFFFFFFFFull);
         if (keys_out) keys_out[m] = keys[m];      // the sortable keys themselves (ids offset by `id_offset`)
     }
+    const unsigned long long taken = keys[max(0, min(k, kept) - 1)];
     __syncthreads();
+    return taken;
 }
 
 // One (batch, head, query block) row of the fused routing; called by every thread of the CTA.  With `logits_ready`
-// the row's scaled logits already lie in `sorted + row * Nkv` (written by this CTA).
+// the row's scaled logits already lie in `sorted + row * Nkv`.
 __device__ __forceinline__ void route_row(const long long row, const bool logits_ready, const float *__restrict__ qp,
                                           const float *__restrict__ kp, int B, int H, int Nq, int Nkv, int n_pow2, int D, float scale,
                                           float tau_min, float tau_span, const int32_t *__restrict__ fixed_num, float *sorted,
                                           int32_t *__restrict__ index, int32_t *num, float *__restrict__ thresholds, float *gini_rows,
                                           int *counters, const SchedJob &job, unsigned long long *keys, float *probs, double *red,
-                                          float &bcast, int &last_flag, const bool select_only) {
+                                          float &bcast, int &last_flag, const bool select_only, const int key_slots) {
     const int T = blockDim.x, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, nwarps = T >> 5;
     const long long bh = row / Nq;
     const int h = (int)(bh % H);
@@ -750,26 +811,13 @@ __device__ __forceinline__ void route_row(const long long row, const bool logits
 
     if (select_only) {
         // fixed per-head count and nobody asked for the whole order or the thresholds: pick the head's k best blocks
-        select_top_blocks(probs, Nkv, max(0, min(fixed_num[h], Nkv)), keys, max(n_pow2, T), index + row * Nkv);
+        const int want = max(0, min(fixed_num[h], Nkv));
+        unsigned long long from = 0ull;
+        for (int at = 0; at < want; at += key_slots)
+            from = select_top_blocks(probs, Nkv, min(want - at, key_slots), keys, key_slots, index + row * Nkv + at, 0, nullptr, from, Nkv - at) + 1ull;
     } else if (n_pow2 <= T) {
-        // one key per thread in a register: exchange distances below 32 go through shuffles, the rest through smem
-        unsigned long long key = tid < Nkv ? (((unsigned long long)descending_key(probs[tid]) << 32) | (unsigned)tid)
-                                           : 0xFFFFFFFFFFFFFFFFull;
-        for (int k = 2; k <= n_pow2; k <<= 1) {
-            for (int j = k >> 1; j > 0; j >>= 1) {
-                unsigned long long other;
-                if (j >= 32) {
-                    keys[tid] = key;
-                    __syncthreads();
-                    other = keys[tid ^ j];
-                    __syncthreads();
-                } else {
-                    other = __shfl_xor_sync(0xffffffffu, key, j);
-                }
-                const bool keep_min = ((tid & j) == 0) == ((tid & k) == 0);
-                key = (other < key) == keep_min ? other : key;
-            }
-        }
+        unsigned long long key = sort_key_per_thread(
+            tid < Nkv ? (((unsigned long long)descending_key(probs[tid]) << 32) | (unsigned)tid) : 0xFFFFFFFFFFFFFFFFull, keys, n_pow2);
         keys[tid] = key;
         __syncthreads();
     } else {
@@ -777,22 +825,7 @@ __device__ __forceinline__ void route_row(const long long row, const bool logits
             keys[j] = j < Nkv ? (((unsigned long long)descending_key(probs[j]) << 32) | (unsigned)j)
                               : 0xFFFFFFFFFFFFFFFFull;
         __syncthreads();
-        for (int k = 2; k <= n_pow2; k <<= 1) {
-            for (int j = k >> 1; j > 0; j >>= 1) {
-                for (int i = tid; i < n_pow2; i += T) {
-                    const int ixj = i ^ j;
-                    if (ixj > i) {
-                        const unsigned long long a = keys[i], b = keys[ixj];
-                        const bool up = (i & k) == 0;
-                        if ((a > b) == up) {
-                            keys[i] = b;
-                            keys[ixj] = a;
-                        }
-                    }
-                }
-                __syncthreads();
-            }
-        }
+        sort_keys_smem(keys, n_pow2);
     }
     ROUTE_STAMP(3);
     if (!select_only) {
@@ -950,60 +983,34 @@ __device__ __forceinline__ void route_row(const long long row, const bool logits
 }
 
 // ------------------------------------------------------------------------------------------------
-// The forward's routing in ONE launch.  Each CTA owns one row, or (thousands of key blocks, head_dim 128) four
-// neighbouring rows of a head whose logits it computes in one pass over the pooled keys.
+// The forward's routing: a row per CTA, from its logits on where route_logits_kernel has left them in `sorted`.
 // ------------------------------------------------------------------------------------------------
-template <int ROWS>   // rows per CTA: 1, 4 or 8 (several rows: 512 threads)
-__global__ void __launch_bounds__(ROWS > 1 ? 512 : 1024)
+__global__ void __launch_bounds__(1024)
 route_fused_kernel(const float *__restrict__ qp, const float *__restrict__ kp, int B, int H, int Nq, int Nkv, int n_pow2,
                    int D, float scale, float tau_min, float tau_span, const int32_t *__restrict__ fixed_num,
                    float *sorted, int32_t *__restrict__ index, int32_t *num, float *__restrict__ thresholds,
-                   float *gini_rows, int *counters, SchedJob job, int gate_per_cta, int sm_count, int slots, int groups_per_bh,
-                   int select_only) {
-    constexpr int rows_per_cta = ROWS;
+                   float *gini_rows, int *counters, SchedJob job, int gate_per_cta, int sm_count, int slots, int select_only,
+                   int logits_ready, int key_slots) {
     extern __shared__ __align__(16) unsigned char fused_smem[];
-    unsigned long long *keys = reinterpret_cast<unsigned long long *>(fused_smem);   // max(n_pow2, threads)
-    float *probs = reinterpret_cast<float *>(keys + max(n_pow2, (int)blockDim.x));    // Nkv
+    unsigned long long *keys = reinterpret_cast<unsigned long long *>(fused_smem);   // key_slots
+    float *probs = reinterpret_cast<float *>(keys + key_slots);                      // Nkv
     __shared__ double red[256];
-    __shared__ __align__(16) double q_rows[ROWS > 1 ? ROWS * 128 : 2];
     __shared__ float bcast;
     __shared__ int last_flag;
 
     // CTAs are dealt to the SMs round-robin, so CTAs b, b + sm_count, ... tend to share an SM: give them
     // neighbouring rows (same head, same pooled keys) so that their key reads can meet in L1
-    const long long group = (long long)(blockIdx.x % sm_count) * slots + blockIdx.x / sm_count;
+    const long long row = (long long)(blockIdx.x % sm_count) * slots + blockIdx.x / sm_count;
     // No early release of the attention kernel here: its CTAs, once resident and waiting, slowed the tail of this
     // kernel (the per-head count and the work order are a few CTAs' work) by about 5 us.
     pdl_wait();                 // pooled means and zeroed counters come from the launch before
     if (job.release_at_start) pdl_release_dependents();
-    if (group >= (long long)B * H * groups_per_bh) return;
-    const long long bh = group / groups_per_bh;
-    const int i0 = (int)(group % groups_per_bh) * rows_per_cta, nrows = min(rows_per_cta, Nq - i0);
-    const long long row0 = bh * Nq + i0;
+    if (row >= (long long)B * H * Nq) return;
 
     ROUTE_STAMP(0);
-    if (job.order && job.gate_w) convert_gate_slice(job, (int)group * gate_per_cta, gate_per_cta);
-
-    if constexpr (ROWS > 1) {
-        // the sort keys' shared memory is free until the first row is sorted: the pooled keys are staged through it
-        // (and through the head of the probabilities' memory behind it, which is not in use yet either)
-        const int stage_bytes = max(n_pow2, (int)blockDim.x) * 8 + Nkv * 4;
-        int tile_keys = 128;      // two staging buffers of (tile_keys + 1) x 512 bytes; whole warps of keys
-        while (tile_keys > 32 && 2 * (tile_keys + 1) * 512 > stage_bytes) tile_keys -= 32;
-        row_logits_keys<ROWS>(qp + row0 * D, nrows, kp + bh * (long long)Nkv * D, Nkv, scale, sorted + row0 * Nkv, q_rows,
-                              reinterpret_cast<float4 *>(keys), tile_keys);      // ends with a barrier: the rows below read these logits back
-        ROUTE_STAMP(10);
-    }
-    if constexpr (ROWS == 1) {
-        route_row(row0, false, qp, kp, B, H, Nq, Nkv, n_pow2, D, scale, tau_min, tau_span, fixed_num, sorted, index, num, thresholds,
-                  gini_rows, counters, job, keys, probs, red, bcast, last_flag, select_only != 0);
-        return;
-    }
-    for (int r = 0; r < nrows; ++r) {
-        route_row(row0 + r, true, qp, kp, B, H, Nq, Nkv, n_pow2, D, scale, tau_min, tau_span, fixed_num, sorted, index,
-                  num, thresholds, gini_rows, counters, job, keys, probs, red, bcast, last_flag, select_only != 0);
-        __syncthreads();
-    }
+    if (job.order && job.gate_w) convert_gate_slice(job, (int)row * gate_per_cta, gate_per_cta);
+    route_row(row, logits_ready != 0, qp, kp, B, H, Nq, Nkv, n_pow2, D, scale, tau_min, tau_span, fixed_num, sorted, index, num, thresholds,
+              gini_rows, counters, job, keys, probs, red, bcast, last_flag, select_only != 0, key_slots);
 }
 
 #ifdef WA_ROUTE_TRACE
@@ -1026,26 +1033,6 @@ namespace wa {
 // except where distinct logits round to one probability at the k-th place (there the single-device rule
 // orders by block id, this one by logit).
 // ------------------------------------------------------------------------------------------------
-__device__ __forceinline__ void sort_keys_smem(unsigned long long *keys, int n_pow2) {   // ascending bitonic sort, whole CTA
-    const int T = blockDim.x;
-    for (int k = 2; k <= n_pow2; k <<= 1) {
-        for (int j = k >> 1; j > 0; j >>= 1) {
-            for (int i = threadIdx.x; i < n_pow2; i += T) {
-                const int ixj = i ^ j;
-                if (ixj > i) {
-                    const unsigned long long a = keys[i], b = keys[ixj];
-                    const bool up = (i & k) == 0;
-                    if ((a > b) == up) {
-                        keys[i] = b;
-                        keys[ixj] = a;
-                    }
-                }
-            }
-            __syncthreads();
-        }
-    }
-}
-
 __global__ void __launch_bounds__(1024)
 route_local_candidates_kernel(const float *__restrict__ qp, const float *__restrict__ kp, int Nq, int Nloc, int n_pow2, int D,
                               float scale, int block_lo, int kcap, unsigned long long *__restrict__ cand) {
@@ -1059,7 +1046,7 @@ route_local_candidates_kernel(const float *__restrict__ qp, const float *__restr
     if (n_pow2 > (int)blockDim.x && kcap <= 1024) {
         // a long row: pick the kcap best instead of sorting all of them (same keys, same order)
         const int k = min(kcap, Nloc);
-        select_top_blocks(logits, Nloc, k, keys, n_pow2, nullptr, block_lo, cand + row * kcap);
+        select_top_blocks(logits, Nloc, k, keys, n_pow2, nullptr, block_lo, cand + row * kcap, 0ull, Nloc);
         for (int j = k + threadIdx.x; j < kcap; j += blockDim.x) cand[row * kcap + j] = 0xFFFFFFFFFFFFFFFFull;
         return;
     }
@@ -1304,53 +1291,63 @@ int route_fused_launch(const float *q_pooled, const float *k_pooled, int B, int 
     WA_REQUIRE(rows < (1ll << 31), WA_ERR_UNSUPPORTED, "wa_hsa_forward(routing): too many rows");
     int threads = n_pow2 / 2;
     threads = threads < 256 ? 256 : (threads > 1024 ? 1024 : threads);
-    const size_t smem = (size_t)(n_pow2 > threads ? n_pow2 : threads) * sizeof(unsigned long long) + (size_t)Nkv * sizeof(float);
-    if (smem > 24 * 1024) {   // static shared memory of the kernel takes ~19 KB of the default 48 KB
-        cudaError_t e = cudaFuncSetAttribute(route_fused_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        if (e == cudaSuccess) e = cudaFuncSetAttribute(route_fused_kernel<8>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        if (e == cudaSuccess) e = cudaFuncSetAttribute(route_fused_kernel<4>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        if (e != cudaSuccess) return fail((int)e, "wa_hsa_forward(routing): %s", cudaGetErrorString(e));
-    }
-    // several rows per CTA where a row's keys are megabytes (see row_logits_keys); one row per CTA where the kernel is latency.
-    // More rows per CTA share more key reads and conversions, but the CTAs come in waves of one per SM (their shared memory
-    // fills it) and a CTA's rows are softmaxed and selected one after the other: take the count with the lowest estimate.
-    int dev = 0, sm_count = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess ||
-        cudaDeviceGetAttribute(&sm_count, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || sm_count <= 0)
-        sm_count = 148;
-    int rows_per_cta = 1;
-    if (Nkv > 2048 && D == 128 && ((uintptr_t)q_pooled % 16 == 0) && ((uintptr_t)k_pooled % 16 == 0)) {
-        // measured at 11 700 key blocks (microseconds; everything scales with the block count, so the comparison holds):
-        // scoring one row per CTA 115, R rows per CTA 190 + 29 R, and 21 per row for softmax and selection
-        auto cost = [&](int r) {
-            const long long g = (long long)B * H * ((Nq + r - 1) / r);
-            return ((g + sm_count - 1) / sm_count) * (r == 1 ? 115 + 21 : 190 + (29 + 21) * r);
-        };
-        rows_per_cta = cost(4) < cost(8) ? 4 : 8;
-        if (cost(1) < cost(rows_per_cta)) rows_per_cta = 1;
-        if (const char *e = getenv("WA_B200_ROUTE_ROWS"))      // tuning aid
-            if (e[0] == '1' || e[0] == '4' || e[0] == '8') rows_per_cta = e[0] - '0';
-    }
-    const int groups_per_bh = (Nq + rows_per_cta - 1) / rows_per_cta;
-    const long long groups = (long long)B * H * groups_per_bh;
-    const int gate_per_cta = (int)((128 * 128 + groups - 1) / groups);
-    if (groups < sm_count) sm_count = (int)groups;
-    const int slots = (int)((groups + sm_count - 1) / sm_count);
-    const dim3 grid((unsigned)((long long)sm_count * slots));
-    const float scale = (float)pow((double)D, -0.5), span = (float)(tau_max - tau_min);
-    SchedJob job = job_in;
-    job.release_dependents_after_rows = pdl_mode() == 2;
     // a fixed count per head over more key blocks than one pass of the register sort covers, and nobody reads the whole
     // order or the thresholds: select the best blocks instead of sorting all of them
     const int select_only = fixed_num_per_head && !whole_order && n_pow2 > threads;
-    if (rows_per_cta > 1 && threads > 512) threads = 512;
-    auto launch = [&](auto kernel) {
-        return launch_dependent(kernel, grid, dim3(threads), smem, stream, q_pooled, k_pooled, B, H, Nq, Nkv, n_pow2, D, scale,
-                                (float)tau_min, span, fixed_num_per_head, sorted, index, num, thresholds, gini, counters, job,
-                                gate_per_cta, sm_count, slots, groups_per_bh, select_only);
-    };
-    cudaError_t le = rows_per_cta == 8 ? launch(route_fused_kernel<8>)
-                                       : (rows_per_cta == 4 ? launch(route_fused_kernel<4>) : launch(route_fused_kernel<1>));
+    int key_slots = n_pow2 > threads ? n_pow2 : threads;
+    if (select_only && key_slots > 2048) {      // the selection's keys; several CTAs then share an SM and cover each other's barriers
+        key_slots = 2048;
+        threads = 512;
+    }
+    const size_t smem = (size_t)key_slots * sizeof(unsigned long long) + (size_t)Nkv * sizeof(float);
+    if (smem > 24 * 1024) {   // static shared memory of the kernel takes ~22 KB of the default 48 KB
+        const cudaError_t e = cudaFuncSetAttribute(route_fused_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        if (e != cudaSuccess) return fail((int)e, "wa_hsa_forward(routing): %s", cudaGetErrorString(e));
+    }
+    int sms = sm_count();
+    const float scale = (float)pow((double)D, -0.5), span = (float)(tau_max - tau_min);
+    const long long bh = (long long)B * H;
+
+    // Scoring in a launch of its own costs about 2 us and saves every row its pass over the head's keys: from 65 536 logits on it
+    // pays (444 rows over 256 key blocks, the whole call: 130.7 -> 127.8 us; 888 over 122: 227.9 -> 222.9; 888 over 512: 706.6 ->
+    // 686.4), at 444 rows over 37 the row kernel alone is 2.7 us faster.
+    const bool logits_ready = D == 128 && rows * Nkv >= 65536 && ((uintptr_t)q_pooled % 16 == 0) && ((uintptr_t)k_pooled % 16 == 0);
+    if (logits_ready) {
+        // rows per CTA: those that finish first, a tile of 128 keys being 2.1 us per 16 rows and about 1 us besides
+        const int tiles = (Nkv + RL_TILE - 1) / RL_TILE, row_tiles = (Nq + 15) / 16;
+        auto cost = [&](int mt) { return ((bh * ((row_tiles + mt - 1) / mt) * tiles + sms - 1) / sms) * (21 * mt + 10); };
+        int mt = RL_MAX_MT;
+        for (int m = RL_MAX_MT - 1; m >= 1; --m)
+            if (cost(m) < cost(mt)) mt = m;
+        const int groups = (row_tiles + mt - 1) / mt;
+        const long long units = bh * groups * tiles;
+        const auto launch = [&](auto width) -> cudaError_t {
+            constexpr int MT = decltype(width)::value, BYTES = MT * 16 * 128 * (int)sizeof(double);
+            const auto kernel = route_logits_kernel<MT>;
+            static PerDeviceOnce attr_set;
+            if (!attr_set.done()) {
+                const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, BYTES);
+                if (e != cudaSuccess) return e;
+                attr_set.mark();
+            }
+            return launch_dependent(kernel, dim3((unsigned)(units < sms ? units : sms)), dim3(RL_WARPS * 32), BYTES, stream, q_pooled, k_pooled, Nq, Nkv,
+                                    scale, sorted, groups, tiles, units);
+        };
+        const cudaError_t e = mt == 1 ? launch(std::integral_constant<int, 1>()) : mt == 2 ? launch(std::integral_constant<int, 2>())
+                            : mt == 3 ? launch(std::integral_constant<int, 3>()) : mt == 4 ? launch(std::integral_constant<int, 4>())
+                                      : launch(std::integral_constant<int, 5>());
+        if (e != cudaSuccess) return fail((int)e, "wa_hsa_forward(logits): %s", cudaGetErrorString(e));
+        if (const int rc = check_launch("wa_hsa_forward(logits)")) return rc;
+    }
+    const int gate_per_cta = (int)((128 * 128 + rows - 1) / rows);
+    if (rows < sms) sms = (int)rows;
+    const int slots = (int)((rows + sms - 1) / sms);
+    const dim3 grid((unsigned)((long long)sms * slots));
+    SchedJob job = job_in;
+    job.release_dependents_after_rows = pdl_mode() == 2;
+    const cudaError_t le = launch_dependent(route_fused_kernel, grid, dim3(threads), smem, stream, q_pooled, k_pooled, B, H, Nq, Nkv, n_pow2, D, scale,
+                                            (float)tau_min, span, fixed_num_per_head, sorted, index, num, thresholds, gini, counters, job,
+                                            gate_per_cta, sms, slots, select_only, logits_ready ? 1 : 0, key_slots);
     if (le != cudaSuccess) return fail((int)le, "wa_hsa_forward(routing): %s", cudaGetErrorString(le));
     return check_launch("wa_hsa_forward(routing)");
 }
