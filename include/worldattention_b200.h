@@ -360,6 +360,30 @@ int wa_hkv_build_records(const int32_t *top_ids, int layers, int heads, int topk
  * the installed rows of all layers, in one launch.  max_tokens: the largest n_tokens of the records; elem_size 2 or 4. */
 int wa_hkv_clear_rows(const wa_page_copy *rows, int n, int max_tokens, int row_elems, int elem_size, void *stream);
 
+/* Install of pages of whole frames into the caches of all layers, fused with the compression of what is installed
+ * (cache.py:229-254 and compress_kv, attention.py:64-110): bf16, rows of H*D contiguous values, projection segments of
+ * one frame.  A tensor is one layer's K or V (layer * 2 + (0 K | 1 V)); the arrays are host arrays.  `wa_hkv_install_table`
+ * fills `table` (host memory, wa_hkv_install_table_bytes) or answers WA_ERR_UNSUPPORTED; the caller copies it to the
+ * device and calls `wa_hkv_install_pages` with the same description.  The pages are installed from row 0 on. */
+typedef struct wa_hkv_install {
+    int pages, tensors, segments;      /* segments: frames of all pages together */
+    int B, H, D, frame;                /* frame: tokens of a frame = segment length of the projections */
+    int block_size, proj_rank, proj_cols, n_temporal;
+    const int32_t *page_frames;        /* [pages] frames of each page */
+    const int32_t *page_rot;           /* [pages] row of the rotation table for its keys, or -1 */
+    const unsigned long long *src;     /* [pages][tensors] address of the page's first row */
+    const int64_t *src_batch;          /* [pages][tensors] elements between batch items */
+    const unsigned long long *dst;     /* [tensors] address of the cache's first row */
+    const int64_t *dst_batch;          /* [tensors] */
+    const unsigned long long *coarse;  /* [tensors] address of the first compressed slot */
+    const int64_t *coarse_batch, *coarse_row;   /* [tensors] elements between batch items, between slots */
+    const unsigned long long *proj;    /* [tensors] the layer's projection, [proj_rank, proj_cols] bf16 */
+} wa_hkv_install;
+size_t wa_hkv_install_table_bytes(int pages, int tensors, int segments);
+int wa_hkv_install_table(const wa_hkv_install *p, void *table, size_t bytes);
+/* `rotations`: device float `[R, n_temporal, 2]`, or null. */
+int wa_hkv_install_pages(const wa_hkv_install *p, const void *device_table, const float *rotations, void *stream);
+
 /* Promotion of cold pages (the `.to(device)` of cache.py:229-231 for chunks that live in host memory): one
  * asynchronous host-to-device copy per record of the HOST array `host_records` (src = page-locked host memory,
  * dst = device memory, `rot` ignored), queued on `stream` -- the caller's side stream.  A record whose token rows

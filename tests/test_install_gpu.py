@@ -1,0 +1,68 @@
+"""The fused install (copy, rotation and compression of all layers in one launch) against the page-copy and compress kernels it
+stands in for: the same bits, over frames of whole tiles and of remainders, batches, head sizes, tiers and unequal pages."""
+import numpy as np
+import pytest
+import torch
+
+from tests.helpers import dev
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("frame,heads,d,bsz,block,hot,rerope", [
+    (24, 2, 64, 1, 64, 2, True), (128, 1, 128, 2, 64, 2, True), (136, 3, 128, 1, 64, 0, True), (1560, 2, 128, 1, 128, 2, True),
+    (256, 4, 32, 2, 64, 1, True), (264, 2, 64, 3, 128, 2, False), (8, 1, 128, 1, 64, 2, True)])
+def test_fused_install_equals_the_separate_kernels(monkeypatch, frame, heads, d, bsz, block, hot, rerope):
+    import worldattention_b200 as wa
+    layers, window = 3, 7
+    g = torch.Generator(device=dev()).manual_seed(frame)
+    make = lambda n: torch.randn((bsz, n, heads, d), generator=g, device=dev()).bfloat16()
+    hsa = [wa.hsa.HSAAttention(heads, d, block_size=block, proj_segment_len=frame).to(dev(), torch.bfloat16) for _ in range(layers)]
+    for m in hsa:
+        torch.nn.init.normal_(m.k_proj_mat)
+        torch.nn.init.normal_(m.v_proj_mat)
+    inv = 1.0 / (10000.0 ** (np.arange(d // 2) / (d // 2)))
+    freqs = torch.from_numpy(np.exp(1j * np.outer(np.arange(256.0), inv))[:, : wa.hkv.temporal_complex_dims(d)])
+    hkv = wa.hkv.HKVCache(frame_seq_length=frame, page_size_frames=2, topk_pages=3, stage1_topk_chunks=2, hbm_max_chunks=hot, rerope=rerope)
+    size, slots = window * frame, hsa[0].coarse_cache_size(window * frame)
+    for c in range(2):
+        cache = [{"k": make(size), "v": make(size), "k_coarse": make(slots), "v_coarse": make(slots),
+                  "local_end_index": torch.tensor([size], device=dev()), "global_end_index": torch.tensor([size], device=dev())} for _ in range(layers)]
+        # what lies behind an installed page must not reach its slots
+        for block_cache in cache:
+            block_cache["k"][:, 4 * frame] = float("nan")
+        hkv.store(cache, prompt_embeds=make(1).float()[:, :, 0], current_start_frame=window * (c + 1), temporal_freqs=freqs)
+    torch.cuda.synchronize()
+    calls = []
+    fused = wa.hkv.HKVCache._install_fused
+    monkeypatch.setattr(wa.hkv.HKVCache, "_install_fused", lambda self, *a: calls.append(fused(self, *a)) or calls[-1])
+    # pages of two frames and the last one of one; the pages of the second call do not fit and are cut
+    for pairs, fits in ((((0, 1), (0, 3), (1, 0)), True), (((0, 0), (1, 1), (0, 3), (1, 0), (1, 3)), True)):
+        start = [{n: t.clone() for n, t in b.items()} for b in cache]
+        tokens = hkv.apply(cache, list(pairs), current_start_frame=40, temporal_freqs=freqs, hsa_modules=hsa)
+        assert calls.pop() is fits and tokens % frame == 0
+        with monkeypatch.context() as m:
+            m.setattr(wa.hkv.HKVCache, "_install_fused", lambda self, *a: False)
+            assert hkv.apply(start, list(pairs), current_start_frame=40, temporal_freqs=freqs, hsa_modules=hsa) == tokens
+        for got, want in zip(cache, start):
+            for name in want:
+                assert torch.equal(got[name].view(torch.int16) if got[name].dtype == torch.bfloat16 else got[name],
+                                   want[name].view(torch.int16) if want[name].dtype == torch.bfloat16 else want[name]), name
+
+
+def test_pages_of_broken_frames_take_the_separate_kernels(monkeypatch):
+    import worldattention_b200 as wa
+    frame, heads, d = 16, 1, 128
+    hkv = wa.hkv.HKVCache(frame_seq_length=frame, page_size_frames=2, hbm_max_chunks=1)
+    hsa = [wa.hsa.HSAAttention(heads, d, block_size=64, proj_segment_len=frame).to(dev(), torch.bfloat16)]
+    make = lambda n: torch.randn((1, n, heads, d), device=dev()).bfloat16()
+    cache = [{"k": make(80), "v": make(80), "k_coarse": make(5), "v_coarse": make(5),
+              "local_end_index": torch.tensor([80], device=dev()), "global_end_index": torch.tensor([80], device=dev())}]
+    freqs = torch.polar(torch.ones(64, 22, dtype=torch.float64), torch.randn(64, 22, dtype=torch.float64))
+    hkv.store(cache, prompt_embeds=make(1).float()[:, :, 0], current_start_frame=5, temporal_freqs=freqs)
+    hkv.chunks[0]["page_spans"] = [(0, 32), (40, 72)]          # a page that does not start with a frame
+    done = []
+    fused = wa.hkv.HKVCache._install_fused
+    monkeypatch.setattr(wa.hkv.HKVCache, "_install_fused", lambda self, *a: done.append(fused(self, *a)) or done[-1])
+    assert hkv.apply(cache, [(0, 0), (0, 1)], current_start_frame=9, temporal_freqs=freqs, hsa_modules=hsa) == 64
+    assert done == [False]

@@ -52,6 +52,13 @@ class PageCopy(C.Structure):
                 ("dst_stride", C.c_int64), ("n_tokens", C.c_int32), ("rot", C.c_int32)]
 
 
+class HkvInstall(C.Structure):      # wa_hkv_install
+    _fields_ = [(n, C.c_int32) for n in ("pages", "tensors", "segments", "B", "H", "D", "frame", "block_size", "proj_rank", "proj_cols",
+                                         "n_temporal")] + \
+               [(n, C.c_void_p) for n in ("page_frames", "page_rot", "src", "src_batch", "dst", "dst_batch", "coarse", "coarse_batch",
+                                          "coarse_row", "proj")]
+
+
 _T4P = C.POINTER(Tensor4)
 _vp, _i, _f, _d, _i64 = C.c_void_p, C.c_int, C.c_float, C.c_double, C.c_int64
 
@@ -95,10 +102,13 @@ SIGNATURES = {
     "wa_hkv_build_records": [_vp, _i, _i, _i, _vp, _i, C.c_longlong, C.c_longlong, _vp, C.c_longlong, C.c_longlong,
                              _i, _i, _i, _i, _vp, _vp, _vp],
     "wa_hkv_promote_pages": [_vp, _i, _i, _i, _vp],
+    "wa_hkv_install_table_bytes": [_i, _i, _i],
+    "wa_hkv_install_table": [_vp, _vp, C.c_size_t],
+    "wa_hkv_install_pages": [_vp, _vp, _vp, _vp],
     "wa_hkv_clear_rows": [_vp, _i, _i, _i, _i, _vp],
     "wa_hkv_gather_pages": [_vp, _i, _i, _i, _i, _i, _vp, _i, _vp],
 }
-_RESTYPES = {"wa_last_error": C.c_char_p, "wa_hsa_workspace_bytes": C.c_size_t, "wa_hsa_params_size": C.c_size_t, "wa_kv_append_workspace_bytes": C.c_size_t,
+_RESTYPES = {"wa_last_error": C.c_char_p, "wa_hkv_install_table_bytes": C.c_size_t, "wa_hsa_workspace_bytes": C.c_size_t, "wa_hsa_params_size": C.c_size_t, "wa_kv_append_workspace_bytes": C.c_size_t,
              "wa_launch_count": C.c_ulonglong}
 
 _lib: Optional[C.CDLL] = None

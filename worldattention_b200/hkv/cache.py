@@ -9,10 +9,10 @@ behaviour follow the reference.  What changes is where the bytes move:
   on a side stream, and builds the page index from layer 0's keys with one pooling kernel that
   removes the temporal rotation on the fly;
 * `retrieve` scores and selects pages in one kernel launch and reads back only the chosen ids;
-* `apply` installs all pages of all layers with one page-copy kernel launch (keys re-rotated in
-  flight, values verbatim), promoting host-resident pages through page-locked async copies on a
-  side stream, clears only the tail of the cache beyond the installed span, and rebuilds the
-  compressed tier with the compress kernel writing straight into the cache slots.
+* `apply` installs all pages of all layers with one launch (keys re-rotated in flight, values
+  verbatim), promoting host-resident pages through page-locked async copies on a side stream, and
+  clears only the tail of the cache beyond the installed span.  Pages of whole frames are compressed
+  by the same launch, straight into the cache slots; others by the compress kernel behind it.
 
 Online cache contract: a list with one dict per transformer block holding `k`, `v`
 (`[B, capacity, H, D]`), scalar tensors `global_end_index`, `local_end_index`, and optionally
@@ -20,6 +20,7 @@ Online cache contract: a list with one dict per transformer block holding `k`, `
 """
 from __future__ import annotations
 
+import ctypes
 from typing import List, Optional, Sequence, Tuple
 
 import numpy as np
@@ -197,15 +198,19 @@ class HKVCache:
         # everything before them.  They go first, so that the device is at work while the copy records are put together.
         sources = self._install_sources(kv_cache, plan, blobs, k0.dtype) if tokens > 0 else None
         self._clear_tails(kv_cache, tokens, hsa_modules if compressed else None, dev)
-        if tokens > 0:
-            self._install(kv_cache, plan, sources, temporal_freqs, dev, k0.dtype)
+        if tokens > 0 and not self._install(kv_cache, plan, sources, temporal_freqs, dev, k0.dtype, hsa_modules if compressed else None):
+            if compressed:
+                for layer, block in enumerate(kv_cache):
+                    self._write_coarse(block, hsa_modules[layer], tokens)
 
-        end_token = current_start_frame * self.frame_seq_length
-        for layer, block in enumerate(kv_cache):
-            if compressed and tokens > 0:
-                self._write_coarse(block, hsa_modules[layer], tokens)
-            block["global_end_index"].fill_(end_token)
-            block["local_end_index"].fill_(tokens)
+        for name, value in (("global_end_index", current_start_frame * self.frame_seq_length), ("local_end_index", tokens)):
+            ends = list({id(block[name]): block[name] for block in kv_cache}.values())
+            if len({t.data_ptr() for t in ends}) == len(ends) and all(t.is_cuda and t.dtype == torch.long for t in ends):
+                torch._foreach_zero_(ends)           # two launches for all layers
+                torch._foreach_add_(ends, value)
+            else:
+                for t in ends:
+                    t.fill_(value)
         return tokens
 
     _PLAN_DTYPE = np.dtype([("chunk", "<i8"), ("src", "<i8"), ("count", "<i8"), ("dst", "<i8"),
@@ -354,8 +359,11 @@ class HKVCache:
                     single.append((layer, name, i, page, slot))
         return whole, single, staged_elems
 
-    def _install(self, kv_cache, plan, sources, temporal_freqs, dev, dtype) -> None:
-        """One page-copy launch for every (layer, page, K|V, batch item) of the plan."""
+    def _install(self, kv_cache, plan, sources, temporal_freqs, dev, dtype, hsa_modules=None) -> bool:
+        """The plan's pages into the caches of all layers in one launch.
+
+        With `hsa_modules` and where the fused kernel covers the call, the compressed slots are written by that launch too
+        (True); otherwise one page-copy launch for every (layer, page, K|V, batch item) (False)."""
         whole, single, staged_elems = sources
         k0 = kv_cache[0]["k"]
         bsz, _, heads, head_dim = k0.shape
@@ -372,14 +380,20 @@ class HKVCache:
         # behind its copy, so that nothing reads a landing buffer early
         staging = torch.empty((max(staged_elems, 1),), dtype=dtype, device=dev) if staged_elems else None
         keep_alive = [staging]
-        promote, pages = [], []      # pages: (src, dst, src_stride, n_tokens, rot)
+        promote = []
         promoted = False
+        # first row of every (page, tensor, batch item) on the device, elements between its rows; a tensor is (layer, K|V)
+        tensors = [block[name] for block in kv_cache for name in ("k", "v")]
+        batch = np.arange(bsz, dtype=np.int64) * esize
+        starts = lambda ts: (np.array([t.data_ptr() for t in ts], dtype=np.int64)[:, None]
+                             + np.array([t.stride(0) for t in ts], dtype=np.int64)[:, None] * batch)
+        src = np.zeros((len(plan), len(tensors), bsz), dtype=np.int64)
+        src_stride = np.full((len(plan), len(tensors)), row_elems, dtype=np.int64)
         for layer, name, i, page, slot in single:
             row = plan[i]
             n = int(row["count"])
-            dst = kv_cache[layer][name]
             if slot is not None:
-                src_ptr, src_batch, src_stride = staging.data_ptr() + slot * esize, n * row_elems, row_elems
+                src_ptr, src_batch, stride = staging.data_ptr() + slot * esize, n * row_elems, row_elems
                 for b in range(bsz):
                     promote.append(_lib.PageCopy(page.data_ptr() + b * page.stride(0) * esize,
                                                  src_ptr + b * src_batch * esize, row_elems, row_elems, n, -1))
@@ -394,10 +408,13 @@ class HKVCache:
                 else:
                     page = self._as_cache_rows(page, dtype, head_dim)
                 keep_alive.append(page)
-                src_ptr, src_batch, src_stride = page.data_ptr(), page.stride(0), page.stride(1)
-            for b in range(bsz):
-                pages.append((src_ptr + b * src_batch * esize, dst.data_ptr() + (b * dst.stride(0) + int(row["dst"]) * row_elems) * esize,
-                              src_stride, n, i if (name == "k" and rot is not None) else -1))
+                src_ptr, src_batch, stride = page.data_ptr(), page.stride(0), page.stride(1)
+            at = 2 * layer + (name == "v")
+            src[i, at] = src_ptr + batch * src_batch
+            src_stride[i, at] = stride
+        for chunk_id, held in whole.items():
+            mine = np.flatnonzero(plan["chunk"] == chunk_id)
+            src[mine] = starts(held) + (plan["src"][mine] * (row_elems * esize))[:, None, None]
         if promote:
             arr = (_lib.PageCopy * len(promote))(*promote)
             side.wait_stream(main)            # the staging block may be recycled memory that the main stream still uses
@@ -407,37 +424,72 @@ class HKVCache:
             promoted = True
         if promoted:
             main.wait_stream(side)
-        parts = [np.array(pages, dtype=np.int64).reshape(-1, 5)]
-        if whole:
-            # [tensor (layer, K|V), batch item] addresses of the cache, and of every chunk: a page is an offset into both
-            batch = np.arange(bsz, dtype=np.int64) * esize
-            starts = lambda ts: (np.array([t.data_ptr() for t in ts], dtype=np.int64)[:, None]
-                                 + np.array([t.stride(0) for t in ts], dtype=np.int64)[:, None] * batch)
-            to = starts([block[name] for block in kv_cache for name in ("k", "v")])
-            origin = {chunk_id: starts(held) for chunk_id, held in whole.items()}
-            is_key = (np.arange(len(to)) % 2 == 0)[:, None]
-            for i, row in enumerate(plan):
-                if row["count"] == 0 or int(row["chunk"]) not in whole:
-                    continue
-                part = np.empty(to.shape + (5,), dtype=np.int64)
-                part[..., 0] = origin[int(row["chunk"])] + int(row["src"]) * row_elems * esize
-                part[..., 1] = to + int(row["dst"]) * row_elems * esize
-                part[..., 2], part[..., 3] = row_elems, row["count"]
-                part[..., 4] = np.where(is_key, i if rot is not None else -1, -1)
-                parts.append(part.reshape(-1, 5))
-        table = np.concatenate(parts)
-        records = np.zeros(len(table), dtype=RECORD_DTYPE)
-        records["src"], records["dst"] = table[:, 0].astype(np.uint64), table[:, 1].astype(np.uint64)
-        records["src_stride"], records["dst_stride"] = table[:, 2], row_elems
-        records["n_tokens"], records["rot"] = table[:, 3], table[:, 4]
+        used = np.flatnonzero(plan["count"] > 0)
+        dst = starts(tensors)
         rot_dev = to_device(rot, dev) if rot is not None else None
-        gather_records_device(to_device(records.view(np.uint8), dev), max_tokens=int(plan["count"].max()), row_elems=row_elems,
-                              head_dim=head_dim, dtype=dtype, rotations=rot_dev, n_temporal=nt)
+        fused = hsa_modules is not None and bool((src_stride[used] == row_elems).all()) and self._install_fused(
+            kv_cache, plan[used], src[used], dst, used if rot is not None else np.full(len(used), -1), rot_dev, nt, dev, hsa_modules)
+        if not fused:
+            records = np.zeros((len(used),) + dst.shape, dtype=RECORD_DTYPE)
+            records["src"] = src[used].astype(np.uint64)
+            records["dst"] = (dst + (plan["dst"][used] * (row_elems * esize))[:, None, None]).astype(np.uint64)
+            records["src_stride"], records["dst_stride"] = src_stride[used][:, :, None], row_elems
+            records["n_tokens"] = plan["count"][used][:, None, None]
+            records["rot"] = -1
+            if rot is not None:
+                records["rot"][:, ::2] = used[:, None, None]
+            gather_records_device(to_device(records.reshape(-1).view(np.uint8), dev), max_tokens=int(plan["count"].max()), row_elems=row_elems,
+                                  head_dim=head_dim, dtype=dtype, rotations=rot_dev, n_temporal=nt)
         storages = {t.untyped_storage().data_ptr(): t for t in keep_alive if t is not None and t.is_cuda}
         for held in whole.values():
             storages.update((t.untyped_storage().data_ptr(), t) for t in held)
         for t in storages.values():
             t.record_stream(main)
+        return fused
+
+    def _install_fused(self, kv_cache, plan, src, dst, rot_rows, rot_dev, nt, dev, hsa_modules) -> bool:
+        """Copy, rotation and compression of all layers in one launch: bf16, pages of whole frames, projection segments of one
+        frame, one shape of projection for all layers.  False (nothing launched): not covered."""
+        k0 = kv_cache[0]["k"]
+        bsz, _, heads, head_dim = k0.shape
+        frame, esize = self.frame_seq_length, k0.element_size()
+        if k0.dtype != torch.bfloat16 or (plan["count"] % frame).any() or (plan["src"] % frame).any():
+            return False
+        first = hsa_modules[0]
+        shape, block = first.k_proj_mat.shape, first.block_size
+        if first.proj_segment_len != frame or shape[1] < frame:
+            return False
+        slots = first.token_range_to_coarse(0, int(plan["count"].sum()))[1]
+        coarse, proj = [], []
+        for layer, hsa in zip(kv_cache, hsa_modules):
+            kc, vc = layer["k_coarse"], layer["v_coarse"]
+            if hsa.proj_segment_len != frame or hsa.block_size != block or kc.stride() != vc.stride():
+                return False
+            for cache, t, p in ((layer["k"], kc, hsa.k_proj_mat), (layer["v"], vc, hsa.v_proj_mat)):
+                if (cache.dtype != torch.bfloat16 or cache.shape[0] != bsz or t.dtype != torch.bfloat16 or p.dtype != torch.bfloat16
+                        or t.device != dev or p.device != dev or p.shape != shape or not p.is_contiguous() or t.shape[0] < bsz
+                        or t.shape[1] < slots or t.shape[2:] != k0.shape[2:] or t.stride(3) != 1 or t.stride(2) != head_dim):
+                    return False
+                coarse.append(t)
+                proj.append(p)
+        address = lambda ts: np.array([t.data_ptr() for t in ts], dtype=np.uint64)
+        step = lambda ts, dim: np.array([t.stride(dim) for t in ts], dtype=np.int64)
+        between = lambda a: np.ascontiguousarray((a[..., 1] - a[..., 0]) // esize if bsz > 1 else np.zeros(a.shape[:-1], dtype=np.int64))
+        frames = (plan["count"] // frame).astype(np.int32)
+        arrays = dict(page_frames=frames, page_rot=rot_rows.astype(np.int32), src=np.ascontiguousarray(src[..., 0]).astype(np.uint64),
+                      src_batch=between(src), dst=dst[:, 0].astype(np.uint64), dst_batch=between(dst), coarse=address(coarse),
+                      coarse_batch=step(coarse, 0), coarse_row=step(coarse, 1), proj=address(proj))
+        job = _lib.HkvInstall(len(plan), len(dst), int(frames.sum()), bsz, heads, head_dim, frame, block, shape[0], shape[1],
+                              nt if rot_dev is not None else 0, *(arrays[n].ctypes.data for n, _ in _lib.HkvInstall._fields_[11:]))
+        lib = _lib.lib()
+        table = np.empty((lib.wa_hkv_install_table_bytes(job.pages, job.tensors, job.segments),), dtype=np.uint8)
+        with _lib.device_guard(dev):
+            rc = lib.wa_hkv_install_table(ctypes.byref(job), table.ctypes.data, table.nbytes)
+            if rc == _lib.WA_ERR_UNSUPPORTED:
+                return False
+            _lib.check(rc)
+            _lib.check(lib.wa_hkv_install_pages(ctypes.byref(job), to_device(table, dev).data_ptr(), _lib.ptr(rot_dev), _lib.stream_ptr(dev)))
+        return True
 
     @staticmethod
     def _as_cache_rows(page: torch.Tensor, dtype: torch.dtype, head_dim: int) -> torch.Tensor:
