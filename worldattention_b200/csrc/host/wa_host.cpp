@@ -484,6 +484,41 @@ PyObject *gated_residual(PyObject *const *a, Py_ssize_t n) {
     return THPVariable_Wrap(std::move(out));
 }
 
+// ---- tensor_table(tensors) -> bytes: twelve int64 per tensor -------------------------------------
+// address, device index (-1: host), scalar type, dimensions, the first four sizes, the first four strides.  A prompt switch looks
+// at some hundred tensors; asked for one attribute at a time from Python that took longer than the copies.
+PyObject *tensor_table(PyObject *const *a, Py_ssize_t n) {
+    expect_args(n, 1);
+    PyObject *seq = PySequence_Fast(a[0], "expected a sequence of tensors");
+    if (!seq) throw PyFailure();
+    const Py_ssize_t count = PySequence_Fast_GET_SIZE(seq);
+    PyObject *out = PyBytes_FromStringAndSize(nullptr, count * 12 * (Py_ssize_t)sizeof(int64_t));
+    if (!out) {
+        Py_DECREF(seq);
+        throw PyFailure();
+    }
+    int64_t *row = reinterpret_cast<int64_t *>(PyBytes_AS_STRING(out));
+    try {
+        for (Py_ssize_t i = 0; i < count; ++i, row += 12) {
+            const Tensor &t = tensor(PySequence_Fast_GET_ITEM(seq, i), "every element");
+            row[0] = reinterpret_cast<int64_t>(t.data_ptr());
+            row[1] = t.is_cuda() ? t.device().index() : -1;
+            row[2] = (int64_t)t.scalar_type();
+            row[3] = t.dim();
+            for (int d = 0; d < 4; ++d) {
+                row[4 + d] = d < t.dim() ? t.size(d) : 1;
+                row[8 + d] = d < t.dim() ? t.stride(d) : 0;
+            }
+        }
+    } catch (...) {
+        Py_DECREF(seq);
+        Py_DECREF(out);
+        throw;
+    }
+    Py_DECREF(seq);
+    return out;
+}
+
 // ---- bind(addresses: dict name -> int, status_word, raise_if_failed) ----------------------------
 PyObject *bind(PyObject *const *a, Py_ssize_t n) {
     expect_args(n, 3);
@@ -534,7 +569,7 @@ PyObject *entry(PyObject *, PyObject *const *args, Py_ssize_t n) {
 
 #define WA_ENTRY(name) {#name, (PyCFunction)(void (*)(void))entry<name>, METH_FASTCALL, nullptr}
 PyMethodDef methods[] = {WA_ENTRY(bind), WA_ENTRY(hsa_forward), WA_ENTRY(run_forward), WA_ENTRY(qk_norm_rope), WA_ENTRY(append_kv), WA_ENTRY(ln_modulate),
-                         WA_ENTRY(gated_residual), {nullptr, nullptr, 0, nullptr}};
+                         WA_ENTRY(gated_residual), WA_ENTRY(tensor_table), {nullptr, nullptr, 0, nullptr}};
 PyModuleDef module = {PyModuleDef_HEAD_INIT, "_host", nullptr, -1, methods, nullptr, nullptr, nullptr, nullptr};
 
 }  // namespace

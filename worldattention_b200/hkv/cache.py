@@ -35,6 +35,25 @@ from .tiering import HKVTierManager
 __all__ = ["HKVCache"]
 
 
+class _Table:
+    """Addresses, sizes and strides of a list of tensors as arrays."""
+
+    def __init__(self, tensors):
+        t = np.frombuffer(_lib.host().tensor_table(tensors), dtype=np.int64).reshape(-1, 12)
+        self.ptr, self.device, self.dtype, self.dim, self.size, self.stride = t[:, 0], t[:, 1], t[:, 2], t[:, 3], t[:, 4:8], t[:, 8:]
+
+    def cache_rows(self, like: "_Table") -> np.ndarray:
+        """Which tensors hold token rows of the heads, type and device of `like`'s first without gaps inside a row or between rows."""
+        heads, head_dim = like.size[0, 2:]
+        return ((self.dim == 4) & (self.dtype == like.dtype[0]) & (self.device == like.device[0]) & (self.size[:, 2] == heads)
+                & (self.size[:, 3] == head_dim) & (self.stride[:, 3] == 1) & (self.stride[:, 2] == head_dim)
+                & (self.stride[:, 1] == heads * head_dim))
+
+    def starts(self, batch: int, esize: int) -> np.ndarray:
+        """`[tensor, batch item]` addresses."""
+        return self.ptr[:, None] + self.stride[:, :1] * (np.arange(batch, dtype=np.int64) * esize)
+
+
 class HKVCache:
     """KV bank with two-stage page retrieval and multi-tier residency.
 
@@ -59,6 +78,7 @@ class HKVCache:
         self.rerope = bool(rerope)
         self._tier_kwargs = dict(cpu_max_chunks=cpu_max_chunks, nvme_enabled=nvme_enabled, nvme_dir=nvme_dir,
                                  hbm_max_chunks=hbm_max_chunks)
+        self._table_stream: Optional[torch.cuda.Stream] = None
         self.reset()
 
     def reset(self) -> None:
@@ -74,6 +94,28 @@ class HKVCache:
     def page_tokens(self) -> int:
         return self.page_size_frames * self.frame_seq_length
 
+    def _fetch_table(self, temporal_freqs):
+        """The frequency table on its way to the host, on a stream that carries nothing else: a function that waits for it (and
+        not for the copies launched meanwhile)."""
+        if not (isinstance(temporal_freqs, torch.Tensor) and temporal_freqs.is_cuda):
+            table = host_table(temporal_freqs)
+            return lambda: table
+        dev = temporal_freqs.device
+        if self._table_stream is None or self._table_stream.device != dev:
+            self._table_stream = torch.cuda.Stream(dev)
+        self._table_stream.wait_stream(torch.cuda.current_stream(dev))
+        with torch.cuda.stream(self._table_stream):
+            landed = torch.empty(temporal_freqs.shape, dtype=temporal_freqs.dtype, pin_memory=True)
+            landed.copy_(temporal_freqs.detach(), non_blocking=True)
+            done = torch.cuda.Event()
+            done.record()
+        temporal_freqs.record_stream(self._table_stream)
+
+        def wait():
+            done.synchronize()
+            return landed.numpy()
+        return wait
+
     # ------------------------------------------------------------------ store
     def store(self, kv_cache: Sequence[dict], *, prompt_embeds: torch.Tensor, current_start_frame: int,
               temporal_freqs: torch.Tensor) -> int:
@@ -85,23 +127,23 @@ class HKVCache:
         if valid_tokens <= 0:
             return -1
         _lib.require_cuda(kv_cache[0]["k"])
-        short = next((block[name] for block in kv_cache for name in ("k", "v") if block[name].shape[1] < valid_tokens), None)
-        if short is not None:          # the copy kernel takes addresses: nothing behind it would stop at the end of a cache
-            raise RuntimeError(f"local_end_index says {valid_tokens} tokens, but an online cache tensor holds {short.shape[1]} rows")
-        temporal_freqs = host_table(temporal_freqs)     # before the copies: it waits for the device
+        tensors = [block[name] for name in ("k", "v") for block in kv_cache]
+        table = _Table(tensors)
+        if (table.size[:, 1] < valid_tokens).any():      # the copy kernel takes addresses: nothing behind it would stop at the end of a cache
+            raise RuntimeError(f"local_end_index says {valid_tokens} tokens, but an online cache tensor holds {table.size[:, 1].min()} rows")
+        temporal_freqs = self._fetch_table(temporal_freqs)
 
         chunk_id = len(self.chunks)
         # one allocation for the whole chunk (views per layer) instead of one per layer and tensor: growing the
         # allocator's pool costs a driver call per allocation, which at 60 calls per stored window showed as stalls of
         # up to a second at a prompt switch
         first = kv_cache[0]["k"]
-        uniform = all(block[name].shape == first.shape and block[name].dtype == first.dtype and block[name].device == first.device
-                      for block in kv_cache for name in ("k", "v"))
+        uniform = bool((table.size == table.size[0]).all() and (table.dtype == table.dtype[0]).all() and (table.device == table.device[0]).all())
         blob = {"k": [], "v": []}
         if uniform:
             slab = torch.empty((2, len(kv_cache), first.shape[0], valid_tokens) + tuple(first.shape[2:]), dtype=first.dtype,
                                device=first.device)
-            self._copy_rows([block[name] for name in ("k", "v") for block in kv_cache], slab, valid_tokens)
+            self._copy_rows(tensors, table, slab, valid_tokens)
             for which, name in enumerate(("k", "v")):
                 blob[name] = list(slab[which])
         else:
@@ -113,7 +155,7 @@ class HKVCache:
                       for start in range(0, valid_tokens, self.page_tokens)]
         start_frame = int(current_start_frame - valid_tokens // self.frame_seq_length)
         page_index = page_key_index(blob["k"][0], page_spans, frame_seq_length=self.frame_seq_length,
-                                    start_frame=start_frame, temporal_freqs=temporal_freqs)
+                                    start_frame=start_frame, temporal_freqs=temporal_freqs())
         self.chunks.append({
             "chunk_id": chunk_id,
             "valid_tokens": valid_tokens,
@@ -185,7 +227,7 @@ class HKVCache:
         dev = _lib.require_cuda(k0)
         tokens = int(plan["count"].sum())
         if self.rerope and tokens > 0:
-            temporal_freqs = host_table(temporal_freqs)     # before anything is launched: it waits for the device
+            temporal_freqs = self._fetch_table(temporal_freqs)
 
         compressed = all(name in kv_cache[0] for name in ("k_coarse", "v_coarse"))
         if compressed and hsa_modules is None:
@@ -258,33 +300,25 @@ class HKVCache:
         return plan, blobs
 
     @staticmethod
-    def _cache_rows(t: torch.Tensor, like: torch.Tensor) -> bool:
-        """Whether `t` holds token rows of `like`'s heads, type and device without gaps inside a row or between rows."""
-        heads, head_dim = like.shape[2:]
-        return (t.dtype == like.dtype and t.device == like.device and t.shape[2:] == like.shape[2:] and t.stride(3) == 1
-                and t.stride(2) == head_dim and t.stride(1) == heads * head_dim)
-
-    @staticmethod
     def _copied_by_kernel(like: torch.Tensor) -> bool:
         """Whether the page-copy kernel takes rows of this type and head size."""
         return like.dtype in (torch.float32, torch.bfloat16) and like.shape[3] % 2 == 0
 
     @classmethod
-    def _copy_rows(cls, sources, slab: torch.Tensor, tokens: int) -> None:
+    def _copy_rows(cls, sources, table: _Table, slab: torch.Tensor, tokens: int) -> None:
         """The first `tokens` rows of the cache tensors into `slab` `[2, layers, B, tokens, H, D]`: one launch of the page-copy
         kernel (6 GB read and written for a full window of 30 blocks: 1.75 ms against 2.05 ms as a copy per tensor)."""
         like = sources[0]
-        rows = list(slab.view(-1, *slab.shape[2:]))
-        if not (cls._copied_by_kernel(like) and all(cls._cache_rows(t, like) for t in sources)):
+        rows = slab.view(-1, *slab.shape[2:])
+        if not (cls._copied_by_kernel(like) and table.cache_rows(table).all()):
             for dst, t in zip(rows, sources):
                 dst.copy_(t[:, :tokens].detach())
             return
-        records = np.zeros((len(rows), like.shape[0]), dtype=RECORD_DTYPE)
-        batch = np.arange(like.shape[0], dtype=np.int64) * like.element_size()
-        for name, tensors in (("src", sources), ("dst", rows)):
-            base, step = (np.array(x, dtype=np.int64)[:, None] for x in ([t.data_ptr() for t in tensors], [t.stride(0) for t in tensors]))
-            records[name] = (base + step * batch).astype(np.uint64)
-        row_elems = like.shape[2] * like.shape[3]
+        records = np.zeros((len(sources), like.shape[0]), dtype=RECORD_DTYPE)
+        row_elems, esize = like.shape[2] * like.shape[3], like.element_size()
+        items = np.arange(len(sources) * like.shape[0], dtype=np.int64).reshape(records.shape)
+        records["src"] = table.starts(like.shape[0], esize).astype(np.uint64)
+        records["dst"] = (slab.data_ptr() + items * (tokens * row_elems * esize)).astype(np.uint64)
         records["src_stride"] = records["dst_stride"] = row_elems
         records["n_tokens"], records["rot"] = tokens, -1
         gather_records_device(to_device(records.reshape(-1).view(np.uint8), like.device), max_tokens=tokens, row_elems=row_elems,
@@ -295,54 +329,51 @@ class HKVCache:
         """Zero everything behind the installed tokens (and, with `hsa_modules`, behind their compressed slots) in all
         layers in one launch."""
         k0 = kv_cache[0]["k"]
-        row_elems = k0.shape[2] * k0.shape[3]
-        direct = cls._copied_by_kernel(k0)
-        dst, count = [], []
+        row_elems, esize = k0.shape[2] * k0.shape[3], k0.element_size()
+        tensors, ends = [], []
         for layer, block in enumerate(kv_cache):
-            ends = {"k": tokens, "v": tokens}
+            tensors += [block["k"], block["v"]]
+            ends += [tokens, tokens]
             if hsa_modules is not None:
                 slots = hsa_modules[layer].token_range_to_coarse(0, tokens)[1] if tokens > 0 else 0
-                ends.update(k_coarse=slots, v_coarse=slots)
-            for name, end in ends.items():
-                t = block[name]
-                rows = t.shape[1] - end
-                if rows <= 0:
-                    continue
-                if not direct or not cls._cache_rows(t, k0):
-                    t[:, end:].zero_()
-                    continue
-                for b in range(t.shape[0]):
-                    dst.append(t.data_ptr() + (b * t.stride(0) + end * row_elems) * t.element_size())
-                    count.append(rows)
-        if not dst:
+                tensors += [block["k_coarse"], block["v_coarse"]]
+                ends += [slots, slots]
+        table, ends = _Table(tensors), np.array(ends, dtype=np.int64)
+        rows = table.size[:, 1] - ends
+        direct = table.cache_rows(table) if cls._copied_by_kernel(k0) else np.zeros(len(rows), dtype=bool)
+        for i in np.flatnonzero((rows > 0) & ~direct):
+            tensors[i][:, int(ends[i]):].zero_()
+        mine = np.flatnonzero((rows > 0) & direct)
+        if mine.size == 0:
             return
-        records = np.zeros(len(dst), dtype=RECORD_DTYPE)
-        records["dst"], records["n_tokens"] = dst, count
-        records["dst_stride"] = row_elems
-        clear_rows_device(to_device(records.view(np.uint8), dev), max_tokens=max(count), row_elems=row_elems, elem_size=k0.element_size())
+        items = np.repeat(mine, table.size[mine, 0])                                     # a record per tensor and batch item
+        batch = np.concatenate([np.arange(n) for n in table.size[mine, 0]])
+        records = np.zeros(len(items), dtype=RECORD_DTYPE)
+        records["dst"] = (table.ptr[items] + (batch * table.stride[items, 0] + ends[items] * row_elems) * esize).astype(np.uint64)
+        records["n_tokens"], records["dst_stride"] = rows[items], row_elems
+        clear_rows_device(to_device(records.view(np.uint8), dev), max_tokens=int(rows[mine].max()), row_elems=row_elems, elem_size=esize)
 
     def _install_sources(self, kv_cache, plan, blobs, dtype):
         """Where the pages come from: `(whole, single, staged_elems)`.
 
-        `whole` maps a chunk that lies on the device in the cache's own layout to the tensors of all layers (its pages are
-        rows of those); `single` lists the pages of every other chunk one by one, as (layer, name, plan row, tensor or host
+        `whole` maps a chunk that lies on the device in the cache's own layout to the tensors of all layers and their table (its
+        pages are rows of those); `single` lists the pages of every other chunk one by one, as (layer, name, plan row, tensor or host
         page, offset in the staging buffer or None), and `staged_elems` is that buffer's size.
         """
         k0 = kv_cache[0]["k"]
         bsz, _, heads, head_dim = k0.shape
         row_elems = heads * head_dim
         _lib.dtype_code(dtype)               # raises for a type that the page-copy kernel does not take
-        for block in kv_cache:
-            for name in ("k", "v"):
-                dst = block[name]
-                if dst.stride(3) != 1 or dst.stride(2) != head_dim or dst.stride(1) != row_elems:
-                    raise ValueError("online cache tensors must be contiguous [B, capacity, H, D]")
+        caches = _Table([block[name] for block in kv_cache for name in ("k", "v")])
+        if (caches.stride[:, 1:] != (row_elems, head_dim, 1)).any():
+            raise ValueError("online cache tensors must be contiguous [B, capacity, H, D]")
         whole = {}
         for chunk_id, held in blobs.items():
             if not callable(held):
                 tensors = [held[name][layer] for layer in range(len(kv_cache)) for name in ("k", "v")]
-                if all(self._cache_rows(t, k0) and t.dtype == dtype and t.shape[0] == bsz for t in tensors):
-                    whole[chunk_id] = tensors
+                table = _Table(tensors)
+                if table.cache_rows(caches).all() and (table.size[:, 0] == bsz).all():
+                    whole[chunk_id] = (tensors, table)
         single, staged_elems = [], 0
         rows = [(i, int(row["chunk"]), int(row["src"]), int(row["count"])) for i, row in enumerate(plan)]
         rows = [row for row in rows if row[3] and row[1] not in whole]
@@ -372,7 +403,7 @@ class HKVCache:
         nt = temporal_complex_dims(head_dim)
         rot = None
         if self.rerope:
-            rot = rotation_table(temporal_freqs, plan["frame_to"].tolist(), plan["frame_from"].tolist(), nt)
+            rot = rotation_table(temporal_freqs(), plan["frame_to"].tolist(), plan["frame_from"].tolist(), nt)
 
         main = torch.cuda.current_stream(dev)
         side = self.tier.side_stream(dev)
@@ -383,12 +414,11 @@ class HKVCache:
         promote = []
         promoted = False
         # first row of every (page, tensor, batch item) on the device, elements between its rows; a tensor is (layer, K|V)
-        tensors = [block[name] for block in kv_cache for name in ("k", "v")]
+        caches = _Table([block[name] for block in kv_cache for name in ("k", "v")])
+        dst = caches.starts(bsz, esize)
         batch = np.arange(bsz, dtype=np.int64) * esize
-        starts = lambda ts: (np.array([t.data_ptr() for t in ts], dtype=np.int64)[:, None]
-                             + np.array([t.stride(0) for t in ts], dtype=np.int64)[:, None] * batch)
-        src = np.zeros((len(plan), len(tensors), bsz), dtype=np.int64)
-        src_stride = np.full((len(plan), len(tensors)), row_elems, dtype=np.int64)
+        src = np.zeros((len(plan),) + dst.shape, dtype=np.int64)
+        src_stride = np.full(src.shape[:2], row_elems, dtype=np.int64)
         for layer, name, i, page, slot in single:
             row = plan[i]
             n = int(row["count"])
@@ -412,9 +442,9 @@ class HKVCache:
             at = 2 * layer + (name == "v")
             src[i, at] = src_ptr + batch * src_batch
             src_stride[i, at] = stride
-        for chunk_id, held in whole.items():
+        for chunk_id, (_, table) in whole.items():
             mine = np.flatnonzero(plan["chunk"] == chunk_id)
-            src[mine] = starts(held) + (plan["src"][mine] * (row_elems * esize))[:, None, None]
+            src[mine] = table.starts(bsz, esize) + (plan["src"][mine] * (row_elems * esize))[:, None, None]
         if promote:
             arr = (_lib.PageCopy * len(promote))(*promote)
             side.wait_stream(main)            # the staging block may be recycled memory that the main stream still uses
@@ -425,10 +455,9 @@ class HKVCache:
         if promoted:
             main.wait_stream(side)
         used = np.flatnonzero(plan["count"] > 0)
-        dst = starts(tensors)
         rot_dev = to_device(rot, dev) if rot is not None else None
         fused = hsa_modules is not None and bool((src_stride[used] == row_elems).all()) and self._install_fused(
-            kv_cache, plan[used], src[used], dst, used if rot is not None else np.full(len(used), -1), rot_dev, nt, dev, hsa_modules)
+            kv_cache, plan[used], src[used], caches, dst, used if rot is not None else np.full(len(used), -1), rot_dev, nt, dev, hsa_modules)
         if not fused:
             records = np.zeros((len(used),) + dst.shape, dtype=RECORD_DTYPE)
             records["src"] = src[used].astype(np.uint64)
@@ -441,13 +470,13 @@ class HKVCache:
             gather_records_device(to_device(records.reshape(-1).view(np.uint8), dev), max_tokens=int(plan["count"].max()), row_elems=row_elems,
                                   head_dim=head_dim, dtype=dtype, rotations=rot_dev, n_temporal=nt)
         storages = {t.untyped_storage().data_ptr(): t for t in keep_alive if t is not None and t.is_cuda}
-        for held in whole.values():
+        for held, _ in whole.values():
             storages.update((t.untyped_storage().data_ptr(), t) for t in held)
         for t in storages.values():
             t.record_stream(main)
         return fused
 
-    def _install_fused(self, kv_cache, plan, src, dst, rot_rows, rot_dev, nt, dev, hsa_modules) -> bool:
+    def _install_fused(self, kv_cache, plan, src, caches, dst, rot_rows, rot_dev, nt, dev, hsa_modules) -> bool:
         """Copy, rotation and compression of all layers in one launch: bf16, pages of whole frames, projection segments of one
         frame, one shape of projection for all layers.  False (nothing launched): not covered."""
         k0 = kv_cache[0]["k"]
@@ -460,25 +489,23 @@ class HKVCache:
         if first.proj_segment_len != frame or shape[1] < frame:
             return False
         slots = first.token_range_to_coarse(0, int(plan["count"].sum()))[1]
-        coarse, proj = [], []
-        for layer, hsa in zip(kv_cache, hsa_modules):
-            kc, vc = layer["k_coarse"], layer["v_coarse"]
-            if hsa.proj_segment_len != frame or hsa.block_size != block or kc.stride() != vc.stride():
-                return False
-            for cache, t, p in ((layer["k"], kc, hsa.k_proj_mat), (layer["v"], vc, hsa.v_proj_mat)):
-                if (cache.dtype != torch.bfloat16 or cache.shape[0] != bsz or t.dtype != torch.bfloat16 or p.dtype != torch.bfloat16
-                        or t.device != dev or p.device != dev or p.shape != shape or not p.is_contiguous() or t.shape[0] < bsz
-                        or t.shape[1] < slots or t.shape[2:] != k0.shape[2:] or t.stride(3) != 1 or t.stride(2) != head_dim):
-                    return False
-                coarse.append(t)
-                proj.append(p)
-        address = lambda ts: np.array([t.data_ptr() for t in ts], dtype=np.uint64)
-        step = lambda ts, dim: np.array([t.stride(dim) for t in ts], dtype=np.int64)
+        if any(hsa.proj_segment_len != frame or hsa.block_size != block for hsa in hsa_modules):
+            return False
+        coarse = _Table([layer[name] for layer in kv_cache for name in ("k_coarse", "v_coarse")])
+        proj = _Table([p for hsa in hsa_modules[: len(kv_cache)] for p in (hsa.k_proj_mat, hsa.v_proj_mat)])
+        if len(proj.ptr) != len(dst) or not (
+                (caches.dtype == caches.dtype[0]).all() and (caches.size[:, 0] == bsz).all() and (coarse.dim == 4).all() and (proj.dim == 2).all()
+                and all((t.dtype == caches.dtype[0]).all() and (t.device == caches.device[0]).all() for t in (coarse, proj))
+                and (proj.size[:, :2] == shape).all() and (proj.stride[:, :2] == (shape[1], 1)).all()
+                and (coarse.stride[::2] == coarse.stride[1::2]).all() and (coarse.size[:, 0] >= bsz).all() and (coarse.size[:, 1] >= slots).all()
+                and (coarse.size[:, 2:] == (heads, head_dim)).all() and (coarse.stride[:, 2:] == (head_dim, 1)).all()):
+            return False
         between = lambda a: np.ascontiguousarray((a[..., 1] - a[..., 0]) // esize if bsz > 1 else np.zeros(a.shape[:-1], dtype=np.int64))
+        whole = lambda a: np.ascontiguousarray(a)
         frames = (plan["count"] // frame).astype(np.int32)
         arrays = dict(page_frames=frames, page_rot=rot_rows.astype(np.int32), src=np.ascontiguousarray(src[..., 0]).astype(np.uint64),
-                      src_batch=between(src), dst=dst[:, 0].astype(np.uint64), dst_batch=between(dst), coarse=address(coarse),
-                      coarse_batch=step(coarse, 0), coarse_row=step(coarse, 1), proj=address(proj))
+                      src_batch=between(src), dst=dst[:, 0].astype(np.uint64), dst_batch=between(dst), coarse=coarse.ptr.astype(np.uint64),
+                      coarse_batch=whole(coarse.stride[:, 0]), coarse_row=whole(coarse.stride[:, 1]), proj=proj.ptr.astype(np.uint64))
         job = _lib.HkvInstall(len(plan), len(dst), int(frames.sum()), bsz, heads, head_dim, frame, block, shape[0], shape[1],
                               nt if rot_dev is not None else 0, *(arrays[n].ctypes.data for n, _ in _lib.HkvInstall._fields_[11:]))
         lib = _lib.lib()
