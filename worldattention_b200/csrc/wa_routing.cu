@@ -926,11 +926,16 @@ __device__ __forceinline__ void route_row(const long long row, const bool logits
                         }
                     }
 #pragma unroll
-                    for (int u = 0; u < QLOADS; ++u)
-                        if (rr[u] >= 0) {
-                            const int n = (c[u].x < thr) + (c[u].y < thr) + (c[u].z < thr) + (c[u].w < thr);
-                            if (n) atomicAdd(&row_count[rr[u]], n);
+                    for (int u = 0; u < QLOADS; ++u) {
+                        const int n = rr[u] >= 0 ? (c[u].x < thr) + (c[u].y < thr) + (c[u].z < thr) + (c[u].w < thr) : 0;
+                        const int first = __shfl_sync(0xffffffffu, rr[u], 0);
+                        if (__all_sync(0xffffffffu, rr[u] == first)) {   // the warp is inside one row: one addition for all lanes
+                            const int all = __reduce_add_sync(0xffffffffu, n);
+                            if (lane == 0 && all) atomicAdd(&row_count[first], all);
+                        } else if (n) {
+                            atomicAdd(&row_count[rr[u]], n);
                         }
+                    }
                 }
             } else {
             const int total = nr * Nkv;   // <= 128 * 16384
@@ -1438,6 +1443,7 @@ int route_fused_launch(const float *q_pooled, const float *k_pooled, int B, int 
     WA_REQUIRE(rows < (1ll << 31), WA_ERR_UNSUPPORTED, "wa_hsa_forward(routing): too many rows");
     int threads = n_pow2 / 2;
     threads = threads < 256 ? 256 : (threads > 1024 ? 1024 : threads);
+    if (n_pow2 == 512) threads = 512;      // a key per thread: 45 passes through shared memory took 13 of a row's 19 us, with shuffles 4
     // a fixed count per head over more key blocks than one pass of the register sort covers, and nobody reads the whole
     // order or the thresholds: select the best blocks instead of sorting all of them
     const int select_only = fixed_num_per_head && !whole_order && n_pow2 > threads;
