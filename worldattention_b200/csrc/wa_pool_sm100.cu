@@ -7,7 +7,10 @@
 // item, each thread two neighbouring columns of it, so no sum crosses a thread.  The rows are added in float64:
 // a sum of a few hundred bf16 values is exact there, so the pooled value, and the discrete routing decision that
 // is taken on it, do not depend on the order of the additions.  The float64 conversion is what bounds the
-// arithmetic (16 per clock per SM); three groups with four boxes in flight each measured fastest (22.5 us for 100 MB, 4.5 TB/s).
+// arithmetic (16 per clock per SM); three groups with four boxes in flight each measured fastest (22.5 us for 100 MB, 4.5 TB/s),
+// four groups with three boxes for long inputs (2.3 GB: 430 -> 393 us, 5.9 TB/s; six with two 401; boxes of 16 rows 500).  Taken
+// back: odd columns added up as shifted bits instead of converted (fewer conversions, more registers and integer
+// instructions: 424 us).
 #include "wa_internal.cuh"
 #include "wa_sm100_ptx.cuh"
 
@@ -18,18 +21,15 @@ namespace pool {
 constexpr int COLS = 256;            // columns of a work item: one 512-byte row piece per token
 constexpr int SUB_ROWS = 32;         // token rows of one TMA box: 16 KB
 constexpr int STAGE_BYTES = SUB_ROWS * COLS * 2;
-#ifndef WA_POOLT_GROUPS
-#define WA_POOLT_GROUPS 3
-#endif
-constexpr int GROUPS = WA_POOLT_GROUPS, GROUP_THREADS = COLS / 2;   // a thread owns two neighbouring columns of its group's item
-constexpr int THREADS = 32 + GROUPS * GROUP_THREADS;                // warp 0 issues the loads
+constexpr int GROUP_THREADS = COLS / 2;             // a thread owns two neighbouring columns of its group's item
+constexpr int BOXES = 12;                                           // in flight per CTA
+constexpr int threads_of(int groups) { return 32 + groups * GROUP_THREADS; }   // warp 0 issues the loads
 // Every group has a ring of its own.  With one ring shared by all groups a group could be asked for a box two laps
 // ahead of a slower group's, and a phase-parity wait cannot tell "two laps behind" from "done".
-constexpr int STAGES = 12 / GROUPS;                                 // boxes in flight per group
-constexpr int SMEM_BYTES = GROUPS * STAGES * STAGE_BYTES + 1024;
+constexpr int SMEM_BYTES = BOXES * STAGE_BYTES + 1024;
 
 struct Barriers {
-    uint64_t full[GROUPS][STAGES], empty[GROUPS][STAGES];
+    uint64_t full[BOXES], empty[BOXES];      // [group][stage]
     int abort_flag;
 };
 
@@ -47,19 +47,21 @@ __device__ int g_status;
 
 // The row pieces of a box are 512 bytes wide on purpose: the copy engine issues one request per row piece, and with
 // 128-byte pieces (64 columns) that request rate, not HBM, bounded the stream at 2.7 TB/s.
-__global__ void __launch_bounds__(THREADS, 1)
+template <int GROUPS>
+__global__ void __launch_bounds__(threads_of(GROUPS), 1)
 pool_stream_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constant__ CUtensorMap tm_y, const Job job) {
+    constexpr int STAGES = BOXES / GROUPS, THREADS = threads_of(GROUPS);   // boxes in flight per group
     extern __shared__ __align__(1024) uint8_t smem[];
-    Barriers *bar = reinterpret_cast<Barriers *>(smem + GROUPS * STAGES * STAGE_BYTES);
+    Barriers *bar = reinterpret_cast<Barriers *>(smem + BOXES * STAGE_BYTES);
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     volatile int *abort_flag = &bar->abort_flag;
     const FailSink sink{job.status, job.status_mirror};
 
     if (threadIdx.x == 0) {
         bar->abort_flag = 0;
-        for (int i = 0; i < GROUPS * STAGES; ++i) {
-            mbar_init(&bar->full[0][i], 1);
-            mbar_init(&bar->empty[0][i], GROUP_THREADS / 32);   // one arrival per warp of the group that read the box
+        for (int i = 0; i < BOXES; ++i) {
+            mbar_init(&bar->full[i], 1);
+            mbar_init(&bar->empty[i], GROUP_THREADS / 32);   // one arrival per warp of the group that read the box
         }
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
@@ -83,10 +85,10 @@ pool_stream_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_consta
                 const uint32_t g = n_item % GROUPS;
                 for (int sub = 0; sub < subs; ++sub) {
                     const uint32_t count = (n_item / GROUPS) * subs + sub, s = count % STAGES;
-                    if (!mbar_wait(&bar->empty[g][s], ((count / STAGES) & 1u) ^ 1u, abort_flag, sink, 201)) return;   // 201, 202: wait sites of this kernel in the status word
-                    mbar_expect_tx(&bar->full[g][s], (uint32_t)STAGE_BYTES);
+                    if (!mbar_wait(&bar->empty[g * STAGES + s], ((count / STAGES) & 1u) ^ 1u, abort_flag, sink, 201)) return;   // 201, 202: wait sites of this kernel in the status word
+                    mbar_expect_tx(&bar->full[g * STAGES + s], (uint32_t)STAGE_BYTES);
                     // rows past the end of the tensor arrive as zeros
-                    tma_load_3d(smem + (g * STAGES + s) * STAGE_BYTES, second ? &tm_y : &tm_x, &bar->full[g][s], ct * COLS,
+                    tma_load_3d(smem + (g * STAGES + s) * STAGE_BYTES, second ? &tm_y : &tm_x, &bar->full[g * STAGES + s], ct * COLS,
                                 nb * job.block_size + sub * SUB_ROWS, b);
                 }
             }
@@ -107,7 +109,7 @@ pool_stream_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_consta
         bool ok = true;
         for (int sub = 0; sub < subs; ++sub) {
             const uint32_t count = (n_item / GROUPS) * subs + sub, s = count % STAGES;
-            ok = mbar_wait(&bar->full[gid][s], (count / STAGES) & 1u, abort_flag, sink, 202);
+            ok = mbar_wait(&bar->full[gid * STAGES + s], (count / STAGES) & 1u, abort_flag, sink, 202);
             if (!ok) break;
             const uint32_t *box = reinterpret_cast<const uint32_t *>(smem + (gid * STAGES + s) * STAGE_BYTES) + t;
 #pragma unroll
@@ -122,7 +124,7 @@ pool_stream_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_consta
                 }
             }
             __syncwarp();
-            if (lane == 0) mbar_arrive(&bar->empty[gid][s]);
+            if (lane == 0) mbar_arrive(&bar->empty[gid * STAGES + s]);
         }
         if (!ok) break;
         const double s0 = (lo[0] + lo[1]) + (lo[2] + lo[3]), s1 = (hi[0] + hi[1]) + (hi[2] + hi[3]);
@@ -198,7 +200,8 @@ int pool_sm100_launch(const wa_tensor4 *x, int Lx, float *px, const wa_tensor4 *
     if (!y) ty = tx;
     static PerDeviceOnce attr_set;
     if (!attr_set.done()) {
-        cudaError_t e = cudaFuncSetAttribute(pool_stream_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES);
+        cudaError_t e = cudaFuncSetAttribute(pool_stream_kernel<3>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES);
+        if (e == cudaSuccess) e = cudaFuncSetAttribute(pool_stream_kernel<4>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES);
         if (e != cudaSuccess) return fail((int)e, "%s: %s", what, cudaGetErrorString(e));
         attr_set.mark();
     }
@@ -218,7 +221,11 @@ int pool_sm100_launch(const wa_tensor4 *x, int Lx, float *px, const wa_tensor4 *
     const long long items = (long long)B * (job.nbx + job.nby) * job.tiles;
     WA_REQUIRE(items < (1ll << 40), WA_ERR_UNSUPPORTED, "%s: too many blocks", what);
     const int grid = items < sms ? (int)items : sms;
-    const cudaError_t le = launch_dependent(pool_stream_kernel, dim3(grid), dim3(THREADS), SMEM_BYTES, stream, tx, ty, job);
+    // The fourth group pays where the stream is long: 480 frames, the whole call, 1126 -> 1100 us; over a window of 21 (115 MB) the call is
+    // 4 % slower with it and over three frames 1 %, the next launch finding less room beside it.
+    const bool four = (long long)B * (Lx + (y ? Ly : 0)) * H * D * 2 > (512ll << 20);
+    const cudaError_t le = four ? launch_dependent(pool_stream_kernel<4>, dim3(grid), dim3(threads_of(4)), SMEM_BYTES, stream, tx, ty, job)
+                                : launch_dependent(pool_stream_kernel<3>, dim3(grid), dim3(threads_of(3)), SMEM_BYTES, stream, tx, ty, job);
     if (le != cudaSuccess) return fail((int)le, "%s: %s", what, cudaGetErrorString(le));
     return check_launch(what);
 }
