@@ -354,11 +354,11 @@ class HKVCache:
         clear_rows_device(to_device(records.view(np.uint8), dev), max_tokens=int(rows[mine].max()), row_elems=row_elems, elem_size=esize)
 
     def _install_sources(self, kv_cache, plan, blobs, dtype):
-        """Where the pages come from: `(whole, single, staged_elems)`.
+        """Where the pages come from: `(whole, single, staging)`; cold pages are on their way to the staging buffer.
 
         `whole` maps a chunk that lies on the device in the cache's own layout to the tensors of all layers and their table (its
         pages are rows of those); `single` lists the pages of every other chunk one by one, as (layer, name, plan row, tensor or host
-        page, offset in the staging buffer or None), and `staged_elems` is that buffer's size.
+        page, offset in the staging buffer or None).
         """
         k0 = kv_cache[0]["k"]
         bsz, _, heads, head_dim = k0.shape
@@ -388,14 +388,34 @@ class HKVCache:
                         slot = staged_elems                      # cold page in the cache's own layout: one block copy per item
                         staged_elems += bsz * n * row_elems
                     single.append((layer, name, i, page, slot))
-        return whole, single, staged_elems
+        return whole, single, self._promote(single, staged_elems, k0) if staged_elems else None
+
+    def _promote(self, single, staged_elems: int, k0: torch.Tensor) -> torch.Tensor:
+        """Cold pages in the cache's own layout cross on the side stream into ONE staging buffer, one block copy per item: the first
+        thing that is launched, since the link is what a cold install waits for."""
+        dev = k0.device
+        bsz, _, heads, head_dim = k0.shape
+        row_elems, esize = heads * head_dim, k0.element_size()
+        staging = torch.empty((staged_elems,), dtype=k0.dtype, device=dev)
+        promote = []
+        for _, _, _, page, slot in single:
+            if slot is not None:
+                n = page.shape[1]
+                promote += [_lib.PageCopy(page.data_ptr() + b * page.stride(0) * esize, staging.data_ptr() + (slot + b * n * row_elems) * esize,
+                                          row_elems, row_elems, n, -1) for b in range(bsz)]
+        main, side = torch.cuda.current_stream(dev), self.tier.side_stream(dev)
+        side.wait_stream(main)            # the staging block may be recycled memory that the main stream still uses
+        staging.record_stream(side)
+        with _lib.device_guard(dev):
+            _lib.check(_lib.lib().wa_hkv_promote_pages((_lib.PageCopy * len(promote))(*promote), len(promote), row_elems, esize, side.cuda_stream))
+        return staging
 
     def _install(self, kv_cache, plan, sources, temporal_freqs, dev, dtype, hsa_modules=None) -> bool:
         """The plan's pages into the caches of all layers in one launch.
 
         With `hsa_modules` and where the fused kernel covers the call, the compressed slots are written by that launch too
         (True); otherwise one page-copy launch for every (layer, page, K|V, batch item) (False)."""
-        whole, single, staged_elems = sources
+        whole, single, staging = sources
         k0 = kv_cache[0]["k"]
         bsz, _, heads, head_dim = k0.shape
         row_elems = heads * head_dim
@@ -407,12 +427,10 @@ class HKVCache:
 
         main = torch.cuda.current_stream(dev)
         side = self.tier.side_stream(dev)
-        # cold pages cross on the side stream into ONE staging buffer; whatever conversion a page needs runs on that stream too,
-        # behind its copy, so that nothing reads a landing buffer early
-        staging = torch.empty((max(staged_elems, 1),), dtype=dtype, device=dev) if staged_elems else None
+        # whatever conversion a cold page needs runs on the side stream too, behind its copy, so that nothing reads a landing
+        # buffer early
         keep_alive = [staging]
-        promote = []
-        promoted = False
+        promoted = staging is not None
         # first row of every (page, tensor, batch item) on the device, elements between its rows; a tensor is (layer, K|V)
         caches = _Table([block[name] for block in kv_cache for name in ("k", "v")])
         dst = caches.starts(bsz, esize)
@@ -424,10 +442,6 @@ class HKVCache:
             n = int(row["count"])
             if slot is not None:
                 src_ptr, src_batch, stride = staging.data_ptr() + slot * esize, n * row_elems, row_elems
-                for b in range(bsz):
-                    promote.append(_lib.PageCopy(page.data_ptr() + b * page.stride(0) * esize,
-                                                 src_ptr + b * src_batch * esize, row_elems, row_elems, n, -1))
-                keep_alive.append(page)
             else:
                 if not page.is_cuda:
                     with torch.cuda.stream(side):
@@ -445,13 +459,6 @@ class HKVCache:
         for chunk_id, (_, table) in whole.items():
             mine = np.flatnonzero(plan["chunk"] == chunk_id)
             src[mine] = table.starts(bsz, esize) + (plan["src"][mine] * (row_elems * esize))[:, None, None]
-        if promote:
-            arr = (_lib.PageCopy * len(promote))(*promote)
-            side.wait_stream(main)            # the staging block may be recycled memory that the main stream still uses
-            staging.record_stream(side)
-            with _lib.device_guard(dev):
-                _lib.check(_lib.lib().wa_hkv_promote_pages(arr, len(promote), row_elems, esize, side.cuda_stream))
-            promoted = True
         if promoted:
             main.wait_stream(side)
         used = np.flatnonzero(plan["count"] > 0)
