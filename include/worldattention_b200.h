@@ -360,6 +360,12 @@ int wa_hkv_build_records(const int32_t *top_ids, int layers, int heads, int topk
  * the installed rows of all layers, in one launch.  max_tokens: the largest n_tokens of the records; elem_size 2 or 4. */
 int wa_hkv_clear_rows(const wa_page_copy *rows, int n, int max_tokens, int row_elems, int elem_size, void *stream);
 
+/* Mean of `x` [B, tokens, D] (float32 or bf16, strides in elements) over the tokens, then over the batch, divided by its
+ * length (at least 1e-12): `out` [D] float32 (prompt_index, retrieval.py:32-38).  WA_ERR_UNSUPPORTED: D no multiple of 8, or rows
+ * that are not 16-byte aligned. */
+int wa_hkv_prompt_index(const void *x, int dtype, int B, int tokens, int D, int64_t stride_b, int64_t stride_t, float *out,
+                        void *stream);
+
 /* Install of pages of whole frames into the caches of all layers, fused with the compression of what is installed
  * (cache.py:229-254 and compress_kv, attention.py:64-110): bf16, rows of H*D contiguous values, projection segments of
  * one frame.  A tensor is one layer's K or V (layer * 2 + (0 K | 1 V)); the arrays are host arrays.  `wa_hkv_install_table`

@@ -1,0 +1,21 @@
+"""The prompt index in two launches against float64, and the tensor expressions it leaves other layouts to."""
+import pytest
+import torch
+
+from tests.helpers import dev
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("b,tokens,dim", [(1, 512, 4096), (1, 1, 8), (2, 31, 72), (3, 257, 1528), (1, 300, 12)])
+def test_prompt_index(dtype, b, tokens, dim):
+    from worldattention_b200.hkv.retrieval import prompt_index
+    g = torch.Generator(device=dev()).manual_seed(dim)
+    x = torch.randn((b, tokens + 2, dim), generator=g, device=dev()).to(dtype)
+    for t in (x[:, :tokens], x[:, 2:], x.transpose(1, 2).contiguous().transpose(1, 2)[:, :tokens]):
+        mean = t.double().mean(1).mean(0)
+        # the means are rounded to float32 (2^-24 of the largest value of a column's terms), the quotient once more
+        assert float((prompt_index(t).double() - mean / mean.norm()).abs().max()) < 2e-6
+    zero = prompt_index(torch.zeros(1, 4, 16, device=dev(), dtype=dtype))
+    assert not zero.any() and bool(prompt_index(torch.full((1, 4, 16), float("nan"), device=dev(), dtype=dtype)).isnan().all())

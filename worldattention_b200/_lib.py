@@ -102,6 +102,7 @@ SIGNATURES = {
     "wa_hkv_build_records": [_vp, _i, _i, _i, _vp, _i, C.c_longlong, C.c_longlong, _vp, C.c_longlong, C.c_longlong,
                              _i, _i, _i, _i, _vp, _vp, _vp],
     "wa_hkv_promote_pages": [_vp, _i, _i, _i, _vp],
+    "wa_hkv_prompt_index": [_vp, _i, _i, _i, _i, _i64, _i64, _vp, _vp],
     "wa_hkv_install_table_bytes": [_i, _i, _i],
     "wa_hkv_install_table": [_vp, _vp, C.c_size_t],
     "wa_hkv_install_pages": [_vp, _vp, _vp, _vp],

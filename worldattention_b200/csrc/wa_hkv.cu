@@ -207,6 +207,83 @@ page_centroid_vec_kernel(const __nv_bfloat16 *__restrict__ keys, long long sb, l
 }
 
 // ------------------------------------------------------------------------------------------------
+// Prompt index: mean over the tokens, then over the batch, then a unit vector (prompt_index, pipeline/hkv/retrieval.py:32-38).
+// A CTA of the first kernel takes 64 columns, eight threads of 16 bytes (8 bf16 or two times 4 float32) across and 32 tokens at
+// a time, eight loads in flight each; the second is one CTA over the pooled vector.  Float64 sums, each mean rounded once to
+// float32.  As tensor expressions these are six launches and a float32 copy of the tokens: 512 x 4096 bf16 33 us, here 12 + 2.
+// ------------------------------------------------------------------------------------------------
+constexpr int PI_COLS = 64, PI_ROWS = 32, PI_FLIGHT = 8;
+
+template <typename T>
+__global__ void __launch_bounds__(256)
+prompt_mean_kernel(const T *__restrict__ x, long long sb, long long st, int B, int tokens, int D, float *__restrict__ out) {
+    constexpr int VE = 16 / sizeof(T), PER = 8 / VE;             // values of a load; loads that make a thread's eight columns
+    __shared__ double part[PI_ROWS][PI_COLS + 2];
+    const int cx = threadIdx.x & 7, ty = threadIdx.x >> 3, col = blockIdx.x * PI_COLS + cx * 8;
+    double total = 0.0;                                          // of column threadIdx.x, over the batch
+    for (int b = 0; b < B; ++b) {
+        double acc[8] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
+        if (col < D) {
+            const T *base = x + b * sb + col;
+            for (int t0 = ty; t0 < tokens; t0 += PI_ROWS * PI_FLIGHT) {
+                uint4 v[PI_FLIGHT][PER];
+#pragma unroll
+                for (int u = 0; u < PI_FLIGHT; ++u)
+#pragma unroll
+                    for (int i = 0; i < PER; ++i)
+                        v[u][i] = t0 + u * PI_ROWS < tokens ? __ldg(reinterpret_cast<const uint4 *>(base + (t0 + u * PI_ROWS) * st + i * VE))
+                                                            : make_uint4(0u, 0u, 0u, 0u);
+#pragma unroll
+                for (int u = 0; u < PI_FLIGHT; ++u)
+#pragma unroll
+                    for (int i = 0; i < PER; ++i) {
+                        const uint32_t w[4] = {v[u][i].x, v[u][i].y, v[u][i].z, v[u][i].w};
+#pragma unroll
+                        for (int e = 0; e < 4; ++e) {
+                            if (sizeof(T) == 2) {
+                                acc[2 * e] += (double)__uint_as_float(w[e] << 16);
+                                acc[2 * e + 1] += (double)__uint_as_float(w[e] & 0xffff0000u);
+                            } else {
+                                acc[i * 4 + e] += (double)__uint_as_float(w[e]);
+                            }
+                        }
+                    }
+            }
+        }
+#pragma unroll
+        for (int e = 0; e < 8; ++e) part[ty][cx * 8 + e] = acc[e];
+        __syncthreads();
+        if (threadIdx.x < PI_COLS) {
+            double sum = 0.0;
+            for (int y = 0; y < PI_ROWS; ++y) sum += part[y][threadIdx.x];
+            total += (double)(float)(sum / (double)tokens);
+        }
+        __syncthreads();
+    }
+    if (threadIdx.x < PI_COLS && blockIdx.x * PI_COLS + threadIdx.x < D) out[blockIdx.x * PI_COLS + threadIdx.x] = (float)(total / (double)B);
+}
+
+__global__ void __launch_bounds__(1024)
+unit_vector_kernel(float *__restrict__ x, int D) {
+    __shared__ double red[32];
+    __shared__ float length;
+    pdl_wait();
+    double sq = 0.0;
+    for (int d = threadIdx.x; d < D; d += 1024) sq += (double)x[d] * (double)x[d];
+    sq = warp_sum_d(sq);
+    if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = sq;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        double t = 0.0;
+        for (int w = 0; w < 32; ++w) t += red[w];
+        const float norm = (float)sqrt(t);
+        length = norm < 1e-12f ? 1e-12f : norm;
+    }
+    __syncthreads();
+    for (int d = threadIdx.x; d < D; d += 1024) x[d] = __fdiv_rn(x[d], length);
+}
+
+// ------------------------------------------------------------------------------------------------
 // Page scores and top-k.  One CTA per score group (1 = whole vector, H = per head).
 // ------------------------------------------------------------------------------------------------
 constexpr int ST_THREADS = 256;
@@ -575,6 +652,24 @@ extern "C" int wa_hkv_page_centroids(const wa_tensor4 *keys, int B, int T, int H
     page_centroid_kernel<<<grid, block, 0, (cudaStream_t)stream>>>(
         make_view(keys), B, H, D, spans, reinterpret_cast<const float2 *>(derope), n_frames, n_temporal,
         frame_seq_length, page_index);
+    return check_launch(what);
+}
+
+extern "C" int wa_hkv_prompt_index(const void *x, int dtype, int B, int tokens, int D, int64_t stride_b, int64_t stride_t, float *out, void *stream) {
+    const char *what = "wa_hkv_prompt_index";
+    WA_REQUIRE(x && out, WA_ERR_ARG, "%s: null pointer", what);
+    WA_REQUIRE(valid_dtype(dtype) && B > 0 && tokens > 0 && D > 0, WA_ERR_ARG, "%s: bad type or sizes", what);
+    const int per = dtype == WA_BF16 ? 8 : 4;
+    WA_REQUIRE(D % 8 == 0 && (uintptr_t)x % 16 == 0 && (B == 1 || stride_b % per == 0) && stride_t % per == 0, WA_ERR_UNSUPPORTED,
+               "%s: rows of a multiple of eight values, 16-byte aligned", what);
+    const unsigned grid = (unsigned)ceil_div(D, PI_COLS);
+    if (dtype == WA_BF16)
+        prompt_mean_kernel<<<grid, 256, 0, (cudaStream_t)stream>>>((const __nv_bfloat16 *)x, (long long)stride_b, (long long)stride_t, B, tokens, D, out);
+    else
+        prompt_mean_kernel<<<grid, 256, 0, (cudaStream_t)stream>>>((const float *)x, (long long)stride_b, (long long)stride_t, B, tokens, D, out);
+    if (const int rc = check_launch(what)) return rc;
+    const cudaError_t e = launch_dependent(unit_vector_kernel, dim3(1), dim3(1024), 0, (cudaStream_t)stream, out, D);
+    if (e != cudaSuccess) return fail((int)e, "%s: %s", what, cudaGetErrorString(e));
     return check_launch(what);
 }
 

@@ -22,6 +22,18 @@ __all__ = ["prompt_index", "query_index", "page_key_index", "score_pages", "sele
 
 def prompt_index(prompt_embeds: torch.Tensor) -> torch.Tensor:
     """Mean-pool `[B, tokens, dim]` into a unit vector `[dim]` (retrieval.py:32-38)."""
+    if (type(prompt_embeds) is torch.Tensor and prompt_embeds.is_cuda and prompt_embeds.dim() == 3 and prompt_embeds.numel() > 0
+            and prompt_embeds.dtype in (torch.float32, torch.bfloat16) and prompt_embeds.stride(2) == 1
+            and not (torch.is_grad_enabled() and prompt_embeds.requires_grad)):
+        bsz, tokens, dim = prompt_embeds.shape
+        out = torch.empty((dim,), device=prompt_embeds.device, dtype=torch.float32)
+        with _lib.device_guard(prompt_embeds.device):
+            rc = _lib.lib().wa_hkv_prompt_index(prompt_embeds.data_ptr(), _lib.dtype_code(prompt_embeds.dtype), bsz, tokens, dim,
+                                                prompt_embeds.stride(0), prompt_embeds.stride(1), out.data_ptr(),
+                                                _lib.stream_ptr(prompt_embeds.device))
+        if rc != _lib.WA_ERR_UNSUPPORTED:
+            _lib.check(rc)
+            return out
     pooled = prompt_embeds.float().mean(dim=1).mean(dim=0)
     return F.normalize(pooled, dim=0)
 
