@@ -163,7 +163,7 @@ int pool_launch(const wa_tensor4 *x, int Lx, float *px, const wa_tensor4 *y, int
                 int block_size, cudaStream_t stream, int *zero = nullptr, int n_zero = 0, int y_first_block = 0,
                 int *status_mirror = nullptr);   // host-visible word that receives a non-zero code if a bounded wait of the TMA kernel runs out
 
-// routing (wa_routing.cu): scores, sort, Gini thresholds and counts in ONE launch (plus `job` when its order is set).
+// routing (wa_routing.cu): scores, sort, Gini thresholds and counts, in one launch or, with many logits, two (plus `job` when its order is set).
 // `sorted` ([rows, Nkv] float32) and `gini` ([rows]) are scratch; `counters` are H + 1 ints that are zero on entry.
 int route_fused_launch(const float *q_pooled, const float *k_pooled, int B, int H, int Nq, int Nkv, int D, double tau_min,
                        double tau_max, const int32_t *fixed_num_per_head, float *sorted, int32_t *index, int32_t *num,

@@ -587,8 +587,8 @@ route_count_kernel(const float *__restrict__ attn, const int32_t *__restrict__ i
 }
 
 // ------------------------------------------------------------------------------------------------
-// The forward's routing in ONE launch.  Each CTA owns a (batch, head, query block) row: scores,
-// softmax, sort and the row's Gini term, with the probabilities kept in shared memory.  The CTA that
+// The forward's routing, a CTA per (batch, head, query block) row (route_row, route_fused_kernel): scores where
+// route_logits_kernel has not left them, softmax, sort and the row's Gini term, with the probabilities kept in shared memory.  The CTA that
 // finishes a head last (a counter per head) turns the head's Gini rows into its threshold and counts
 // every row of that head, a warp per row over the sorted probabilities; the CTA that finishes the
 // last head prepares the attention kernel's launch (work order, counters).  Same arithmetic as the
