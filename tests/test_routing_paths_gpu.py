@@ -21,7 +21,8 @@ def _inputs(b, h, lq, lkv, seed, spread=1.0):
                                         (1, 40, 1, 1700), (1, 2, 97, 513), (1, 1, 15, 4096), (1, 1, 2, 128),
                                         # short rows: a CTA per head, one, two or four keys per lane, and just beyond
                                         (1, 3, 1, 1), (2, 3, 7, 19), (1, 2, 37, 37), (1, 2, 64, 128), (2, 2, 32, 64), (1, 1, 16, 8), (1, 2, 33, 33),
-                                        (4, 2, 16, 127), (1, 2, 65, 40), (1, 2, 64, 129)])
+                                        (4, 2, 16, 127), (4, 2, 8, 127), (1, 2, 32, 128), (1, 2, 33, 80), (1, 2, 64, 64),
+                                        (1, 2, 65, 40), (1, 2, 64, 129)])
 @pytest.mark.parametrize("ragged", [0, 3])
 def test_forward_routing_equals_the_separate_functions(b, h, nq, nkv, ragged):
     from worldattention_b200.hsa import routing as R

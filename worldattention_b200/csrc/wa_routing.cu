@@ -1026,8 +1026,8 @@ route_fused_kernel(const float *__restrict__ qp, const float *__restrict__ kp, i
 }
 
 // ------------------------------------------------------------------------------------------------
-// The whole routing of short rows (head_dim 128, up to 128 key blocks and 64 query blocks of a head over the batch): a CTA per
-// head.  There the kernel above is a chain of waits: some twenty barriers of a row, a counter per head, the last CTA's walk
+// The whole routing of short rows (head_dim 128, up to 64 query blocks of a head over the batch and 64 key blocks, or 128 where one
+// round of the CTA's warps does): a CTA per head.  There the kernel above is a chain of waits: some twenty barriers of a row, a counter per head, the last CTA's walk
 // over all rows of the head, a second counter.  Here the logits come from the float64 matrix instruction, a 16 x 8 tile per
 // warp, a row's softmax, sort and sums stay inside a warp (K keys per lane, exchanges by shuffles), and the head's threshold
 // and counts need two barriers.  Same sums (float64, rounded where the reference rounds) and the same order.
@@ -1468,8 +1468,11 @@ int route_fused_launch(const float *q_pooled, const float *k_pooled, int B, int 
     const float scale = (float)pow((double)D, -0.5), span = (float)(tau_max - tau_min);
     const long long bh = (long long)B * H;
 
-    // A CTA takes 32 rows at a time and a row is a warp's work, so the line lies where that is no longer the shorter way.
-    if (D == 128 && Nkv <= RH_MAX_KEYS && (long long)B * Nq <= RH_MAX_ROWS && ((uintptr_t)q_pooled % 16 == 0) && ((uintptr_t)k_pooled % 16 == 0)) {
+    // A CTA takes 32 rows and 32 tiles of logits at a time.  Two rounds of rows pay up to 64 keys (37 rows over 37: 16.5 us against 22.6);
+    // beyond, one round of rows or of tiles does (25 rows over 74: 14.7 against 20; whole calls: 37 over 74 144.9 against 147.8,
+    // but 37 over 110, two rounds of both, 108.7 against 101.6).
+    const bool one_round = (long long)B * Nq <= RH_WARPS || (long long)B * ((Nq + 15) / 16) * ((Nkv + 7) / 8) <= RH_WARPS;
+    if (D == 128 && Nkv <= RH_MAX_KEYS && (long long)B * Nq <= RH_MAX_ROWS && (Nkv <= 64 || one_round) && ((uintptr_t)q_pooled % 16 == 0) && ((uintptr_t)k_pooled % 16 == 0)) {
         const auto launch = [&](auto width) -> cudaError_t {
             constexpr int K = decltype(width)::value, BYTES = RH_MAX_ROWS * K * 32 * (int)sizeof(float);
             const auto kernel = route_head_kernel<K>;
