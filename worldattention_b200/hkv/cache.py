@@ -489,7 +489,7 @@ class HKVCache:
         k0 = kv_cache[0]["k"]
         bsz, _, heads, head_dim = k0.shape
         frame, esize = self.frame_seq_length, k0.element_size()
-        if k0.dtype != torch.bfloat16 or (plan["count"] % frame).any() or (plan["src"] % frame).any():
+        if k0.dtype != torch.bfloat16 or kv_cache[0]["k_coarse"].dtype != torch.bfloat16 or (plan["count"] % frame).any() or (plan["src"] % frame).any():
             return False
         first = hsa_modules[0]
         shape, block = first.k_proj_mat.shape, first.block_size
