@@ -177,6 +177,12 @@ def dtype_code(dtype: torch.dtype) -> int:
     raise ValueError(f"worldattention_b200 kernels take float32 or bfloat16 tensors, got {dtype}")
 
 
+def is_plain(t) -> bool:
+    """A tensor whose memory stands for it: no subclass, no wrapper of a function transform (vmap, jvp, grad) and, outside a
+    forward-mode level, no tangent."""
+    return type(t) is torch.Tensor and not torch._C._functorch.is_functorch_wrapped_tensor(t) and torch.autograd.forward_ad._current_level < 0
+
+
 def require_cuda(*tensors: torch.Tensor) -> torch.device:
     dev = None
     for t in tensors:
