@@ -26,3 +26,19 @@ def test_rows_of_every_width(c):
     # the same rounding points; float32 statistics in another order put a normalised value at most one bf16 step away, whose
     # product with 1 + scale (below 4 here) is rounded again: two steps of the largest value
     assert float(diff.max()) <= 2 * 2 ** -8 * float(want.abs().max()) and float((diff > 0).float().mean()) < 0.02
+
+
+def test_a_modulation_holds_a_vector_for_every_frame():
+    """The kernels take the vector of row / tokens_per_frame: rows behind the last frame are refused, not read with what lies there."""
+    from worldattention_b200.causal_dit import gated_residual, ln_modulate
+    dev = torch.device("cuda:0")
+    x, e = torch.randn(1, 33, 64, device=dev).bfloat16(), torch.randn(1, 3, 1, 64, device=dev).bfloat16()
+    for tokens in (10, 1):
+        for call in (lambda: ln_modulate(x, 1e-6, scale=e, tokens_per_frame=tokens), lambda: ln_modulate(x, 1e-6, shift=e, tokens_per_frame=tokens),
+                     lambda: gated_residual(x, x, e, tokens_per_frame=tokens)):
+            with pytest.raises(ValueError, match="frames"):
+                call()
+    with pytest.raises(ValueError, match="modulation"):
+        gated_residual(x, x, e[..., :56], tokens_per_frame=11)
+    gated_residual(x, x, e, tokens_per_frame=11)
+    gated_residual(x, x, e, tokens_per_frame=40)             # frames that no row reaches

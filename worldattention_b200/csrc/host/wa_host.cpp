@@ -423,13 +423,16 @@ PyObject *append_kv(PyObject *const *a, Py_ssize_t n) {
 
 // ---- the element-wise steps of a block (causal_dit.py) ------------------------------------------
 // `[B, F, 1, C]` or `[B, F, C]` modulation view -> (pointer, elements between consecutive frames); it must step uniformly
-// over (b, f)
-const void *frame_vectors(const Tensor *e, int64_t dim, Tensor &keep, long long &stride) {
+// over (b, f) and hold a vector for every `tokens` of the `rows` rows: the kernels take the vector of row / tokens
+const void *frame_vectors(const Tensor *e, int64_t rows, int64_t tokens, int64_t dim, Tensor &keep, long long &stride) {
     if (!e) return nullptr;
     const Tensor *t = e;
-    if (e->dim() < 2) fail(PyExc_ValueError, "expected a [B, F, 1, C] or [B, F, C] modulation, got shape " + shape_of(*e));
+    if (e->dim() < 3 || e->size(-1) < dim) fail(PyExc_ValueError, "expected a [B, F, 1, C] or [B, F, C] modulation, got shape " + shape_of(*e));
     const int64_t b = e->size(0), f = e->size(1);
-    if (e->stride(-1) != 1 || e->size(-1) != dim || (b > 1 && e->stride(0) != f * e->stride(1))) {
+    if (tokens > 0 && (rows + tokens - 1) / tokens > b * f)
+        fail(PyExc_ValueError, std::to_string(rows) + " rows of " + std::to_string(tokens) + " tokens per frame need more than the modulation's " +
+                                   std::to_string(b * f) + " frames");
+    if (e->stride(-1) != 1 || (b > 1 && e->stride(0) != f * e->stride(1))) {
         keep = e->contiguous();
         t = &keep;
     }
@@ -459,10 +462,11 @@ PyObject *ln_modulate(PyObject *const *a, Py_ssize_t n) {
     const Tensor *w = tensor_or_null(a[2], "weight"), *b = tensor_or_null(a[3], "bias");
     const Tensor *scale = tensor_or_null(a[4], "scale"), *shift = tensor_or_null(a[5], "shift");
     long long ss = 0, hs = 0;
-    const void *sp = frame_vectors(scale, c, keep[1], ss), *hp = frame_vectors(shift, c, keep[2], hs);
+    const int64_t rows = c ? x.numel() / c : 0, tokens = (int)integer(a[6]);
+    const void *sp = frame_vectors(scale, rows, tokens, c, keep[1], ss), *hp = frame_vectors(shift, rows, tokens, c, keep[2], hs);
     if (sp && hp && ss != hs) fail(PyExc_ValueError, "scale and shift must share a layout");
-    check(f_ln(x.data_ptr(), out.data_ptr(), c ? x.numel() / c : 0, (int)c, (float)real(a[1]), w ? w->data_ptr() : nullptr, b ? b->data_ptr() : nullptr,
-               sp, hp, ss ? ss : hs, (int)integer(a[6]), stream));
+    check(f_ln(x.data_ptr(), out.data_ptr(), rows, (int)c, (float)real(a[1]), w ? w->data_ptr() : nullptr, b ? b->data_ptr() : nullptr,
+               sp, hp, ss ? ss : hs, (int)tokens, stream));
     return THPVariable_Wrap(std::move(out));
 }
 
@@ -479,8 +483,9 @@ PyObject *gated_residual(PyObject *const *a, Py_ssize_t n) {
     Tensor out = at::empty(x.sizes(), x.options().requires_grad(false));
     const int64_t c = x.size(-1);
     long long gs = 0;
-    const void *gp = frame_vectors(tensor_or_null(a[2], "gate"), c, keep[2], gs);
-    check(f_residual(x.data_ptr(), y.data_ptr(), out.data_ptr(), c ? x.numel() / c : 0, (int)c, gp, gs, (int)integer(a[3]), stream));
+    const int64_t rows = c ? x.numel() / c : 0, tokens = (int)integer(a[3]);
+    const void *gp = frame_vectors(tensor_or_null(a[2], "gate"), rows, tokens, c, keep[2], gs);
+    check(f_residual(x.data_ptr(), y.data_ptr(), out.data_ptr(), rows, (int)c, gp, gs, (int)tokens, stream));
     return THPVariable_Wrap(std::move(out));
 }
 
