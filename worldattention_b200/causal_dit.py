@@ -266,6 +266,16 @@ class CausalDiT(nn.Module):
             self._table = torch.view_as_real(self.freqs.to(torch.complex128)).to(device=dev, dtype=torch.float64).contiguous()
         return self._table
 
+    def _modulated(self, x, scale, shift):
+        """The output head's norm and modulation: one launch where the blocks' own are, and the norm is the one that the launch computes."""
+        norm, tokens = self.head_norm, self.cfg.frame_tokens
+        if (x.is_cuda and x.dtype == scale.dtype == torch.bfloat16 and not torch.is_grad_enabled() and x.shape[1] == scale.shape[1] * tokens
+                and x.shape[2] % 8 == 0 and x.shape[2] <= 4096 and all(getattr(blk, "fused", False) for blk in self.blocks)
+                and type(norm) is _LayerNorm and norm.weight is None and norm.bias is None and norm.normalized_shape == x.shape[2:]
+                and not (norm._forward_hooks or norm._forward_pre_hooks or "forward" in vars(norm) or nn.modules.module._has_any_global_hook())):
+            return ln_modulate(x, norm.eps, scale=scale, shift=shift, tokens_per_frame=tokens)
+        return (norm(x).unflatten(1, (scale.shape[1], tokens)) * (1 + scale) + shift).flatten(1, 2)
+
     def embed_text(self, prompt_embeds: torch.Tensor) -> torch.Tensor:
         return self.text_embedding(prompt_embeds)
 
@@ -287,10 +297,7 @@ class CausalDiT(nn.Module):
             x = blk(x, e0, context, cache, cross, plan, table)
         m = (self.head_modulation.unsqueeze(1) + e.unflatten(0, (b, f)).unsqueeze(2)).chunk(2, dim=2)
         tokens = cfg.frame_tokens
-        if x.is_cuda and x.dtype == m[0].dtype == torch.bfloat16 and not torch.is_grad_enabled():
-            x = self.head(ln_modulate(x, self.head_norm.eps, scale=m[1], shift=m[0], tokens_per_frame=tokens))
-        else:
-            x = self.head(self.head_norm(x).unflatten(1, (f, tokens)) * (1 + m[1]) + m[0])          # [B, F, tokens, p*C]
+        x = self.head(self._modulated(x, m[1], m[0]).unflatten(1, (f, tokens)))                     # [B, F, tokens, p*C]
         gh, gw = cfg.grid_hw
         x = x.view(b, f, gh, gw, cfg.patch[1], cfg.patch[2], cfg.out_channels)
         return x.permute(0, 1, 6, 2, 4, 3, 5).reshape(b, f, cfg.out_channels, gh * cfg.patch[1], gw * cfg.patch[2])
