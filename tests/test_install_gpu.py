@@ -66,3 +66,30 @@ def test_pages_of_broken_frames_take_the_separate_kernels(monkeypatch):
     monkeypatch.setattr(wa.hkv.HKVCache, "_install_fused", lambda self, *a: done.append(fused(self, *a)) or done[-1])
     assert hkv.apply(cache, [(0, 0), (0, 1)], current_start_frame=9, temporal_freqs=freqs, hsa_modules=hsa) == 64
     assert done == [False]
+
+
+def _small_bank(frame=16, layers=2, frames=5):
+    import worldattention_b200 as wa
+    heads, d = 1, 128
+    hkv = wa.hkv.HKVCache(frame_seq_length=frame, page_size_frames=2, hbm_max_chunks=1)
+    hsa = [wa.hsa.HSAAttention(heads, d, block_size=64, proj_segment_len=frame).to(dev(), torch.bfloat16) for _ in range(layers)]
+    size = frames * frame
+    make = lambda n: torch.randn((1, n, heads, d), device=dev()).bfloat16()
+    cache = [{"k": make(size), "v": make(size), "k_coarse": make(frames), "v_coarse": make(frames),
+              "local_end_index": torch.tensor([size], device=dev()), "global_end_index": torch.tensor([size], device=dev())} for _ in range(layers)]
+    freqs = torch.polar(torch.ones(64, 22, dtype=torch.float64), torch.randn(64, 22, dtype=torch.float64))
+    hkv.store(cache, prompt_embeds=make(1).float()[:, :, 0], current_start_frame=frames, temporal_freqs=freqs)
+    return hkv, hsa, cache, freqs
+
+
+@pytest.mark.parametrize("start", [9, 9.0, 9.25, np.float32(9.25), torch.tensor(9), torch.tensor(9.25), "device"], ids=str)
+@pytest.mark.parametrize("dtype", [torch.int64, torch.int32, torch.float32], ids=str)
+def test_start_frame_of_any_number_type(start, dtype):
+    hkv, hsa, cache, freqs = _small_bank()
+    start = torch.tensor(9.25, device=dev()) if isinstance(start, str) else start
+    for block in cache:
+        block["global_end_index"] = block["global_end_index"].to(dtype)
+    assert hkv.apply(cache, [(0, 1)], current_start_frame=start, temporal_freqs=freqs, hsa_modules=hsa) == 32
+    for block in cache:
+        assert torch.equal(block["global_end_index"].cpu(), torch.zeros(1, dtype=dtype).fill_(float(start) * 16))
+        assert int(block["local_end_index"]) == 32

@@ -225,6 +225,9 @@ class HKVCache:
         if plan is None:
             return 0
         dev = _lib.require_cuda(k0)
+        end_token = current_start_frame * self.frame_seq_length      # a float or a 0-dim tensor as well
+        if isinstance(end_token, torch.Tensor):
+            end_token = end_token.item()
         tokens = int(plan["count"].sum())
         if self.rerope and tokens > 0:
             temporal_freqs = self._fetch_table(temporal_freqs)
@@ -245,15 +248,20 @@ class HKVCache:
                 for layer, block in enumerate(kv_cache):
                     self._write_coarse(block, hsa_modules[layer], tokens)
 
-        for name, value in (("global_end_index", current_start_frame * self.frame_seq_length), ("local_end_index", tokens)):
-            ends = list({id(block[name]): block[name] for block in kv_cache}.values())
-            if len({t.data_ptr() for t in ends}) == len(ends) and all(t.is_cuda and t.dtype == torch.long for t in ends):
-                torch._foreach_zero_(ends)           # two launches for all layers
-                torch._foreach_add_(ends, value)
-            else:
-                for t in ends:
-                    t.fill_(value)
+        self._set_ends(kv_cache, "global_end_index", end_token)
+        self._set_ends(kv_cache, "local_end_index", tokens)
         return tokens
+
+    @staticmethod
+    def _set_ends(kv_cache, name: str, value) -> None:
+        """One index of every layer to `value`, in two launches for all layers where they can be."""
+        ends = list({id(block[name]): block[name] for block in kv_cache}.values())
+        if len({t.data_ptr() for t in ends}) == len(ends) and all(t.is_cuda and t.dtype == torch.long for t in ends):
+            torch._foreach_zero_(ends)
+            torch._foreach_add_(ends, int(value))        # which `fill_` makes of a fraction too
+        else:
+            for t in ends:
+                t.fill_(value)
 
     _PLAN_DTYPE = np.dtype([("chunk", "<i8"), ("src", "<i8"), ("count", "<i8"), ("dst", "<i8"),
                             ("frame_from", "<i8"), ("frame_to", "<i8")])
