@@ -93,3 +93,39 @@ def test_start_frame_of_any_number_type(start, dtype):
     for block in cache:
         assert torch.equal(block["global_end_index"].cpu(), torch.zeros(1, dtype=dtype).fill_(float(start) * 16))
         assert int(block["local_end_index"]) == 32
+
+
+class _Compressor:
+    """A module that offers what a compressed tier of its own kind needs, and nothing else."""
+
+    def __init__(self, hsa):
+        self.token_range_to_coarse, self.compress_kv_cache = hsa.token_range_to_coarse, hsa.compress_kv_cache
+
+
+@pytest.mark.parametrize("tier", ["float32", "float32 in the last layer", "other strides of v", "channels apart"])
+def test_a_tier_of_its_own_kind_asks_its_module_for_the_slots_only(tier):
+    hkv, hsa, cache, freqs = _small_bank()
+    modules = list(hsa)
+    for m in hsa:
+        torch.nn.init.normal_(m.k_proj_mat)
+        torch.nn.init.normal_(m.v_proj_mat)
+    for layer, block in enumerate(cache):
+        if tier == "float32 in the last layer" and layer == 0:
+            continue
+        modules[layer] = _Compressor(hsa[layer])
+        for name in ("k_coarse", "v_coarse") if tier != "other strides of v" else ("v_coarse",):
+            if tier.startswith("float32"):
+                block[name] = block[name].float()
+            else:
+                wide = torch.zeros(1, 5, 1, 256, device=dev(), dtype=torch.bfloat16)
+                block[name] = wide[..., ::2] if tier == "channels apart" else wide[..., :128]
+    assert hkv.apply(cache, [(0, 0), (0, 1)], current_start_frame=9, temporal_freqs=freqs, hsa_modules=modules) == 64
+    for m, block in zip(hsa, cache):
+        want = m.compress_kv_cache(block["k"][:, :64], block["v"][:, :64])
+        for name, slots in zip(("k_coarse", "v_coarse"), want):
+            assert torch.equal(block[name][:, :4], slots.to(block[name].dtype)) and not block[name][:, 4:].any()
+
+
+def test_modules_may_be_keyed_by_layer():
+    hkv, hsa, cache, freqs = _small_bank()
+    assert hkv.apply(cache, [(0, 0)], current_start_frame=9, temporal_freqs=freqs, hsa_modules=dict(enumerate(hsa))) == 32

@@ -497,23 +497,25 @@ class HKVCache:
         k0 = kv_cache[0]["k"]
         bsz, _, heads, head_dim = k0.shape
         frame, esize = self.frame_seq_length, k0.element_size()
-        if k0.dtype != torch.bfloat16 or kv_cache[0]["k_coarse"].dtype != torch.bfloat16 or (plan["count"] % frame).any() or (plan["src"] % frame).any():
+        if k0.dtype != torch.bfloat16 or (plan["count"] % frame).any() or (plan["src"] % frame).any():
             return False
+        # tiers whose slots the compress kernel does not write either are the module's own business (`compress_kv_cache`), and all
+        # that is asked of such a module
+        coarse = _Table([layer[name] for layer in kv_cache for name in ("k_coarse", "v_coarse")])
+        if not ((coarse.dim == 4).all() and (coarse.dtype == caches.dtype[0]).all() and (coarse.device == caches.device[0]).all()
+                and (coarse.stride[::2] == coarse.stride[1::2]).all() and (coarse.size[:, 0] >= bsz).all()
+                and (coarse.size[:, 2:] == (heads, head_dim)).all() and (coarse.stride[:, 2:] == (head_dim, 1)).all()):
+            return False
+        hsa_modules = [hsa_modules[layer] for layer in range(len(kv_cache))]
         first = hsa_modules[0]
         shape, block = first.k_proj_mat.shape, first.block_size
-        if first.proj_segment_len != frame or shape[1] < frame:
+        if first.proj_segment_len != frame or shape[1] < frame or any(hsa.proj_segment_len != frame or hsa.block_size != block for hsa in hsa_modules):
             return False
         slots = first.token_range_to_coarse(0, int(plan["count"].sum()))[1]
-        if any(hsa.proj_segment_len != frame or hsa.block_size != block for hsa in hsa_modules):
-            return False
-        coarse = _Table([layer[name] for layer in kv_cache for name in ("k_coarse", "v_coarse")])
-        proj = _Table([p for hsa in hsa_modules[: len(kv_cache)] for p in (hsa.k_proj_mat, hsa.v_proj_mat)])
-        if len(proj.ptr) != len(dst) or not (
-                (caches.dtype == caches.dtype[0]).all() and (caches.size[:, 0] == bsz).all() and (coarse.dim == 4).all() and (proj.dim == 2).all()
-                and all((t.dtype == caches.dtype[0]).all() and (t.device == caches.device[0]).all() for t in (coarse, proj))
-                and (proj.size[:, :2] == shape).all() and (proj.stride[:, :2] == (shape[1], 1)).all()
-                and (coarse.stride[::2] == coarse.stride[1::2]).all() and (coarse.size[:, 0] >= bsz).all() and (coarse.size[:, 1] >= slots).all()
-                and (coarse.size[:, 2:] == (heads, head_dim)).all() and (coarse.stride[:, 2:] == (head_dim, 1)).all()):
+        proj = _Table([p for hsa in hsa_modules for p in (hsa.k_proj_mat, hsa.v_proj_mat)])
+        if not ((caches.dtype == caches.dtype[0]).all() and (caches.size[:, 0] == bsz).all() and (coarse.size[:, 1] >= slots).all()
+                and (proj.dim == 2).all() and (proj.dtype == caches.dtype[0]).all() and (proj.device == caches.device[0]).all()
+                and (proj.size[:, :2] == shape).all() and (proj.stride[:, :2] == (shape[1], 1)).all()):
             return False
         between = lambda a: np.ascontiguousarray((a[..., 1] - a[..., 0]) // esize if bsz > 1 else np.zeros(a.shape[:-1], dtype=np.int64))
         whole = lambda a: np.ascontiguousarray(a)
