@@ -532,7 +532,8 @@ class HKVCache:
             if rc == _lib.WA_ERR_UNSUPPORTED:
                 return False
             _lib.check(rc)
-            _lib.check(lib.wa_hkv_install_pages(ctypes.byref(job), to_device(table, dev).data_ptr(), _lib.ptr(rot_dev), _lib.stream_ptr(dev)))
+            maps = to_device(table, dev)         # held until the launch is enqueued: its memory then stays ahead of whoever takes it next
+            _lib.check(lib.wa_hkv_install_pages(ctypes.byref(job), maps.data_ptr(), _lib.ptr(rot_dev), _lib.stream_ptr(dev)))
         return True
 
     @staticmethod
