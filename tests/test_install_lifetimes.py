@@ -50,3 +50,29 @@ def test_the_install_holds_its_table_while_it_launches(monkeypatch):
     dst = caches.starts(1, 2)
     assert hkv._install_fused(cache, plan, dst[None], caches, dst, np.full(1, -1), None, 22, torch.device("cpu"), hsa)
     assert lib.seen == [[True]]
+
+
+def test_candidates_of_a_shard_hold_their_contiguous_inputs(monkeypatch):
+    from worldattention_b200 import _lib, sharded
+    made, seen = [], []
+    contiguous = torch.Tensor.contiguous
+
+    def copy(t, *a):
+        out = contiguous(t, *a)
+        made.append(weakref.ref(out))
+        return out
+
+    class Lib:
+        def call(self, *args):
+            seen.append([ref() is not None for ref in made])
+            return 0
+        wa_route_local_candidates = wa_route_merge_candidates = call
+    monkeypatch.setattr(torch.Tensor, "contiguous", copy)
+    monkeypatch.setattr(_lib, "lib", lambda: Lib())
+    monkeypatch.setattr(_lib, "require_cuda", lambda *t: torch.device("cpu"))
+    monkeypatch.setattr(_lib, "stream_ptr", lambda dev: 0)
+    sharded.local_candidates(torch.zeros(1, 3, 2, 8).transpose(1, 2), torch.zeros(1, 5, 2, 8).transpose(1, 2), block_lo=0, topk_max=2)
+    made.clear()
+    sharded.merge_candidates(torch.zeros(6, 2, 2, dtype=torch.int64).transpose(0, 1), (1, 2, 3), topk_per_head=torch.ones(2), blocks_total=9,
+                             block_lo=0, block_hi=5)
+    assert seen == [[True, True], [True, True]]

@@ -183,8 +183,9 @@ def local_candidates(q_pooled, k_pooled_local, *, block_lo: int, topk_max: int) 
     bsz, heads, nq, head_dim = q_pooled.shape
     nloc = k_pooled_local.shape[2]
     cand = torch.empty((bsz * heads * nq, topk_max), dtype=torch.int64, device=dev)
+    q_pooled, k_pooled_local = q_pooled.contiguous(), k_pooled_local.contiguous()      # held until the launch is enqueued
     _lib.check(_lib.lib().wa_route_local_candidates(
-        q_pooled.contiguous().data_ptr(), k_pooled_local.contiguous().data_ptr() if nloc else None, bsz, heads, nq, nloc,
+        q_pooled.data_ptr(), k_pooled_local.data_ptr() if nloc else None, bsz, heads, nq, nloc,
         head_dim, block_lo, topk_max, cand.data_ptr(), _lib.stream_ptr(dev)))
     return cand
 
@@ -200,8 +201,9 @@ def merge_candidates(every: torch.Tensor, shape, *, topk_per_head, blocks_total:
     local_index = torch.empty((bsz, heads, nq, width), dtype=torch.int32, device=dev)
     local_num = torch.empty((bsz, heads, nq), dtype=torch.int32, device=dev)
     topk = topk_per_head.to(device=dev, dtype=torch.int32).contiguous()
+    every = every.contiguous()             # held until the launch is enqueued
     _lib.check(_lib.lib().wa_route_merge_candidates(
-        every.contiguous().data_ptr(), world, bsz, heads, nq, topk_max, topk.data_ptr(), blocks_total, block_lo, block_hi, width,
+        every.data_ptr(), world, bsz, heads, nq, topk_max, topk.data_ptr(), blocks_total, block_lo, block_hi, width,
         local_index.data_ptr(), local_num.data_ptr(), _lib.stream_ptr(dev)))
     return local_index, local_num
 
