@@ -3,6 +3,7 @@ import contextlib
 import weakref
 
 import numpy as np
+import pytest
 import torch
 
 
@@ -76,3 +77,75 @@ def test_candidates_of_a_shard_hold_their_contiguous_inputs(monkeypatch):
     sharded.merge_candidates(torch.zeros(6, 2, 2, dtype=torch.int64).transpose(0, 1), (1, 2, 3), topk_per_head=torch.ones(2), blocks_total=9,
                              block_lo=0, block_hi=5)
     assert seen == [[True, True], [True, True]]
+
+
+def test_promoted_pages_are_known_to_the_allocator_of_host_memory(monkeypatch):
+    from worldattention_b200 import _lib
+    from worldattention_b200.hkv import cache as C
+    order, known = [], [True]
+
+    class Side:
+        stream_id, device_index, cuda_stream = 7, 0, 70
+        wait_stream = lambda self, other: order.append("behind")
+        synchronize = lambda self: order.append("waited for")
+
+    class Lib:
+        wa_hkv_promote_pages = lambda self, records, n, *rest: order.append(("copied", n)) or 0
+
+    class Host:
+        read_on_stream = lambda self, pages, stream_id, device: order.append(("told", [id(p) for p in pages], stream_id, device)) or known[0]
+    monkeypatch.setattr(_lib, "lib", lambda: Lib())
+    monkeypatch.setattr(_lib, "host", lambda: Host())
+    monkeypatch.setattr(_lib, "device_guard", lambda dev: contextlib.nullcontext())
+    monkeypatch.setattr(torch.cuda, "current_stream", lambda dev: None)
+    monkeypatch.setattr(torch.Tensor, "record_stream", lambda t, stream: None)
+    hkv = C.HKVCache(frame_seq_length=4, page_size_frames=2)
+    monkeypatch.setattr(hkv.tier, "side_stream", lambda dev: Side())
+    k0 = torch.zeros(2, 16, 1, 8)
+    pages = [torch.zeros(2, 8, 1, 8) for _ in range(3)]
+    single = [(0, "k", 0, pages[0], 0), (0, "v", 0, pages[1], None), (1, "k", 0, pages[2], 128)]
+    for known[0] in (True, False):
+        order.clear()
+        hkv._promote(single, 256, k0)
+        told = ("told", [id(pages[0]), id(pages[2])], 7, 0)
+        assert order == ["behind", ("copied", 4), told] + ([] if known[0] else ["waited for"])
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("tier", ["file", "host"])
+def test_host_pages_are_not_handed_out_again_while_they_cross(tmp_path, tier):
+    """The copies of a cold install wait behind other work; what is let go and allocated meanwhile must not reach them."""
+    import worldattention_b200 as wa
+    dev, frame, layers = torch.device("cuda:0"), 64, 3
+    hkv = wa.hkv.HKVCache(frame_seq_length=frame, page_size_frames=2, cpu_max_chunks=1, nvme_enabled=tier == "file", nvme_dir=str(tmp_path), rerope=False)
+    make = lambda n: torch.randn((1, n, 2, 128), device=dev).bfloat16()
+    end = lambda: torch.tensor([4 * frame], device=dev)
+    fill = lambda: [{"k": make(4 * frame), "v": make(4 * frame), "local_end_index": end(), "global_end_index": end()} for _ in range(layers)]
+    freqs = torch.polar(torch.ones(64, 22, dtype=torch.float64), torch.randn(64, 22, dtype=torch.float64))
+    first = fill()
+    for window in (first, fill())[: 2 if tier == "file" else 1]:
+        hkv.store(window, prompt_embeds=make(1).float()[:, :, 0], current_start_frame=4, temporal_freqs=freqs)
+    assert hkv.tier.location(0) == ("nvme" if tier == "file" else "cpu")
+    cache = fill()
+    busy = torch.empty(1 << 30, dtype=torch.uint8, device=dev)
+    # page-locking new memory waits for the device: what is wanted below has to be there
+    buffers = lambda: [torch.full((1, n * frame, 2, 128), 7.0, dtype=torch.bfloat16, pin_memory=True) for n in (2, 4) for _ in range(4 * layers)]
+    hkv.apply(fill(), [(0, 0), (0, 1)], current_start_frame=9, temporal_freqs=freqs)
+    small = [torch.empty(1 << bits, dtype=torch.uint8, pin_memory=True) for bits in range(4, 17) for _ in range(8)]
+    spare = buffers() + buffers()
+    torch.cuda.synchronize()
+    del small, spare
+    with torch.cuda.stream(hkv.tier.side_stream(dev)):
+        for _ in range(600):                                    # some 100 ms
+            busy[: 1 << 29].copy_(busy[1 << 29:])
+        done = torch.cuda.Event()
+        done.record()
+    assert hkv.apply(cache, [(0, 0), (0, 1)], current_start_frame=9, temporal_freqs=freqs) == 4 * frame
+    if tier == "host":
+        hkv.reset()
+    others = buffers()
+    assert not done.query(), "the copies were over before anything could reach them: this says nothing"
+    torch.cuda.synchronize()
+    for got, want in zip(cache, first):
+        assert torch.equal(got["k"], want["k"]) and torch.equal(got["v"], want["v"])
+    del others

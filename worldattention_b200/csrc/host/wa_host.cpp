@@ -8,6 +8,7 @@
 // come from.
 #include <torch/extension.h>
 
+#include <ATen/core/CachingHostAllocator.h>
 #include <ATen/cuda/CUDAContext.h>
 #include <c10/cuda/CUDAGuard.h>
 #include <torch/csrc/autograd/python_variable.h>
@@ -524,6 +525,31 @@ PyObject *tensor_table(PyObject *const *a, Py_ssize_t n) {
     return out;
 }
 
+// ---- read_on_stream(tensors, stream_id, device_index) -> bool -------------------------------------
+// Tells PyTorch's allocator of page-locked memory that the stream reads these host tensors, so that it keeps their memory from the
+// next allocation until what the stream carries by then is done, whoever drops them and when: its own copies say so, a copy
+// queued by this library does not.  False: some are page-locked by another hand, and only the caller can keep them.
+PyObject *read_on_stream(PyObject *const *a, Py_ssize_t n) {
+    expect_args(n, 3);
+    const c10::Stream stream = c10::Stream::unpack3(integer(a[1]), (c10::DeviceIndex)integer(a[2]), c10::DeviceType::CUDA);
+    PyObject *seq = PySequence_Fast(a[0], "expected a sequence of tensors");
+    if (!seq) throw PyFailure();
+    bool all = true;
+    try {
+        at::HostAllocator *allocator = at::getHostAllocator(at::kCUDA);
+        for (Py_ssize_t i = 0; i < PySequence_Fast_GET_SIZE(seq); ++i) {
+            const Tensor &t = tensor(PySequence_Fast_GET_ITEM(seq, i), "every element");
+            const c10::DataPtr &memory = t.storage().data_ptr();
+            if (t.numel() && !allocator->record_event(memory.get(), memory.get_context(), stream) && t.is_pinned()) all = false;
+        }
+    } catch (...) {
+        Py_DECREF(seq);
+        throw;
+    }
+    Py_DECREF(seq);
+    return PyBool_FromLong(all);
+}
+
 // ---- bind(addresses: dict name -> int, status_word, raise_if_failed) ----------------------------
 PyObject *bind(PyObject *const *a, Py_ssize_t n) {
     expect_args(n, 3);
@@ -574,7 +600,7 @@ PyObject *entry(PyObject *, PyObject *const *args, Py_ssize_t n) {
 
 #define WA_ENTRY(name) {#name, (PyCFunction)(void (*)(void))entry<name>, METH_FASTCALL, nullptr}
 PyMethodDef methods[] = {WA_ENTRY(bind), WA_ENTRY(hsa_forward), WA_ENTRY(run_forward), WA_ENTRY(qk_norm_rope), WA_ENTRY(append_kv), WA_ENTRY(ln_modulate),
-                         WA_ENTRY(gated_residual), WA_ENTRY(tensor_table), {nullptr, nullptr, 0, nullptr}};
+                         WA_ENTRY(gated_residual), WA_ENTRY(tensor_table), WA_ENTRY(read_on_stream), {nullptr, nullptr, 0, nullptr}};
 PyModuleDef module = {PyModuleDef_HEAD_INIT, "_host", nullptr, -1, methods, nullptr, nullptr, nullptr, nullptr};
 
 }  // namespace

@@ -414,8 +414,14 @@ class HKVCache:
         main, side = torch.cuda.current_stream(dev), self.tier.side_stream(dev)
         side.wait_stream(main)            # the staging block may be recycled memory that the main stream still uses
         staging.record_stream(side)
-        with _lib.device_guard(dev):
-            _lib.check(_lib.lib().wa_hkv_promote_pages((_lib.PageCopy * len(promote))(*promote), len(promote), row_elems, esize, side.cuda_stream))
+        try:
+            with _lib.device_guard(dev):
+                _lib.check(_lib.lib().wa_hkv_promote_pages((_lib.PageCopy * len(promote))(*promote), len(promote), row_elems, esize, side.cuda_stream))
+        finally:
+            # nobody waits here, and a page read from a file is dropped as soon as the install is enqueued, a chunk's when the bank
+            # lets go of it: their page-locked memory must not be handed out again before the copies are done
+            if not _lib.host().read_on_stream([page for _, _, _, page, slot in single if slot is not None], side.stream_id, side.device_index):
+                side.synchronize()
         return staging
 
     def _install(self, kv_cache, plan, sources, temporal_freqs, dev, dtype, hsa_modules=None) -> bool:
