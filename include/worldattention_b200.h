@@ -389,6 +389,10 @@ size_t wa_hkv_install_table_bytes(int pages, int tensors, int segments);
 int wa_hkv_install_table(const wa_hkv_install *p, void *table, size_t bytes);
 /* `rotations`: device float `[R, n_temporal, 2]`, or null. */
 int wa_hkv_install_pages(const wa_hkv_install *p, const void *device_table, const float *rotations, void *stream);
+/* The same; `status_mirror` (page-locked host memory, or null) receives the site code, 301 to 309, when a bounded wait of the
+ * launch runs out: pages and slots are then incomplete.  wa_compress_status reads the same code from the device. */
+int wa_hkv_install_pages_mirrored(const wa_hkv_install *p, const void *device_table, const float *rotations, int32_t *status_mirror,
+                                  void *stream);
 
 /* Promotion of cold pages (the `.to(device)` of cache.py:229-231 for chunks that live in host memory): one
  * asynchronous host-to-device copy per record of the HOST array `host_records` (src = page-locked host memory,

@@ -19,7 +19,8 @@ class _Lib:
     def wa_hkv_install_table(self, *args):
         return 0
 
-    def wa_hkv_install_pages(self, job, table, *args):
+    def wa_hkv_install_pages_mirrored(self, job, table, rotations, mirror, stream):
+        self.mirror = mirror
         self.seen.append([ref() is not None and ref().data_ptr() == table for ref in self.refs])
         return 0
 
@@ -48,9 +49,34 @@ def test_the_install_holds_its_table_while_it_launches(monkeypatch):
     monkeypatch.setattr(_lib, "lib", lambda: lib)
     monkeypatch.setattr(_lib, "device_guard", lambda dev: contextlib.nullcontext())
     monkeypatch.setattr(_lib, "stream_ptr", lambda dev: 0)
+    word = torch.zeros(1, dtype=torch.int32)
+    monkeypatch.setattr(_lib, "status_word", lambda dev: word)
     dst = caches.starts(1, 2)
     assert hkv._install_fused(cache, plan, dst[None], caches, dst, np.full(1, -1), None, 22, torch.device("cpu"), hsa)
-    assert lib.seen == [[True]]
+    assert lib.seen == [[True]] and lib.mirror == word.data_ptr()
+
+
+@pytest.mark.parametrize("call", ["store", "retrieve", "apply"])
+def test_a_launch_that_gave_up_raises_in_the_next_call_of_the_bank(monkeypatch, call):
+    from worldattention_b200 import _lib
+    from worldattention_b200.hkv import HKVCache
+    hkv = HKVCache(frame_seq_length=4, page_size_frames=2)
+    k = torch.zeros(1, 8, 1, 8)
+    cache = [{"k": k, "v": k.clone(), "local_end_index": torch.tensor([8]), "global_end_index": torch.tensor([8])}]
+    hkv.chunks = [{"page_spans": [(0, 8)], "start_frame": 0}]
+    hkv.tier.put(0, {"k": [k], "v": [k]})
+    word = torch.tensor([304], dtype=torch.int32)
+    monkeypatch.setitem(_lib._status_words, 0, word)
+    monkeypatch.setattr(_lib, "require_cuda", lambda *t: torch.device("cuda", 0))
+    on_device = type("T", (), {"is_cuda": True, "device": torch.device("cuda", 0)})()
+    with pytest.raises(RuntimeError, match="HKV install.*304"):
+        if call == "store":
+            hkv.store(cache, prompt_embeds=k[0], current_start_frame=2, temporal_freqs=None)
+        elif call == "retrieve":
+            hkv.retrieve(prompt_embeds=on_device, query_vec=None)
+        else:
+            hkv.apply(cache, [(0, 0)], current_start_frame=2, temporal_freqs=None)
+    assert int(word) == 0 and int(cache[0]["global_end_index"]) == 8
 
 
 def test_candidates_of_a_shard_hold_their_contiguous_inputs(monkeypatch):

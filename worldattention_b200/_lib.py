@@ -106,6 +106,7 @@ SIGNATURES = {
     "wa_hkv_install_table_bytes": [_i, _i, _i],
     "wa_hkv_install_table": [_vp, _vp, C.c_size_t],
     "wa_hkv_install_pages": [_vp, _vp, _vp, _vp],
+    "wa_hkv_install_pages_mirrored": [_vp, _vp, _vp, _vp, _vp],
     "wa_hkv_clear_rows": [_vp, _i, _i, _i, _i, _vp],
     "wa_hkv_gather_pages": [_vp, _i, _i, _i, _i, _i, _vp, _i, _vp],
 }
@@ -204,7 +205,7 @@ _status_words: dict = {}
 
 
 def status_word(device: torch.device) -> torch.Tensor:
-    """The page-locked int32 that the tcgen05 kernel writes its failure code to on `device` (one per device)."""
+    """The page-locked int32 that kernels with bounded waits write their failure code to on `device` (one per device)."""
     key = torch.device(device).index or 0
     word = _status_words.get(key)
     if word is None:
@@ -214,7 +215,7 @@ def status_word(device: torch.device) -> torch.Tensor:
 
 
 def raise_if_failed(device: torch.device) -> None:
-    """Raise if an earlier launch of an HSA forward on `device` gave up at a bounded wait (its output is invalid).
+    """Raise if an earlier launch of an HSA forward or an HKV install on `device` gave up at a bounded wait (its output is invalid).
 
     Reads host memory only: no copy, no synchronisation.  A failure of a launch that is still in flight shows
     at the next call or at the caller's next synchronisation point followed by this check.
@@ -223,6 +224,8 @@ def raise_if_failed(device: torch.device) -> None:
     if word is not None and int(word[0]) != 0:
         code = int(word[0])
         word.zero_()
+        if 301 <= code <= 309:
+            raise RuntimeError(f"an earlier HKV install on {device} gave up at wait site {code}; the installed pages and slots are invalid")
         kernel = "block-pooling (TMA stream)" if code in (201, 202) else "tcgen05 attention"
         raise RuntimeError(f"an earlier {kernel} launch of an HSA forward on {device} gave up at wait site {code}; "
                            "its output is invalid")

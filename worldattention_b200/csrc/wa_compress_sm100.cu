@@ -278,7 +278,7 @@ struct Job {
     Table at;
     const float2 *rotations;
     int tensors, n_seg, tiles_cols, B, D, frame, rank, nt;
-    int *status;
+    int *status, *status_mirror;
 };
 
 struct Barriers {
@@ -301,12 +301,12 @@ install_stream_kernel(const Job job) {
     Barriers *bar = reinterpret_cast<Barriers *>(smem + STAGES * STAGE_BYTES);
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     volatile int *abort_flag = &bar->abort_flag;
-    const FailSink sink{job.status, nullptr};
+    const FailSink sink{job.status, job.status_mirror};      // sites 301 to 309
     const Segment *segments = reinterpret_cast<const Segment *>(job.table + job.at.segments);
 
     if (threadIdx.x == 0) {
         bar->abort_flag = (smem_u32(smem) & 1023u) ? 1 : 0;
-        if (bar->abort_flag) report_failure(sink, 98);
+        if (bar->abort_flag) report_failure(sink, 309);
         for (int i = 0; i < STAGES; ++i) {
             mbar_init(&bar->full[i], 1);
             mbar_init(&bar->ready[i], TURN_WARPS);
@@ -350,7 +350,7 @@ install_stream_kernel(const Job job) {
                 const CUtensorMap *te = acquire_map(job.table + job.at.proj + (size_t)tensor * sizeof(CUtensorMap));
                 for (int t = 0; t < n_tiles && ok; ++t, ++count) {
                     const uint32_t s = count % STAGES;
-                    ok = mbar_wait(&bar->empty[s], ((count / STAGES) & 1u) ^ 1u, abort_flag, sink, 31);
+                    ok = mbar_wait(&bar->empty[s], ((count / STAGES) & 1u) ^ 1u, abort_flag, sink, 301);
                     if (!ok) break;
                     uint8_t *xs = smem + s * STAGE_BYTES, *es = xs + TILE_BYTES;
                     mbar_expect_tx(&bar->full[s], TILE_BYTES + 2 * E_HALF_BYTES);
@@ -369,12 +369,12 @@ install_stream_kernel(const Job job) {
         bool ok = true;
         for (int item = blockIdx.x; item < n_items && ok; item += gridDim.x, ++n_done) {
             const uint32_t buf = n_done & 1u;
-            ok = __all_sync(0xffffffffu, mbar_wait(&bar->acc_empty[buf], ((n_done >> 1) & 1u) ^ 1u, abort_flag, sink, 32));
+            ok = __all_sync(0xffffffffu, mbar_wait(&bar->acc_empty[buf], ((n_done >> 1) & 1u) ^ 1u, abort_flag, sink, 302));
             if (!ok) break;
             for (int t = 0; t < n_tiles && ok; ++t, ++count) {
                 const uint32_t s = count % STAGES;
-                ok = __all_sync(0xffffffffu, mbar_wait(&bar->full[s], (count / STAGES) & 1u, abort_flag, sink, 33) &&
-                                                 mbar_wait(&bar->ready[s], (count / STAGES) & 1u, abort_flag, sink, 34));
+                ok = __all_sync(0xffffffffu, mbar_wait(&bar->full[s], (count / STAGES) & 1u, abort_flag, sink, 303) &&
+                                                 mbar_wait(&bar->ready[s], (count / STAGES) & 1u, abort_flag, sink, 304));
                 if (!ok) break;
                 tc_fence_after();
                 if (leader) {
@@ -401,8 +401,8 @@ install_stream_kernel(const Job job) {
                 const CUtensorMap *td = acquire_map(job.table + job.at.dst + (size_t)tensor * sizeof(CUtensorMap));
                 for (int t = 0; t < n_tiles && ok; ++t, ++count) {
                     const uint32_t s = count % STAGES;
-                    ok = mbar_wait(&bar->full[s], (count / STAGES) & 1u, abort_flag, sink, 35) &&
-                         mbar_wait(&bar->ready[s], (count / STAGES) & 1u, abort_flag, sink, 36);
+                    ok = mbar_wait(&bar->full[s], (count / STAGES) & 1u, abort_flag, sink, 305) &&
+                         mbar_wait(&bar->ready[s], (count / STAGES) & 1u, abort_flag, sink, 306);
                     if (!ok) break;
                     const uint8_t *xs = smem + s * STAGE_BYTES;
                     tma_store_4d(td, xs, ct * TILE, t * TILE, seg, b);
@@ -426,7 +426,7 @@ install_stream_kernel(const Job job) {
             const float2 *turn = job.rotations + (long long)max(rot, 0) * job.nt;
             for (int t = 0; t < n_tiles && ok; ++t, ++count) {
                 const uint32_t s = count % STAGES;
-                ok = __all_sync(0xffffffffu, mbar_wait(&bar->full[s], (count / STAGES) & 1u, abort_flag, sink, 37));
+                ok = __all_sync(0xffffffffu, mbar_wait(&bar->full[s], (count / STAGES) & 1u, abort_flag, sink, 307));
                 if (!ok) break;
                 if (rot >= 0) {
                     uint8_t *line = smem + s * STAGE_BYTES + row * 128;
@@ -462,7 +462,7 @@ install_stream_kernel(const Job job) {
             int ct, seg, tensor, b;
             decode(item, ct, seg, tensor, b);
             const uint32_t buf = n_done & 1u;
-            ok = __all_sync(0xffffffffu, mbar_wait(&bar->acc_full[buf], (n_done >> 1) & 1u, abort_flag, sink, 38));
+            ok = __all_sync(0xffffffffu, mbar_wait(&bar->acc_full[buf], (n_done >> 1) & 1u, abort_flag, sink, 308));
             if (!ok) break;
             tc_fence_after();
             const Slots sl = reinterpret_cast<const Slots *>(job.table + job.at.slots)[tensor];
@@ -702,6 +702,11 @@ extern "C" int wa_hkv_install_table(const wa_hkv_install *p, void *table, size_t
 }
 
 extern "C" int wa_hkv_install_pages(const wa_hkv_install *p, const void *device_table, const float *rotations, void *stream) {
+    return wa_hkv_install_pages_mirrored(p, device_table, rotations, nullptr, stream);
+}
+
+extern "C" int wa_hkv_install_pages_mirrored(const wa_hkv_install *p, const void *device_table, const float *rotations, int32_t *status_mirror,
+                                             void *stream) {
     using namespace wa;
     using namespace wa::sm100::compress;
     const char *what = "wa_hkv_install_pages";
@@ -721,6 +726,7 @@ extern "C" int wa_hkv_install_pages(const wa_hkv_install *p, const void *device_
     job.tiles_cols = p->H * p->D / wa::sm100::TILE;
     job.rank = install_rank(p);
     job.status = status_address();
+    job.status_mirror = status_mirror;
     if (!job.status) return fail(WA_ERR_DEVICE, "%s: no usable current device", what);
     const long long items = (long long)p->B * p->tensors * p->segments * job.tiles_cols;
     const int sms = sm_count();

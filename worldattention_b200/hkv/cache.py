@@ -126,7 +126,7 @@ class HKVCache:
         valid_tokens = int(kv_cache[0]["local_end_index"].item())
         if valid_tokens <= 0:
             return -1
-        _lib.require_cuda(kv_cache[0]["k"])
+        _lib.raise_if_failed(_lib.require_cuda(kv_cache[0]["k"]))
         tensors = [block[name] for name in ("k", "v") for block in kv_cache]
         table = _Table(tensors)
         if (table.size[:, 1] < valid_tokens).any():      # the copy kernel takes addresses: nothing behind it would stop at the end of a cache
@@ -179,6 +179,8 @@ class HKVCache:
         """
         if not self.chunks:
             return []
+        if prompt_embeds.is_cuda:
+            _lib.raise_if_failed(prompt_embeds.device)
         bank = torch.stack(self.prompt_bank, dim=0)
         candidates = select_top_chunks(prompt_index(prompt_embeds).detach(), bank, self.stage1_topk_chunks)
 
@@ -217,7 +219,9 @@ class HKVCache:
               hsa_modules: Optional[Sequence] = None) -> int:
         """Install the selected pages into the online cache, replacing its contents (cache.py:180-254).
 
-        Returns the number of tokens installed; 0 (cache untouched) when nothing resolves.
+        Returns the number of tokens installed; 0 (cache untouched) when nothing resolves.  Nothing waits for the launches: one
+        that gives up at a bounded wait raises in the next call of the bank or of the attention on the device, or when the
+        caller runs `_lib.raise_if_failed` after its own synchronisation.
         """
         k0 = kv_cache[0]["k"]
         plan, blobs = self._install_plan(selected_pairs, capacity=int(k0.shape[1]),
@@ -225,6 +229,7 @@ class HKVCache:
         if plan is None:
             return 0
         dev = _lib.require_cuda(k0)
+        _lib.raise_if_failed(dev)
         end_token = current_start_frame * self.frame_seq_length      # a float or a 0-dim tensor as well
         if isinstance(end_token, torch.Tensor):
             end_token = end_token.item()
@@ -539,7 +544,8 @@ class HKVCache:
                 return False
             _lib.check(rc)
             maps = to_device(table, dev)         # held until the launch is enqueued: its memory then stays ahead of whoever takes it next
-            _lib.check(lib.wa_hkv_install_pages(ctypes.byref(job), maps.data_ptr(), _lib.ptr(rot_dev), _lib.stream_ptr(dev)))
+            _lib.check(lib.wa_hkv_install_pages_mirrored(ctypes.byref(job), maps.data_ptr(), _lib.ptr(rot_dev), _lib.status_word(dev).data_ptr(),
+                                                         _lib.stream_ptr(dev)))
         return True
 
     @staticmethod
