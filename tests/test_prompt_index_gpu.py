@@ -19,3 +19,21 @@ def test_prompt_index(dtype, b, tokens, dim):
         assert float((prompt_index(t).double() - mean / mean.norm()).abs().max()) < 2e-6
     zero = prompt_index(torch.zeros(1, 4, 16, device=dev(), dtype=dtype))
     assert not zero.any() and bool(prompt_index(torch.full((1, 4, 16), float("nan"), device=dev(), dtype=dtype)).isnan().all())
+
+
+def test_prompt_index_under_function_transforms():
+    from worldattention_b200.hkv.retrieval import prompt_index
+    x = torch.randn((3, 2, 16, 8), generator=torch.Generator(device=dev()).manual_seed(1), device=dev())
+    batched = torch.vmap(prompt_index)(x)
+    torch.testing.assert_close(batched, torch.stack([prompt_index(t) for t in x]), rtol=0, atol=2e-6)
+    mean = lambda t: t.mean(1).mean(0)
+    want = torch.func.jvp(lambda t: mean(t) / mean(t).norm(), (x[0].double(),), (x[1].double(),))
+    for got in (torch.func.jvp(prompt_index, (x[0],), (x[1],)), _dual(prompt_index, x[0], x[1])):
+        for a, b in zip(got, want):      # float32 sums of 16 values near 1 and a quotient
+            torch.testing.assert_close(a.double(), b, rtol=0, atol=2e-6)
+
+
+def _dual(f, x, tangent):
+    from torch.autograd import forward_ad
+    with forward_ad.dual_level():
+        return tuple(forward_ad.unpack_dual(f(forward_ad.make_dual(x, tangent))))

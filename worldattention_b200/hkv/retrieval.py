@@ -22,7 +22,7 @@ __all__ = ["prompt_index", "query_index", "page_key_index", "score_pages", "sele
 
 def prompt_index(prompt_embeds: torch.Tensor) -> torch.Tensor:
     """Mean-pool `[B, tokens, dim]` into a unit vector `[dim]` (retrieval.py:32-38)."""
-    if (type(prompt_embeds) is torch.Tensor and prompt_embeds.is_cuda and prompt_embeds.dim() == 3 and prompt_embeds.numel() > 0
+    if (_lib.is_plain(prompt_embeds) and prompt_embeds.is_cuda and prompt_embeds.dim() == 3 and prompt_embeds.numel() > 0
             and prompt_embeds.dtype in (torch.float32, torch.bfloat16) and prompt_embeds.stride(2) == 1
             and not (torch.is_grad_enabled() and prompt_embeds.requires_grad)):
         bsz, tokens, dim = prompt_embeds.shape
