@@ -129,3 +129,22 @@ def test_a_tier_of_its_own_kind_asks_its_module_for_the_slots_only(tier):
 def test_modules_may_be_keyed_by_layer():
     hkv, hsa, cache, freqs = _small_bank()
     assert hkv.apply(cache, [(0, 0)], current_start_frame=9, temporal_freqs=freqs, hsa_modules=dict(enumerate(hsa))) == 32
+
+
+@pytest.mark.parametrize("view", ["conjugate", "imaginary part", "every other row", "band"])
+def test_frequency_tables_on_the_device_in_every_view(view):
+    """A table on the device is fetched without waiting; what comes of it is what the same values on the host give."""
+    frame, heads, d = 16, 1, 128
+    import worldattention_b200 as wa
+    g = torch.Generator().manual_seed(3)
+    base = torch.polar(torch.ones(4096, 64, dtype=torch.float64), torch.randn(4096, 64, generator=g, dtype=torch.float64))
+    take = {"conjugate": lambda t: t[:, :22].conj(), "imaginary part": lambda t: t[:, :22].conj().imag, "every other row": lambda t: t[::2, :22],
+            "band": lambda t: wa.hkv.temporal_band(t, d)}[view]
+    k = torch.randn((1, 80, heads, d), generator=torch.Generator(device=dev()).manual_seed(4), device=dev()).bfloat16()
+    indices = []
+    for freqs in (take(base.to(dev())), take(base).resolve_conj().resolve_neg().clone()):
+        hkv = wa.hkv.HKVCache(frame_seq_length=frame, page_size_frames=2, hbm_max_chunks=1)
+        cache = [{"k": k.clone(), "v": k.clone(), "local_end_index": torch.tensor([80], device=dev()), "global_end_index": torch.tensor([80], device=dev())}]
+        hkv.store(cache, prompt_embeds=torch.ones(1, 1, 8), current_start_frame=900, temporal_freqs=freqs)
+        indices.append(hkv.chunks[0]["page_index"])
+    assert torch.equal(*indices)

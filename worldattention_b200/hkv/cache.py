@@ -106,7 +106,8 @@ class HKVCache:
         self._table_stream.wait_stream(torch.cuda.current_stream(dev))
         with torch.cuda.stream(self._table_stream):
             landed = torch.empty(temporal_freqs.shape, dtype=temporal_freqs.dtype, pin_memory=True)
-            landed.copy_(temporal_freqs.detach(), non_blocking=True)
+            # a lazy conjugate is resolved on the device: copy_ would do it on the host, ahead of what it does not wait for
+            landed.copy_(temporal_freqs.detach().resolve_conj().resolve_neg(), non_blocking=True)
             done = torch.cuda.Event()
             done.record()
         temporal_freqs.record_stream(self._table_stream)
