@@ -72,3 +72,18 @@ def test_bf16_rows_match_the_float64_rotation_bit_for_bit(batch, grid, heads, d)
         x4 = x.view(batch, n, heads, d)
         spread = torch.empty(batch, n, heads, d + 2, dtype=x.dtype, device=dev())[..., :d].copy_(x4)
         assert same(rope.causal_rope_apply(x4, grid, freqs, 5), rope.causal_rope_apply(spread, grid, freqs, 5))
+
+
+def test_factors_below_float32_are_rotated_in_float64():
+    """A table's smallest factors times the largest values: what float32 cannot hold of the factor is not in the rotation's bound."""
+    from worldattention_b200 import rope
+    g = torch.Generator(device=dev()).manual_seed(7)
+    n, heads, d = 12, 2, 128
+    sign = torch.randn(64, d // 2, 2, generator=g, device=dev(), dtype=torch.float64)
+    freqs = torch.view_as_complex(sign * 2.0 ** torch.randint(-170, -90, (64, d // 2, 2), generator=g, device=dev()).double()).cpu()
+    freqs[:, ::3] = freqs[:, ::3].imag * 1j + 1.0
+    x = (torch.randn(1, n, heads, d, generator=g, device=dev()) * 2.0 ** torch.randint(0, 120, (1, n, heads, d), generator=g, device=dev()).float()).bfloat16()
+    x[..., 1::4] = 0
+    spread = torch.empty(1, n, heads, d + 2, dtype=x.dtype, device=dev())[..., :d].copy_(x)
+    got, want = (rope.causal_rope_apply(t, (3, 2, 2), freqs, 5) for t in (x, spread))
+    assert torch.equal(got.contiguous().view(torch.int16), want.contiguous().view(torch.int16))

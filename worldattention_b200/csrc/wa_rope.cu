@@ -170,8 +170,9 @@ qk_norm_rope_rows_kernel(const __nv_bfloat16 *__restrict__ x, long long xsb, lon
 //   * the product with the weight is one bf16x2 instruction (the exact product rounded once);
 //   * the rotation is computed in float32 with the bound 2^-22 (|r| + |p|) on its distance from the float64 one (r the result, p
 //     the product subtracted or added; the factors', the product's and the sum's roundings are 2^-24 of these each): where both
-//     ends of that interval round to the same bf16, that is the result; the other pairs (about one in 3000) and those near zero are
-//     rotated in float64 as in the kernel above.  The results are therefore the same bits;
+//     ends of that interval round to the same bf16, that is the result; the other pairs (about one in 3000), those near zero and
+//     those with a factor below float32's normal range (whose rounding the bound does not cover) are rotated in float64 as in the
+//     kernel above.  The results are therefore the same bits;
 //   * four CTAs per SM: the 4680 tokens of a chunk are resident at once.
 // 12 heads of 128, 4680 tokens: 18.3 us with the general form, 10.5 here (2.7 TB/s; a chunk of q and k prepared and appended: 54.5 -> 39.0).
 template <int NV, bool WEIGHT, bool ROTATE>
@@ -197,6 +198,7 @@ qk_norm_rope_bits_kernel(const __nv_bfloat16 *__restrict__ x, long long xsb, lon
     const double2 *factors[3];                           // table rows of the three bands, at this lane's pairs
     const int ct = c - 2 * (c / 3), ch = c / 3;
     float fx[4], fy[4];
+    uint32_t smallest = 0xffffffffu;                     // exponent of the smallest factor that is not zero
     if constexpr (ROTATE) {
         if (start_frame_dev) start_frame = max(*start_frame_dev, 0);
         const int line = t / grid_w, fr = line / grid_h;
@@ -211,6 +213,7 @@ qk_norm_rope_bits_kernel(const __nv_bfloat16 *__restrict__ x, long long xsb, lon
             const double2 f = __ldg((jp < ct ? factors[0] : (jp < ct + ch ? factors[1] : factors[2])) + e);
             fx[e] = (float)f.x;
             fy[e] = (float)f.y;
+            smallest = min(smallest, min(2u * (uint32_t)__double2hiint(f.x) - 1u, 2u * (uint32_t)__double2hiint(f.y) - 1u));
         }
     }
 
@@ -282,6 +285,11 @@ qk_norm_rope_bits_kernel(const __nv_bfloat16 *__restrict__ x, long long xsb, lon
         }
     }
     if constexpr (ROTATE) {
+        if (smallest < 2u * 0x38100000u - 1u) {          // a factor below 2^-126
+#pragma unroll
+            for (int i = 0; i < NV; ++i)
+                if (i * 32 + lane < nvec) open |= 15u << (4 * i);
+        }
 #pragma unroll 1
         while (open) {
             const int k = __ffs((int)open) - 1;
