@@ -19,6 +19,11 @@ def _inputs(b, h, lq, lkv, seed, spread=1.0):
 
 @pytest.mark.parametrize("b,h,nq,nkv", [(1, 16, 16, 256), (1, 32, 17, 129), (2, 4, 80, 127), (1, 3, 81, 300), (1, 1, 33, 2049),
                                         (1, 40, 1, 1700), (1, 2, 97, 513), (1, 1, 15, 4096), (1, 1, 2, 128),
+                                        # on 148 SMs a CTA of the logits kernel holds one row tile of those above from 65 536 logits
+                                        # on, and two, three, four and five of these
+                                        (1, 40, 17, 129), (1, 24, 97, 129), (1, 40, 49, 300), (1, 40, 65, 300),
+                                        # a key per thread, and passes through shared memory beyond
+                                        (1, 3, 5, 257), (1, 3, 70, 512), (1, 3, 5, 513), (1, 3, 70, 1024),
                                         # short rows: a CTA per head, one, two or four keys per lane, and just beyond
                                         (1, 3, 1, 1), (2, 3, 7, 19), (1, 2, 37, 37), (1, 2, 64, 128), (2, 2, 32, 64), (1, 1, 16, 8), (1, 2, 33, 33),
                                         (4, 2, 16, 127), (4, 2, 8, 127), (1, 2, 32, 128), (1, 2, 33, 80), (1, 2, 64, 64),
