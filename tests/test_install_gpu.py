@@ -36,7 +36,7 @@ def test_fused_install_equals_the_separate_kernels(monkeypatch, frame, heads, d,
     calls = []
     fused = wa.hkv.HKVCache._install_fused
     monkeypatch.setattr(wa.hkv.HKVCache, "_install_fused", lambda self, *a: calls.append(fused(self, *a)) or calls[-1])
-    # pages of two frames and the last one of one; the pages of the second call do not fit and are cut
+    # pages of two frames and the last one of one; the last page of the second call does not fit and is left out
     for pairs, fits in ((((0, 1), (0, 3), (1, 0)), True), (((0, 0), (1, 1), (0, 3), (1, 0), (1, 3)), True)):
         start = [{n: t.clone() for n, t in b.items()} for b in cache]
         tokens = hkv.apply(cache, list(pairs), current_start_frame=40, temporal_freqs=freqs, hsa_modules=hsa)
@@ -75,7 +75,8 @@ def _small_bank(frame=16, layers=2, frames=5):
     hsa = [wa.hsa.HSAAttention(heads, d, block_size=64, proj_segment_len=frame).to(dev(), torch.bfloat16) for _ in range(layers)]
     size = frames * frame
     make = lambda n: torch.randn((1, n, heads, d), device=dev()).bfloat16()
-    cache = [{"k": make(size), "v": make(size), "k_coarse": make(frames), "v_coarse": make(frames),
+    slots = hsa[0].coarse_cache_size(size)
+    cache = [{"k": make(size), "v": make(size), "k_coarse": make(slots), "v_coarse": make(slots),
               "local_end_index": torch.tensor([size], device=dev()), "global_end_index": torch.tensor([size], device=dev())} for _ in range(layers)]
     freqs = torch.polar(torch.ones(64, 22, dtype=torch.float64), torch.randn(64, 22, dtype=torch.float64))
     hkv.store(cache, prompt_embeds=make(1).float()[:, :, 0], current_start_frame=frames, temporal_freqs=freqs)
@@ -148,3 +149,40 @@ def test_frequency_tables_on_the_device_in_every_view(view):
         hkv.store(cache, prompt_embeds=torch.ones(1, 1, 8), current_start_frame=900, temporal_freqs=freqs)
         indices.append(hkv.chunks[0]["page_index"])
     assert torch.equal(*indices)
+
+
+@pytest.mark.parametrize("frame", [16, 136])
+@pytest.mark.parametrize("half_frames,pages,installed", [(14, 4, 7), (15, 3, 6), (14, 3, 6), (3, 1, None)])
+def test_fused_install_at_the_end_of_the_cache(monkeypatch, frame, half_frames, pages, installed):
+    """A page of two frames cut to one, a capacity that is no multiple of a frame, and one that cuts a frame (refused: its slots
+    would be of a part of a segment)."""
+    hkv, hsa, bank, freqs = _small_bank(frame, frames=8)
+    capacity, slots = half_frames * frame // 2, (half_frames + 1) // 2 * hsa[0].proj_rank
+    make = lambda n: torch.randn((1, n, 1, 128), device=dev()).bfloat16()
+    for m in hsa:
+        torch.nn.init.normal_(m.k_proj_mat)
+        torch.nn.init.normal_(m.v_proj_mat)
+    cache = [{"k": make(capacity), "v": make(capacity), "k_coarse": make(slots), "v_coarse": make(slots),
+              "local_end_index": torch.tensor([0], device=dev()), "global_end_index": torch.tensor([0], device=dev())} for _ in hsa]
+    other = [{n: t.clone() for n, t in b.items()} for b in cache]
+    done = []
+    fused = wa_cache()._install_fused
+    monkeypatch.setattr(wa_cache(), "_install_fused", lambda self, *a: done.append(fused(self, *a)) or done[-1])
+    call = lambda c: hkv.apply(c, [(0, p) for p in range(pages)], current_start_frame=9, temporal_freqs=freqs, hsa_modules=hsa)
+    if installed is None:
+        with pytest.raises(ValueError, match="segment-aligned"):
+            call(cache)
+        return
+    assert call(cache) == installed * frame and done == [True]
+    monkeypatch.setattr(wa_cache(), "_install_fused", lambda self, *a: False)
+    assert call(other) == installed * frame
+    for got, want in zip(cache, other):
+        for name in want:
+            assert torch.equal(got[name], want[name]), name
+    for b, stored in zip(cache, hkv.tier.get(0)["v"]):
+        assert torch.equal(b["v"][:, :installed * frame], stored[:, :installed * frame]) and not b["v"][:, installed * frame:].any()
+
+
+def wa_cache():
+    from worldattention_b200.hkv import HKVCache
+    return HKVCache
