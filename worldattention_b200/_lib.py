@@ -221,8 +221,8 @@ def raise_if_failed(device: torch.device) -> None:
     at the next call or at the caller's next synchronisation point followed by this check.
     """
     word = _status_words.get(torch.device(device).index or 0)
-    if word is not None and int(word[0]) != 0:
-        code = int(word[0])
+    code = 0 if word is None else word.item()
+    if code != 0:
         word.zero_()
         if 301 <= code <= 309:
             raise RuntimeError(f"an earlier HKV install on {device} gave up at wait site {code}; the installed pages and slots are invalid")
