@@ -206,7 +206,8 @@ extern "C" int wa_hsa_forward(const wa_hsa_params *p, int *used_tuned, void *str
         index = const_cast<int32_t *>(p->index_in);
         num = const_cast<int32_t *>(p->num_in);
     } else {
-        // pooling, then scores + sort + thresholds + counts (+ the tcgen05 kernel's work order) in one launch
+        // pooling, then scores + sort + thresholds + counts (+ the tcgen05 kernel's work order): one launch, or two where the
+        // scores of many rows come from a kernel of their own
         int *counters = (int *)(ws + w.counters);
         if ((rc = pool_launch(&p->q, p->Lq, q_pooled, &p->k, p->Lkv, k_pooled, p->B, p->H, p->D, p->block_size, stream,
                               counters, p->H + 1, k_first, p->status_mirror)))

@@ -221,8 +221,10 @@ int pool_sm100_launch(const wa_tensor4 *x, int Lx, float *px, const wa_tensor4 *
     const long long items = (long long)B * (job.nbx + job.nby) * job.tiles;
     WA_REQUIRE(items < (1ll << 40), WA_ERR_UNSUPPORTED, "%s: too many blocks", what);
     const int grid = items < sms ? (int)items : sms;
-    // The fourth group pays where the stream is long: 480 frames, the whole call, 1126 -> 1100 us; over a window of 21 (115 MB) the call is
-    // 4 % slower with it and over three frames 1 %, the next launch finding less room beside it.
+    // The fourth group pays where the stream is long (whole calls with 64-token blocks, three and four groups: 526 MB 422 and 415 us, 745 MB
+    // 517 and 508, 1111 MB 664 and 649, 2.2 GB 1114 and 1086).  Below the difference is small and goes either way with what runs next: 1 to
+    // 1.5 % for four groups over 110 to 480 MB with 64-token blocks, 4 % against them over a window of 115 MB with 128-token blocks, the next
+    // launch finding less room beside them.
     const bool four = (long long)B * (Lx + (y ? Ly : 0)) * H * D * 2 > (512ll << 20);
     const cudaError_t le = four ? launch_dependent(pool_stream_kernel<4>, dim3(grid), dim3(threads_of(4)), SMEM_BYTES, stream, tx, ty, job)
                                 : launch_dependent(pool_stream_kernel<3>, dim3(grid), dim3(threads_of(3)), SMEM_BYTES, stream, tx, ty, job);

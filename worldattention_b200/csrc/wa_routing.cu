@@ -639,9 +639,9 @@ __device__ __forceinline__ void sort_keys_smem(unsigned long long *keys, int n_p
 // the full bitonic sort (105 passes over 16384 keys) was two thirds of the routing kernel.  Keys are the sort's own
 // 64-bit keys (descending probability, then ascending id; all distinct).  A most-significant-byte-first radix select
 // narrows down the k-th smallest key (histogram passes over the row: it stops as soon as one histogram bin holds exactly the
-// keys still needed, or the keys at or below the bin are at most 1024), the keys at or below it are collected and only
-// they are sorted.  `idx[0..k)` receive the same ids in the same order as the full sort; slots past k are not written.
-// `keys` is shared memory for `key_slots` >= max(1024, pow2(k)) entries.  Called by every thread of the CTA (>= 256 threads).
+// keys still needed, or the keys at or below the bin are no more than the CTA's threads), the keys at or below it are collected
+// and only they are sorted.  `idx[0..k)` receive the same ids in the same order as the full sort; slots past k are not written.
+// `keys` is shared memory for `key_slots` >= max(threads, pow2(k)) entries.  Called by every thread of the CTA (256 to 1024 of them).
 // A larger k is selected in pieces: `from` is the smallest key still to be had and `n_left` how many there are of those; returns
 // the largest key taken.
 __device__ __forceinline__ unsigned long long select_top_blocks(const float *probs, int Nkv, int k, unsigned long long *keys, int key_slots,
@@ -1450,7 +1450,11 @@ int route_fused_launch(const float *q_pooled, const float *k_pooled, int B, int 
     WA_REQUIRE(rows < (1ll << 31), WA_ERR_UNSUPPORTED, "wa_hsa_forward(routing): too many rows");
     int threads = n_pow2 / 2;
     threads = threads < 256 ? 256 : (threads > 1024 ? 1024 : threads);
-    if (n_pow2 == 512) threads = 512;      // a key per thread: 45 passes through shared memory took 13 of a row's 19 us, with shuffles 4
+    // A key per thread up to 512 key blocks: 45 passes through shared memory took 13 of a row's 19 us there, with shuffles 4 (whole calls
+    // with 256 and 512 threads, 74 rows of 12 heads over 257 blocks: 190 and 175 us; over 512: 242 and 229).  Beyond, a row's CTA
+    // of 1024 threads fills half an SM, and what the sort gains is lost on the other steps (512 and 1024 threads, 74 over 585: 301 and
+    // 299 us; over 700: 316 and 315; over 1024: 388 and 389; 37 over 513: 201 and 192).
+    if (n_pow2 == 512) threads = 512;
     // a fixed count per head over more key blocks than one pass of the register sort covers, and nobody reads the whole
     // order or the thresholds: select the best blocks instead of sorting all of them
     const int select_only = fixed_num_per_head && !whole_order && n_pow2 > threads;
