@@ -175,3 +175,19 @@ def test_host_pages_are_not_handed_out_again_while_they_cross(tmp_path, tier):
     for got, want in zip(cache, first):
         assert torch.equal(got["k"], want["k"]) and torch.equal(got["v"], want["v"])
     del others
+
+
+@pytest.mark.parametrize("frame,heads,head_dim", [(218, 1, 128), (1500, 1, 128), (16, 3, 64), (16, 32, 4)])
+def test_an_install_that_is_not_covered_puts_no_tables_together(monkeypatch, frame, heads, head_dim):
+    from worldattention_b200.hkv import cache as C
+    from worldattention_b200.hsa import HSAAttention
+    hkv = C.HKVCache(frame_seq_length=frame, page_size_frames=2)
+    make = lambda n: torch.zeros(1, n, heads, head_dim, dtype=torch.bfloat16)
+    cache = [{"k": make(2 * frame), "v": make(2 * frame), "k_coarse": make(48), "v_coarse": make(48)}]
+    caches = C._Table([cache[0]["k"], cache[0]["v"]])
+    hsa = [HSAAttention(heads, head_dim, block_size=64, proj_segment_len=frame)]
+    plan = np.zeros(1, dtype=hkv._PLAN_DTYPE)
+    plan["count"] = 2 * frame
+    monkeypatch.setattr(C, "_Table", lambda tensors: pytest.fail("put together for nothing"))
+    dst = caches.starts(1, 2)
+    assert hkv._install_fused(cache, plan, dst[None], caches, dst, np.full(1, -1), None, 22, torch.device("cpu"), hsa) is False

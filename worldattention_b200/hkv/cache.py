@@ -40,14 +40,14 @@ class _Table:
 
     def __init__(self, tensors):
         t = np.frombuffer(_lib.host().tensor_table(tensors), dtype=np.int64).reshape(-1, 12)
+        self.columns = t
         self.ptr, self.device, self.dtype, self.dim, self.size, self.stride = t[:, 0], t[:, 1], t[:, 2], t[:, 3], t[:, 4:8], t[:, 8:]
 
     def cache_rows(self, like: "_Table") -> np.ndarray:
         """Which tensors hold token rows of the heads, type and device of `like`'s first without gaps inside a row or between rows."""
-        heads, head_dim = like.size[0, 2:]
-        return ((self.dim == 4) & (self.dtype == like.dtype[0]) & (self.device == like.device[0]) & (self.size[:, 2] == heads)
-                & (self.size[:, 3] == head_dim) & (self.stride[:, 3] == 1) & (self.stride[:, 2] == head_dim)
-                & (self.stride[:, 1] == heads * head_dim))
+        _, device, dtype, _, _, _, heads, head_dim = like.columns[0, :8].tolist()
+        # device, type, dimensions; heads and channels; strides of rows, heads and channels
+        return (self.columns[:, (1, 2, 3, 6, 7, 9, 10, 11)] == (device, dtype, 4, heads, head_dim, heads * head_dim, head_dim, 1)).all(axis=1)
 
     def starts(self, batch: int, esize: int) -> np.ndarray:
         """`[tensor, batch item]` addresses."""
@@ -360,19 +360,20 @@ class HKVCache:
         mine = np.flatnonzero((rows > 0) & direct)
         if mine.size == 0:
             return
-        items = np.repeat(mine, table.size[mine, 0])                                     # a record per tensor and batch item
-        batch = np.concatenate([np.arange(n) for n in table.size[mine, 0]])
+        items, batch = mine, 0                                                           # a record per tensor and batch item
+        if (table.size[mine, 0] != 1).any():
+            items, batch = np.repeat(mine, table.size[mine, 0]), np.concatenate([np.arange(n) for n in table.size[mine, 0]])
         records = np.zeros(len(items), dtype=RECORD_DTYPE)
         records["dst"] = (table.ptr[items] + (batch * table.stride[items, 0] + ends[items] * row_elems) * esize).astype(np.uint64)
         records["n_tokens"], records["dst_stride"] = rows[items], row_elems
         clear_rows_device(to_device(records.view(np.uint8), dev), max_tokens=int(rows[mine].max()), row_elems=row_elems, elem_size=esize)
 
     def _install_sources(self, kv_cache, plan, blobs, dtype):
-        """Where the pages come from: `(whole, single, staging)`; cold pages are on their way to the staging buffer.
+        """Where the pages come from and go to: `(whole, single, staging, caches)`; cold pages are on their way to the staging buffer.
 
         `whole` maps a chunk that lies on the device in the cache's own layout to the tensors of all layers and their table (its
         pages are rows of those); `single` lists the pages of every other chunk one by one, as (layer, name, plan row, tensor or host
-        page, offset in the staging buffer or None).
+        page, offset in the staging buffer or None); `caches` is the table of the online tensors, (layer, K|V).
         """
         k0 = kv_cache[0]["k"]
         bsz, _, heads, head_dim = k0.shape
@@ -402,7 +403,7 @@ class HKVCache:
                         slot = staged_elems                      # cold page in the cache's own layout: one block copy per item
                         staged_elems += bsz * n * row_elems
                     single.append((layer, name, i, page, slot))
-        return whole, single, self._promote(single, staged_elems, k0) if staged_elems else None
+        return whole, single, self._promote(single, staged_elems, k0) if staged_elems else None, caches
 
     def _promote(self, single, staged_elems: int, k0: torch.Tensor) -> torch.Tensor:
         """Cold pages in the cache's own layout cross on the side stream into ONE staging buffer, one block copy per item: the first
@@ -435,7 +436,7 @@ class HKVCache:
 
         With `hsa_modules` and where the fused kernel covers the call, the compressed slots are written by that launch too
         (True); otherwise one page-copy launch for every (layer, page, K|V, batch item) (False)."""
-        whole, single, staging = sources
+        whole, single, staging, caches = sources
         k0 = kv_cache[0]["k"]
         bsz, _, heads, head_dim = k0.shape
         row_elems = heads * head_dim
@@ -451,8 +452,7 @@ class HKVCache:
         # buffer early
         keep_alive = [staging]
         promoted = staging is not None
-        # first row of every (page, tensor, batch item) on the device, elements between its rows; a tensor is (layer, K|V)
-        caches = _Table([block[name] for block in kv_cache for name in ("k", "v")])
+        # first row of every (page, tensor, batch item) on the device, elements between its rows
         dst = caches.starts(bsz, esize)
         batch = np.arange(bsz, dtype=np.int64) * esize
         src = np.zeros((len(plan),) + dst.shape, dtype=np.int64)
@@ -509,7 +509,11 @@ class HKVCache:
         k0 = kv_cache[0]["k"]
         bsz, _, heads, head_dim = k0.shape
         frame, esize = self.frame_seq_length, k0.element_size()
-        if k0.dtype != torch.bfloat16 or (plan["count"] % frame).any() or (plan["src"] % frame).any():
+        # most of what the native call would refuse, before the tables that it looks at are put together (a projection of 218 or 1500
+        # tokens: 150 us of host work for nothing)
+        proj = getattr(hsa_modules[0], "k_proj_mat", None)
+        if (k0.dtype != torch.bfloat16 or heads * head_dim % 128 or head_dim % 8 or not isinstance(proj, torch.Tensor) or proj.dim() != 2
+                or proj.shape[1] % 8 or proj.dtype != k0.dtype or (plan["count"] % frame).any() or (plan["src"] % frame).any()):
             return False
         # tiers whose slots the compress kernel does not write either are the module's own business (`compress_kv_cache`), and all
         # that is asked of such a module
