@@ -174,7 +174,7 @@ qk_norm_rope_rows_kernel(const __nv_bfloat16 *__restrict__ x, long long xsb, lon
 //     those with a factor below float32's normal range (whose rounding the bound does not cover) are rotated in float64 as in the
 //     kernel above.  The results are therefore the same bits;
 //   * four CTAs per SM: the 4680 tokens of a chunk are resident at once.
-// 12 heads of 128, 4680 tokens: 18.3 us with the general form, 10.5 here (2.7 TB/s; a chunk of q and k prepared and appended: 54.5 -> 39.0).
+// 12 heads of 128, 4680 tokens: 18.3 us with the general form, 10.1 here (2.8 TB/s; a chunk of q and k prepared and appended: 54.5 -> 39.0).
 template <int NV, bool WEIGHT, bool ROTATE>
 __global__ void __launch_bounds__(RN_WARPS * 32, NV > 6 ? 3 : 4)
 qk_norm_rope_bits_kernel(const __nv_bfloat16 *__restrict__ x, long long xsb, long long xsl, __nv_bfloat16 *__restrict__ out,
