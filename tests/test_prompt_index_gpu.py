@@ -37,3 +37,15 @@ def _dual(f, x, tangent):
     from torch.autograd import forward_ad
     with forward_ad.dual_level():
         return tuple(forward_ad.unpack_dual(f(forward_ad.make_dual(x, tangent))))
+
+
+def test_prompt_index_is_recorded_as_tensor_expressions():
+    from torch.fx.experimental.proxy_tensor import make_fx
+    from torch.utils.flop_counter import FlopCounterMode
+    from worldattention_b200.hkv.retrieval import prompt_index
+    first, other = (torch.randn((2, 16, 8), generator=torch.Generator(device=dev()).manual_seed(s), device=dev()) for s in (1, 2))
+    recorded = [torch.jit.trace(prompt_index, first), make_fx(prompt_index)(first), torch.compile(prompt_index, backend="eager", fullgraph=True)]
+    for f in recorded:       # of another input: a result that was computed while recording would be the first one's
+        torch.testing.assert_close(f(other), prompt_index(other), rtol=0, atol=2e-6)
+    with FlopCounterMode(display=False):
+        torch.testing.assert_close(prompt_index(first), recorded[1](first), rtol=0, atol=2e-6)

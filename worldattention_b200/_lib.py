@@ -179,9 +179,12 @@ def dtype_code(dtype: torch.dtype) -> int:
 
 
 def is_plain(t) -> bool:
-    """A tensor whose memory stands for it: no subclass, no wrapper of a function transform (vmap, jvp, grad) and, outside a
-    forward-mode level, no tangent."""
-    return type(t) is torch.Tensor and not torch._C._functorch.is_functorch_wrapped_tensor(t) and torch.autograd.forward_ad._current_level < 0
+    """A tensor whose memory stands for it, in a call that only its result is wanted of: no subclass, no wrapper of a function
+    transform (vmap, jvp, grad), no tangent of a forward-mode level, and nobody recording operations (tracing, compiling, a
+    dispatch mode)."""
+    return (not torch.compiler.is_compiling() and type(t) is torch.Tensor and not torch._C._functorch.is_functorch_wrapped_tensor(t)
+            and torch.autograd.forward_ad._current_level < 0 and torch._C._get_tracing_state() is None
+            and torch._C._len_torch_dispatch_stack() == 0)
 
 
 def require_cuda(*tensors: torch.Tensor) -> torch.device:
