@@ -178,20 +178,28 @@ class _CrossAttention(nn.Module):   # model.py:165-200 (text-to-video), keys/val
         return self.o(y.transpose(1, 2).reshape(b, s, d))
 
 
+def _unobserved(*modules) -> bool:
+    """Whether calling these modules is calling their class's `forward` and nothing else: no hooks, no `forward` of an instance."""
+    for m in modules:
+        if m._forward_hooks or m._forward_pre_hooks or "forward" in m.__dict__:
+            return False
+    return not nn.modules.module._has_any_global_hook()
+
+
 def feed_forward(ffn: nn.Module, x: torch.Tensor) -> torch.Tensor:
     """`ffn(x)`; of a Linear, a tanh GELU and a Linear without gradients, the GELU in the first product's epilogue, on its float32
     sums: the separate launch reads and writes the widest activation of a block once more (4680 x 8960: 131.5 -> 95.5 us; distance
-    of the hidden values from float64 2.7e-3 -> 1.7e-3, there being one rounding to bf16 less)."""
-    if (type(ffn) is nn.Sequential and [type(m) for m in ffn] == [nn.Linear, nn.GELU, nn.Linear] and _lib.is_plain(x) and x.is_cuda
-            and x.dtype == torch.bfloat16 and x.numel() > 0 and not torch.is_grad_enabled() and not torch.is_autocast_enabled("cuda")):
-        first, act, second = ffn
-        # a weight or bias of another type (quantised, distributed, swapped in by a transform) and whatever hangs on the modules' calls
-        # go through the modules
-        if (type(first.weight) is nn.Parameter and type(first.bias) is nn.Parameter and first.weight.dtype == x.dtype and act.approximate == "tanh"
-                and not nn.modules.module._has_any_global_hook()
-                and not any(m._forward_hooks or m._forward_pre_hooks or "forward" in vars(m) for m in (ffn, first, act))):
-            h = torch._addmm_activation(first.bias, x.reshape(-1, x.shape[-1]), first.weight.t(), use_gelu=True)
-            return second(h.view(*x.shape[:-1], -1))
+    of the hidden values from float64 2.7e-3 -> 1.7e-3, there being one rounding to bf16 less).  `x` is the result of a launch of
+    this library, so no transform's wrapper and no tangent."""
+    if x.is_cuda and x.dtype == torch.bfloat16 and type(ffn) is nn.Sequential and len(ffn._modules) == 3 and not torch.is_grad_enabled():
+        first, act, second = ffn._modules.values()
+        if type(first) is nn.Linear and type(act) is nn.GELU and type(second) is nn.Linear and act.approximate == "tanh":
+            # a weight or bias of another type (quantised, distributed, swapped in by a transform) goes through the module
+            weight, bias = first._parameters.get("weight"), first._parameters.get("bias")
+            if (type(weight) is nn.Parameter and type(bias) is nn.Parameter and weight.dtype == x.dtype and _unobserved(ffn, first, act)
+                    and not torch.is_autocast_enabled("cuda")):
+                b, n, c = x.shape
+                return second(torch._addmm_activation(bias, x.view(b * n, c), weight.t(), use_gelu=True).view(b, n, weight.shape[0]))
     return ffn(x)
 
 
@@ -270,9 +278,8 @@ class CausalDiT(nn.Module):
         """The output head's norm and modulation: one launch where the blocks' own are, and the norm is the one that the launch computes."""
         norm, tokens = self.head_norm, self.cfg.frame_tokens
         if (x.is_cuda and x.dtype == scale.dtype == torch.bfloat16 and not torch.is_grad_enabled() and x.shape[1] == scale.shape[1] * tokens
-                and x.shape[2] % 8 == 0 and x.shape[2] <= 4096 and all(getattr(blk, "fused", False) for blk in self.blocks)
-                and type(norm) is _LayerNorm and norm.weight is None and norm.bias is None and norm.normalized_shape == x.shape[2:]
-                and not (norm._forward_hooks or norm._forward_pre_hooks or "forward" in vars(norm) or nn.modules.module._has_any_global_hook())):
+                and x.shape[2] % 8 == 0 and x.shape[2] <= 4096 and type(norm) is _LayerNorm and not norm.elementwise_affine
+                and norm.normalized_shape == x.shape[2:] and _unobserved(norm) and all([getattr(blk, "fused", False) for blk in self.blocks])):
             return ln_modulate(x, norm.eps, scale=scale, shift=shift, tokens_per_frame=tokens)
         return (norm(x).unflatten(1, (scale.shape[1], tokens)) * (1 + scale) + shift).flatten(1, 2)
 
@@ -297,7 +304,7 @@ class CausalDiT(nn.Module):
             x = blk(x, e0, context, cache, cross, plan, table)
         m = (self.head_modulation.unsqueeze(1) + e.unflatten(0, (b, f)).unsqueeze(2)).chunk(2, dim=2)
         tokens = cfg.frame_tokens
-        x = self.head(self._modulated(x, m[1], m[0]).unflatten(1, (f, tokens)))                     # [B, F, tokens, p*C]
+        x = self.head(self._modulated(x, m[1], m[0]).view(b, f, tokens, cfg.dim))                   # [B, F, tokens, p*C]
         gh, gw = cfg.grid_hw
         x = x.view(b, f, gh, gw, cfg.patch[1], cfg.patch[2], cfg.out_channels)
         return x.permute(0, 1, 6, 2, 4, 3, 5).reshape(b, f, cfg.out_channels, gh * cfg.patch[1], gw * cfg.patch[2])
