@@ -50,3 +50,19 @@ def test_best_blocks_of_long_rows(topk, spread):
     picked = hsa_attention(*qkv, topk_per_head=counts, **kwargs)
     whole, (_, num, _, _) = hsa_attention(*qkv, topk_per_head=counts, return_routing=True, **kwargs)
     assert num.unique().tolist() == sorted(set(topk)) and torch.equal(picked, whole)
+
+
+# fixed counts: one row per CTA of 128 (logits ready), 256 or 512 threads, up to 32 blocks per thread; few and many best blocks
+# collected, ordered by counting, by sorting, or (beyond 2048) in pieces
+@pytest.mark.parametrize("nq,nkv,topk", [(3, 1, (1, 0, 1)), (3, 129, (4, 129, 0)), (90, 256, (16, 127, 256)), (90, 255, (1, 33, 128)),
+                                         (60, 511, (32, 129, 511)), (3, 257, (31, 256, 257)), (30, 2048, (8, 257, 2047)),
+                                         (2, 2049, (64, 513, 2049)), (2, 4097, (32, 512, 3000)), (2, 8193, (1, 100, 600)),
+                                         (2, 16384, (32, 16384, 2048))])
+@pytest.mark.parametrize("spread", [1.0, 0.0])
+def test_best_blocks_by_count(nq, nkv, topk, spread):
+    from worldattention_b200.hsa import hsa_attention
+    qkv, kwargs = _inputs(1, 3, nq * BLOCK, nkv * BLOCK - 3, nkv, spread)
+    counts = torch.tensor(topk, dtype=torch.int32)
+    picked = hsa_attention(*qkv, topk_per_head=counts, **kwargs)
+    whole, (_, num, _, _) = hsa_attention(*qkv, topk_per_head=counts, return_routing=True, **kwargs)
+    assert num.unique().tolist() == sorted(set(topk)) and torch.equal(picked, whole)

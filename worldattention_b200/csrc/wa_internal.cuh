@@ -125,28 +125,33 @@ __device__ __forceinline__ void sort_items_by_head(Count count_of, int n_items, 
     }
 }
 
-// Work order of the items (a row of `num`, or two neighbouring ones of a head), heavy first (weight: selected blocks; of a
+// Work order of the items (a row of the routing, or two neighbouring ones of a head), heavy first (weight: selected blocks; of a
 // pair of rows the larger count).  Called by every thread of ONE CTA whose size is a power of two between 32 and 1024.
-// The counts were written by other CTAs of this launch: they are read past L1.
-__device__ inline void schedule_items(const int32_t *num, int rows, int Nq, int Nkv, const SchedJob &job) {
+// `num_of(row)` is a row's count.
+template <typename Num>
+__device__ __forceinline__ void schedule_items_by(Num num_of, int rows, int Nq, int Nkv, const SchedJob &job) {
     __shared__ int hist[SCHED_BINS];
     __shared__ int warp_tot[32];
     if (!job.paired) {
-        sort_items([&](int i) { return __ldcg(num + i); }, rows, Nkv, hist, warp_tot, job.order, job.work_counter, job.error_flag);
+        sort_items(num_of, rows, Nkv, hist, warp_tot, job.order, job.work_counter, job.error_flag);
         return;
     }
     const int each = (Nq + 1) >> 1, heads = rows / Nq, n_items = heads * each;
     // without branches, so that a thread's look-ups are all on their way at once (one after the other they cost the call 3 us)
     auto count_of = [&](int i) {
-        const int head = i / each, q = 2 * (i - head * each);
-        const int32_t *at = num + (long long)head * Nq + q;
-        return max(__ldcg(at), __ldcg(at + (q + 1 < Nq ? 1 : 0)));
+        const int head = i / each, q = 2 * (i - head * each), at = head * Nq + q;
+        return max(num_of(at), num_of(at + (q + 1 < Nq ? 1 : 0)));
     };
     // calls with so many items that ranking them against one another would take too long are sorted over all heads
     if (job.by_head && heads <= SCHED_HEADS && n_items <= SCHED_BINS - 2 * SCHED_HEADS && (long long)n_items * each <= 2048ll * blockDim.x)
         sort_items_by_head(count_of, n_items, each, Nkv, hist, job.order, job.work_counter, job.error_flag);
     else
         sort_items(count_of, n_items, Nkv, hist, warp_tot, job.order, job.work_counter, job.error_flag);
+}
+
+// The counts were written by other CTAs of this launch: they are read past L1.
+__device__ inline void schedule_items(const int32_t *num, int rows, int Nq, int Nkv, const SchedJob &job) {
+    schedule_items_by([&](int row) { return __ldcg(num + row); }, rows, Nq, Nkv, job);
 }
 
 // Elements [first, first + count) of the gate weight -> bf16 (it is an MMA operand) and of the bias -> float32.

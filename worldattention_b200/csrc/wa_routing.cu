@@ -800,7 +800,7 @@ __device__ __forceinline__ void route_row(const long long row, const bool logits
                                           float tau_min, float tau_span, const int32_t *__restrict__ fixed_num, float *sorted,
                                           int32_t *__restrict__ index, int32_t *num, float *__restrict__ thresholds, float *gini_rows,
                                           int *counters, const SchedJob &job, unsigned long long *keys, float *probs, double *red,
-                                          float &bcast, int &last_flag, const bool select_only, const int key_slots) {
+                                          float &bcast, int &last_flag) {
     const int T = blockDim.x, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, nwarps = T >> 5;
     const long long bh = row / Nq;
     const int h = (int)(bh % H);
@@ -816,13 +816,7 @@ __device__ __forceinline__ void route_row(const long long row, const bool logits
     row_softmax(Nkv, probs, red, &bcast);
     ROUTE_STAMP(2);
 
-    if (select_only) {
-        // fixed per-head count and nobody asked for the whole order or the thresholds: pick the head's k best blocks
-        const int want = max(0, min(fixed_num[h], Nkv));
-        unsigned long long from = 0ull;
-        for (int at = 0; at < want; at += key_slots)
-            from = select_top_blocks(probs, Nkv, min(want - at, key_slots), keys, key_slots, index + row * Nkv + at, 0, nullptr, from, Nkv - at) + 1ull;
-    } else if (n_pow2 <= T) {
+    if (n_pow2 <= T) {
         unsigned long long key = sort_key_per_thread(
             tid < Nkv ? (((unsigned long long)descending_key(probs[tid]) << 32) | (unsigned)tid) : 0xFFFFFFFFFFFFFFFFull, keys, n_pow2);
         keys[tid] = key;
@@ -835,25 +829,23 @@ __device__ __forceinline__ void route_row(const long long row, const bool logits
         sort_keys_smem(keys, n_pow2);
     }
     ROUTE_STAMP(3);
-    if (!select_only) {
-        int32_t *idx = index + row * Nkv;
-        double acc = 0.0;
-        for (int m = tid; m < Nkv; m += T) {
-            const int id = (int)(keys[m] & 0xFFFFFFFFull);
-            idx[m] = id;
-            const float w = __fsub_rn((float)(Nkv + 1), __fmul_rn(2.0f, (float)(m + 1)));
-            acc += (double)__fmul_rn(w, probs[id]);
-        }
-        acc = warp_sum_d(acc);
-        if (lane == 0) red[warp] = acc;
-        __syncthreads();
-        if (tid == 0) {
-            double t = 0.0;
-            for (int w = 0; w < nwarps; ++w) t += red[w];
-            gini_rows[row] = __fdiv_rn((float)t, (float)Nkv);
-        }
-        __syncthreads();
+    int32_t *idx = index + row * Nkv;
+    double acc = 0.0;
+    for (int m = tid; m < Nkv; m += T) {
+        const int id = (int)(keys[m] & 0xFFFFFFFFull);
+        idx[m] = id;
+        const float w = __fsub_rn((float)(Nkv + 1), __fmul_rn(2.0f, (float)(m + 1)));
+        acc += (double)__fmul_rn(w, probs[id]);
     }
+    acc = warp_sum_d(acc);
+    if (lane == 0) red[warp] = acc;
+    __syncthreads();
+    if (tid == 0) {
+        double t = 0.0;
+        for (int w = 0; w < nwarps; ++w) t += red[w];
+        gini_rows[row] = __fdiv_rn((float)t, (float)Nkv);
+    }
+    __syncthreads();
     if (!fixed_num) {
         // What the count needs of this row once the head's threshold is known: for every sorted position the
         // cumulative mass before it, fl32(fl64 prefix including m) - p_m.  A contiguous run of positions per thread,
@@ -893,8 +885,8 @@ __device__ __forceinline__ void route_row(const long long row, const bool logits
     if (!last_flag) return;
     __threadfence();
 
-    const float thr = select_only ? 0.f : head_threshold(gini_rows, B, H, Nq, h, tau_min, tau_span, red, &bcast);
-    if (tid == 0 && !select_only) thresholds[h] = thr;
+    const float thr = head_threshold(gini_rows, B, H, Nq, h, tau_min, tau_span, red, &bcast);
+    if (tid == 0) thresholds[h] = thr;
     ROUTE_STAMP(8);
     if (fixed_num) {
         const int n = max(0, min(fixed_num[h], Nkv));
@@ -1001,8 +993,7 @@ __global__ void __launch_bounds__(1024)
 route_fused_kernel(const float *__restrict__ qp, const float *__restrict__ kp, int B, int H, int Nq, int Nkv, int n_pow2,
                    int D, float scale, float tau_min, float tau_span, const int32_t *__restrict__ fixed_num,
                    float *sorted, int32_t *__restrict__ index, int32_t *num, float *__restrict__ thresholds,
-                   float *gini_rows, int *counters, SchedJob job, int gate_per_cta, int sm_count, int slots, int select_only,
-                   int logits_ready, int key_slots) {
+                   float *gini_rows, int *counters, SchedJob job, int gate_per_cta, int sm_count, int slots, int logits_ready, int key_slots) {
     extern __shared__ __align__(16) unsigned char fused_smem[];
     unsigned long long *keys = reinterpret_cast<unsigned long long *>(fused_smem);   // key_slots
     float *probs = reinterpret_cast<float *>(keys + key_slots);                      // Nkv
@@ -1022,7 +1013,7 @@ route_fused_kernel(const float *__restrict__ qp, const float *__restrict__ kp, i
     ROUTE_STAMP(0);
     if (job.order && job.gate_w) convert_gate_slice(job, (int)row * gate_per_cta, gate_per_cta);
     route_row(row, logits_ready != 0, qp, kp, B, H, Nq, Nkv, n_pow2, D, scale, tau_min, tau_span, fixed_num, sorted, index, num, thresholds,
-              gini_rows, counters, job, keys, probs, red, bcast, last_flag, select_only != 0, key_slots);
+              gini_rows, counters, job, keys, probs, red, bcast, last_flag);
 }
 
 // ------------------------------------------------------------------------------------------------
@@ -1170,6 +1161,146 @@ route_head_kernel(const float *__restrict__ qp, const float *__restrict__ kp, in
     if (!last_flag || !job.order) return;
     __threadfence();
     schedule_items(num, B * H * Nq, Nq, Nkv, job);
+}
+
+// ------------------------------------------------------------------------------------------------
+// Routing with a fixed count per head where nobody reads the whole order or the thresholds: a row per CTA, V blocks per thread
+// in registers from the logit to the key, and only the best blocks are ordered.  Every warp sorts its lanes' best keys; with
+// W warps and c = ceil(count / W), at least W * c >= count blocks lie at or below the worst of the warps' c-th keys, so what lies
+// above it cannot be among the best.  The few blocks at or below it (26 of 256 for a count of 16, about 90 of 11 700 for 32) are
+// collected and each counts how many of them come before it, which is its place.  Same probabilities and keys as route_row,
+// hence the same ids in the same order.  The counts are known without the routing, so the attention kernel's work order is
+// made by a CTA of its own (the first) beside the rows instead of by the last one after them.
+// Bound by latency (a row is a chain of four block-wide exchanges) and, over thousands of blocks, by the float64 exponentials.
+// 128 threads a row up to 512 blocks; 256 where the row makes its own logits (a warp per eight dot products) or has up to
+// 2048; beyond, 512 threads with two CTAs per SM.
+// Before, a row was sorted (or, beyond 1024 blocks, selected by radix passes) with its Gini term, and two counters led to the last CTA.
+// 12 heads, 37 rows over 256 blocks: 16.7 -> 7.8 us, the call 134.0 -> 128.6; 74 rows over 11 700: 117 -> 78, the call 1150 -> 1125.
+// ------------------------------------------------------------------------------------------------
+template <int T, int V>
+__global__ void __launch_bounds__(T, 1024 / T)
+route_topk_kernel(const float *__restrict__ qp, const float *__restrict__ kp, int H, int Nq, int Nkv, int D, float scale,
+                  const int32_t *__restrict__ fixed_num, float *logits, int32_t *__restrict__ index, int32_t *__restrict__ num, SchedJob job,
+                  int rows, int gate_per_cta, int sm_count, int per_sm, int logits_ready) {
+    constexpr int W = T / 32, SLOTS = V * T < 2048 ? V * T : 2048;
+    extern __shared__ float own_logits[];                // Nkv, where the row makes them
+    __shared__ __align__(16) unsigned long long keys[SLOTS];
+    __shared__ float top[W];
+    __shared__ double sums[W];
+    __shared__ uint32_t bounds[W];
+    __shared__ int n_near;
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    pdl_wait();                 // pooled means, or logits, come from the launch before
+    if (job.release_at_start) pdl_release_dependents();
+    if (blockIdx.x == 0) {
+        if (job.order)
+            schedule_items_by([&](int row) { return __ldg(fixed_num + (row / Nq) % H); }, rows, Nq, Nkv, job);
+        return;
+    }
+    // neighbouring rows (same head, same pooled keys) on one SM, as in route_fused_kernel
+    const int at = blockIdx.x - 1, row = (at % sm_count) * per_sm + at / sm_count;
+    if (row >= rows) return;
+    if (job.order && job.gate_w) convert_gate_slice(job, row * gate_per_cta, gate_per_cta);
+
+    const int want = max(0, min(fixed_num[(row / Nq) % H], Nkv));
+    if (tid == 0) {
+        num[row] = want;
+        n_near = 0;
+    }
+    if (want == 0) return;
+    float *lrow = logits + (long long)row * Nkv;
+    if (!logits_ready) {
+        row_logits(qp + (long long)row * D, kp + (long long)(row / Nq) * Nkv * D, Nkv, D, scale, own_logits);
+        __syncthreads();
+    }
+    float e[V], m = -INFINITY;
+#pragma unroll
+    for (int u = 0; u < V; ++u) {
+        const int j = u * T + tid;
+        e[u] = j < Nkv ? (logits_ready ? __ldcg(lrow + j) : own_logits[j]) : -INFINITY;
+    }
+#pragma unroll
+    for (int u = 0; u < V; ++u) m = fmaxf(m, e[u]);
+    m = warp_max(m);
+    if (lane == 0) top[warp] = m;
+    __syncthreads();
+#pragma unroll
+    for (int w = 0; w < W; ++w) m = fmaxf(m, top[w]);
+    double sum = 0.0;
+#pragma unroll
+    for (int u = 0; u < V; ++u)
+        if (u * T + tid < Nkv) {
+            e[u] = (float)exp((double)__fsub_rn(e[u], m));
+            sum += (double)e[u];
+        }
+    sum = warp_sum_d(sum);
+    if (lane == 0) sums[warp] = sum;
+    __syncthreads();
+    sum = 0.0;
+#pragma unroll
+    for (int w = 0; w < W; ++w) sum += sums[w];
+    const float denom = (float)sum;
+    uint32_t key[V], best = 0xFFFFFFFFu;                 // upper half of the sort's key; the id is the lower one
+#pragma unroll
+    for (int u = 0; u < V; ++u) {
+        key[u] = u * T + tid < Nkv ? descending_key(__fdiv_rn(e[u], denom)) : 0xFFFFFFFFu;
+        best = min(best, key[u]);
+    }
+    const int nth = (want + W - 1) / W;
+    uint32_t bound = 0xFFFFFFFFu;
+    if (nth <= 32) {
+#pragma unroll
+        for (int k = 2; k <= 32; k <<= 1)
+#pragma unroll
+            for (int j = k >> 1; j > 0; j >>= 1) {
+                const uint32_t other = __shfl_xor_sync(0xffffffffu, best, j);
+                const bool keep_min = ((lane & j) == 0) == ((lane & k) == 0);
+                best = keep_min ? min(best, other) : max(best, other);
+            }
+        bound = __shfl_sync(0xffffffffu, best, nth - 1);
+    }
+    if (lane == 0) bounds[warp] = bound;
+    __syncthreads();
+    bound = 0u;
+#pragma unroll
+    for (int w = 0; w < W; ++w) bound = max(bound, bounds[w]);
+#pragma unroll
+    for (int u = 0; u < V; ++u) {
+        const bool near = u * T + tid < Nkv && key[u] <= bound;
+        const unsigned voters = __ballot_sync(0xffffffffu, near);
+        if (voters) {
+            int base = 0;
+            if (lane == 0) base = atomicAdd(&n_near, __popc(voters));
+            const int pos = __shfl_sync(0xffffffffu, base, 0) + __popc(voters & ((1u << lane) - 1u));
+            if (near && pos < SLOTS) keys[pos] = ((unsigned long long)key[u] << 32) | (unsigned)(u * T + tid);
+        }
+    }
+    __syncthreads();
+    const int n = n_near;        // >= want
+    int32_t *idx = index + (long long)row * Nkv;
+    if (n <= T) {
+        if (tid < n) {
+            const unsigned long long mine = keys[tid];
+            int place = 0;
+            for (int j = 0; j < n; ++j) place += keys[j] < mine;
+            if (place < want) idx[place] = (int32_t)(mine & 0xFFFFFFFFull);
+        }
+    } else if (V * T <= SLOTS || n <= SLOTS) {           // a large count, or many equal probabilities
+        int n_pow2 = 1;
+        while (n_pow2 < n) n_pow2 <<= 1;                 // <= SLOTS, a power of two
+        for (int j = n + tid; j < n_pow2; j += T) keys[j] = 0xFFFFFFFFFFFFFFFFull;
+        __syncthreads();
+        sort_keys_smem(keys, n_pow2);
+        for (int j = tid; j < want; j += T) idx[j] = (int32_t)(keys[j] & 0xFFFFFFFFull);
+    } else if constexpr (V * T > SLOTS) {
+#pragma unroll
+        for (int u = 0; u < V; ++u)
+            if (u * T + tid < Nkv) lrow[u * T + tid] = value_of_key((unsigned long long)key[u] << 32);
+        __syncthreads();
+        unsigned long long from = 0ull;
+        for (int first = 0; first < want; first += SLOTS)
+            from = select_top_blocks(lrow, Nkv, min(want - first, SLOTS), keys, SLOTS, idx + first, 0, nullptr, from, Nkv - first) + 1ull;
+    }
 }
 
 #ifdef WA_ROUTE_TRACE
@@ -1455,14 +1586,7 @@ int route_fused_launch(const float *q_pooled, const float *k_pooled, int B, int 
     // of 1024 threads fills half an SM, and what the sort gains is lost on the other steps (512 and 1024 threads, 74 over 585: 301 and
     // 299 us; over 700: 316 and 315; over 1024: 388 and 389; 37 over 513: 201 and 192).
     if (n_pow2 == 512) threads = 512;
-    // a fixed count per head over more key blocks than one pass of the register sort covers, and nobody reads the whole
-    // order or the thresholds: select the best blocks instead of sorting all of them
-    const int select_only = fixed_num_per_head && !whole_order && n_pow2 > threads;
-    int key_slots = n_pow2 > threads ? n_pow2 : threads;
-    if (select_only && key_slots > 2048) {      // the selection's keys; several CTAs then share an SM and cover each other's barriers
-        key_slots = 2048;
-        threads = 512;
-    }
+    const int key_slots = n_pow2 > threads ? n_pow2 : threads;
     const size_t smem = (size_t)key_slots * sizeof(unsigned long long) + (size_t)Nkv * sizeof(float);
     if (smem > 24 * 1024) {   // static shared memory of the kernel takes ~22 KB of the default 48 KB
         const cudaError_t e = cudaFuncSetAttribute(route_fused_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
@@ -1530,12 +1654,37 @@ int route_fused_launch(const float *q_pooled, const float *k_pooled, int B, int 
     const int gate_per_cta = (int)((128 * 128 + rows - 1) / rows);
     if (rows < sms) sms = (int)rows;
     const int slots = (int)((rows + sms - 1) / sms);
+    if (fixed_num_per_head && !whole_order) {
+        const auto launch = [&](auto threads_c, auto values_c) -> cudaError_t {
+            constexpr int T = decltype(threads_c)::value, V = decltype(values_c)::value;
+            const size_t bytes = logits_ready ? 0 : (size_t)Nkv * sizeof(float);       // at most 64 KB
+            const auto kernel = route_topk_kernel<T, V>;
+            static PerDeviceOnce attr_set;
+            if (!attr_set.done()) {
+                const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, T * V * (int)sizeof(float));
+                if (e != cudaSuccess) return e;
+                attr_set.mark();
+            }
+            return launch_dependent(kernel, dim3((unsigned)((long long)sms * slots) + 1), dim3(T), bytes, stream, q_pooled, k_pooled, H, Nq, Nkv, D,
+                                    scale, fixed_num_per_head, sorted, index, num, job_in, (int)rows, gate_per_cta, sms, slots, logits_ready ? 1 : 0);
+        };
+        using std::integral_constant;
+        const cudaError_t e = logits_ready && Nkv <= 256    ? launch(integral_constant<int, 128>(), integral_constant<int, 2>())
+                              : logits_ready && Nkv <= 512  ? launch(integral_constant<int, 128>(), integral_constant<int, 4>())
+                              : Nkv <= 256                  ? launch(integral_constant<int, 256>(), integral_constant<int, 1>())
+                              : Nkv <= 2048                 ? launch(integral_constant<int, 256>(), integral_constant<int, 8>())
+                              : Nkv <= 4096                 ? launch(integral_constant<int, 512>(), integral_constant<int, 8>())
+                              : Nkv <= 8192                 ? launch(integral_constant<int, 512>(), integral_constant<int, 16>())
+                                                            : launch(integral_constant<int, 512>(), integral_constant<int, 32>());
+        if (e != cudaSuccess) return fail((int)e, "wa_hsa_forward(routing by count): %s", cudaGetErrorString(e));
+        return check_launch("wa_hsa_forward(routing by count)");
+    }
     const dim3 grid((unsigned)((long long)sms * slots));
     SchedJob job = job_in;
     job.release_dependents_after_rows = pdl_mode() == 2;
     const cudaError_t le = launch_dependent(route_fused_kernel, grid, dim3(threads), smem, stream, q_pooled, k_pooled, B, H, Nq, Nkv, n_pow2, D, scale,
                                             (float)tau_min, span, fixed_num_per_head, sorted, index, num, thresholds, gini, counters, job,
-                                            gate_per_cta, sms, slots, select_only, logits_ready ? 1 : 0, key_slots);
+                                            gate_per_cta, sms, slots, logits_ready ? 1 : 0, key_slots);
     if (le != cudaSuccess) return fail((int)le, "wa_hsa_forward(routing): %s", cudaGetErrorString(le));
     return check_launch("wa_hsa_forward(routing)");
 }
