@@ -563,102 +563,119 @@ hsa_fwd_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
             for (int phase = 0; phase < 2 && ok; ++phase) {
                 const int t0 = phase == 0 ? 0 : n_sel, t1 = phase == 0 ? n_sel : n_kv;
                 float mA = -INFINITY, mB = -INFINITY, lA = 0.f, lB = 0.f;   // l: this thread's columns only
-                // One tile of 8 * STEPS key columns: scores at s_addr -> probabilities at p_addr, the accumulator rescaled
-                // where a running maximum outgrew it.  Columns of the first 64 keys are real below lim_lo, the others below lim_hi.
-                auto softmax_tile = [&](auto steps, uint32_t s_addr, uint32_t p_addr, bool full, int lim_lo, int lim_hi, bool later) {
-                    constexpr int STEPS = decltype(steps)::value;
-                    uint32_t r[4 * STEPS];
-                    if constexpr (STEPS == 16) TMEM_LDQ64(s_addr, r);
-                    else TMEM_LDQ32(s_addr, r);
-                    tmem_wait_ld();
-                    float xa0 = -INFINITY, xa1 = -INFINITY, xb0 = -INFINITY, xb1 = -INFINITY;
-                    if (full) {
+                bool started = false;      // every row of the warp has its reference point
+                // One tile of 64 * halves key columns: scores at s_addr -> probabilities at p_addr.  Columns of the first half are
+                // real below lim_lo, the others below lim_hi.  The reference point m of a row (the exponentials are 2^(s - m)) is
+                // the maximum of the row's first real tile; later tiles are computed against it WITHOUT looking for their own
+                // maximum: any m gives the same quotients as long as nothing overflows, and the sums, which are needed anyway,
+                // show when a row has outgrown its m.  Only then is the tile's maximum found, the accumulator rescaled and the tile
+                // computed again (its scores are still in tensor memory).  So a tile needs no pass over its scores before the
+                // exponentials, and the next 32 columns are fetched while 32 are at work.
+                // ONE copy of the exponentials, for 64 columns, serves full tiles, ragged ones (masked scores are -inf) and the
+                // half tiles of PAIR: what bounds these warps is the fetching of instructions (the loop is run by warps that take
+                // turns with four other roles' code) and latency, not a pipe: the special-function unit is 30 % busy.  (4680 queries, the
+                // kernel: 72.8 -> 68.8 us over 3 frames, 75.6 -> 70.8 over 21; 64-token blocks 559 -> 512 and, over 480 frames, 450 -> 423.)
+                auto softmax_tile = [&](int halves, uint32_t s_addr, uint32_t p_addr, bool full, int lim_lo, int lim_hi, bool later) {
+                    constexpr float OUTGROWN = 256.0f;       // sum over a thread's columns, a quarter of a row's: no probability exceeds it
+                    constexpr uint32_t MASKED = 0xff800000u; // -inf
+                    uint32_t lo[16], hi[16], pk0[16], pk1[16];
+                    float sumA, sumB;
+                    bool with_max = !started;
+                    auto mask = [&](uint32_t (&r)[16], int col0) {
+                        const int left = (col0 < HALF ? lim_lo : lim_hi) - col0 - 2 * c2;
 #pragma unroll
-                        for (int j = 0; j < STEPS; ++j) {
-                            xa0 = fmaxf(xa0, __uint_as_float(r[4 * j]));
-                            xa1 = fmaxf(xa1, __uint_as_float(r[4 * j + 1]));
-                            xb0 = fmaxf(xb0, __uint_as_float(r[4 * j + 2]));
-                            xb1 = fmaxf(xb1, __uint_as_float(r[4 * j + 3]));
+                        for (int j = 0; j < 4; ++j) {
+                            if (8 * j >= left) r[4 * j] = r[4 * j + 2] = MASKED;
+                            if (8 * j + 1 >= left) r[4 * j + 1] = r[4 * j + 3] = MASKED;
                         }
-                    } else {
+                    };
+                    while (true) {
+                        if (with_max) {
+                            float xa = -INFINITY, xb = -INFINITY;
+#pragma unroll 1
+                            for (int c = 0; c < 2 * halves; ++c) {
+                                TMEM_LDQ16(s_addr + 32 * c, lo);
+                                tmem_wait_ld16(lo);
+                                if (!full) mask(lo, 32 * c);
 #pragma unroll
-                        for (int j = 0; j < STEPS; ++j) {
-                            const int col = 8 * j + 2 * c2, lim = j < 8 ? lim_lo : lim_hi;
-                            if (col < lim) {
-                                xa0 = fmaxf(xa0, __uint_as_float(r[4 * j]));
-                                xb0 = fmaxf(xb0, __uint_as_float(r[4 * j + 2]));
+                                for (int j = 0; j < 4; ++j) {
+                                    xa = fmaxf(xa, fmaxf(__uint_as_float(lo[4 * j]), __uint_as_float(lo[4 * j + 1])));
+                                    xb = fmaxf(xb, fmaxf(__uint_as_float(lo[4 * j + 2]), __uint_as_float(lo[4 * j + 3])));
+                                }
                             }
-                            if (col + 1 < lim) {
-                                xa1 = fmaxf(xa1, __uint_as_float(r[4 * j + 1]));
-                                xb1 = fmaxf(xb1, __uint_as_float(r[4 * j + 3]));
+                            const float mxA = quad_max(xa) * p.scale_log2, mxB = quad_max(xb) * p.scale_log2;
+                            WA_TRACE(8);
+                            const bool growA = mxA > mA, growB = mxB > mB;
+                            const float mA_new = growA ? mxA : mA, mB_new = growB ? mxB : mB;
+                            if (__any_sync(0xffffffffu, (growA || growB) && later)) {
+                                // every PV requested so far must have landed before the accumulator is touched
+                                ok = __all_sync(0xffffffffu, mbar_wait(&bar->v_empty[(pv_count - 1u) % V_STAGES],
+                                                                       ((pv_count - 1u) / V_STAGES) & 1u, abort_flag, sink, 9));
+                                if (!ok) return;
+                                tc_fence_after();
+                                const float fA = (growA && later) ? ex2(mA - mA_new) : 1.0f, fB = (growB && later) ? ex2(mB - mB_new) : 1.0f;
+                                lA *= fA;
+                                lB *= fB;
+#pragma unroll 1
+                                for (int c = 0; c < 4; ++c) {   // 32 columns at a time
+                                    TMEM_LDQ16(tmem_o + lane_addr + c * 32, lo);
+                                    tmem_wait_ld16(lo);
+#pragma unroll
+                                    for (int j = 0; j < 4; ++j) {
+                                        lo[4 * j] = __float_as_uint(__uint_as_float(lo[4 * j]) * fA);
+                                        lo[4 * j + 1] = __float_as_uint(__uint_as_float(lo[4 * j + 1]) * fA);
+                                        lo[4 * j + 2] = __float_as_uint(__uint_as_float(lo[4 * j + 2]) * fB);
+                                        lo[4 * j + 3] = __float_as_uint(__uint_as_float(lo[4 * j + 3]) * fB);
+                                    }
+                                    TMEM_STQ16(tmem_o + lane_addr + c * 32, lo);
+                                }
+                                tmem_wait_st();
+                            }
+                            mA = mA_new;
+                            mB = mB_new;
+                            started = __all_sync(0xffffffffu, mA > -INFINITY && mB > -INFINITY);   // (a row without a real key yet: look again)
+                        }
+                        // p = 2^(s*c - m), row sums, pack to bf16.  A row that has seen no key yet and sees none here keeps sums of zero.
+                        const bool any_real = full || lim_lo > 0 || lim_hi > HALF;
+                        const float nA = any_real || mA > -INFINITY ? -mA : 0.f, nB = any_real || mB > -INFINITY ? -mB : 0.f;
+                        const float2 nmA = make_float2(nA, nA), nmB = make_float2(nB, nB);
+                        float2 accA = make_float2(0.f, 0.f), accB = make_float2(0.f, 0.f);
+                        auto exp32 = [&](const uint32_t (&r)[16], uint32_t *pk) {       // 32 columns of the row pair
+                            exp_step<true>(r[0], r[1], r[2], r[3], sc, nmA, nmB, accA, accB, pk[0], pk[1]);
+#pragma unroll
+                            for (int j = 1; j < 4; ++j)
+                                exp_step<false>(r[4 * j], r[4 * j + 1], r[4 * j + 2], r[4 * j + 3], sc, nmA, nmB, accA, accB, pk[2 * j], pk[2 * j + 1]);
+                        };
+                        TMEM_LDQ16(s_addr, lo);
+#pragma unroll 1
+                        for (int c = 0; c < halves; ++c) {
+                            tmem_wait_ld16(lo);
+                            TMEM_LDQ16(s_addr + 64 * c + 32, hi);
+                            if (!full) mask(lo, 64 * c);
+                            exp32(lo, pk1);
+                            tmem_wait_ld16(hi);
+                            if (c + 1 < halves) TMEM_LDQ16(s_addr + 64 * c + 64, lo);
+                            if (!full) mask(hi, 64 * c + 32);
+                            exp32(hi, pk1 + 8);
+                            if (c + 1 < halves) {
+#pragma unroll
+                                for (int j = 0; j < 16; ++j) pk0[j] = pk1[j];
                             }
                         }
-                    }
-                    const float mxA = quad_max(fmaxf(xa0, xa1)) * p.scale_log2, mxB = quad_max(fmaxf(xb0, xb1)) * p.scale_log2;
-                    WA_TRACE(8);
-                    // lazy rescale: only when a running maximum grows by more than 2^8
-                    float mA_new = mA, mB_new = mB;
-                    const bool growA = mxA > mA + 8.0f, growB = mxB > mB + 8.0f;
-                    if (growA) mA_new = mxA;
-                    if (growB) mB_new = mxB;
-                    if (__any_sync(0xffffffffu, (growA || growB) && later)) {
-                        // every PV requested so far must have landed before the accumulator is touched
-                        ok = __all_sync(0xffffffffu, mbar_wait(&bar->v_empty[(pv_count - 1u) % V_STAGES],
-                                                               ((pv_count - 1u) / V_STAGES) & 1u, abort_flag, sink, 9));
-                        if (!ok) return;
-                        tc_fence_after();
-                        const float fA = (growA && later) ? ex2(mA - mA_new) : 1.0f, fB = (growB && later) ? ex2(mB - mB_new) : 1.0f;
-                        lA *= fA;
-                        lB *= fB;
-#pragma unroll
-                        for (int c = 0; c < 4; ++c) {   // 32 columns at a time
-                            uint32_t ro[16];
-                            TMEM_LDQ16(tmem_o + lane_addr + c * 32, ro);
-                            tmem_wait_ld();
-#pragma unroll
-                            for (int j = 0; j < 4; ++j) {
-                                ro[4 * j] = __float_as_uint(__uint_as_float(ro[4 * j]) * fA);
-                                ro[4 * j + 1] = __float_as_uint(__uint_as_float(ro[4 * j + 1]) * fA);
-                                ro[4 * j + 2] = __float_as_uint(__uint_as_float(ro[4 * j + 2]) * fB);
-                                ro[4 * j + 3] = __float_as_uint(__uint_as_float(ro[4 * j + 3]) * fB);
-                            }
-                            TMEM_STQ16(tmem_o + lane_addr + c * 32, ro);
-                        }
-                        tmem_wait_st();
-                    }
-                    mA = mA_new;
-                    mB = mB_new;
-                    // p = 2^(s*c - m), row sums, pack to bf16, write P over the consumed S columns
-                    uint32_t pk[2 * STEPS];
-                    const float2 nmA = make_float2(-mA, -mA), nmB = make_float2(-mB, -mB);
-                    float2 accA = make_float2(0.f, 0.f), accB = make_float2(0.f, 0.f);
-                    if (full) {
-#pragma unroll
-                        for (int j = 0; j < STEPS; ++j) {
-                            if (j % POLY_EVERY == 0)
-                                exp_step<true, false>(r[4 * j], r[4 * j + 1], r[4 * j + 2], r[4 * j + 3], sc, nmA, nmB, accA, accB,
-                                                      pk[2 * j], pk[2 * j + 1], 0, 0);
-                            else
-                                exp_step<false, false>(r[4 * j], r[4 * j + 1], r[4 * j + 2], r[4 * j + 3], sc, nmA, nmB, accA, accB,
-                                                       pk[2 * j], pk[2 * j + 1], 0, 0);
-                        }
-                    } else {
-                        // ragged tile (the last one of a branch): 8-column steps without a real token cost nothing
-#pragma unroll
-                        for (int j = 0; j < STEPS; ++j) {
-                            const int lim = j < 8 ? lim_lo : lim_hi;
-                            if (8 * j < lim)
-                                exp_step<false, true>(r[4 * j], r[4 * j + 1], r[4 * j + 2], r[4 * j + 3], sc, nmA, nmB, accA, accB,
-                                                      pk[2 * j], pk[2 * j + 1], 8 * j + 2 * c2, lim);
-                            else
-                                pk[2 * j] = pk[2 * j + 1] = 0u;
-                        }
+                        sumA = accA.x + accA.y;
+                        sumB = accB.x + accB.y;
+                        if (with_max || !__any_sync(0xffffffffu, !(sumA <= OUTGROWN) || !(sumB <= OUTGROWN))) break;
+                        with_max = true;
                     }
                     WA_TRACE(20);
-                    if constexpr (STEPS == 16) TMEM_STP32(p_addr, pk);
-                    else TMEM_STP16(p_addr, pk);
-                    lA += accA.x + accA.y;
-                    lB += accB.x + accB.y;
+                    if (halves == 2) {       // over the consumed S columns
+                        TMEM_STP16(p_addr, pk0);
+                        TMEM_STP16(p_addr + 32, pk1);
+                    } else {
+                        TMEM_STP16(p_addr, pk1);
+                    }
+                    lA += sumA;
+                    lB += sumB;
                     tmem_wait_st();
                 };
                 for (int t = t0; t < t1 && ok; ++t) {
@@ -674,9 +691,9 @@ hsa_fwd_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
                     const int v0 = vword & 0xff, v1 = (vword >> 8) & 0xff;
                     if (PAIR && phase == 0 && t >= n_both) {
                         const int v = second_block ? v1 : v0;
-                        softmax_tile(std::integral_constant<int, 8>(), s_addr + second_block * HALF, s_addr, v == HALF, v, 0, t > t0);
+                        softmax_tile(1, s_addr + second_block * HALF, s_addr, v == HALF, v, 0, t > t0);
                     } else {
-                        softmax_tile(std::integral_constant<int, 16>(), s_addr, s_addr, vword == (HALF | (HALF << 8)), v0, HALF + v1, t > t0);
+                        softmax_tile(2, s_addr, s_addr, vword == (HALF | (HALF << 8)), v0, HALF + v1, t > t0);
                     }
                     if (!ok) break;
                     WA_TRACE(21);
