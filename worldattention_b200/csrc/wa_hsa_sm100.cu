@@ -34,10 +34,18 @@ constexpr int REGS_SOFTMAX = 224;    // register budget per thread after the rol
 constexpr int REGS_OTHER = 56;       // ... and of the warpgroup that holds the four single-purpose warps; 256*224 + 128*56 = 384*168
 constexpr int TMEM_COLS = 512;       // three S buffers: columns [0,128), [128,256), [256,384); O: [384,512)
 constexpr int S_BUFS = 3;            // score products run up to two tiles ahead of the softmax
-constexpr int Q_STAGES = 2;          // the staged output of item j leaves from one Q buffer while item j+1 loads the other
 constexpr int KV_STAGES = 3;         // shared-memory ring depth for K tiles
-constexpr int V_STAGES = 2;          // shared-memory ring depth for V tiles
-constexpr int SMEM_BYTES = (Q_STAGES + KV_STAGES + V_STAGES) * TILE_BYTES + 3072 /*barriers, bias*/;
+constexpr int QV_STAGES = 4;         // shared-memory stages of Q and V together, see Stages
+constexpr int SMEM_BYTES = (KV_STAGES + QV_STAGES) * TILE_BYTES + 3072 /*barriers, bias*/;
+
+// With two Q stages the staged output of item j leaves from one while item j + 1 loads the other.  Pairs of 64-token query blocks
+// have long items of tiles that need 64 KB of keys and values each but only half a tile's arithmetic: there a third V stage (a
+// V load may then be two tiles ahead of its product instead of one) is worth more than the waits between items (21 frames, counts from
+// the mass: 512 -> 499 us; with one Q stage 128-token calls over the same window lose 6 us of 72).
+template <bool PAIR>
+struct Stages {
+    static constexpr int Q = PAIR ? 1 : 2, V = QV_STAGES - Q;
+};
 
 // Optional event trace for kernel tuning (compile with -DWA_SM100_TRACE): CTA 0 appends
 // (event id, clock) pairs from one thread per role to a global buffer.
@@ -90,8 +98,8 @@ __device__ __forceinline__ unsigned wa_smid() {
 
 struct Barriers {
     uint64_t item_full[2], item_empty[2];
-    uint64_t q_full[Q_STAGES], q_empty[Q_STAGES], out_ready[Q_STAGES];
-    uint64_t k_full[KV_STAGES], k_empty[KV_STAGES], v_full[V_STAGES], v_empty[V_STAGES];
+    uint64_t q_full[2], q_empty[2], out_ready[2];
+    uint64_t k_full[KV_STAGES], k_empty[KV_STAGES], v_full[3], v_empty[3];
     // K-type tile g (global count) lives in S buffer g % S_BUFS; it is that buffer's occupancy number g / S_BUFS, which
     // is the phase of s_full / p_full the tile completes (every tile completes exactly one phase of each).
     uint64_t s_full[S_BUFS], p_full[S_BUFS];
@@ -132,6 +140,7 @@ hsa_fwd_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
                      const __grid_constant__ CUtensorMap tm_out, const Params p) {
     static_assert(!PAIR || BLK == HALF, "query blocks are paired where a block is half a tile");
     constexpr int Q_ROWS = PAIR ? TILE : BLK;    // query rows of a work item
+    constexpr int Q_STAGES = Stages<PAIR>::Q, V_STAGES = Stages<PAIR>::V;
     extern __shared__ __align__(1024) uint8_t smem[];   // swizzled TMA tiles need 1024-byte alignment (checked below)
     uint8_t *q_s = smem, *k_s = smem + Q_STAGES * TILE_BYTES, *v_s = smem + (Q_STAGES + KV_STAGES) * TILE_BYTES;
     Barriers *bar = reinterpret_cast<Barriers *>(smem + (Q_STAGES + KV_STAGES + V_STAGES) * TILE_BYTES);
