@@ -145,7 +145,7 @@ hsa_fwd_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
     uint8_t *q_s = smem, *k_s = smem + Q_STAGES * TILE_BYTES, *v_s = smem + (Q_STAGES + KV_STAGES) * TILE_BYTES;
     Barriers *bar = reinterpret_cast<Barriers *>(smem + (Q_STAGES + KV_STAGES + V_STAGES) * TILE_BYTES);
 
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;   // (known to be uniform)
     volatile int *abort_flag = &bar->abort_flag;
     const FailSink sink{p.error_flag, p.status_mirror};
 
@@ -573,21 +573,39 @@ hsa_fwd_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
                 const int t0 = phase == 0 ? 0 : n_sel, t1 = phase == 0 ? n_sel : n_kv;
                 float mA = -INFINITY, mB = -INFINITY, lA = 0.f, lB = 0.f;   // l: this thread's columns only
                 bool started = false;      // every row of the warp has its reference point
-                // One tile of 64 * halves key columns: scores at s_addr -> probabilities at p_addr.  Columns of the first half are
-                // real below lim_lo, the others below lim_hi.  The reference point m of a row (the exponentials are 2^(s - m)) is
-                // the maximum of the row's first real tile; later tiles are computed against it WITHOUT looking for their own
-                // maximum: any m gives the same quotients as long as nothing overflows, and the sums, which are needed anyway,
-                // show when a row has outgrown its m.  Only then is the tile's maximum found, the accumulator rescaled and the tile
-                // computed again (its scores are still in tensor memory).  So a tile needs no pass over its scores before the
-                // exponentials, and the next 32 columns are fetched while 32 are at work.
-                // ONE copy of the exponentials, for 64 columns, serves full tiles, ragged ones (masked scores are -inf) and the
-                // half tiles of PAIR: what bounds these warps is the fetching of instructions (the loop is run by warps that take
-                // turns with four other roles' code) and latency, not a pipe: the special-function unit is 30 % busy.  (4680 queries, the
-                // kernel: 72.8 -> 68.8 us over 3 frames, 75.6 -> 70.8 over 21; 64-token blocks 559 -> 512 and, over 480 frames, 450 -> 423.)
-                auto softmax_tile = [&](int halves, uint32_t s_addr, uint32_t p_addr, bool full, int lim_lo, int lim_hi, bool later) {
-                    constexpr float OUTGROWN = 256.0f;       // sum over a thread's columns, a quarter of a row's: no probability exceeds it
-                    constexpr uint32_t MASKED = 0xff800000u; // -inf
-                    uint32_t lo[16], hi[16], pk0[16], pk1[16];
+                // The reference point m of a row (the exponentials are 2^(s - m)) is the maximum of the row's first real tile; later
+                // tiles are computed against it WITHOUT looking for their own maximum: any m gives the same quotients as long as
+                // nothing overflows, and the sums, which are needed anyway, show when a row has outgrown its m.  Only then is the
+                // tile's maximum found, the accumulator rescaled and the tile computed again (its scores are still in tensor
+                // memory).  So a tile needs no pass over its scores before the exponentials, the next 32 columns are fetched
+                // while 32 are at work (fetching the next tile's first ones before this one's probabilities are handed over delays that: 421 ->
+                // 448 us over 480 frames).
+                // ONE copy of the exponentials of full tiles, for 64 columns, without masks (branches among them cost a tenth);
+                // ragged tiles, the last of a branch, have a small loop of their own.  What bounds these warps is latency and the
+                // fetching of instructions, not a pipe: the special-function unit is 30 % busy.  SOFTMAX_FIGURES
+                constexpr float OUTGROWN = 256.0f;       // sum over a thread's columns, a quarter of a row's: no probability exceeds it
+                constexpr uint32_t MASKED = 0xff800000u; // -inf
+                for (int t = t0; t < t1 && ok; ++t) {
+                    const int buf = (sg + t) % S_BUFS;
+                    const uint32_t p_addr = tmem_s + buf * TILE + lane_addr;
+                    const uint32_t s_addr = p_addr + (PAIR && phase == 0 && t >= n_both ? second_block * HALF : 0);
+                    uint32_t lo[16];
+                    ok = __all_sync(0xffffffffu, mbar_wait(&bar->s_full[buf], ((sg + t) / S_BUFS) & 1u, abort_flag, sink, 8));
+                    if (!ok) break;
+                    tc_fence_after();
+                    TMEM_LDQ16(s_addr, lo);
+                    WA_TRACE(2);
+                    // real tokens of the tile's first and last 64 keys (the producer wrote the counts): columns of the first half are
+                    // real below lim_lo, the others below lim_hi
+                    const int vword = bar->valid[(sg + t) & 7];
+                    int lim_lo = vword & 0xff, lim_hi = HALF + ((vword >> 8) & 0xff), halves = 2;
+                    if (PAIR && phase == 0 && t >= n_both) {
+                        lim_lo = second_block ? lim_hi - HALF : lim_lo;
+                        lim_hi = HALF;
+                        halves = 1;
+                    }
+                    const bool full = lim_lo == HALF && lim_hi == HALF * halves, later = t > t0;
+                    uint32_t hi[16], pk0[16], pk1[16];
                     float sumA, sumB;
                     bool with_max = !started;
                     auto mask = [&](uint32_t (&r)[16], int col0) {
@@ -599,8 +617,9 @@ hsa_fwd_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
                         }
                     };
                     while (true) {
-                        if (with_max) {
+                        if (__builtin_expect(with_max, 0)) {
                             float xa = -INFINITY, xb = -INFINITY;
+                            tmem_wait_ld16(lo);
 #pragma unroll 1
                             for (int c = 0; c < 2 * halves; ++c) {
                                 TMEM_LDQ16(s_addr + 32 * c, lo);
@@ -620,7 +639,7 @@ hsa_fwd_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
                                 // every PV requested so far must have landed before the accumulator is touched
                                 ok = __all_sync(0xffffffffu, mbar_wait(&bar->v_empty[(pv_count - 1u) % V_STAGES],
                                                                        ((pv_count - 1u) / V_STAGES) & 1u, abort_flag, sink, 9));
-                                if (!ok) return;
+                                if (!ok) break;
                                 tc_fence_after();
                                 const float fA = (growA && later) ? ex2(mA - mA_new) : 1.0f, fB = (growB && later) ? ex2(mB - mB_new) : 1.0f;
                                 lA *= fA;
@@ -643,11 +662,10 @@ hsa_fwd_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
                             mA = mA_new;
                             mB = mB_new;
                             started = __all_sync(0xffffffffu, mA > -INFINITY && mB > -INFINITY);   // (a row without a real key yet: look again)
+                            TMEM_LDQ16(s_addr, lo);
                         }
-                        // p = 2^(s*c - m), row sums, pack to bf16.  A row that has seen no key yet and sees none here keeps sums of zero.
-                        const bool any_real = full || lim_lo > 0 || lim_hi > HALF;
-                        const float nA = any_real || mA > -INFINITY ? -mA : 0.f, nB = any_real || mB > -INFINITY ? -mB : 0.f;
-                        const float2 nmA = make_float2(nA, nA), nmB = make_float2(nB, nB);
+                        // p = 2^(s*c - m), row sums, pack to bf16
+                        float2 nmA = make_float2(-mA, -mA), nmB = make_float2(-mB, -mB);
                         float2 accA = make_float2(0.f, 0.f), accB = make_float2(0.f, 0.f);
                         auto exp32 = [&](const uint32_t (&r)[16], uint32_t *pk) {       // 32 columns of the row pair
                             exp_step<true>(r[0], r[1], r[2], r[3], sc, nmA, nmB, accA, accB, pk[0], pk[1]);
@@ -655,27 +673,54 @@ hsa_fwd_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
                             for (int j = 1; j < 4; ++j)
                                 exp_step<false>(r[4 * j], r[4 * j + 1], r[4 * j + 2], r[4 * j + 3], sc, nmA, nmB, accA, accB, pk[2 * j], pk[2 * j + 1]);
                         };
-                        TMEM_LDQ16(s_addr, lo);
+                        if (__builtin_expect(full, 1)) {
 #pragma unroll 1
-                        for (int c = 0; c < halves; ++c) {
-                            tmem_wait_ld16(lo);
-                            TMEM_LDQ16(s_addr + 64 * c + 32, hi);
-                            if (!full) mask(lo, 64 * c);
-                            exp32(lo, pk1);
-                            tmem_wait_ld16(hi);
-                            if (c + 1 < halves) TMEM_LDQ16(s_addr + 64 * c + 64, lo);
-                            if (!full) mask(hi, 64 * c + 32);
-                            exp32(hi, pk1 + 8);
-                            if (c + 1 < halves) {
+                            for (int c = 0; c < halves; ++c) {
+                                tmem_wait_ld16(lo);
+                                TMEM_LDQ16(s_addr + 64 * c + 32, hi);
+                                exp32(lo, pk1);
+                                tmem_wait_ld16(hi);
+                                if (c + 1 < halves) TMEM_LDQ16(s_addr + 64 * c + 64, lo);
+                                exp32(hi, pk1 + 8);
+                                if (c + 1 < halves) {
 #pragma unroll
-                                for (int j = 0; j < 16; ++j) pk0[j] = pk1[j];
+                                    for (int j = 0; j < 16; ++j) pk0[j] = pk1[j];
+                                }
+                            }
+                        } else {
+                            // A row that has seen no key yet and sees none here keeps sums of zero.
+                            const bool any_real = lim_lo > 0 || lim_hi > HALF;
+                            if (!any_real && mA == -INFINITY) nmA = make_float2(0.f, 0.f);
+                            if (!any_real && mB == -INFINITY) nmB = make_float2(0.f, 0.f);
+                            tmem_wait_ld16(lo);
+#pragma unroll 1
+                            for (int c = 0; c < 2 * halves; ++c) {
+                                uint32_t w[8];
+                                if (32 * c < (c < 2 ? lim_lo : lim_hi)) {
+                                    TMEM_LDQ16(s_addr + 32 * c, lo);
+                                    tmem_wait_ld16(lo);
+                                    mask(lo, 32 * c);
+                                    exp32(lo, w);
+                                } else {                                    // no real token: costs nothing
+#pragma unroll
+                                    for (int j = 0; j < 8; ++j) w[j] = 0u;
+                                }
+#pragma unroll
+                                for (int j = 0; j < 8; ++j) {               // a queue of four: pk0, pk1
+                                    pk0[j] = pk0[8 + j];
+                                    pk0[8 + j] = pk1[j];
+                                    pk1[j] = pk1[8 + j];
+                                    pk1[8 + j] = w[j];
+                                }
                             }
                         }
                         sumA = accA.x + accA.y;
                         sumB = accB.x + accB.y;
                         if (with_max || !__any_sync(0xffffffffu, !(sumA <= OUTGROWN) || !(sumB <= OUTGROWN))) break;
                         with_max = true;
+                        TMEM_LDQ16(s_addr, lo);
                     }
+                    if (!ok) break;
                     WA_TRACE(20);
                     if (halves == 2) {       // over the consumed S columns
                         TMEM_STP16(p_addr, pk0);
@@ -686,31 +731,12 @@ hsa_fwd_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
                     lA += sumA;
                     lB += sumB;
                     tmem_wait_st();
-                };
-                for (int t = t0; t < t1 && ok; ++t) {
-                    const int buf = (sg + t) % S_BUFS;
-                    const uint32_t s_addr = tmem_s + buf * TILE + lane_addr;
-                    ok = __all_sync(0xffffffffu, mbar_wait(&bar->s_full[buf], ((sg + t) / S_BUFS) & 1u, abort_flag, sink, 8));
-                    if (!ok) break;
-                    WA_TRACE(2);
-                    tc_fence_after();
-                    // real tokens of the tile's first and last 64 keys (the producer wrote the counts); key column c is real
-                    // when c < v0 (c < 64) or c - 64 < v1: per 8-column step j that is c < lim(j)
-                    const int vword = bar->valid[(sg + t) & 7];
-                    const int v0 = vword & 0xff, v1 = (vword >> 8) & 0xff;
-                    if (PAIR && phase == 0 && t >= n_both) {
-                        const int v = second_block ? v1 : v0;
-                        softmax_tile(1, s_addr + second_block * HALF, s_addr, v == HALF, v, 0, t > t0);
-                    } else {
-                        softmax_tile(2, s_addr, s_addr, vword == (HALF | (HALF << 8)), v0, HALF + v1, t > t0);
-                    }
-                    if (!ok) break;
                     WA_TRACE(21);
                     tc_fence_before();
                     warp_arrive(&bar->p_full[buf]);
                     WA_TRACE(3);
                     ++pv_count;
-                    if (phase == 1 && t == t0 && n_sel > 0) {
+                    if (__builtin_expect(phase == 1 && t == t0 && n_sel > 0, 0)) {
                         // The sparse branch's accumulator: its last PV product had this whole tile to land.  Normalise,
                         // round to bf16 (the reference stores this branch in bf16) and park it in registers until the
                         // combine; then the linear branch's first PV product may overwrite it.
@@ -719,9 +745,14 @@ hsa_fwd_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
                         ph_od ^= 1u;
                         tc_fence_after();
                         WA_TRACE(12);
-#pragma unroll
-                        for (int c = 0; c < 4; ++c) {   // 32 columns at a time
+#pragma unroll 1
+                        for (int c = 0; c < 4; ++c) {   // 32 columns at a time, queued into the arrays (rolled: see below)
                             uint32_t ro[16];
+#pragma unroll
+                            for (int j = 0; j < 24; ++j) {
+                                park[j] = park[j + 8];
+                                if (p.part_sparse) gpk[j] = gpk[j + 8];
+                            }
                             TMEM_LDQ16(tmem_o + lane_addr + c * 32, ro);
                             tmem_wait_ld();
 #pragma unroll
@@ -729,14 +760,14 @@ hsa_fwd_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
                                 const float a0 = __uint_as_float(ro[4 * j]) * inv_spA, a1 = __uint_as_float(ro[4 * j + 1]) * inv_spA;
                                 const float b0 = __uint_as_float(ro[4 * j + 2]) * inv_spB, b1 = __uint_as_float(ro[4 * j + 3]) * inv_spB;
                                 if (p.part_sparse) {
-                                    park[2 * (4 * c + j)] = __float_as_uint(a0);
-                                    park[2 * (4 * c + j) + 1] = __float_as_uint(a1);
-                                    gpk[2 * (4 * c + j)] = __float_as_uint(b0);
-                                    gpk[2 * (4 * c + j) + 1] = __float_as_uint(b1);
+                                    park[24 + 2 * j] = __float_as_uint(a0);
+                                    park[25 + 2 * j] = __float_as_uint(a1);
+                                    gpk[24 + 2 * j] = __float_as_uint(b0);
+                                    gpk[25 + 2 * j] = __float_as_uint(b1);
                                 } else {
                                     __nv_bfloat162 ha = __floats2bfloat162_rn(a0, a1), hbv = __floats2bfloat162_rn(b0, b1);
-                                    park[2 * (4 * c + j)] = *reinterpret_cast<uint32_t *>(&ha);
-                                    park[2 * (4 * c + j) + 1] = *reinterpret_cast<uint32_t *>(&hbv);
+                                    park[24 + 2 * j] = *reinterpret_cast<uint32_t *>(&ha);
+                                    park[25 + 2 * j] = *reinterpret_cast<uint32_t *>(&hbv);
                                 }
                             }
                         }
@@ -795,9 +826,14 @@ hsa_fwd_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
                 tc_fence_after();
                 WA_TRACE(13);
                 if (!p.part_linear) {
-#pragma unroll
+                    // Rolled, here and in the combine below, with the arrays as queues: this code runs once per item, and fetching its
+                    // instructions for the first time cost more than the work (unrolled, the gate took 3800 cycles in a CTA's first
+                    // item and 1600 in its third).
+#pragma unroll 1
                     for (int c = 0; c < 4; ++c) {   // 32 columns at a time
                         uint32_t gsc[16];
+#pragma unroll
+                        for (int j = 0; j < 24; ++j) gpk[j] = gpk[j + 8];
                         if (p.has_gate) {
                             TMEM_LDQ16(tmem_s + gbuf * TILE + lane_addr + c * 32, gsc);
                             tmem_wait_ld();
@@ -826,8 +862,8 @@ hsa_fwd_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
                                                                        fmaf(tanh_approx(0.5f * zA1), 0.5f, 0.5f));
                             __nv_bfloat162 gb = __floats2bfloat162_rn(fmaf(tanh_approx(0.5f * zB0), 0.5f, 0.5f),
                                                                        fmaf(tanh_approx(0.5f * zB1), 0.5f, 0.5f));
-                            gpk[2 * jj] = *reinterpret_cast<uint32_t *>(&ga);
-                            gpk[2 * jj + 1] = *reinterpret_cast<uint32_t *>(&gb);
+                            gpk[24 + 2 * j] = *reinterpret_cast<uint32_t *>(&ga);
+                            gpk[25 + 2 * j] = *reinterpret_cast<uint32_t *>(&gb);
                         }
                     }
                 }
@@ -905,7 +941,7 @@ hsa_fwd_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
                     if (c & 1) flush(p.part_linear, c >> 1);
                 }
             } else if (ok) {
-#pragma unroll
+#pragma unroll 1
                 for (int c = 0; c < 4; ++c) {   // 32 columns at a time
                     uint32_t o[16];
                     TMEM_LDQ16(tmem_o + lane_addr + c * 32, o);
@@ -921,7 +957,7 @@ hsa_fwd_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
                         const int jj = 4 * c + j;
                         const float a0 = __uint_as_float(o[4 * j]) * inv_linA, a1 = __uint_as_float(o[4 * j + 1]) * inv_linA;
                         const float b0 = __uint_as_float(o[4 * j + 2]) * inv_linB, b1 = __uint_as_float(o[4 * j + 3]) * inv_linB;
-                        const uint32_t spA = park[2 * jj], spB = park[2 * jj + 1], gA = gpk[2 * jj], gB = gpk[2 * jj + 1];   // low half = even column
+                        const uint32_t spA = park[2 * j], spB = park[2 * j + 1], gA = gpk[2 * j], gB = gpk[2 * j + 1];   // low half = even column
                         __nv_bfloat162 ra = __floats2bfloat162_rn(fmaf(a0, __uint_as_float(gA << 16), __uint_as_float(spA << 16)),
                                                                    fmaf(a1, __uint_as_float(gA & 0xffff0000u), __uint_as_float(spA & 0xffff0000u)));
                         __nv_bfloat162 rb = __floats2bfloat162_rn(fmaf(b0, __uint_as_float(gB << 16), __uint_as_float(spB << 16)),
@@ -929,6 +965,11 @@ hsa_fwd_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
                         // the finished tile is staged in the shared-memory stage that held Q (the layout the TMA store expects)
                         *reinterpret_cast<uint32_t *>(q_stage + tile_off(rowA, jj)) = *reinterpret_cast<uint32_t *>(&ra);
                         *reinterpret_cast<uint32_t *>(q_stage + tile_off(rowB, jj)) = *reinterpret_cast<uint32_t *>(&rb);
+                    }
+#pragma unroll
+                    for (int j = 0; j < 24; ++j) {
+                        park[j] = park[j + 8];
+                        gpk[j] = gpk[j + 8];
                     }
                     WA_TRACE(15);
                 }
