@@ -249,8 +249,6 @@ __host__ __device__ constexpr uint32_t instr_desc(bool b_mn_major, int n) {
 // issue slot for two results).  2^x on the FMA pipe: split x into round(x) + f, f in [-0.5, 0.5], evaluate a
 // cubic for 2^f and add round(x) to the exponent field; relative error < 2^-10, below the bf16 rounding of P.  Below -127
 // the result is zero (at -127 the cubic is exactly one and the exponent field comes out empty).
-// The special-function unit (16 results per clock per SM) is the narrowest pipe of the softmax, so every
-// fourth pair of columns takes the polynomial instead.
 __device__ __forceinline__ float2 ex2_poly2(float2 x) {
     x.x = fmaxf(x.x, -127.0f);
     x.y = fmaxf(x.y, -127.0f);
