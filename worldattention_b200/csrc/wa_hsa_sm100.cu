@@ -219,7 +219,7 @@ hsa_fwd_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
                     row0 = PAIR ? (long long)(item / p.q_items) * p.Nq + 2 * (item % p.q_items) : item;
                     n_sel = max(0, min(p.num[row0], p.Nkv));
                     if (PAIR && 2 * (item % p.q_items) + 1 < p.Nq) n_sel2 = max(0, min(p.num[row0 + 1], p.Nkv));
-                    if (PAIR) n_both = p.both[item] >> 1;
+                    if (PAIR) n_both = (p.both[item] & 0xffff) >> 1;
                 }
                 // the other roles count sparse TILES: with 64-token blocks a tile holds two selected blocks
                 const int n_st = BLK == TILE ? n_sel : PAIR ? max(n_sel, n_sel2) - n_both : (n_sel + 1) >> 1;
@@ -998,84 +998,102 @@ hsa_fwd_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
 // ---- the lists of a pair: [blocks of both | the row's others], each part in ascending order ------------------------
 // A warp per item.  Ascending, so that the CTAs that work on a head sweep its keys side by side and find in L2 what the
 // first of them fetched.  A list that names a block twice (only a caller's own routing can) stays as it is.
-constexpr int PL_WARPS = 4;
+// `both` receives the number of common blocks (lower half) and the item's sparse tiles (upper half).  The CTA that finishes
+// last makes the work order from the latter: what an item costs is its tiles, and two query blocks that share their blocks have
+// far fewer of them than their counts say.
+constexpr int PL_WARPS = 8;
 __global__ void __launch_bounds__(PL_WARPS * 32)
 pair_lists_kernel(const int32_t *__restrict__ index, const int32_t *__restrict__ num, int Nq, int Nkv, int q_items, int n_items,
-                  int32_t *__restrict__ lists, int32_t *__restrict__ both) {
+                  int32_t *__restrict__ lists, int32_t *both, int ctas, SchedJob job) {
     extern __shared__ uint32_t pl_smem[];
+    __shared__ int hist[SCHED_BINS], warp_tot[32], last_cta;
     const int words = (Nkv + 31) >> 5, lane = threadIdx.x & 31;
     uint32_t *bits[2] = {pl_smem + (threadIdx.x >> 5) * 2 * words, pl_smem + ((threadIdx.x >> 5) * 2 + 1) * words};
     pdl_wait();                 // the routing comes from the launch before
     const int item = blockIdx.x * PL_WARPS + (threadIdx.x >> 5);
-    if (item >= n_items) return;
-    const long long row0 = (long long)(item / q_items) * Nq + 2 * (item % q_items);
-    const bool two = 2 * (item % q_items) + 1 < Nq;
-    int n[2], distinct[2] = {0, 0}, shared = 0;
-    for (int w = lane; w < words; w += 32) bits[0][w] = bits[1][w] = 0u;
-    __syncwarp();
-    auto id_of = [&](int side, int i) { return max(0, min(index[(row0 + side) * Nkv + i], Nkv - 1)); };
+    if (item < n_items) {
+        const long long row0 = (long long)(item / q_items) * Nq + 2 * (item % q_items);
+        const bool two = 2 * (item % q_items) + 1 < Nq;
+        int n[2], distinct[2] = {0, 0}, shared = 0;
+        for (int w = lane; w < words; w += 32) bits[0][w] = bits[1][w] = 0u;
+        __syncwarp();
+        auto id_of = [&](int side, int i) { return max(0, min(index[(row0 + side) * Nkv + i], Nkv - 1)); };
 #pragma unroll
-    for (int side = 0; side < 2; ++side) {
-        n[side] = side == 0 || two ? max(0, min(num[row0 + side], Nkv)) : 0;
-        for (int i = lane; i < n[side]; i += 32) {
-            const int id = id_of(side, i);
-            atomicOr(&bits[side][id >> 5], 1u << (id & 31));
+        for (int side = 0; side < 2; ++side) {
+            n[side] = side == 0 || two ? max(0, min(num[row0 + side], Nkv)) : 0;
+            for (int i = lane; i < n[side]; i += 32) {
+                const int id = id_of(side, i);
+                atomicOr(&bits[side][id >> 5], 1u << (id & 31));
+            }
         }
-    }
-    __syncwarp();
-    for (int w = lane; w < words; w += 32) {
-        distinct[0] += __popc(bits[0][w]);
-        distinct[1] += __popc(bits[1][w]);
-        shared += __popc(bits[0][w] & bits[1][w]);
-    }
+        __syncwarp();
+        for (int w = lane; w < words; w += 32) {
+            distinct[0] += __popc(bits[0][w]);
+            distinct[1] += __popc(bits[1][w]);
+            shared += __popc(bits[0][w] & bits[1][w]);
+        }
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-        distinct[0] += __shfl_xor_sync(0xffffffffu, distinct[0], o);
-        distinct[1] += __shfl_xor_sync(0xffffffffu, distinct[1], o);
-        shared += __shfl_xor_sync(0xffffffffu, shared, o);
-    }
-    const bool plain = distinct[0] != n[0] || distinct[1] != n[1];
-    const int n_both = plain ? 0 : shared;
-    int32_t *own = lists + row0 * Nkv;
-    if (plain) {
+        for (int o = 16; o > 0; o >>= 1) {
+            distinct[0] += __shfl_xor_sync(0xffffffffu, distinct[0], o);
+            distinct[1] += __shfl_xor_sync(0xffffffffu, distinct[1], o);
+            shared += __shfl_xor_sync(0xffffffffu, shared, o);
+        }
+        const bool plain = distinct[0] != n[0] || distinct[1] != n[1];
+        const int n_both = plain ? 0 : shared;
+        int32_t *own = lists + row0 * Nkv;
+        if (plain) {
 #pragma unroll
-        for (int side = 0; side < 2; ++side)
-            for (int i = lane; i < n[side]; i += 32) own[(long long)side * Nkv + i] = id_of(side, i);
-    } else {
-        int at[3] = {0, n_both, n_both};            // next place of a block of both, of the first row's others, of the second's
-        for (int w0 = 0; w0 < words; w0 += 32) {
-            const uint32_t a = w0 + lane < words ? bits[0][w0 + lane] : 0u, b = w0 + lane < words ? bits[1][w0 + lane] : 0u;
-            const uint32_t part[3] = {a & b, a & ~b, b & ~a};
+            for (int side = 0; side < 2; ++side)
+                for (int i = lane; i < n[side]; i += 32) own[(long long)side * Nkv + i] = id_of(side, i);
+        } else {
+            int at[3] = {0, n_both, n_both};            // next place of a block of both, of the first row's others, of the second's
+            for (int w0 = 0; w0 < words; w0 += 32) {
+                const uint32_t a = w0 + lane < words ? bits[0][w0 + lane] : 0u, b = w0 + lane < words ? bits[1][w0 + lane] : 0u;
+                const uint32_t part[3] = {a & b, a & ~b, b & ~a};
 #pragma unroll
-            for (int k = 0; k < 3; ++k) {
-                const int mine = __popc(part[k]);
-                int incl = mine;
+                for (int k = 0; k < 3; ++k) {
+                    const int mine = __popc(part[k]);
+                    int incl = mine;
 #pragma unroll
-                for (int o = 1; o < 32; o <<= 1) {
-                    const int v = __shfl_up_sync(0xffffffffu, incl, o);
-                    if (lane >= o) incl += v;
-                }
-                int pos = at[k] + incl - mine;
-                at[k] += __shfl_sync(0xffffffffu, incl, 31);
-                for (uint32_t m = part[k]; m; m &= m - 1, ++pos) {
-                    const int id = (w0 + lane) * 32 + __ffs(m) - 1;
-                    if (k != 2) own[pos] = id;
-                    if (k != 1 && two) own[Nkv + pos] = id;
+                    for (int o = 1; o < 32; o <<= 1) {
+                        const int v = __shfl_up_sync(0xffffffffu, incl, o);
+                        if (lane >= o) incl += v;
+                    }
+                    int pos = at[k] + incl - mine;
+                    at[k] += __shfl_sync(0xffffffffu, incl, 31);
+                    for (uint32_t m = part[k]; m; m &= m - 1, ++pos) {
+                        const int id = (w0 + lane) * 32 + __ffs(m) - 1;
+                        if (k != 2) own[pos] = id;
+                        if (k != 1 && two) own[Nkv + pos] = id;
+                    }
                 }
             }
         }
+        if (lane == 0) both[item] = n_both | ((max(n[0], n[1]) - (n_both >> 1)) << 16);
     }
-    if (lane == 0) both[item] = n_both;
+    __threadfence();
+    __syncthreads();
+    if (threadIdx.x == 0) last_cta = atomicAdd(job.pairs_done, 1) == (int)gridDim.x - 1;
+    __syncthreads();
+    if (!last_cta) return;
+    __threadfence();
+    auto tiles_of = [&](int i) { return (int)((uint32_t)__ldcg(both + i) >> 16); };
+    // calls with so many items that ranking them against one another would take too long are sorted over all heads
+    if (job.by_head && n_items / q_items <= SCHED_HEADS && n_items <= SCHED_BINS - 2 * SCHED_HEADS && (long long)n_items * (q_items + ctas) <= 1ll << 19)
+        sort_items_by_head(tiles_of, n_items, q_items, Nkv, ctas, hist, job.order, job.work_counter, job.error_flag);
+    else
+        sort_items(tiles_of, n_items, Nkv, hist, warp_tot, job.order, job.work_counter, job.error_flag);
 }
 
 // ---- launch preparation as a kernel of its own (used when the routing kernel has not done it) --------
 __global__ void __launch_bounds__(1024)
-schedule_kernel(const int32_t *__restrict__ num, int rows, int Nq, int Nkv, SchedJob job) {
+schedule_kernel(const int32_t *__restrict__ num, int rows, int Nkv, SchedJob job) {
     if (blockIdx.x > 0) {
-        if (job.gate_w) convert_gate_slice(job, (blockIdx.x - 1) * 1024, 1024);
+        convert_gate_slice(job, (blockIdx.x - 1) * 1024, 1024);
         return;
     }
-    schedule_items(num, rows, Nq, Nkv, job);
+    if (!job.gate_w) convert_gate_slice(job, 0, 0);
+    schedule_items(num, rows, Nkv, job);
 }
 
 // ---- host side -----------------------------------------------------------------------------------
@@ -1150,7 +1168,7 @@ static TunedWs tuned_plan(const wa_hsa_params *p) {
     size_t c = 0;
     const size_t items = (size_t)p->B * p->H * ceil_div(p->Lq, p->block_size < TILE ? p->block_size : TILE);
     w.order = c; c = align_up(c + items * sizeof(int32_t), 256);
-    w.counter = c; c = align_up(c + 2 * sizeof(int), 256);
+    w.counter = c; c = align_up(c + 3 * sizeof(int), 256);
     w.w_bf16 = c; c = align_up(c + (size_t)TILE * TILE * 2, 256);
     w.bias = c; c = align_up(c + TILE * sizeof(float), 256);
     w.zeros = c; c = align_up(c + items * sizeof(int32_t), 256);   // an all-zero `num` for the linear-branch-only launch
@@ -1192,6 +1210,7 @@ SchedJob hsa_sm100_sched_job(const wa_hsa_params *p, void *workspace) {
     job.order = (int32_t *)(ws + w.order);
     job.work_counter = (int *)(ws + w.counter);
     job.error_flag = job.work_counter + 1;
+    job.pairs_done = job.work_counter + 2;
     job.gate_w = p->gate_w; job.gate_b = p->gate_b; job.gate_dt = p->gate_dtype;
     job.w_out = (__nv_bfloat16 *)(ws + w.w_bf16);
     job.b_out = (float *)(ws + w.bias);
@@ -1253,16 +1272,25 @@ int hsa_sm100_launch(const wa_hsa_params *p, int Lc, const wa_tensor4 *kc, const
     if ((rc = make_map_w(&tw, w_bf16))) return rc;
     if ((rc = make_map_4d(&tout, p->part_sparse ? &p->q : &p->out, p->B, p->Lq, p->H, "out", pair ? TILE : blk))) return rc;   // unused in partial mode
 
+    static PerDeviceOnce attr_set;
+    if (!attr_set.done()) {
+        cudaError_t e = cudaSuccess;
+        for (auto kernel : {hsa_fwd_sm100_kernel<TILE, false>, hsa_fwd_sm100_kernel<HALF, false>, hsa_fwd_sm100_kernel<HALF, true>})
+            if (e == cudaSuccess) e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES);
+        if (e == cudaSuccess) e = cudaFuncSetAttribute(pair_lists_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 32 * 1024);
+        if (e != cudaSuccess) return fail((int)e, "wa_hsa_forward(tcgen05): %s", cudaGetErrorString(e));
+        attr_set.mark();
+    }
     const int rows = p->B * p->H * Nq, q_items = pair ? (Nq + 1) / 2 : Nq, n_items = p->B * p->H * q_items;
     if (!prepared) {
-        schedule_kernel<<<p->gate_w ? 1 + TILE * TILE / 1024 : 1, 1024, 0, stream>>>(num, rows, Nq, Nkv, job);
+        schedule_kernel<<<p->gate_w ? 1 + TILE * TILE / 1024 : 1, 1024, 0, stream>>>(num, rows, Nkv, job);
         if ((rc = check_launch("wa_hsa_forward(schedule)"))) return rc;
     }
 
     if (pair) {
-        const size_t smem = (size_t)PL_WARPS * 2 * ((Nkv + 31) / 32) * sizeof(uint32_t);   // at most 16 KB
+        const size_t smem = (size_t)PL_WARPS * 2 * ((Nkv + 31) / 32) * sizeof(uint32_t);   // at most 32 KB beside 17 KB for the order
         const cudaError_t e = launch_dependent(pair_lists_kernel, dim3(ceil_div(n_items, PL_WARPS)), dim3(PL_WARPS * 32), smem, stream, index, num, Nq,
-                                               Nkv, q_items, n_items, lists, both);
+                                               Nkv, q_items, n_items, lists, both, n_items < max_grid() ? n_items : max_grid(), job);
         if (e != cudaSuccess) return fail((int)e, "wa_hsa_forward(pairs): %s", cudaGetErrorString(e));
         if ((rc = check_launch("wa_hsa_forward(pairs)"))) return rc;
         index = lists;
@@ -1297,14 +1325,6 @@ int hsa_sm100_launch(const wa_hsa_params *p, int Lc, const wa_tensor4 *kc, const
     }
 
 
-    static PerDeviceOnce attr_set;
-    if (!attr_set.done()) {
-        cudaError_t e = cudaSuccess;
-        for (auto kernel : {hsa_fwd_sm100_kernel<TILE, false>, hsa_fwd_sm100_kernel<HALF, false>, hsa_fwd_sm100_kernel<HALF, true>})
-            if (e == cudaSuccess) e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES);
-        if (e != cudaSuccess) return fail((int)e, "wa_hsa_forward(tcgen05): %s", cudaGetErrorString(e));
-        attr_set.mark();
-    }
     int grid = n_items < max_grid() ? n_items : max_grid();
 #ifdef WA_SM100_TRACE
     if (getenv("WA_SM100_ONE_CTA") && grid > max_grid() / 2) grid = max_grid() / 2;   // tuning aid: one CTA per SM

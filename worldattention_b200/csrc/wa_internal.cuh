@@ -15,8 +15,9 @@ struct SchedJob {
     int gate_dt;
     __nv_bfloat16 *w_out;   // [128 x 128] bf16
     float *b_out;           // [128] float32
-    bool paired;            // a work item is two neighbouring query blocks (rows of `num`) of one head
+    bool paired;            // a work item is two neighbouring query blocks (rows of `num`) of one head: pair_lists_kernel makes the order
     bool by_head;           // paired: work order head by head (see sort_items_by_head)
+    int *pairs_done;        // paired: CTAs of pair_lists_kernel that are done; zero before it runs
     bool release_at_start;  // the next launch does not wait for the routing (it compresses K and V meanwhile)
     int release_dependents_after_rows;   // timing experiment (WA_B200_PDL=2), see route_row
 };
@@ -91,11 +92,13 @@ __device__ __forceinline__ void sort_items(Count count_of, int n_items, int Nkv,
 }
 
 // Head by head, the head with the most work first and a head's items heaviest first, so that the CTAs at work at a time read
-// the keys of a few heads (counts from the mass over a window of 21 frames: 797 against 716 us a call).  Taken back: only the
-// heavier 60 % of a head's items so and the rest by weight over all heads, which evens out the end but mixes the heads again
-// (764 us).
+// the keys of a few heads (counts from the mass over a window of 21 frames: 797 against 716 us a call).  The last heads, as many as
+// the CTAs work on at a time, are taken together, heaviest item first: the keys are no more than before, and the items that come last
+// are then the lightest of all these and not the lightest of one head behind heavier ones (with weights that are tiles, see
+// pair_lists_kernel, 496 -> 465 us).  Taken
+// back: only the heavier 60 % of a head's items by head and the rest by weight over all heads, which mixes the heads again (764 us).
 template <typename Count>
-__device__ __forceinline__ void sort_items_by_head(Count count_of, int n_items, int each, int Nkv, int *hist, int32_t *__restrict__ order,
+__device__ __forceinline__ void sort_items_by_head(Count count_of, int n_items, int each, int Nkv, int ctas, int *hist, int32_t *__restrict__ order,
                                                    int *work_counter, int *error_flag) {
     const int T = blockDim.x, tid = threadIdx.x, heads = n_items / each;
     int *head_sum = hist + SCHED_BINS - 2 * SCHED_HEADS, *head_rank = head_sum + SCHED_HEADS;   // behind the items' weights
@@ -107,7 +110,7 @@ __device__ __forceinline__ void sort_items_by_head(Count count_of, int n_items, 
     __syncthreads();
     for (int i = tid; i < n_items; i += T) {
         const int w = max(0, min(count_of(i), Nkv));
-        hist[i] = w;
+        hist[i] = (w << 12) | (SCHED_BINS - 1 - i);      // all different: an item's rank is the number of larger ones
         atomicAdd(&head_sum[i / each], w);
     }
     __syncthreads();
@@ -117,45 +120,37 @@ __device__ __forceinline__ void sort_items_by_head(Count count_of, int n_items, 
         head_rank[i] = rank;
     }
     __syncthreads();
+    const int alone = max(0, heads - (ctas + each - 1) / each);      // heads that keep to themselves
     for (int i = tid; i < n_items; i += T) {
-        const int head = i / each, first = head * each, w = hist[i];
+        const int head = i / each, mine = hist[i], by_itself = head_rank[head] < alone;
         int rank = 0;
-        for (int j = first; j < first + each; ++j) rank += hist[j] > w || (hist[j] == w && j < i);
-        order[head_rank[head] * each + rank] = i;
+        for (int other = by_itself ? head : 0; other < (by_itself ? head + 1 : heads); ++other) {
+            if (!by_itself && head_rank[other] < alone) continue;
+#pragma unroll 8
+            for (int j = 0; j < each; ++j) rank += hist[other * each + j] > mine;
+        }
+        order[(by_itself ? head_rank[head] : alone) * each + rank] = i;
     }
 }
 
-// Work order of the items (a row of the routing, or two neighbouring ones of a head), heavy first (weight: selected blocks; of a
-// pair of rows the larger count).  Called by every thread of ONE CTA whose size is a power of two between 32 and 1024.
-// `num_of(row)` is a row's count.
-template <typename Num>
-__device__ __forceinline__ void schedule_items_by(Num num_of, int rows, int Nq, int Nkv, const SchedJob &job) {
+// Work order of single rows, heaviest first.  Called by every thread of ONE CTA whose size is a power of two between 32 and 1024.
+// `count_of(row)` is a row's number of selected blocks.
+template <typename Count>
+__device__ __forceinline__ void schedule_rows(Count count_of, int rows, int Nkv, const SchedJob &job) {
     __shared__ int hist[SCHED_BINS];
     __shared__ int warp_tot[32];
-    if (!job.paired) {
-        sort_items(num_of, rows, Nkv, hist, warp_tot, job.order, job.work_counter, job.error_flag);
-        return;
-    }
-    const int each = (Nq + 1) >> 1, heads = rows / Nq, n_items = heads * each;
-    // without branches, so that a thread's look-ups are all on their way at once (one after the other they cost the call 3 us)
-    auto count_of = [&](int i) {
-        const int head = i / each, q = 2 * (i - head * each), at = head * Nq + q;
-        return max(num_of(at), num_of(at + (q + 1 < Nq ? 1 : 0)));
-    };
-    // calls with so many items that ranking them against one another would take too long are sorted over all heads
-    if (job.by_head && heads <= SCHED_HEADS && n_items <= SCHED_BINS - 2 * SCHED_HEADS && (long long)n_items * each <= 2048ll * blockDim.x)
-        sort_items_by_head(count_of, n_items, each, Nkv, hist, job.order, job.work_counter, job.error_flag);
-    else
-        sort_items(count_of, n_items, Nkv, hist, warp_tot, job.order, job.work_counter, job.error_flag);
+    sort_items(count_of, rows, Nkv, hist, warp_tot, job.order, job.work_counter, job.error_flag);
 }
 
-// The counts were written by other CTAs of this launch: they are read past L1.
-__device__ inline void schedule_items(const int32_t *num, int rows, int Nq, int Nkv, const SchedJob &job) {
-    schedule_items_by([&](int row) { return __ldcg(num + row); }, rows, Nq, Nkv, job);
+// The same after a routing kernel, whose counts were written by other CTAs of this launch: they are read past L1.
+__device__ inline void schedule_items(const int32_t *num, int rows, int Nkv, const SchedJob &job) {
+    if (!job.paired) schedule_rows([&](int row) { return __ldcg(num + row); }, rows, Nkv, job);
 }
 
 // Elements [first, first + count) of the gate weight -> bf16 (it is an MMA operand) and of the bias -> float32.
 __device__ inline void convert_gate_slice(const SchedJob &job, int first, int count) {
+    if (first == 0 && threadIdx.x == 0 && job.pairs_done) *job.pairs_done = 0;
+    if (!job.gate_w) return;
     for (int i = first + threadIdx.x; i < first + count && i < 128 * 128; i += blockDim.x) {
         job.w_out[i] = __float2bfloat16_rn(load_elem(job.gate_w, job.gate_dt, i));
         if (i < 128) job.b_out[i] = job.gate_b ? load_elem(job.gate_b, job.gate_dt, i) : 0.f;

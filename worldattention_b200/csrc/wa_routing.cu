@@ -982,7 +982,7 @@ __device__ __forceinline__ void route_row(const long long row, const bool logits
     __syncthreads();
     if (!last_flag || !job.order) return;
     __threadfence();
-    schedule_items(num, B * H * Nq, Nq, Nkv, job);
+    schedule_items(num, B * H * Nq, Nkv, job);
     ROUTE_STAMP(7);
 }
 
@@ -1011,7 +1011,7 @@ route_fused_kernel(const float *__restrict__ qp, const float *__restrict__ kp, i
     if (row >= (long long)B * H * Nq) return;
 
     ROUTE_STAMP(0);
-    if (job.order && job.gate_w) convert_gate_slice(job, (int)row * gate_per_cta, gate_per_cta);
+    if (job.order) convert_gate_slice(job, (int)row * gate_per_cta, gate_per_cta);
     route_row(row, logits_ready != 0, qp, kp, B, H, Nq, Nkv, n_pow2, D, scale, tau_min, tau_span, fixed_num, sorted, index, num, thresholds,
               gini_rows, counters, job, keys, probs, red, bcast, last_flag);
 }
@@ -1044,7 +1044,7 @@ route_head_kernel(const float *__restrict__ qp, const float *__restrict__ kp, in
     const int h = blockIdx.x, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t = lane & 3, rows = B * Nq;
     pdl_wait();                 // pooled means and zeroed counters come from the launch before
     if (job.release_at_start) pdl_release_dependents();
-    if (job.order && job.gate_w) convert_gate_slice(job, h * gate_per_cta, gate_per_cta);
+    if (job.order) convert_gate_slice(job, h * gate_per_cta, gate_per_cta);
 
     const int row_tiles = (Nq + 15) / 16, key_tiles = (Nkv + 7) / 8;
     for (int u = warp; u < B * row_tiles * key_tiles; u += RH_WARPS) {
@@ -1160,7 +1160,7 @@ route_head_kernel(const float *__restrict__ qp, const float *__restrict__ kp, in
     __syncthreads();
     if (!last_flag || !job.order) return;
     __threadfence();
-    schedule_items(num, B * H * Nq, Nq, Nkv, job);
+    schedule_items(num, B * H * Nq, Nkv, job);
 }
 
 // ------------------------------------------------------------------------------------------------
@@ -1193,14 +1193,13 @@ route_topk_kernel(const float *__restrict__ qp, const float *__restrict__ kp, in
     pdl_wait();                 // pooled means, or logits, come from the launch before
     if (job.release_at_start) pdl_release_dependents();
     if (blockIdx.x == 0) {
-        if (job.order)
-            schedule_items_by([&](int row) { return __ldg(fixed_num + (row / Nq) % H); }, rows, Nq, Nkv, job);
+        if (job.order && !job.paired) schedule_rows([&](int row) { return __ldg(fixed_num + (row / Nq) % H); }, rows, Nkv, job);
         return;
     }
     // neighbouring rows (same head, same pooled keys) on one SM, as in route_fused_kernel
     const int at = blockIdx.x - 1, row = (at % sm_count) * per_sm + at / sm_count;
     if (row >= rows) return;
-    if (job.order && job.gate_w) convert_gate_slice(job, row * gate_per_cta, gate_per_cta);
+    if (job.order) convert_gate_slice(job, row * gate_per_cta, gate_per_cta);
 
     const int want = max(0, min(fixed_num[(row / Nq) % H], Nkv));
     if (tid == 0) {
