@@ -58,7 +58,7 @@ extern "C" const char *wa_last_error(void) { return last_error_buffer(); }
 namespace {
 
 struct Workspace {
-    size_t q_pooled, k_pooled, block_attn, index, num, gini, thresholds, counters, kc, vc, sparse, linear, tuned, total;
+    size_t q_pooled, k_pooled, block_attn, index, num, gini, thresholds, counters, kc, vc, sparse, linear, tuned, kv16, total;
     int Nq, Nkv, Lc_inline;
 };
 
@@ -77,6 +77,14 @@ int inline_coarse_len(const wa_hsa_params *p) {
         total += r < p->proj_rank ? r : p->proj_rank;
     }
     return total;
+}
+
+// Keys and values of a float32 call are rounded once for all query blocks: a pass over memory that pays where a key block is
+// selected several times and the chip is full (12 heads over 4680 keys, 64-token blocks, the whole call without and with it: 4 query
+// blocks 210 and 219 us, 12 245 and 242, 14 286 and 278, 25 323 and 317; over 9360 keys 25 blocks 576 and 551).
+bool keeps_rounded_kv(const wa_hsa_params *p) {
+    return p->k.dtype == WA_F32 && p->v.dtype == WA_F32 && p->D == 128 &&
+           (long long)p->B * p->H * ceil_div(p->Lq, p->block_size) >= sm_count();
 }
 
 Workspace plan(const wa_hsa_params *p) {
@@ -101,6 +109,7 @@ Workspace plan(const wa_hsa_params *p) {
     w.sparse = take(c, tokens * sizeof(__nv_bfloat16));
     w.linear = take(c, tokens * sizeof(float));
     w.tuned = take(c, hsa_sm100_workspace_bytes(p));
+    w.kv16 = take(c, keeps_rounded_kv(p) ? 2 * (size_t)p->B * p->Lkv * p->H * p->D * sizeof(__nv_bfloat16) : 0);
     w.total = c;
     return w;
 }
@@ -202,6 +211,7 @@ extern "C" int wa_hsa_forward(const wa_hsa_params *p, int *used_tuned, void *str
                "%s: a partial-output layout other than the contiguous one needs the tcgen05 kernel", what);
 
     bool prepared = false;
+    const int32_t *order = nullptr;
     if (p->index_in) {
         index = const_cast<int32_t *>(p->index_in);
         num = const_cast<int32_t *>(p->num_in);
@@ -213,7 +223,13 @@ extern "C" int wa_hsa_forward(const wa_hsa_params *p, int *used_tuned, void *str
                               counters, p->H + 1, k_first, p->status_mirror)))
             return rc;
         SchedJob job{};
-        if (tuned) job = hsa_sm100_sched_job(p, ws + w.tuned);
+        const bool ordered = !tuned && !partial && p->D == 128;
+        if (tuned || ordered) job = hsa_sm100_sched_job(p, ws + w.tuned);
+        if (ordered) {      // the sparse branch takes its rows heaviest first as well, one by one
+            job.paired = job.by_head = false;
+            job.gate_w = job.gate_b = nullptr;
+            order = job.order;
+        }
         job.release_at_start = compress_inline;
         if ((rc = route_fused_launch(q_pooled, k_pooled, p->B, p->H, w.Nq, w.Nkv, p->D, p->tau_min, p->tau_max,
                                      p->topk_per_head, block_attn, index, num, thresholds, gini, counters, job, stream,
@@ -222,9 +238,11 @@ extern "C" int wa_hsa_forward(const wa_hsa_params *p, int *used_tuned, void *str
         prepared = tuned;
     }
 
+    const bool rounded = !tuned && !partial && keeps_rounded_kv(p) && round_kv_supported(&p->k, &p->v, p->D);
     if (compress_inline) {
         if ((rc = compress_kv_launch(&p->k, &p->v, &kc, &vc, p->B, p->Lkv, p->H, p->D, p->proj_segment_len, p->block_size, p->k_proj,
-                                     p->v_proj, p->proj_dtype, p->proj_rank, p->proj_cols, /*beside_routing=*/!p->index_in, stream)))
+                                     p->v_proj, p->proj_dtype, p->proj_rank, p->proj_cols, /*beside_routing=*/!p->index_in, stream,
+                                     /*ahead=*/rounded && !p->index_in)))
             return rc;
     }
 
@@ -256,18 +274,30 @@ extern "C" int wa_hsa_forward(const wa_hsa_params *p, int *used_tuned, void *str
     sparse.stride_h = linear.stride_h = p->D;
     sparse.stride_l = linear.stride_l = (int64_t)p->H * p->D;
     sparse.stride_b = linear.stride_b = (int64_t)p->Lq * p->H * p->D;
+    wa_tensor4 ks = p->k, vs = p->v;
+    if (rounded) {
+        // beside the compression, or whatever else came last: only the keys and values themselves are read
+        if ((rc = round_kv_launch(&p->k, &p->v, p->B, p->Lkv, p->H, p->D, ws + w.kv16, /*beside=*/!p->index_in, stream))) return rc;
+        ks.dtype = vs.dtype = WA_BF16;
+        ks.ptr = ws + w.kv16;
+        vs.ptr = (__nv_bfloat16 *)ks.ptr + (size_t)p->B * p->Lkv * p->H * p->D;
+        ks.stride_h = vs.stride_h = p->D;
+        ks.stride_l = vs.stride_l = (int64_t)p->H * p->D;
+        ks.stride_b = vs.stride_b = (int64_t)p->Lkv * p->H * p->D;
+    }
+    const bool linear_tuned = !(p->flags & WA_HSA_FORCE_GENERIC) && hsa_sm100_linear_supported(p, Lc, &kc, &vc);
     profile_mark(true, stream);
-    rc = wa_block_sparse_forward(&p->q, &p->k, &p->v, &sparse, p->B, p->H, p->Lq, p->Lkv, p->D, p->block_size, index,
-                                 num, w.Nkv, nullptr, /*round_in=*/1, /*round_out=*/1, nullptr, stream);
+    rc = block_sparse_run(&p->q, &ks, &vs, &sparse, p->B, p->H, p->Lq, p->Lkv, p->D, p->block_size, index, num, w.Nkv, nullptr,
+                          /*round_in=*/1, /*round_out=*/1, nullptr, order, /*ahead=*/!linear_tuned, stream);
     profile_mark(false, stream);
     if (rc) return rc;
-    if (!(p->flags & WA_HSA_FORCE_GENERIC) && hsa_sm100_linear_supported(p, Lc, &kc, &vc)) {
+    if (linear_tuned) {
         // routing block size other than 128: the sparse branch ran on the SIMT kernel above, but the linear branch
         // does not depend on the block size and takes the tcgen05 kernel (float32 result, as in the fused path)
         linear.dtype = WA_F32;
         if ((rc = hsa_sm100_launch_linear(p, Lc, &kc, &vc, (float *)linear.ptr, ws + w.tuned, stream))) return rc;
-    } else if ((rc = wa_linear_branch(&p->q, &kc, &vc, &linear, p->B, p->H, p->Lq, Lc, p->D, lin_dtype == WA_BF16, nullptr,
-                                      stream))) {
+    } else if ((rc = linear_run(&p->q, &kc, &vc, &linear, p->B, p->H, p->Lq, Lc, p->D, lin_dtype == WA_BF16, nullptr, /*beside=*/true,
+                                stream))) {
         return rc;
     }
     return wa_gate_combine(&p->q, &sparse, &linear, &p->out, p->B, p->Lq, p->H, p->D, p->gate_w, p->gate_b,

@@ -36,6 +36,8 @@ struct GenericAttnParams {
     int round_in, round_out;
     float scale;
     float *lse;
+    const int32_t *order;   // split kernel, not dense: routing rows in the order in which CTAs take them, or null
+    int ahead, beside;      // split kernel: the next launch may start while this one runs; this one started while the one before it ran
 };
 
 __global__ void __launch_bounds__(GA_THREADS)
@@ -181,13 +183,20 @@ generic_attention_kernel(GenericAttnParams p) {
 // 9.2e-7 -> 2.6e-7, 4680 rounded keys 1.25e-6 -> 2.9e-7; the log-sum-exp has the same error within 6 % or less.
 // The SIMT kernel above is bound by shared-memory reads (one per four multiply-adds).  12 heads, 1560 queries: a third of
 // 4680 keys in 64-token blocks 1480 -> 238 us, 75 float32 slots 92 -> 57 us.
+//
+// DIRECT: keys and values that are bf16 in memory (aligned rows) go to shared memory by asynchronous copies, the next chunk
+// while one is at work, with one barrier a chunk.  Float32 layers get there by rounding keys and values once (round_kv_kernel, see
+// wa_hsa_forward) instead of in every CTA that selects them: 238 -> 202 us.  Rows of
+// different counts then left a third of the chip idle at the end (mean 240 of 368 kcycles per SM): they are taken heaviest first
+// (-> 156 us), and the linear branch's launch starts on what the last of them leave free (`ahead`, `beside`: the two branches
+// 261 -> 216 us from the first's start to the second's end).
 // ------------------------------------------------------------------------------------------------
 constexpr int SA_ROWS = 64;                  // query rows of a CTA
 constexpr int SA_THREADS = 256;
 constexpr int SA_D = 128;
 constexpr int SA_LD = SA_D + 8;              // bf16 elements of a shared-memory row: ldmatrix without bank conflicts
 constexpr int sa_keys(int ns) { return ns == 1 ? 64 : 32; }
-constexpr size_t sa_smem(int ns) { return (size_t)ns * (SA_ROWS + 2 * sa_keys(ns)) * SA_LD * 2 + 32; }
+constexpr size_t sa_smem(int ns, int stages) { return (size_t)ns * (SA_ROWS + stages * 2 * sa_keys(ns)) * SA_LD * 2 + stages * 32; }
 
 __device__ __forceinline__ uint32_t sa_u32(const void *p) { return (uint32_t)__cvta_generic_to_shared(p); }
 __device__ __forceinline__ void ldsm4(uint32_t (&r)[4], uint32_t addr) {
@@ -254,18 +263,36 @@ __device__ __forceinline__ float4 fetch4(const void *base, int dtype, long long 
     return make_float4(a.x, a.y, b.x, b.y);
 }
 
-template <int NS>
+__device__ __forceinline__ void copy16_async(uint32_t dst, const void *src, bool real) {      // zeros if not real
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(real ? 16 : 0) : "memory");
+}
+
+template <int NS, bool DIRECT>
 __global__ void __launch_bounds__(SA_THREADS, NS == 1 ? 2 : 1)
 split_attention_kernel(GenericAttnParams p) {
+    static_assert(!DIRECT || NS == 1, "asynchronous copies bring bf16 values");
     constexpr int KC = sa_keys(NS), KW = KC / 2, NT = KW / 8, RW = KC / 8;   // keys of a chunk and of a warp; 8-key tiles; rows a warp stages
     extern __shared__ __align__(16) uint8_t sa_raw[];
     __nv_bfloat16 *qs = reinterpret_cast<__nv_bfloat16 *>(sa_raw);   // [NS][SA_ROWS][SA_LD]
     __nv_bfloat16 *ks = qs + NS * SA_ROWS * SA_LD;                    // [NS][KC][SA_LD]
     __nv_bfloat16 *vs = ks + NS * KC * SA_LD;                         // [NS][KC][SA_LD]
-    unsigned *real = reinterpret_cast<unsigned *>(vs + NS * KC * SA_LD);   // per warp: which of the rows it staged are real keys
+    constexpr int STAGES = DIRECT ? 2 : 1, STAGE_ELEMS = 2 * NS * KC * SA_LD;
+    unsigned *real = reinterpret_cast<unsigned *>(ks + STAGES * STAGE_ELEMS);   // per stage and warp: which of the rows it staged are real keys
 
-    const int qb = blockIdx.x / p.tiles_per_block, tile = blockIdx.x % p.tiles_per_block;
-    const int h = blockIdx.y, b = blockIdx.z;
+    if (p.ahead) pdl_release_dependents();
+    // what is left of the chip at the end of the launch before this one is used; whoever waits for this launch waits for both
+    struct Both {
+        int beside;
+        __device__ ~Both() { if (beside) pdl_wait(); }
+    } both{p.beside};
+    int qb = blockIdx.x / p.tiles_per_block, h = blockIdx.y, b = blockIdx.z;
+    const int tile = blockIdx.x % p.tiles_per_block, n_qb = (p.Lq + p.q_block - 1) / p.q_block;
+    if (p.order) {
+        const int item = p.order[qb];
+        qb = item % n_qb;
+        h = item / n_qb % p.H;
+        b = item / n_qb / p.H;
+    }
     const int row0 = qb * p.q_block + tile * p.q_tile;
     const int rows_here = max(0, min(min(p.q_tile, p.q_block - tile * p.q_tile), p.Lq - row0));
     if (rows_here <= 0) return;
@@ -299,20 +326,47 @@ split_attention_kernel(GenericAttnParams p) {
     const uint32_t va = sa_u32(vs + (half_keys * KW + (lane & 15)) * SA_LD + (lane >> 4) * 8);
     constexpr uint32_t Q_PART = SA_ROWS * SA_LD * 2, K_PART = KC * SA_LD * 2;   // bytes between the parts of an operand
 
-    for (long long c0 = 0; c0 < total; c0 += KC) {
-        __syncthreads();   // the chunk before this one has been read
-        // this warp stages rows warp * RW ... of the chunk; lane i looks up the i-th of them
-        int token = -1;
-        if (lane < RW) {
-            const long long j = c0 + warp * RW + lane;
-            if (j < total) {
-                const int s = (int)(j / p.kv_block), off = (int)(j - (long long)s * p.kv_block);
-                const int id = max(0, min(p.dense ? s : ids[s], p.n_kv_blocks - 1));
-                int size = p.block_sizes ? p.block_sizes[id] : p.Lkv - id * p.kv_block;
-                size = max(0, min(size, min(p.kv_block, p.Lkv - id * p.kv_block)));
-                if (off < size) token = id * p.kv_block + off;
-            }
+    // this warp stages rows warp * RW ... of a chunk; lane i looks up the block of the i-th of them, then its token
+    auto block_of = [&](long long c0) -> int {
+        const long long j = c0 + warp * RW + lane;
+        if (lane >= RW || j >= total) return -1;
+        const int s = (int)(j / p.kv_block);
+        return max(0, min(p.dense ? s : ids[s], p.n_kv_blocks - 1));
+    };
+    auto token_of = [&](long long c0, int id) -> int {
+        if (id < 0) return -1;
+        const int off = (int)((c0 + warp * RW + lane) % p.kv_block);
+        int size = p.block_sizes ? p.block_sizes[id] : p.Lkv - id * p.kv_block;
+        size = max(0, min(size, min(p.kv_block, p.Lkv - id * p.kv_block)));
+        return off < size ? id * p.kv_block + off : -1;
+    };
+    int stage = 0, next_block = block_of(0);
+    // DIRECT: the chunk at c0 into a stage; the blocks of the chunk behind it are looked up on the way
+    auto copy_chunk = [&](long long c0, int to) {
+        const int token = token_of(c0, next_block);
+        next_block = block_of(c0 + KC);
+        const unsigned found = __ballot_sync(0xffffffffu, token >= 0);
+        if (lane == 0) real[to * 8 + warp] = found;
+        const uint32_t dst = sa_u32(ks + to * STAGE_ELEMS + (warp * RW + (lane >> 4)) * SA_LD + (lane & 15) * 8);
+#pragma unroll
+        for (int r = 0; r < RW; r += 2) {
+            const int t = __shfl_sync(0xffffffffu, token, r + (lane >> 4));
+            const long long row = max(t, 0);
+            copy16_async(dst + r * SA_LD * 2, (const __nv_bfloat16 *)p.k.ptr + kbase + row * p.k.sl + (lane & 15) * 8, t >= 0);
+            copy16_async(dst + (KC + r) * SA_LD * 2, (const __nv_bfloat16 *)p.v.ptr + vbase + row * p.v.sl + (lane & 15) * 8, t >= 0);
         }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+    if (DIRECT && total > 0) copy_chunk(0, 0);
+
+    for (long long c0 = 0; c0 < total; c0 += KC, stage ^= DIRECT ? 1 : 0) {
+        if (DIRECT) {
+            asm volatile("cp.async.wait_group 0;" ::: "memory");
+            __syncthreads();      // this chunk has arrived, and the one before it, in the other stage, has been read
+            if (c0 + KC < total) copy_chunk(c0 + KC, stage ^ 1);
+        } else {
+        __syncthreads();   // the chunk before this one has been read
+        const int token = token_of(c0, block_of(c0));
         const unsigned found = __ballot_sync(0xffffffffu, token >= 0);
         if (lane == 0) real[warp] = found;
 #pragma unroll
@@ -335,10 +389,12 @@ split_attention_kernel(GenericAttnParams p) {
             }
         }
         __syncthreads();
+        }
+        const uint32_t at = stage * STAGE_ELEMS * 2;      // bytes
         if (!rows_mine) continue;
         unsigned keep = 0;   // this warp's keys that are real
 #pragma unroll
-        for (int w = 0; w < 4; ++w) keep |= real[4 * half_keys + w] << (w * RW);
+        for (int w = 0; w < 4; ++w) keep |= real[stage * 8 + 4 * half_keys + w] << (w * RW);
         if (keep == 0) continue;
         any_key = 1;
         const bool full = keep == (KW == 32 ? ~0u : (1u << (KW & 31)) - 1);
@@ -357,7 +413,7 @@ split_attention_kernel(GenericAttnParams p) {
 #pragma unroll
                 for (int i = NS - 1; i >= 0; --i) {
                     uint32_t kb[4];
-                    ldsm4(kb, ka + i * K_PART + (uint32_t)(j * 8 * SA_LD + kk * 16) * 2);
+                    ldsm4(kb, ka + at + i * K_PART + (uint32_t)(j * 8 * SA_LD + kk * 16) * 2);
 #pragma unroll
                     for (int u = NS - 1; u >= 0; --u) mma_step(i == NS - 1 && u == NS - 1, x0, x1, a[u], kb);
                 }
@@ -422,7 +478,7 @@ split_attention_kernel(GenericAttnParams p) {
 #pragma unroll
                 for (int i = NS - 1; i >= 0; --i) {
                     uint32_t vb[4];
-                    ldsm4_t(vb, va + i * K_PART + (uint32_t)(kk * 16 * SA_LD + j * 8) * 2);
+                    ldsm4_t(vb, va + at + i * K_PART + (uint32_t)(kk * 16 * SA_LD + j * 8) * 2);
 #pragma unroll
                     for (int u = 2; u >= 0; --u) mma_step(i == NS - 1 && u == 2, x0, x1, a[u], vb);
                 }
@@ -490,25 +546,88 @@ split_attention_kernel(GenericAttnParams p) {
     }
 }
 
-template <int NS>
+template <int NS, bool DIRECT>
 int launch_split_attention(GenericAttnParams &p, int B, int n_q_blocks, cudaStream_t stream, const char *what) {
     p.q_tile = p.q_block < SA_ROWS ? p.q_block : SA_ROWS;
     p.tiles_per_block = ceil_div(p.q_block, p.q_tile);
     const long long gx = (long long)n_q_blocks * p.tiles_per_block;
+    if (p.order && gx * p.H * B >= (1ll << 31)) p.order = nullptr;
     WA_REQUIRE(gx < (1ll << 31) && p.H <= 65535 && B <= 65535, WA_ERR_UNSUPPORTED, "%s: grid too large", what);
     static PerDeviceOnce attr_set;
     if (!attr_set.done()) {
-        const cudaError_t e = cudaFuncSetAttribute(split_attention_kernel<NS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sa_smem(NS));
+        const cudaError_t e = cudaFuncSetAttribute(split_attention_kernel<NS, DIRECT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                                   (int)sa_smem(NS, DIRECT ? 2 : 1));
         if (e != cudaSuccess) return fail((int)e, "%s: %s", what, cudaGetErrorString(e));
         attr_set.mark();
     }
-    split_attention_kernel<NS><<<dim3((unsigned)gx, p.H, B), SA_THREADS, sa_smem(NS), stream>>>(p);
+    const dim3 grid = p.order ? dim3((unsigned)(gx * p.H * B)) : dim3((unsigned)gx, p.H, B);
+    const size_t smem = sa_smem(NS, DIRECT ? 2 : 1);
+    if (p.beside) {
+        const cudaError_t e = launch_dependent(split_attention_kernel<NS, DIRECT>, grid, dim3(SA_THREADS), smem, stream, p);
+        if (e != cudaSuccess) return fail((int)e, "%s: %s", what, cudaGetErrorString(e));
+    } else {
+        split_attention_kernel<NS, DIRECT><<<grid, SA_THREADS, smem, stream>>>(p);
+    }
     return check_launch(what);
 }
 
 // four consecutive elements of every row as one load or store
 static bool rows_of_four(const void *ptr, int dtype, long long sb, long long sl, long long sh) {
     return (uintptr_t)ptr % (4 * dtype_size(dtype)) == 0 && sb % 4 == 0 && sl % 4 == 0 && sh % 4 == 0;
+}
+
+// Float32 keys and values -> bf16, contiguous `[B, L, H, D]` one behind the other at `dst`: what every CTA of the sparse branch would
+// round for itself.  One pass over memory: 2 x 4680 tokens of 1536 channels (57 MB read, 29 written) 13.3 us
+// alone; it runs beside the compression of the call's keys and values.
+constexpr int RK_THREADS = 256, RK_AT_ONCE = 4;
+__global__ void __launch_bounds__(RK_THREADS)
+round_kv_kernel(View4 k, View4 v, long long pieces, int L, int H, int D8, uint4 *__restrict__ dst, int beside) {
+    const View4 &src = blockIdx.y ? v : k;
+    uint4 *out = dst + blockIdx.y * pieces;                      // a piece: eight channels
+    float4 x[RK_AT_ONCE][2];
+    const long long first = (long long)blockIdx.x * RK_THREADS * RK_AT_ONCE + threadIdx.x;
+#pragma unroll
+    for (int u = 0; u < RK_AT_ONCE; ++u) {
+        const long long i = first + u * RK_THREADS;
+        if (i < pieces) {
+            const long long head = i / D8, token = head / H, b = token / L;
+            const float4 *at = reinterpret_cast<const float4 *>((const float *)src.ptr + b * src.sb + (token - b * L) * src.sl + (head - token * H) * src.sh) +
+                               2 * (i - head * D8);
+            x[u][0] = __ldg(at);
+            x[u][1] = __ldg(at + 1);
+        }
+    }
+#pragma unroll
+    for (int u = 0; u < RK_AT_ONCE; ++u) {
+        const long long i = first + u * RK_THREADS;
+        if (i < pieces) {
+            const __nv_bfloat162 a = __floats2bfloat162_rn(x[u][0].x, x[u][0].y), b = __floats2bfloat162_rn(x[u][0].z, x[u][0].w);
+            const __nv_bfloat162 c = __floats2bfloat162_rn(x[u][1].x, x[u][1].y), d = __floats2bfloat162_rn(x[u][1].z, x[u][1].w);
+            out[i] = make_uint4(*reinterpret_cast<const uint32_t *>(&a), *reinterpret_cast<const uint32_t *>(&b),
+                                *reinterpret_cast<const uint32_t *>(&c), *reinterpret_cast<const uint32_t *>(&d));
+        }
+    }
+    if (beside) pdl_wait();
+}
+
+bool round_kv_supported(const wa_tensor4 *k, const wa_tensor4 *v, int D) {
+    const auto ok = [](const wa_tensor4 *t) {
+        return t->dtype == WA_F32 && rows_of_four(t->ptr, t->dtype, t->stride_b, t->stride_l, t->stride_h);
+    };
+    return D == SA_D && ok(k) && ok(v);
+}
+
+int round_kv_launch(const wa_tensor4 *k, const wa_tensor4 *v, int B, int L, int H, int D, void *dst, bool beside, cudaStream_t stream) {
+    const long long pieces = (long long)B * L * H * (D / 8), blocks = (pieces + RK_THREADS * RK_AT_ONCE - 1) / (RK_THREADS * RK_AT_ONCE);
+    WA_REQUIRE(blocks < (1ll << 31), WA_ERR_UNSUPPORTED, "wa_hsa_forward(rounding): too many keys");
+    const View4 kv = make_view(k), vv = make_view(v);
+    if (beside) {
+        const cudaError_t e = launch_dependent(round_kv_kernel, dim3((unsigned)blocks, 2), dim3(RK_THREADS), 0, stream, kv, vv, pieces, L, H, D / 8, (uint4 *)dst, 1);
+        if (e != cudaSuccess) return fail((int)e, "wa_hsa_forward(rounding): %s", cudaGetErrorString(e));
+    } else {
+        round_kv_kernel<<<dim3((unsigned)blocks, 2), RK_THREADS, 0, stream>>>(kv, vv, pieces, L, H, D / 8, (uint4 *)dst, 0);
+    }
+    return check_launch("wa_hsa_forward(rounding)");
 }
 
 int launch_generic_attention(GenericAttnParams &p, int B, int n_q_blocks, cudaStream_t stream,
@@ -521,7 +640,11 @@ int launch_generic_attention(GenericAttnParams &p, int B, int n_q_blocks, cudaSt
             p.q_block = SA_ROWS;
         }
         const bool exact = p.round_in || (p.q.dtype == WA_BF16 && p.k.dtype == WA_BF16 && p.v.dtype == WA_BF16);
-        return exact ? launch_split_attention<1>(p, B, n_q_blocks, stream, what) : launch_split_attention<3>(p, B, n_q_blocks, stream, what);
+        const auto rows_of_eight = [](const View4 &t) {      // 16 bytes at a time
+            return t.dtype == WA_BF16 && (uintptr_t)t.ptr % 16 == 0 && t.sb % 8 == 0 && t.sl % 8 == 0 && t.sh % 8 == 0;
+        };
+        if (exact && rows_of_eight(p.k) && rows_of_eight(p.v)) return launch_split_attention<1, true>(p, B, n_q_blocks, stream, what);
+        return exact ? launch_split_attention<1, false>(p, B, n_q_blocks, stream, what) : launch_split_attention<3, false>(p, B, n_q_blocks, stream, what);
     }
     p.q_tile = p.q_block < GA_QT ? p.q_block : GA_QT;
     p.tiles_per_block = ceil_div(p.q_block, p.q_tile);
@@ -763,11 +886,10 @@ static int check_view(const wa_tensor4 *t, const char *what, const char *name) {
 
 using namespace wa;
 
-extern "C" int wa_block_sparse_forward(const wa_tensor4 *q, const wa_tensor4 *k, const wa_tensor4 *v,
-                                       const wa_tensor4 *out, int B, int H, int Lq, int Lkv, int D,
-                                       int block_size, const int32_t *index, const int32_t *num,
-                                       int index_stride, const int32_t *block_sizes, int round_inputs_bf16,
-                                       int round_output_bf16, float *lse, void *stream) {
+namespace wa {
+int block_sparse_run(const wa_tensor4 *q, const wa_tensor4 *k, const wa_tensor4 *v, const wa_tensor4 *out, int B, int H, int Lq, int Lkv, int D,
+                     int block_size, const int32_t *index, const int32_t *num, int index_stride, const int32_t *block_sizes, int round_inputs_bf16,
+                     int round_output_bf16, float *lse, const int32_t *order, bool ahead, cudaStream_t stream) {
     const char *what = "wa_block_sparse_forward";
     int rc;
     if ((rc = check_view(q, what, "q")) || (rc = check_view(k, what, "k")) || (rc = check_view(v, what, "v")) ||
@@ -785,12 +907,12 @@ extern "C" int wa_block_sparse_forward(const wa_tensor4 *q, const wa_tensor4 *k,
     p.round_in = round_inputs_bf16; p.round_out = round_output_bf16;
     p.scale = (float)(1.0 / sqrt((double)D));
     p.lse = lse;
-    return launch_generic_attention(p, B, ceil_div(Lq, block_size), (cudaStream_t)stream, what);
+    p.order = order; p.ahead = ahead;
+    return launch_generic_attention(p, B, ceil_div(Lq, block_size), stream, what);
 }
 
-extern "C" int wa_linear_branch(const wa_tensor4 *q, const wa_tensor4 *k_coarse, const wa_tensor4 *v_coarse,
-                                const wa_tensor4 *out, int B, int H, int Lq, int Lc, int D,
-                                int round_output_bf16, float *lse, void *stream) {
+int linear_run(const wa_tensor4 *q, const wa_tensor4 *k_coarse, const wa_tensor4 *v_coarse, const wa_tensor4 *out, int B, int H, int Lq, int Lc,
+               int D, int round_output_bf16, float *lse, bool beside, cudaStream_t stream) {
     const char *what = "wa_linear_branch";
     int rc;
     if ((rc = check_view(q, what, "q")) || (rc = check_view(k_coarse, what, "k_coarse")) ||
@@ -806,7 +928,24 @@ extern "C" int wa_linear_branch(const wa_tensor4 *q, const wa_tensor4 *k_coarse,
     p.round_in = 0; p.round_out = round_output_bf16;
     p.scale = (float)pow((double)D, -0.5);
     p.lse = lse;
-    return launch_generic_attention(p, B, ceil_div(Lq, GA_QT), (cudaStream_t)stream, what);
+    p.beside = beside;
+    return launch_generic_attention(p, B, ceil_div(Lq, GA_QT), stream, what);
+}
+}  // namespace wa
+
+extern "C" int wa_block_sparse_forward(const wa_tensor4 *q, const wa_tensor4 *k, const wa_tensor4 *v,
+                                       const wa_tensor4 *out, int B, int H, int Lq, int Lkv, int D,
+                                       int block_size, const int32_t *index, const int32_t *num,
+                                       int index_stride, const int32_t *block_sizes, int round_inputs_bf16,
+                                       int round_output_bf16, float *lse, void *stream) {
+    return block_sparse_run(q, k, v, out, B, H, Lq, Lkv, D, block_size, index, num, index_stride, block_sizes, round_inputs_bf16,
+                            round_output_bf16, lse, nullptr, false, (cudaStream_t)stream);
+}
+
+extern "C" int wa_linear_branch(const wa_tensor4 *q, const wa_tensor4 *k_coarse, const wa_tensor4 *v_coarse,
+                                const wa_tensor4 *out, int B, int H, int Lq, int Lc, int D,
+                                int round_output_bf16, float *lse, void *stream) {
+    return linear_run(q, k_coarse, v_coarse, out, B, H, Lq, Lc, D, round_output_bf16, lse, false, (cudaStream_t)stream);
 }
 
 extern "C" int wa_gate_combine(const wa_tensor4 *q, const wa_tensor4 *sparse, const wa_tensor4 *linear,

@@ -102,7 +102,8 @@ template <int R, typename T>
 __global__ void __launch_bounds__(CF_WARPS * 32)
 compress_cluster_kernel(const T *__restrict__ k, const T *__restrict__ v, long long xsb, long long xsl, T *__restrict__ ok,
                         T *__restrict__ ov, long long osb, long long osl, int L, int segment_len, int block_size, const void *pk,
-                        const void *pv, int pdt, int proj_rank, int proj_cols, int rank_full, int split, int tokens_per_split) {
+                        const void *pv, int pdt, int proj_rank, int proj_cols, int rank_full, int split, int tokens_per_split, int ahead) {
+    if (ahead) pdl_release_dependents();
     extern __shared__ __align__(16) float cc_smem[];
     constexpr int LD = R + 4;
     constexpr size_t HEAD = compress_cluster_smem<R, T>() / sizeof(float) - (size_t)R * 128;
@@ -205,7 +206,7 @@ inline int compress_split(long long groups, int longest, int ctas) {
 template <int R, typename T>
 int compress_cluster_launch(const wa_tensor4 *k, const wa_tensor4 *v, const wa_tensor4 *ok, const wa_tensor4 *ov, int B, int L, int HD,
                             int segment_len, int block_size, const void *k_proj, const void *v_proj, int proj_dtype, int proj_rank,
-                            int proj_cols, int rank_full, bool beside, cudaStream_t stream, const char *what) {
+                            int proj_cols, int rank_full, bool beside, bool ahead, cudaStream_t stream, const char *what) {
     const auto kernel = compress_cluster_kernel<R, T>;
     constexpr size_t smem = compress_cluster_smem<R, T>();
     static PerDeviceOnce attr_set;
@@ -233,7 +234,7 @@ int compress_cluster_launch(const wa_tensor4 *k, const wa_tensor4 *v, const wa_t
     cfg.numAttrs = beside && pdl_enabled() ? 2 : 1;
     const cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, (const T *)k->ptr, (const T *)v->ptr, (long long)k->stride_b, (long long)k->stride_l,
                                              (T *)ok->ptr, (T *)ov->ptr, (long long)ok->stride_b, (long long)ok->stride_l, L, segment_len,
-                                             block_size, k_proj, v_proj, proj_dtype, proj_rank, proj_cols, rank_full, split, tokens);
+                                             block_size, k_proj, v_proj, proj_dtype, proj_rank, proj_cols, rank_full, split, tokens, ahead ? 1 : 0);
     if (e != cudaSuccess) return fail((int)e, "%s: %s", what, cudaGetErrorString(e));
     return check_launch(what);
 }
@@ -361,7 +362,7 @@ extern "C" int wa_compress_kv(const wa_tensor4 *k, const wa_tensor4 *v, const wa
 
 int wa::compress_kv_launch(const wa_tensor4 *k, const wa_tensor4 *v, const wa_tensor4 *out_k, const wa_tensor4 *out_v, int B, int L, int H,
                            int D, int segment_len, int block_size, const void *k_proj, const void *v_proj, int proj_dtype, int proj_rank,
-                           int proj_cols, bool beside_routing, cudaStream_t stream) {
+                           int proj_cols, bool beside_routing, cudaStream_t stream, bool ahead) {
     const char *what = "wa_compress_kv";
     WA_REQUIRE(k && v && out_k && out_v && k->ptr && v->ptr && out_k->ptr && out_v->ptr && k_proj && v_proj,
                WA_ERR_ARG, "%s: null pointer", what);
@@ -393,7 +394,7 @@ int wa::compress_kv_launch(const wa_tensor4 *k, const wa_tensor4 *v, const wa_te
         const auto launch = k->dtype == WA_BF16 ? (rank_full <= 16 ? compress_cluster_launch<16, __nv_bfloat16> : compress_cluster_launch<32, __nv_bfloat16>)
                                                 : (rank_full <= 16 ? compress_cluster_launch<16, float> : compress_cluster_launch<32, float>);
         return launch(k, v, out_k, out_v, B, L, H * D, segment_len, block_size, k_proj, v_proj, proj_dtype, proj_rank, proj_cols, rank_full,
-                      beside_routing, stream, what);
+                      beside_routing, ahead, stream, what);
     }
     dim3 grid(ceil_div(H * D, CK_THREADS), n_seg, 2 * B);
     compress_kernel<<<grid, CK_THREADS, 0, stream>>>(

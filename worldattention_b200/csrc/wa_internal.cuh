@@ -203,12 +203,27 @@ int compress_sm100_launch(const wa_tensor4 *k, const wa_tensor4 *v, const wa_ten
                           int segment_len, int block_size, const void *k_proj, const void *v_proj, int proj_rank, int proj_cols,
                           int slot0, int slot_stride, cudaStream_t stream, bool beside_routing = false);
 
+// wa_block_sparse_forward and wa_linear_branch for wa_hsa_forward.  `order`: routing rows in the order in which they are taken (heaviest
+// first), or null.  `ahead`: the launch after this one may start while it runs; `beside`: this launch reads nothing that the one before it
+// writes and starts on what that leaves free, but completes only after it (head_dim 128; otherwise one after the other).
+int block_sparse_run(const wa_tensor4 *q, const wa_tensor4 *k, const wa_tensor4 *v, const wa_tensor4 *out, int B, int H, int Lq, int Lkv, int D,
+                     int block_size, const int32_t *index, const int32_t *num, int index_stride, const int32_t *block_sizes, int round_inputs_bf16,
+                     int round_output_bf16, float *lse, const int32_t *order, bool ahead, cudaStream_t stream);
+int linear_run(const wa_tensor4 *q, const wa_tensor4 *k_coarse, const wa_tensor4 *v_coarse, const wa_tensor4 *out, int B, int H, int Lq, int Lc,
+               int D, int round_output_bf16, float *lse, bool beside, cudaStream_t stream);
+
+// float32 keys and values rounded to bf16, both contiguous `[B, L, H, D]` at dst, for the sparse branch (wa_attention_generic.cu)
+bool round_kv_supported(const wa_tensor4 *k, const wa_tensor4 *v, int D);
+// `beside`: it starts on what the launch before it leaves free, and completes only after that one.
+int round_kv_launch(const wa_tensor4 *k, const wa_tensor4 *v, int B, int L, int H, int D, void *dst, bool beside, cudaStream_t stream);
+
 // compress_kv by whichever kernel covers the call (wa_compress.cu).  `beside_routing`: the launch before this one on the
 // stream is a routing kernel that released its dependents at its start (SchedJob::release_at_start).  The two share nothing, so
 // the compression runs on what the routing leaves free of the chip; it completes only after the routing has, so that
-// whatever waits for it may read both.  (One latent frame of 390 tokens over three: the call 49.5 -> 43.1 us.)
+// whatever waits for it may read both.  (One latent frame of 390 tokens over three: the call 49.5 -> 43.1 us.)  `ahead`: the launch
+// after this one reads nothing of it and may start while it runs (where the kernel that covers the call does so).
 int compress_kv_launch(const wa_tensor4 *k, const wa_tensor4 *v, const wa_tensor4 *out_k, const wa_tensor4 *out_v, int B, int L, int H, int D,
                        int segment_len, int block_size, const void *k_proj, const void *v_proj, int proj_dtype, int proj_rank, int proj_cols,
-                       bool beside_routing, cudaStream_t stream);
+                       bool beside_routing, cudaStream_t stream, bool ahead = false);
 
 }  // namespace wa
