@@ -1176,6 +1176,8 @@ route_head_kernel(const float *__restrict__ qp, const float *__restrict__ kp, in
 // 2048; beyond, 512 threads with two CTAs per SM.
 // Before, a row was sorted (or, beyond 1024 blocks, selected by radix passes) with its Gini term, and two counters led to the last CTA.
 // 12 heads, 37 rows over 256 blocks: 16.7 -> 7.8 us, the call 134.0 -> 128.6; 74 rows over 11 700: 117 -> 78, the call 1150 -> 1125.
+// Rows of few blocks, which were route_head_kernel's, the whole call: 4 over 4 26.5 -> 21.0, 7 over 19 34.1 -> 29.8, 37 over 37 78.6 -> 68.7,
+// 37 over 74 88.3 -> 75.3, 25 over 49 of a batch of two 102.1 -> 94.7.
 // ------------------------------------------------------------------------------------------------
 template <int T, int V>
 __global__ void __launch_bounds__(T, 1024 / T)
@@ -1599,7 +1601,8 @@ int route_fused_launch(const float *q_pooled, const float *k_pooled, int B, int 
     // beyond, one round of rows or of tiles does (25 rows over 74: 14.7 against 20; whole calls: 37 over 74 144.9 against 147.8,
     // but 37 over 110, two rounds of both, 108.7 against 101.6).
     const bool one_round = (long long)B * Nq <= RH_WARPS || (long long)B * ((Nq + 15) / 16) * ((Nkv + 7) / 8) <= RH_WARPS;
-    if (D == 128 && Nkv <= RH_MAX_KEYS && (long long)B * Nq <= RH_MAX_ROWS && (Nkv <= 64 || one_round) && ((uintptr_t)q_pooled % 16 == 0) && ((uintptr_t)k_pooled % 16 == 0)) {
+    const bool by_count = fixed_num_per_head && !whole_order;      // route_topk_kernel, whatever the size
+    if (!by_count && D == 128 && Nkv <= RH_MAX_KEYS && (long long)B * Nq <= RH_MAX_ROWS && (Nkv <= 64 || one_round) && ((uintptr_t)q_pooled % 16 == 0) && ((uintptr_t)k_pooled % 16 == 0)) {
         const auto launch = [&](auto width) -> cudaError_t {
             constexpr int K = decltype(width)::value, BYTES = RH_MAX_ROWS * K * 32 * (int)sizeof(float);
             const auto kernel = route_head_kernel<K>;
@@ -1653,7 +1656,7 @@ int route_fused_launch(const float *q_pooled, const float *k_pooled, int B, int 
     const int gate_per_cta = (int)((128 * 128 + rows - 1) / rows);
     if (rows < sms) sms = (int)rows;
     const int slots = (int)((rows + sms - 1) / sms);
-    if (fixed_num_per_head && !whole_order) {
+    if (by_count) {
         const auto launch = [&](auto threads_c, auto values_c) -> cudaError_t {
             constexpr int T = decltype(threads_c)::value, V = decltype(values_c)::value;
             const size_t bytes = logits_ready ? 0 : (size_t)Nkv * sizeof(float);       // at most 64 KB
