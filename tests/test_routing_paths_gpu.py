@@ -27,7 +27,9 @@ def _inputs(b, h, lq, lkv, seed, spread=1.0):
                                         # short rows: a CTA per head, one, two or four keys per lane, and just beyond
                                         (1, 3, 1, 1), (2, 3, 7, 19), (1, 2, 37, 37), (1, 2, 64, 128), (2, 2, 32, 64), (1, 1, 16, 8), (1, 2, 33, 33),
                                         (4, 2, 16, 127), (4, 2, 8, 127), (1, 2, 32, 128), (1, 2, 33, 80), (1, 2, 64, 64),
-                                        (1, 2, 65, 40), (1, 2, 64, 129)])
+                                        (1, 2, 65, 40), (1, 2, 64, 129),
+                                        # ... spread over clusters of one, two, four and eight
+                                        (1, 2, 8, 19), (1, 3, 9, 65), (1, 2, 17, 128), (1, 3, 57, 33)])
 @pytest.mark.parametrize("ragged", [0, 3])
 def test_forward_routing_equals_the_separate_functions(b, h, nq, nkv, ragged):
     from worldattention_b200.hsa import routing as R
@@ -56,7 +58,7 @@ def test_best_blocks_of_long_rows(topk, spread):
 # collected, ordered by counting, by sorting, or (beyond 2048) in pieces
 @pytest.mark.parametrize("nq,nkv,topk", [(3, 1, (1, 0, 1)), (3, 129, (4, 129, 0)), (90, 256, (16, 127, 256)), (90, 255, (1, 33, 128)),
                                          (60, 511, (32, 129, 511)), (3, 257, (31, 256, 257)), (30, 2048, (8, 257, 2047)),
-                                         (2, 2049, (64, 513, 2049)), (2, 4097, (32, 512, 3000)), (2, 8193, (1, 100, 600)),
+                                         (37, 37, (4, 37, 1)), (64, 128, (31, 33, 128)), (2, 2049, (64, 513, 2049)), (2, 4097, (32, 512, 3000)), (2, 8193, (1, 100, 600)),
                                          (2, 16384, (32, 16384, 2048))])
 @pytest.mark.parametrize("spread", [1.0, 0.0])
 def test_best_blocks_by_count(nq, nkv, topk, spread):

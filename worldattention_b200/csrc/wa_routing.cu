@@ -4,6 +4,8 @@
 // of Q and K, then a few hundred short rows), so the kernels are plain coalesced / warp-shuffle
 // code; every reduction that feeds the discrete selection accumulates in float64 and rounds once,
 // which makes the chosen block ids independent of the summation order.
+#include <cooperative_groups.h>
+
 #include <type_traits>
 
 #include "wa_internal.cuh"
@@ -1017,14 +1019,17 @@ route_fused_kernel(const float *__restrict__ qp, const float *__restrict__ kp, i
 }
 
 // ------------------------------------------------------------------------------------------------
-// The whole routing of short rows (head_dim 128, up to 64 query blocks of a head over the batch and 64 key blocks, or 128 where one
-// round of the CTA's warps does): a CTA per head.  There the kernel above is a chain of waits: some twenty barriers of a row, a counter per head, the last CTA's walk
+// The whole routing of short rows (head_dim 128, up to 64 query blocks of a head over the batch and 128 key blocks; with a batch 64, or
+// 128 where one round of the CTA's warps does): a cluster, or a CTA, per head.  There the kernel above is a chain of waits: some twenty barriers of a row, a counter per head, the last CTA's walk
 // over all rows of the head, a second counter.  Here the logits come from the float64 matrix instruction, a 16 x 8 tile per
 // warp, a row's softmax, sort and sums stay inside a warp (K keys per lane, exchanges by shuffles), and the head's threshold
 // and counts need two barriers.  Same sums (float64, rounded where the reference rounds) and the same order.
 // 12 heads, the whole call: 7 query blocks over 19 key blocks 40.5 -> 37.0 us, 37 over 37 100.1 -> 96.2 (the routing itself 20.6 -> 11.5 and
 // 22.6 -> 15.9).
 // ------------------------------------------------------------------------------------------------
+// Without a batch the rows of a head are spread over a cluster of up to eight CTAs, so that every row has a warp of its own and the whole
+// chip fetches its instructions at once; the Gini terms go to all of them through distributed shared memory (37 query blocks over 37:
+// 17.8 -> 11.1 us, the call 87.5 -> 81.5; 63 over 125, which the row kernel took before, 166 -> 149 us a call).
 constexpr int RH_WARPS = 32, RH_MAX_KEYS = 128, RH_MAX_ROWS = 64;
 
 __device__ __forceinline__ float value_of_key(unsigned long long key) {      // the probability that descending_key was given
@@ -1032,8 +1037,8 @@ __device__ __forceinline__ float value_of_key(unsigned long long key) {      // 
     return __uint_as_float((u & 0x80000000u) ? (u & 0x7fffffffu) : ~u);
 }
 
-template <int K>
-__global__ void __launch_bounds__(RH_WARPS * 32)
+template <int K, int WARPS>
+__global__ void __launch_bounds__(WARPS * 32)
 route_head_kernel(const float *__restrict__ qp, const float *__restrict__ kp, int B, int H, int Nq, int Nkv, float scale, float tau_min,
                   float tau_span, const int32_t *__restrict__ fixed_num, int32_t *__restrict__ index, int32_t *num,
                   float *__restrict__ thresholds, int *counters, SchedJob job, int gate_per_cta) {
@@ -1041,20 +1046,25 @@ route_head_kernel(const float *__restrict__ qp, const float *__restrict__ kp, in
     extern __shared__ __align__(16) float row_values[];      // [rows of the head][W]: logits, then the mass before each sorted position
     __shared__ float gini[RH_MAX_ROWS], threshold;
     __shared__ int last_flag;
-    const int h = blockIdx.x, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t = lane & 3, rows = B * Nq;
+    const auto cluster = cooperative_groups::this_cluster();
+    const int parts = (int)cluster.num_blocks(), part = (int)cluster.block_rank(), h = blockIdx.x / parts;
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t = lane & 3, rows = B * Nq;
+    // this CTA's rows of the head (a batch has one CTA per head)
+    const int per = (rows + parts - 1) / parts, first = part * per, mine_n = max(0, min(per, rows - first));
+    if (parts > 1) asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory");      // everybody is there before anything is left with others
     pdl_wait();                 // pooled means and zeroed counters come from the launch before
     if (job.release_at_start) pdl_release_dependents();
-    if (job.order) convert_gate_slice(job, h * gate_per_cta, gate_per_cta);
+    if (job.order) convert_gate_slice(job, (int)blockIdx.x * gate_per_cta, gate_per_cta);
 
-    const int row_tiles = (Nq + 15) / 16, key_tiles = (Nkv + 7) / 8;
-    for (int u = warp; u < B * row_tiles * key_tiles; u += RH_WARPS) {
-        const int b = u / (row_tiles * key_tiles), rest = u - b * row_tiles * key_tiles, i0 = rest / key_tiles * 16, j0 = rest % key_tiles * 8;
+    const int in_item = B == 1 ? mine_n : Nq, row_tiles = (in_item + 15) / 16, key_tiles = (Nkv + 7) / 8;      // in_item: rows of a batch item here
+    for (int u = warp; u < B * row_tiles * key_tiles; u += WARPS) {
+        const int b = u / (row_tiles * key_tiles), rest = u - b * row_tiles * key_tiles, i0 = first + rest / key_tiles * 16, j0 = rest % key_tiles * 8;
         const float *qb = qp + (long long)(b * H + h) * Nq * 128;
         const float4 *qa = reinterpret_cast<const float4 *>(qb + min(i0 + g, Nq - 1) * 128) + t;
         const float4 *qc = reinterpret_cast<const float4 *>(qb + min(i0 + g + 8, Nq - 1) * 128) + t;
         const float4 *kv = reinterpret_cast<const float4 *>(kp + ((long long)(b * H + h) * Nkv + min(j0 + g, Nkv - 1)) * 128) + t;
         double acc[4] = {0.0, 0.0, 0.0, 0.0};
-#pragma unroll 2
+#pragma unroll(WARPS < 32 ? 8 : 2)
         for (int step = 0; step < 8; ++step) {
             const float4 x = __ldg(qa + 4 * step), y = __ldg(qc + 4 * step), z = __ldg(kv + 4 * step);
             const double a[8] = {x.x, y.x, x.y, y.y, x.z, y.z, x.w, y.w}, k[4] = {z.x, z.y, z.z, z.w};
@@ -1063,13 +1073,15 @@ route_head_kernel(const float *__restrict__ qp, const float *__restrict__ kp, in
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
             const int row = i0 + g + 8 * (i >> 1), key = j0 + 2 * t + (i & 1);
-            if (row < Nq && key < Nkv) row_values[(b * Nq + row) * W + key] = __fmul_rn((float)acc[i], scale);
+            if (row < first + in_item && key < Nkv) row_values[(b * Nq + row - first) * W + key] = __fmul_rn((float)acc[i], scale);
         }
     }
     __syncthreads();
 
-    for (int r = warp; r < rows; r += RH_WARPS) {
-        float *mine = row_values + r * W + lane;
+    if (parts > 1) asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+    for (int i = warp; i < mine_n; i += WARPS) {
+        const int r = first + i;
+        float *mine = row_values + i * W + lane;
         const long long row = (long long)(r / Nq * H + h) * Nq + r % Nq;
         float e[K], m = -INFINITY;
 #pragma unroll
@@ -1133,30 +1145,32 @@ route_head_kernel(const float *__restrict__ qp, const float *__restrict__ kp, in
             mine[u * 32] = real ? __fsub_rn((float)mass, p) : INFINITY;
         }
         spread = warp_sum_d(spread);
-        if (lane == 0) gini[r] = __fdiv_rn((float)spread, (float)Nkv);
+        if (lane < parts) *cluster.map_shared_rank(&gini[r], lane) = __fdiv_rn((float)spread, (float)Nkv);
     }
-    __syncthreads();
+    cluster.sync();
     if (warp == 0) {
         double total = 0.0;
         for (int r = lane; r < rows; r += 32) total += (double)gini[r];
         total = warp_sum_d(total);
-        if (lane == 0) threshold = thresholds[h] = __fadd_rn(tau_min, __fmul_rn((float)(total / (double)rows), tau_span));
+        if (lane == 0) threshold = __fadd_rn(tau_min, __fmul_rn((float)(total / (double)rows), tau_span));
+        if (lane == 0 && part == 0) thresholds[h] = threshold;
     }
     __syncthreads();
-    for (int r = warp; r < rows; r += RH_WARPS) {
+    for (int i = warp; i < mine_n; i += WARPS) {
+        const int r = first + i;
         int n = 0;
         if (fixed_num) {
             n = max(0, min(fixed_num[h], Nkv));
         } else {
 #pragma unroll
-            for (int u = 0; u < K; ++u) n += __popc(__ballot_sync(0xffffffffu, row_values[r * W + u * 32 + lane] < threshold));
+            for (int u = 0; u < K; ++u) n += __popc(__ballot_sync(0xffffffffu, row_values[i * W + u * 32 + lane] < threshold));
         }
         if (lane == 0) num[(long long)(r / Nq * H + h) * Nq + r % Nq] = n;
     }
     // the CTA that finishes the last head prepares the attention kernel's launch
     __threadfence();
     __syncthreads();
-    if (tid == 0) last_flag = atomicAdd(&counters[0], 1) == H - 1;
+    if (tid == 0) last_flag = atomicAdd(&counters[0], 1) == (int)gridDim.x - 1;
     __syncthreads();
     if (!last_flag || !job.order) return;
     __threadfence();
@@ -1597,27 +1611,44 @@ int route_fused_launch(const float *q_pooled, const float *k_pooled, int B, int 
     const float scale = (float)pow((double)D, -0.5), span = (float)(tau_max - tau_min);
     const long long bh = (long long)B * H;
 
-    // A CTA takes 32 rows and 32 tiles of logits at a time.  Two rounds of rows pay up to 64 keys (37 rows over 37: 16.5 us against 22.6);
+    // With a batch a CTA takes 32 rows and 32 tiles of logits at a time.  Two rounds of rows pay up to 64 keys (37 rows over 37: 16.5 us against 22.6);
     // beyond, one round of rows or of tiles does (25 rows over 74: 14.7 against 20; whole calls: 37 over 74 144.9 against 147.8,
     // but 37 over 110, two rounds of both, 108.7 against 101.6).
     const bool one_round = (long long)B * Nq <= RH_WARPS || (long long)B * ((Nq + 15) / 16) * ((Nkv + 7) / 8) <= RH_WARPS;
     const bool by_count = fixed_num_per_head && !whole_order;      // route_topk_kernel, whatever the size
-    if (!by_count && D == 128 && Nkv <= RH_MAX_KEYS && (long long)B * Nq <= RH_MAX_ROWS && (Nkv <= 64 || one_round) && ((uintptr_t)q_pooled % 16 == 0) && ((uintptr_t)k_pooled % 16 == 0)) {
-        const auto launch = [&](auto width) -> cudaError_t {
-            constexpr int K = decltype(width)::value, BYTES = RH_MAX_ROWS * K * 32 * (int)sizeof(float);
-            const auto kernel = route_head_kernel<K>;
+    if (!by_count && D == 128 && Nkv <= RH_MAX_KEYS && (long long)B * Nq <= RH_MAX_ROWS && (B == 1 || Nkv <= 64 || one_round) &&
+        ((uintptr_t)q_pooled % 16 == 0) && ((uintptr_t)k_pooled % 16 == 0)) {
+        const auto launch = [&](auto width, auto warps) -> cudaError_t {
+            constexpr int K = decltype(width)::value, WARPS = decltype(warps)::value, BYTES = RH_MAX_ROWS * K * 32 * (int)sizeof(float);
+            const auto kernel = route_head_kernel<K, WARPS>;
             static PerDeviceOnce attr_set;
             if (!attr_set.done()) {
                 const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, BYTES);
                 if (e != cudaSuccess) return e;
                 attr_set.mark();
             }
-            return launch_dependent(kernel, dim3(H), dim3(RH_WARPS * 32), (size_t)B * Nq * K * 32 * sizeof(float), stream, q_pooled, k_pooled, B, H, Nq, Nkv,
-                                    scale, (float)tau_min, span, fixed_num_per_head, index, num, thresholds, counters, job_in,
-                                    (128 * 128 + H - 1) / H);
+            constexpr int parts = WARPS < RH_WARPS ? RH_MAX_ROWS / WARPS : 1;    // 8: a warp per row, whatever the number of rows
+            cudaLaunchConfig_t cfg{};
+            cfg.gridDim = dim3(H * parts);
+            cfg.blockDim = dim3(WARPS * 32);
+            cfg.dynamicSmemBytes = (size_t)B * ((Nq + parts - 1) / parts) * K * 32 * sizeof(float);
+            cfg.stream = stream;
+            cudaLaunchAttribute attr[2];
+            attr[0].id = cudaLaunchAttributeClusterDimension;
+            attr[0].val.clusterDim.x = parts;
+            attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+            attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+            attr[1].val.programmaticStreamSerializationAllowed = 1;
+            cfg.attrs = attr;
+            cfg.numAttrs = pdl_enabled() ? 2 : 1;
+            return cudaLaunchKernelEx(&cfg, kernel, q_pooled, k_pooled, B, H, Nq, Nkv, scale, (float)tau_min, span, fixed_num_per_head, index, num,
+                                      thresholds, counters, job_in, (128 * 128 + H * parts - 1) / (H * parts));
         };
-        const cudaError_t e = Nkv <= 32 ? launch(std::integral_constant<int, 1>())
-                                        : Nkv <= 64 ? launch(std::integral_constant<int, 2>()) : launch(std::integral_constant<int, 4>());
+        const auto launch_width = [&](auto warps) {
+            return Nkv <= 32 ? launch(std::integral_constant<int, 1>(), warps)
+                             : Nkv <= 64 ? launch(std::integral_constant<int, 2>(), warps) : launch(std::integral_constant<int, 4>(), warps);
+        };
+        const cudaError_t e = B == 1 ? launch_width(std::integral_constant<int, 8>()) : launch_width(std::integral_constant<int, RH_WARPS>());
         if (e != cudaSuccess) return fail((int)e, "wa_hsa_forward(routing of short rows): %s", cudaGetErrorString(e));
         return check_launch("wa_hsa_forward(routing of short rows)");
     }
