@@ -212,14 +212,37 @@ hsa_fwd_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
                 const uint32_t slot = jcount & 1u;
                 ok = mbar_wait(&bar->item_empty[slot], ((jcount >> 1) & 1u) ^ 1u, abort_flag, sink, 11);
                 if (!ok) break;
-                int item = -1, n_sel = 0, n_sel2 = 0, n_both = 0;   // PAIR: of the item's first and second query block; tiles for both
-                long long row0 = 0;                                 // routing row of the item's (first) query block
-                if (at < p.n_items) {
-                    item = p.order[at];
-                    row0 = PAIR ? (long long)(item / p.q_items) * p.Nq + 2 * (item % p.q_items) : item;
-                    n_sel = max(0, min(p.num[row0], p.Nkv));
-                    if (PAIR && 2 * (item % p.q_items) + 1 < p.Nq) n_sel2 = max(0, min(p.num[row0 + 1], p.Nkv));
-                    if (PAIR) n_both = (p.both[item] & 0xffff) >> 1;
+                // Whatever of the item lies in memory is asked for at once -- its counts and the first blocks of its lists, whether it turns
+                // out to have any or not -- and Q's load leaves before the answers are there (a launch begins with this chain).
+                const int item = at < p.n_items ? p.order[at] : -1;
+                int n_sel = 0, n_sel2 = 0, n_both = 0;      // PAIR: of the item's first and second query block; tiles for both
+                int qb = 0, h = 0, b = 0, first = 0, first2 = 0, other = 0;
+                const int32_t *ids = p.index;
+                const uint32_t qs = jcount % Q_STAGES, q_phase = ((jcount / Q_STAGES) & 1u) ^ 1u;
+                auto load_q = [&]() {
+                    uint8_t *qdst = q_s + qs * TILE_BYTES;
+                    mbar_expect_tx(&bar->q_full[qs], TILE_BYTES);
+                    tma_load_4d(qdst, &tm_q, &bar->q_full[qs], 0, h, qb * Q_ROWS, b);
+                    tma_load_4d(qdst + HALF_BYTES, &tm_q, &bar->q_full[qs], 64, h, qb * Q_ROWS, b);
+                };
+                bool q_sent = false;
+                if (item >= 0) {
+                    const int bh = item / p.q_items;
+                    qb = item - bh * p.q_items, b = bh / p.H, h = bh - b * p.H;
+                    const long long row0 = PAIR ? (long long)bh * p.Nq + 2 * qb : item;      // routing row of the (first) query block
+                    const bool second = PAIR && 2 * qb + 1 < p.Nq;
+                    ids += row0 * p.Nkv;
+                    n_sel = p.num[row0];
+                    if (second) n_sel2 = p.num[row0 + 1];
+                    if (PAIR) n_both = p.both[item];
+                    first = ids[0];
+                    if (BLK != TILE) first2 = ids[min(1, p.Nkv - 1)];
+                    if (second) other = ids[p.Nkv];
+                    q_sent = mbar_test(&bar->q_empty[qs], q_phase);
+                    if (q_sent) load_q();
+                    n_sel = max(0, min(n_sel, p.Nkv));
+                    n_sel2 = max(0, min(n_sel2, p.Nkv));
+                    n_both = (n_both & 0xffff) >> 1;
                 }
                 // the other roles count sparse TILES: with 64-token blocks a tile holds two selected blocks
                 const int n_st = BLK == TILE ? n_sel : PAIR ? max(n_sel, n_sel2) - n_both : (n_sel + 1) >> 1;
@@ -229,8 +252,6 @@ hsa_fwd_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
                 mbar_arrive(&bar->item_full[slot]);
                 if (item < 0) break;
                 at = (int)gridDim.x + atomicAdd(p.work_counter, 1);   // consumed at the top of the next round
-                const int qb = item % p.q_items, h = (item / p.q_items) % p.H, b = item / (p.q_items * p.H);
-                const int32_t *ids = p.index + row0 * p.Nkv;
                 // The blocks of sparse tile t as the lists name them (PAIR: one past the end of the shorter list lies beyond the keys
                 // and loads as zeros; a missing second block of a single item repeats the first and is masked out).  They are
                 // fetched a tile ahead: a look-up on the way of each load, for K and again for V, is what the tiles of 64-token
@@ -243,18 +264,16 @@ hsa_fwd_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
                     return make_int2(t + n_both < n_sel ? ids[t + n_both] : INT_MAX, t + n_both < n_sel2 ? ids[p.Nkv + t + n_both] : INT_MAX);
                 };
                 auto block_row = [&](int id) { return PAIR && id == INT_MAX ? p.Nkv : max(0, min(id, p.Nkv - 1)); };
-                int2 next = make_int2(0, 0);
-                if (n_st > 0) next = fetch_blocks(0);
+                int2 next = make_int2(first, n_sel > 1 ? first2 : first);
+                if (PAIR && n_both == 0) next = make_int2(n_sel > 0 ? first : INT_MAX, n_sel2 > 0 ? other : INT_MAX);
                 const int n_kv = n_st + lin_tiles;
                 WA_STATS_ITEM(n_kv + 1);
 
-                const uint32_t qs = jcount % Q_STAGES;
-                ok = mbar_wait(&bar->q_empty[qs], ((jcount / Q_STAGES) & 1u) ^ 1u, abort_flag, sink, 12);
-                if (!ok) break;
-                uint8_t *qdst = q_s + qs * TILE_BYTES;
-                mbar_expect_tx(&bar->q_full[qs], TILE_BYTES);
-                tma_load_4d(qdst, &tm_q, &bar->q_full[qs], 0, h, qb * Q_ROWS, b);
-                tma_load_4d(qdst + HALF_BYTES, &tm_q, &bar->q_full[qs], 64, h, qb * Q_ROWS, b);
+                if (!q_sent) {
+                    ok = mbar_wait(&bar->q_empty[qs], q_phase, abort_flag, sink, 12);
+                    if (!ok) break;
+                    load_q();
+                }
 
                 // K tiles and V tiles advance on cursors of their own: the V ring is shallower and its stages come back
                 // later (after the PV product), and a K load that queued behind a V wait would reach the QK warp late.
@@ -827,9 +846,9 @@ hsa_fwd_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
                 tc_fence_after();
                 WA_TRACE(13);
                 if (!p.part_linear) {
-                    // Rolled, here and in the combine below, with the arrays as queues: this code runs once per item, and fetching its
-                    // instructions for the first time cost more than the work (unrolled, the gate took 3800 cycles in a CTA's first
-                    // item and 1600 in its third).
+                    // Rolled, with the array as a queue: this code runs once per item, and fetching its instructions for the first time cost
+                    // more than the work (unrolled, the gate took 3800 cycles in a CTA's first item and 1600 in its third; rolled 2300).
+                    // The combine below is short enough as it stands (1900 cycles; rolled 3500).
 #pragma unroll 1
                     for (int c = 0; c < 4; ++c) {   // 32 columns at a time
                         uint32_t gsc[16];
@@ -942,7 +961,7 @@ hsa_fwd_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
                     if (c & 1) flush(p.part_linear, c >> 1);
                 }
             } else if (ok) {
-#pragma unroll 1
+#pragma unroll
                 for (int c = 0; c < 4; ++c) {   // 32 columns at a time
                     uint32_t o[16];
                     TMEM_LDQ16(tmem_o + lane_addr + c * 32, o);
@@ -958,7 +977,7 @@ hsa_fwd_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
                         const int jj = 4 * c + j;
                         const float a0 = __uint_as_float(o[4 * j]) * inv_linA, a1 = __uint_as_float(o[4 * j + 1]) * inv_linA;
                         const float b0 = __uint_as_float(o[4 * j + 2]) * inv_linB, b1 = __uint_as_float(o[4 * j + 3]) * inv_linB;
-                        const uint32_t spA = park[2 * j], spB = park[2 * j + 1], gA = gpk[2 * j], gB = gpk[2 * j + 1];   // low half = even column
+                        const uint32_t spA = park[2 * jj], spB = park[2 * jj + 1], gA = gpk[2 * jj], gB = gpk[2 * jj + 1];   // low half = even column
                         __nv_bfloat162 ra = __floats2bfloat162_rn(fmaf(a0, __uint_as_float(gA << 16), __uint_as_float(spA << 16)),
                                                                    fmaf(a1, __uint_as_float(gA & 0xffff0000u), __uint_as_float(spA & 0xffff0000u)));
                         __nv_bfloat162 rb = __floats2bfloat162_rn(fmaf(b0, __uint_as_float(gB << 16), __uint_as_float(spB << 16)),
@@ -966,11 +985,6 @@ hsa_fwd_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
                         // the finished tile is staged in the shared-memory stage that held Q (the layout the TMA store expects)
                         *reinterpret_cast<uint32_t *>(q_stage + tile_off(rowA, jj)) = *reinterpret_cast<uint32_t *>(&ra);
                         *reinterpret_cast<uint32_t *>(q_stage + tile_off(rowB, jj)) = *reinterpret_cast<uint32_t *>(&rb);
-                    }
-#pragma unroll
-                    for (int j = 0; j < 24; ++j) {
-                        park[j] = park[j + 8];
-                        gpk[j] = gpk[j + 8];
                     }
                     WA_TRACE(15);
                 }
