@@ -1,0 +1,53 @@
+"""Rows whose later key blocks outgrow the reference point that the tcgen05 kernel took from an earlier one, and the work order of
+calls whose keys and values are more than L2 keeps, both against the library's float32 path."""
+import pytest
+import torch
+
+from tests.helpers import attention_error, dev, to_np
+
+pytestmark = pytest.mark.gpu
+D = 128
+MAX_ABS, MEAN_REL = 2e-2, 1e-2      # as for the other calls (bf16 operands and result, values of unit variance)
+
+
+# 128-token blocks; 64-token blocks, one query block per work item and two.  A step of 3 stays below what makes a row look again, 20
+# does not, and 200 is beyond the range of the exponential.
+@pytest.mark.parametrize("block,heads,nq", [(128, 3, 2), (64, 3, 2), (64, 24, 8)])
+@pytest.mark.parametrize("step", [3.0, 20.0, 200.0])
+def test_later_blocks_outgrow_earlier_ones(block, heads, nq, step):
+    from worldattention_b200.hsa.branches import hsa_partials
+    g = torch.Generator(device=dev()).manual_seed(block + heads)
+    draw = lambda n: torch.randn(1, n, heads, D, generator=g, device=dev())
+    nkv, slots = 9, 300
+    q, k, v, kc, vc = draw(nq * block - 5) * 0.3, draw(nkv * block - 17) * 0.3, draw(nkv * block - 17), draw(slots) * 0.3, draw(slots)
+    # logits in powers of two: `step` per block for most rows, the same downwards for every third
+    q[..., 0] = 8.0
+    q[:, ::3, :, 0] = -8.0
+    unit = step / (8.0 * D ** -0.5 * 1.4426950408889634)
+    k[..., 0] = (torch.arange(k.shape[1], device=dev()) // block)[None, :, None] * unit
+    kc[..., 0] = (torch.arange(slots, device=dev()) // 100)[None, :, None] * unit
+    args = [t.bfloat16() for t in (q, k, v, kc, vc)]
+    index = torch.arange(nkv, dtype=torch.int32, device=dev()).expand(1, heads, nq, nkv).contiguous()
+    num = torch.full((1, heads, nq), nkv, dtype=torch.int32, device=dev())
+    num[0, 0, 0] = 4
+    got, want = (hsa_partials(*args, index, num, block, force_generic=generic) for generic in (False, True))
+    assert got[4] and not want[4]
+    for a, b in zip(got[:4], want[:4]):
+        a, b = to_np(a), to_np(b)
+        max_abs, mean_rel = attention_error(a, b)
+        assert max_abs < max(MAX_ABS, 1e-5 * abs(b).max()) and mean_rel < MEAN_REL      # the normalisers reach a thousand
+
+
+@pytest.mark.parametrize("heads,q_blocks,kv", [(12, 13, 11003), (5, 75, 30000), (24, 7, 6000)])
+def test_every_item_of_a_call_ordered_by_heads_is_done(heads, q_blocks, kv):
+    from worldattention_b200.hsa import hsa_attention
+    assert heads * q_blocks > torch.cuda.get_device_properties(0).multi_processor_count and 4 * heads * kv * D > 64 << 20
+    g = torch.Generator(device=dev()).manual_seed(kv)
+    draw = lambda n: torch.randn(1, n, heads, D, generator=g, device=dev())
+    q, k, v, kc, vc = (t.bfloat16() for t in (draw(q_blocks * 64 - 9) * 0.5, draw(kv) * 0.5, draw(kv), draw(60), draw(60)))
+    kwargs = dict(k_coarse=kc, v_coarse=vc, k_proj_mat=None, v_proj_mat=None, block_size=64)
+    out, (_, num, _, used) = hsa_attention(q, k, v, return_routing=True, check_status=True, **kwargs)
+    want, (_, num_g, _, used_g) = hsa_attention(q, k, v, return_routing=True, force_generic=True, **kwargs)
+    assert used and not used_g and torch.equal(num, num_g)
+    max_abs, mean_rel = attention_error(to_np(out), to_np(want))
+    assert max_abs < 2 * 2 ** -6 and mean_rel < MEAN_REL      # |v| < 4 of a mean of hundreds: a step of bf16 each way
