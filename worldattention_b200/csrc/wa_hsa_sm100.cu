@@ -202,7 +202,11 @@ hsa_fwd_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
     asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(REGS_OTHER));
     if (warp == 8) {
         // ================= producer: work queue + TMA =================
-        if (lane == 0) {
+        // One thread, and what it has to do for a tile of two 64-token blocks was as long as the tile: its loads are as few as the
+        // layouts allow, and it is elected, not picked by its lane, which lets the compiler keep the loads' operands in uniform registers
+        // (21 frames, 64-token blocks, counts from the mass: 462 us with two loads per half a block, 442 with three per block, 417
+        // elected; 480 frames 422 -> 414).
+        if (elect_one()) {
             uint32_t jcount = 0, kcount = 0, vcount = 0;
             bool ok = true;
             // Work queue: the first item of a CTA is fixed by its index (no round trip to the counter before the first
@@ -285,19 +289,10 @@ hsa_fwd_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
                     mbar_expect_tx(&bar->v_full[vs], TILE_BYTES);
                     if (tv < n_st) {
                         const int id = bar->blocks[tv & 7].x, id2 = bar->blocks[tv & 7].y;
-                        if (BLK == TILE) {
-                            tma_load_4d(vdst, &tm_v, &bar->v_full[vs], 0, h, id * TILE, b);
-                            tma_load_4d(vdst + HALF_BYTES, &tm_v, &bar->v_full[vs], 64, h, id * TILE, b);
-                        } else {
-                            tma_load_4d(vdst, &tm_v, &bar->v_full[vs], 0, h, id * HALF, b);
-                            tma_load_4d(vdst + HALF_BYTES / 2, &tm_v, &bar->v_full[vs], 0, h, id2 * HALF, b);
-                            tma_load_4d(vdst + HALF_BYTES, &tm_v, &bar->v_full[vs], 64, h, id * HALF, b);
-                            tma_load_4d(vdst + HALF_BYTES + HALF_BYTES / 2, &tm_v, &bar->v_full[vs], 64, h, id2 * HALF, b);
-                        }
+                        tma_load_5d(vdst, &tm_v, &bar->v_full[vs], 0, id * BLK, 0, h, b);      // both halves of the channels
+                        if (BLK == HALF) tma_load_5d(vdst + HALF_BYTES, &tm_v, &bar->v_full[vs], 0, id2 * HALF, 0, h, b);
                     } else {
-                        const int c = (tv - n_st) * TILE;
-                        tma_load_4d(vdst, &tm_vc, &bar->v_full[vs], 0, h, c, b);
-                        tma_load_4d(vdst + HALF_BYTES, &tm_vc, &bar->v_full[vs], 64, h, c, b);
+                        tma_load_5d(vdst, &tm_vc, &bar->v_full[vs], 0, (tv - n_st) * TILE, 0, h, b);
                     }
                     ++tv;
                 };
@@ -349,18 +344,16 @@ hsa_fwd_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
                     mbar_expect_tx(&bar->k_full[ks], TILE_BYTES);
                     if (t < n_st) {
                         if (BLK == TILE) {
-                            tma_load_4d(kdst, &tm_k, &bar->k_full[ks], 0, h, id * TILE, b);
-                            tma_load_4d(kdst + HALF_BYTES, &tm_k, &bar->k_full[ks], 64, h, id * TILE, b);
+                            tma_load_5d(kdst, &tm_k, &bar->k_full[ks], 0, id * TILE, 0, h, b);
                         } else {   // 64-row boxes: rows 0..63 of each half-tile from the first block, 64..127 from the second
-                            tma_load_4d(kdst, &tm_k, &bar->k_full[ks], 0, h, id * HALF, b);
-                            tma_load_4d(kdst + HALF_BYTES / 2, &tm_k, &bar->k_full[ks], 0, h, id2 * HALF, b);
-                            tma_load_4d(kdst + HALF_BYTES, &tm_k, &bar->k_full[ks], 64, h, id * HALF, b);
-                            tma_load_4d(kdst + HALF_BYTES + HALF_BYTES / 2, &tm_k, &bar->k_full[ks], 64, h, id2 * HALF, b);
+                            tma_load_5d(kdst, &tm_k, &bar->k_full[ks], 0, id * HALF, 0, h, b);
+                            tma_load_5d(kdst + HALF_BYTES / 2, &tm_k, &bar->k_full[ks], 0, id2 * HALF, 0, h, b);
+                            tma_load_5d(kdst + HALF_BYTES, &tm_k, &bar->k_full[ks], 0, id * HALF, 1, h, b);
+                            tma_load_5d(kdst + HALF_BYTES + HALF_BYTES / 2, &tm_k, &bar->k_full[ks], 0, id2 * HALF, 1, h, b);
                         }
                     } else if (t < n_kv) {
                         const int c = (t - n_st) * TILE;
-                        tma_load_4d(kdst, &tm_kc, &bar->k_full[ks], 0, h, c, b);
-                        tma_load_4d(kdst + HALF_BYTES, &tm_kc, &bar->k_full[ks], 64, h, c, b);
+                        tma_load_5d(kdst, &tm_kc, &bar->k_full[ks], 0, c, 0, h, b);
                     } else {
                         tma_load_2d(kdst, &tm_w, &bar->k_full[ks], 0, 0);
                         tma_load_2d(kdst + HALF_BYTES, &tm_w, &bar->k_full[ks], 64, 0);
@@ -478,7 +471,10 @@ hsa_fwd_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
                 }
                 tc_fence_after();
                 if (leader) {
-                    const uint64_t vd = smem_desc(smem_u32(v_s + vs * TILE_BYTES), HALF_BYTES, 1024);
+                    // values of 64-token blocks lie block by block, both halves of the channels of one before the other's
+                    const bool by_block = BLK == HALF && t < n_sel;
+                    const uint64_t vd = smem_desc(smem_u32(v_s + vs * TILE_BYTES), by_block ? HALF_BYTES / 2 : HALF_BYTES, 1024);
+                    const uint64_t upper = (uint64_t)((by_block ? HALF_BYTES : HALF_BYTES / 2) >> 4);     // keys 64 ..
                     if (PAIR && t >= n_both && t < n_sel) {
                         // both halves of the rows left their probabilities in the same 32 columns
 #pragma unroll
@@ -487,12 +483,12 @@ hsa_fwd_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
                                                !(first && kk == 0));
 #pragma unroll
                         for (int kk = 0; kk < 4; ++kk)
-                            mma_ts_half<true>(tmem_o, tmem_s + buf * TILE + kk * 8, vd + (uint64_t)(((kk + 4) * 2048) >> 4), IDESC_PV,
+                            mma_ts_half<true>(tmem_o, tmem_s + buf * TILE + kk * 8, vd + upper + (uint64_t)((kk * 2048) >> 4), IDESC_PV,
                                               !(first && kk == 0));
                     } else {
 #pragma unroll
                         for (int kk = 0; kk < 8; ++kk)
-                            mma_ts(tmem_o, tmem_s + buf * TILE + kk * 8, vd + (uint64_t)((kk * 2048) >> 4), IDESC_PV,
+                            mma_ts(tmem_o, tmem_s + buf * TILE + kk * 8, vd + (kk >> 2) * upper + (uint64_t)(((kk & 3) * 2048) >> 4), IDESC_PV,
                                    !(first && kk == 0));
                     }
                     tc_commit(&bar->s_free[buf]);   // first: the next score product waits for it
@@ -1146,6 +1142,24 @@ static int make_map_4d(CUtensorMap *map, const wa_tensor4 *t, int B, int L, int 
     return 0;
 }
 
+// The same view as a 5-D map (64 channels, token, half of the channels, h, batch): one load brings `rows` tokens with both halves
+// `halves` = 2, [half][token][64 channels] in shared memory, or one of them.
+static int make_map_5d(CUtensorMap *map, const wa_tensor4 *t, int B, int L, int H, const char *name, int rows, int halves) {
+    EncodeTiledFn fn = encode_fn();
+    WA_REQUIRE(fn, WA_ERR_DEVICE, "tcgen05 path: cuTensorMapEncodeTiled is unavailable");
+    cuuint64_t dims[5] = {64, (cuuint64_t)L, 2, (cuuint64_t)H, (cuuint64_t)B};
+    cuuint64_t strides[4] = {(cuuint64_t)t->stride_l * 2, 128, (cuuint64_t)t->stride_h * 2, (cuuint64_t)t->stride_b * 2};
+    if (B == 1) strides[3] = strides[0] * (cuuint64_t)L;   // unused extent: any legal stride
+    if (H == 1) strides[2] = 256;
+    cuuint32_t box[5] = {64, (cuuint32_t)rows, (cuuint32_t)halves, 1, 1};
+    cuuint32_t elem[5] = {1, 1, 1, 1, 1};
+    CUresult r = fn(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 5, t->ptr, dims, strides, box, elem,
+                    CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+                    CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    WA_REQUIRE(r == CUDA_SUCCESS, WA_ERR_ALIGN, "tcgen05 path: tensor map for %s rejected (CUresult %d)", name, (int)r);
+    return 0;
+}
+
 static int make_map_w(CUtensorMap *map, const void *w) {
     EncodeTiledFn fn = encode_fn();
     WA_REQUIRE(fn, WA_ERR_DEVICE, "tcgen05 path: cuTensorMapEncodeTiled is unavailable");
@@ -1279,10 +1293,11 @@ int hsa_sm100_launch(const wa_hsa_params *p, int Lc, const wa_tensor4 *kc, const
     int rc;
     if ((rc = make_map_4d(&tq, &p->q, p->B, p->Lq, p->H, "q"))) return rc;
     const int blk = p->block_size == HALF ? HALF : TILE;   // the linear-branch-only launch (other sizes) never loads k / v
-    if ((rc = make_map_4d(&tk, &p->k, p->B, p->Lkv, p->H, "k", blk))) return rc;
-    if ((rc = make_map_4d(&tv, &p->v, p->B, p->Lkv, p->H, "v", blk))) return rc;
-    if ((rc = make_map_4d(&tkc, kc, p->B, Lc, p->H, "k_coarse"))) return rc;
-    if ((rc = make_map_4d(&tvc, vc, p->B, Lc, p->H, "v_coarse"))) return rc;
+    // a load instruction costs the one thread that issues them 100 to 190 cycles: as few as the layouts allow
+    if ((rc = make_map_5d(&tk, &p->k, p->B, p->Lkv, p->H, "k", blk, blk == TILE ? 2 : 1))) return rc;
+    if ((rc = make_map_5d(&tv, &p->v, p->B, p->Lkv, p->H, "v", blk, 2))) return rc;
+    if ((rc = make_map_5d(&tkc, kc, p->B, Lc, p->H, "k_coarse", TILE, 2))) return rc;
+    if ((rc = make_map_5d(&tvc, vc, p->B, Lc, p->H, "v_coarse", TILE, 2))) return rc;
     if ((rc = make_map_w(&tw, w_bf16))) return rc;
     if ((rc = make_map_4d(&tout, p->part_sparse ? &p->q : &p->out, p->B, p->Lq, p->H, "out", pair ? TILE : blk))) return rc;   // unused in partial mode
 
