@@ -1182,8 +1182,8 @@ route_head_kernel(const float *__restrict__ qp, const float *__restrict__ kp, in
 }
 
 // ------------------------------------------------------------------------------------------------
-// Routing with a fixed count per head where nobody reads the whole order or the thresholds: a row per CTA, V blocks per thread
-// in registers from the logit to the key, and only the best blocks are ordered.  Every warp sorts its lanes' best keys; with
+// Routing with a fixed count per head where nobody reads the whole order or the thresholds: a row per CTA, up to 2048 blocks in
+// registers (V per thread) from the logit to the key, more in shared memory, and only the best blocks are ordered.  Every warp sorts its lanes' best keys; with
 // W warps and c = ceil(count / W), at least W * c >= count blocks lie at or below the worst of the warps' c-th keys, so what lies
 // above it cannot be among the best.  The few blocks at or below it (26 of 256 for a count of 16, about 90 of 11 700 for 32) are
 // collected and each counts how many of them come before it, which is its place.  Same probabilities and keys as route_row,
@@ -1191,19 +1191,20 @@ route_head_kernel(const float *__restrict__ qp, const float *__restrict__ kp, in
 // made by a CTA of its own (the first) beside the rows instead of by the last one after them.
 // Bound by latency (a row is a chain of four block-wide exchanges) and, over thousands of blocks, by the float64 exponentials.
 // 128 threads a row up to 512 blocks; 256 where the row makes its own logits (a warp per eight dot products) or has up to
-// 2048; beyond, 512 threads with two CTAs per SM.
+// 2048; beyond, 512 threads with three CTAs per SM.
 // Before, a row was sorted (or, beyond 1024 blocks, selected by radix passes) with its Gini term, and two counters led to the last CTA.
-// 12 heads, 37 rows over 256 blocks: 16.7 -> 7.8 us, the call 134.0 -> 128.6; 74 rows over 11 700: 117 -> 78, the call 1150 -> 1125.
+// 12 heads, 37 rows over 256 blocks: 16.7 -> 7.8 us, the call 134.0 -> 128.6; 74 rows over 11 700: 117 -> 78 with the values in registers (two
+// CTAs per SM and spills), 56 in shared memory.
 // Rows of few blocks, which were route_head_kernel's, the whole call: 4 over 4 26.5 -> 21.0, 7 over 19 34.1 -> 29.8, 37 over 37 78.6 -> 68.7,
 // 37 over 74 88.3 -> 75.3, 25 over 49 of a batch of two 102.1 -> 94.7.
 // ------------------------------------------------------------------------------------------------
-template <int T, int V>
-__global__ void __launch_bounds__(T, 1024 / T)
+template <int T, int V>      // V = 0: the row's values in shared memory, any number of them
+__global__ void __launch_bounds__(T, V ? 1024 / T : 3)
 route_topk_kernel(const float *__restrict__ qp, const float *__restrict__ kp, int H, int Nq, int Nkv, int D, float scale,
                   const int32_t *__restrict__ fixed_num, float *logits, int32_t *__restrict__ index, int32_t *__restrict__ num, SchedJob job,
                   int rows, int gate_per_cta, int sm_count, int per_sm, int logits_ready) {
-    constexpr int W = T / 32, SLOTS = V * T < 2048 ? V * T : 2048;
-    extern __shared__ float own_logits[];                // Nkv, where the row makes them
+    constexpr int W = T / 32, SLOTS = V == 0 ? 1024 : V * T < 2048 ? V * T : 2048, N = V ? V : 1;
+    extern __shared__ float own_logits[];                // Nkv, where the row makes them or keeps its values
     __shared__ __align__(16) unsigned long long keys[SLOTS];
     __shared__ float top[W];
     __shared__ double sums[W];
@@ -1232,38 +1233,69 @@ route_topk_kernel(const float *__restrict__ qp, const float *__restrict__ kp, in
         row_logits(qp + (long long)row * D, kp + (long long)(row / Nq) * Nkv * D, Nkv, D, scale, own_logits);
         __syncthreads();
     }
-    float e[V], m = -INFINITY;
-#pragma unroll
-    for (int u = 0; u < V; ++u) {
-        const int j = u * T + tid;
-        e[u] = j < Nkv ? (logits_ready ? __ldcg(lrow + j) : own_logits[j]) : -INFINITY;
-    }
-#pragma unroll
-    for (int u = 0; u < V; ++u) m = fmaxf(m, e[u]);
-    m = warp_max(m);
-    if (lane == 0) top[warp] = m;
-    __syncthreads();
-#pragma unroll
-    for (int w = 0; w < W; ++w) m = fmaxf(m, top[w]);
+    float e[N], m = -INFINITY;
+    uint32_t key[N], best = 0xFFFFFFFFu;                 // upper half of the sort's key; the id is the lower one
     double sum = 0.0;
+    auto total_of = [&]() -> float {                     // the row's sum, rounded once
+        sum = warp_sum_d(sum);
+        if (lane == 0) sums[warp] = sum;
+        __syncthreads();
+        sum = 0.0;
 #pragma unroll
-    for (int u = 0; u < V; ++u)
-        if (u * T + tid < Nkv) {
-            e[u] = (float)exp((double)__fsub_rn(e[u], m));
-            sum += (double)e[u];
+        for (int w = 0; w < W; ++w) sum += sums[w];
+        return (float)sum;
+    };
+    auto largest_of = [&]() {
+        m = warp_max(m);
+        if (lane == 0) top[warp] = m;
+        __syncthreads();
+#pragma unroll
+        for (int w = 0; w < W; ++w) m = fmaxf(m, top[w]);
+    };
+    auto exponential = [&](float x) { return (float)exp((double)__fsub_rn(x, m)); };
+    if constexpr (V > 0) {
+#pragma unroll
+        for (int u = 0; u < V; ++u) {
+            const int j = u * T + tid;
+            e[u] = j < Nkv ? (logits_ready ? __ldcg(lrow + j) : own_logits[j]) : -INFINITY;
         }
-    sum = warp_sum_d(sum);
-    if (lane == 0) sums[warp] = sum;
-    __syncthreads();
-    sum = 0.0;
 #pragma unroll
-    for (int w = 0; w < W; ++w) sum += sums[w];
-    const float denom = (float)sum;
-    uint32_t key[V], best = 0xFFFFFFFFu;                 // upper half of the sort's key; the id is the lower one
+        for (int u = 0; u < V; ++u) m = fmaxf(m, e[u]);
+        largest_of();
 #pragma unroll
-    for (int u = 0; u < V; ++u) {
-        key[u] = u * T + tid < Nkv ? descending_key(__fdiv_rn(e[u], denom)) : 0xFFFFFFFFu;
-        best = min(best, key[u]);
+        for (int u = 0; u < V; ++u)
+            if (u * T + tid < Nkv) {
+                e[u] = exponential(e[u]);
+                sum += (double)e[u];
+            }
+        const float denom = total_of();
+#pragma unroll
+        for (int u = 0; u < V; ++u) {
+            key[u] = u * T + tid < Nkv ? descending_key(__fdiv_rn(e[u], denom)) : 0xFFFFFFFFu;
+            best = min(best, key[u]);
+        }
+    } else {
+        // a thread only touches its own places
+        if (logits_ready) {
+#pragma unroll 8
+            for (int j = tid; j < Nkv; j += T) own_logits[j] = __ldcg(lrow + j);
+        }
+#pragma unroll 8
+        for (int j = tid; j < Nkv; j += T) m = fmaxf(m, own_logits[j]);
+        largest_of();
+#pragma unroll 2
+        for (int j = tid; j < Nkv; j += T) {
+            const float x = exponential(own_logits[j]);
+            own_logits[j] = x;
+            sum += (double)x;
+        }
+        const float denom = total_of();
+#pragma unroll 2
+        for (int j = tid; j < Nkv; j += T) {
+            const uint32_t x = descending_key(__fdiv_rn(own_logits[j], denom));
+            own_logits[j] = __uint_as_float(x);
+            best = min(best, x);
+        }
     }
     const int nth = (want + W - 1) / W;
     uint32_t bound = 0xFFFFFFFFu;
@@ -1283,16 +1315,22 @@ route_topk_kernel(const float *__restrict__ qp, const float *__restrict__ kp, in
     bound = 0u;
 #pragma unroll
     for (int w = 0; w < W; ++w) bound = max(bound, bounds[w]);
-#pragma unroll
-    for (int u = 0; u < V; ++u) {
-        const bool near = u * T + tid < Nkv && key[u] <= bound;
+    auto collect = [&](int j, uint32_t x) {
+        const bool near = j < Nkv && x <= bound;
         const unsigned voters = __ballot_sync(0xffffffffu, near);
         if (voters) {
             int base = 0;
             if (lane == 0) base = atomicAdd(&n_near, __popc(voters));
             const int pos = __shfl_sync(0xffffffffu, base, 0) + __popc(voters & ((1u << lane) - 1u));
-            if (near && pos < SLOTS) keys[pos] = ((unsigned long long)key[u] << 32) | (unsigned)(u * T + tid);
+            if (near && pos < SLOTS) keys[pos] = ((unsigned long long)x << 32) | (unsigned)j;
         }
+    };
+    if constexpr (V > 0) {
+#pragma unroll
+        for (int u = 0; u < V; ++u) collect(u * T + tid, key[u]);
+    } else {
+#pragma unroll 4
+        for (int j0 = 0; j0 < Nkv; j0 += T) collect(j0 + tid, j0 + tid < Nkv ? __float_as_uint(own_logits[j0 + tid]) : 0xFFFFFFFFu);
     }
     __syncthreads();
     const int n = n_near;        // >= want
@@ -1304,17 +1342,15 @@ route_topk_kernel(const float *__restrict__ qp, const float *__restrict__ kp, in
             for (int j = 0; j < n; ++j) place += keys[j] < mine;
             if (place < want) idx[place] = (int32_t)(mine & 0xFFFFFFFFull);
         }
-    } else if (V * T <= SLOTS || n <= SLOTS) {           // a large count, or many equal probabilities
+    } else if ((V > 0 && V * T <= SLOTS) || n <= SLOTS) {        // a large count, or many equal probabilities
         int n_pow2 = 1;
         while (n_pow2 < n) n_pow2 <<= 1;                 // <= SLOTS, a power of two
         for (int j = n + tid; j < n_pow2; j += T) keys[j] = 0xFFFFFFFFFFFFFFFFull;
         __syncthreads();
         sort_keys_smem(keys, n_pow2);
         for (int j = tid; j < want; j += T) idx[j] = (int32_t)(keys[j] & 0xFFFFFFFFull);
-    } else if constexpr (V * T > SLOTS) {
-#pragma unroll
-        for (int u = 0; u < V; ++u)
-            if (u * T + tid < Nkv) lrow[u * T + tid] = value_of_key((unsigned long long)key[u] << 32);
+    } else if constexpr (V == 0) {
+        for (int j = tid; j < Nkv; j += T) lrow[j] = value_of_key((unsigned long long)__float_as_uint(own_logits[j]) << 32);
         __syncthreads();
         unsigned long long from = 0ull;
         for (int first = 0; first < want; first += SLOTS)
@@ -1690,11 +1726,11 @@ int route_fused_launch(const float *q_pooled, const float *k_pooled, int B, int 
     if (by_count) {
         const auto launch = [&](auto threads_c, auto values_c) -> cudaError_t {
             constexpr int T = decltype(threads_c)::value, V = decltype(values_c)::value;
-            const size_t bytes = logits_ready ? 0 : (size_t)Nkv * sizeof(float);       // at most 64 KB
+            const size_t bytes = V > 0 && logits_ready ? 0 : (size_t)Nkv * sizeof(float);       // at most 64 KB
             const auto kernel = route_topk_kernel<T, V>;
             static PerDeviceOnce attr_set;
             if (!attr_set.done()) {
-                const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, T * V * (int)sizeof(float));
+                const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (V > 0 ? T * V : 16384) * (int)sizeof(float));
                 if (e != cudaSuccess) return e;
                 attr_set.mark();
             }
@@ -1706,9 +1742,7 @@ int route_fused_launch(const float *q_pooled, const float *k_pooled, int B, int 
                               : logits_ready && Nkv <= 512  ? launch(integral_constant<int, 128>(), integral_constant<int, 4>())
                               : Nkv <= 256                  ? launch(integral_constant<int, 256>(), integral_constant<int, 1>())
                               : Nkv <= 2048                 ? launch(integral_constant<int, 256>(), integral_constant<int, 8>())
-                              : Nkv <= 4096                 ? launch(integral_constant<int, 512>(), integral_constant<int, 8>())
-                              : Nkv <= 8192                 ? launch(integral_constant<int, 512>(), integral_constant<int, 16>())
-                                                            : launch(integral_constant<int, 512>(), integral_constant<int, 32>());
+                                                            : launch(integral_constant<int, 512>(), integral_constant<int, 0>());
         if (e != cudaSuccess) return fail((int)e, "wa_hsa_forward(routing by count): %s", cudaGetErrorString(e));
         return check_launch("wa_hsa_forward(routing by count)");
     }
