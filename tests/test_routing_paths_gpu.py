@@ -68,3 +68,19 @@ def test_best_blocks_by_count(nq, nkv, topk, spread):
     picked = hsa_attention(*qkv, topk_per_head=counts, **kwargs)
     whole, (_, num, _, _) = hsa_attention(*qkv, topk_per_head=counts, return_routing=True, **kwargs)
     assert num.unique().tolist() == sorted(set(topk)) and torch.equal(picked, whole)
+
+
+# short rows beside the compression of the call's own keys and values (projections of zeros: the coarse blocks are exact zeros), a
+# CTA or a cluster of up to four per head
+@pytest.mark.parametrize("b,nq,nkv", [(1, 1, 1), (1, 8, 33), (1, 9, 64), (1, 17, 65), (1, 64, 128), (2, 3, 22), (2, 32, 64)])
+@pytest.mark.parametrize("fixed", [False, True])
+def test_short_rows_beside_the_compression(b, nq, nkv, fixed):
+    from worldattention_b200.hsa import hsa_attention
+    qkv, kwargs = _inputs(b, 3, nq * BLOCK, nkv * BLOCK, nkv)
+    kwargs.update(k_proj_mat=kwargs["k_proj_mat"].new_zeros(1, nkv * BLOCK), v_proj_mat=kwargs["v_proj_mat"].new_zeros(1, nkv * BLOCK),
+                  k_coarse=torch.zeros_like(kwargs["k_coarse"]), v_coarse=torch.zeros_like(kwargs["v_coarse"]))
+    if fixed:
+        kwargs.update(topk_per_head=torch.tensor([1, nkv, nkv // 2], dtype=torch.int32))
+    given = hsa_attention(*qkv, **kwargs)
+    kwargs.update(k_coarse=None, v_coarse=None)
+    assert torch.equal(hsa_attention(*qkv, **kwargs), given)

@@ -151,6 +151,19 @@ __device__ inline void schedule_items(const int32_t *num, int rows, int Nkv, con
 __device__ inline void convert_gate_slice(const SchedJob &job, int first, int count) {
     if (first == 0 && threadIdx.x == 0 && job.pairs_done) *job.pairs_done = 0;
     if (!job.gate_w) return;
+    if (job.gate_dt == WA_F32 && ((uintptr_t)job.gate_w & 15) == 0 && first % 4 == 0 && count % 4 == 0) {      // four at a time
+        for (int i = first + 4 * threadIdx.x; i < first + count && i < 128 * 128; i += 4 * blockDim.x) {
+            const float4 w = __ldg(reinterpret_cast<const float4 *>((const float *)job.gate_w + i));
+            const __nv_bfloat162 lo = __floats2bfloat162_rn(w.x, w.y), hi = __floats2bfloat162_rn(w.z, w.w);
+            *reinterpret_cast<uint2 *>(job.w_out + i) = make_uint2(*reinterpret_cast<const uint32_t *>(&lo), *reinterpret_cast<const uint32_t *>(&hi));
+            if (i < 128)
+                *reinterpret_cast<float4 *>(job.b_out + i) =
+                    job.gate_b ? make_float4(load_elem(job.gate_b, WA_F32, i), load_elem(job.gate_b, WA_F32, i + 1), load_elem(job.gate_b, WA_F32, i + 2),
+                                             load_elem(job.gate_b, WA_F32, i + 3))
+                               : make_float4(0.f, 0.f, 0.f, 0.f);
+        }
+        return;
+    }
     for (int i = first + threadIdx.x; i < first + count && i < 128 * 128; i += blockDim.x) {
         job.w_out[i] = __float2bfloat16_rn(load_elem(job.gate_w, job.gate_dt, i));
         if (i < 128) job.b_out[i] = job.gate_b ? load_elem(job.gate_b, job.gate_dt, i) : 0.f;

@@ -1651,9 +1651,13 @@ int route_fused_launch(const float *q_pooled, const float *k_pooled, int B, int 
     // beyond, one round of rows or of tiles does (25 rows over 74: 14.7 against 20; whole calls: 37 over 74 144.9 against 147.8,
     // but 37 over 110, two rounds of both, 108.7 against 101.6).
     const bool one_round = (long long)B * Nq <= RH_WARPS || (long long)B * ((Nq + 15) / 16) * ((Nkv + 7) / 8) <= RH_WARPS;
-    const bool by_count = fixed_num_per_head && !whole_order;      // route_topk_kernel, whatever the size
-    if (!by_count && D == 128 && Nkv <= RH_MAX_KEYS && (long long)B * Nq <= RH_MAX_ROWS && (B == 1 || Nkv <= 64 || one_round) &&
-        ((uintptr_t)q_pooled % 16 == 0) && ((uintptr_t)k_pooled % 16 == 0)) {
+    const bool short_rows = D == 128 && Nkv <= RH_MAX_KEYS && (long long)B * Nq <= RH_MAX_ROWS && (B == 1 || Nkv <= 64 || one_round) &&
+                            ((uintptr_t)q_pooled % 16 == 0) && ((uintptr_t)k_pooled % 16 == 0);
+    // route_topk_kernel, whatever the size -- unless the call's keys and values are compressed meanwhile, which is the longer of the two for
+    // short rows: a CTA per row takes room on most SMs from its clusters (2 items of 24 heads, 6 query blocks over 22, whole calls:
+    // 79.0 us, with a CTA per head 76.6)
+    const bool by_count = fixed_num_per_head && !whole_order && !(short_rows && job_in.release_at_start);
+    if (!by_count && short_rows) {
         const auto launch = [&](auto width, auto warps) -> cudaError_t {
             constexpr int K = decltype(width)::value, WARPS = decltype(warps)::value, BYTES = RH_MAX_ROWS * K * 32 * (int)sizeof(float);
             const auto kernel = route_head_kernel<K, WARPS>;
@@ -1663,7 +1667,10 @@ int route_fused_launch(const float *q_pooled, const float *k_pooled, int B, int 
                 if (e != cudaSuccess) return e;
                 attr_set.mark();
             }
-            constexpr int parts = WARPS < RH_WARPS ? RH_MAX_ROWS / WARPS : 1;    // 8: a warp per row, whatever the number of rows
+            // A warp per row: up to eight rows per CTA.  While K and V are compressed beside it, half the CTAs: see above (4 rows over 79, whole
+            // calls: 62.4 us with a cluster of eight and eight warps, 58.5 with one CTA of sixteen).
+            int parts = 1;
+            while (WARPS < RH_WARPS && parts * 8 < Nq && parts < (job_in.release_at_start ? 4 : 8)) parts <<= 1;
             cudaLaunchConfig_t cfg{};
             cfg.gridDim = dim3(H * parts);
             cfg.blockDim = dim3(WARPS * 32);
@@ -1678,13 +1685,17 @@ int route_fused_launch(const float *q_pooled, const float *k_pooled, int B, int 
             cfg.attrs = attr;
             cfg.numAttrs = pdl_enabled() ? 2 : 1;
             return cudaLaunchKernelEx(&cfg, kernel, q_pooled, k_pooled, B, H, Nq, Nkv, scale, (float)tau_min, span, fixed_num_per_head, index, num,
-                                      thresholds, counters, job_in, (128 * 128 + H * parts - 1) / (H * parts));
+                                      thresholds, counters, job_in, (128 * 128 / 4 + H * parts - 1) / (H * parts) * 4);
         };
-        const auto launch_width = [&](auto warps) {
-            return Nkv <= 32 ? launch(std::integral_constant<int, 1>(), warps)
-                             : Nkv <= 64 ? launch(std::integral_constant<int, 2>(), warps) : launch(std::integral_constant<int, 4>(), warps);
+        // Eight warps, or sixteen where a row has up to sixteen tiles of logits (4 rows over 79: 14.4 us with eight, 12.4 with sixteen).
+        const auto launch_width = [&](auto few, auto many) {
+            return Nkv <= 32 ? launch(std::integral_constant<int, 1>(), few)
+                             : Nkv <= 64 ? launch(std::integral_constant<int, 2>(), few) : launch(std::integral_constant<int, 4>(), many);
         };
-        const cudaError_t e = B == 1 ? launch_width(std::integral_constant<int, 8>()) : launch_width(std::integral_constant<int, RH_WARPS>());
+        const std::integral_constant<int, 8> w8;
+        const std::integral_constant<int, 16> w16;
+        const std::integral_constant<int, RH_WARPS> w32;
+        const cudaError_t e = B == 1 ? launch_width(w8, w16) : launch_width(w32, w32);
         if (e != cudaSuccess) return fail((int)e, "wa_hsa_forward(routing of short rows): %s", cudaGetErrorString(e));
         return check_launch("wa_hsa_forward(routing of short rows)");
     }
@@ -1720,7 +1731,7 @@ int route_fused_launch(const float *q_pooled, const float *k_pooled, int B, int 
         if (e != cudaSuccess) return fail((int)e, "wa_hsa_forward(logits): %s", cudaGetErrorString(e));
         if (const int rc = check_launch("wa_hsa_forward(logits)")) return rc;
     }
-    const int gate_per_cta = (int)((128 * 128 + rows - 1) / rows);
+    const int gate_per_cta = (int)((128 * 128 / 4 + rows - 1) / rows) * 4;
     if (rows < sms) sms = (int)rows;
     const int slots = (int)((rows + sms - 1) / sms);
     if (by_count) {
