@@ -70,17 +70,18 @@ def test_best_blocks_by_count(nq, nkv, topk, spread):
     assert num.unique().tolist() == sorted(set(topk)) and torch.equal(picked, whole)
 
 
-# short rows beside the compression of the call's own keys and values (projections of zeros: the coarse blocks are exact zeros), a
-# CTA or a cluster of up to four per head
-@pytest.mark.parametrize("b,nq,nkv", [(1, 1, 1), (1, 8, 33), (1, 9, 64), (1, 17, 65), (1, 64, 128), (2, 3, 22), (2, 32, 64)])
+# beside the compression of the call's own keys and values (projections of zeros: the coarse blocks are exact zeros): short rows by
+# one or two CTAs per head; pairs of 64-token blocks, which the routing then orders by counts, in every routing kernel
+@pytest.mark.parametrize("b,h,nq,nkv,block", [(1, 3, 1, 1, 8), (1, 3, 8, 33, 8), (1, 3, 9, 64, 8), (1, 3, 17, 65, 8), (1, 3, 64, 128, 8), (2, 3, 3, 22, 8),
+                                              (2, 3, 32, 64, 8), (1, 40, 9, 5, 64), (2, 20, 4, 7, 64), (1, 3, 101, 30, 64), (1, 2, 75, 129, 64)])
 @pytest.mark.parametrize("fixed", [False, True])
-def test_short_rows_beside_the_compression(b, nq, nkv, fixed):
+def test_routing_beside_the_compression(b, h, nq, nkv, block, fixed):
     from worldattention_b200.hsa import hsa_attention
-    qkv, kwargs = _inputs(b, 3, nq * BLOCK, nkv * BLOCK, nkv)
-    kwargs.update(k_proj_mat=kwargs["k_proj_mat"].new_zeros(1, nkv * BLOCK), v_proj_mat=kwargs["v_proj_mat"].new_zeros(1, nkv * BLOCK),
-                  k_coarse=torch.zeros_like(kwargs["k_coarse"]), v_coarse=torch.zeros_like(kwargs["v_coarse"]))
+    qkv, kwargs = _inputs(b, h, nq * block - 1, nkv * block, nkv)
+    proj = torch.zeros(1, nkv * block, device=dev(), dtype=torch.bfloat16)
+    kwargs.update(block_size=block, k_proj_mat=proj, v_proj_mat=proj, k_coarse=qkv[1].new_zeros(b, 16, h, D), v_coarse=qkv[1].new_zeros(b, 16, h, D))
     if fixed:
-        kwargs.update(topk_per_head=torch.tensor([1, nkv, nkv // 2], dtype=torch.int32))
+        kwargs.update(topk_per_head=torch.tensor([1, nkv, nkv // 2], dtype=torch.int32).repeat(h)[:h])
     given = hsa_attention(*qkv, **kwargs)
     kwargs.update(k_coarse=None, v_coarse=None)
     assert torch.equal(hsa_attention(*qkv, **kwargs), given)

@@ -6,15 +6,14 @@
 // 246-259) for bf16, head_dim 128, 128- or 64-token routing blocks.
 //
 // Work item = (batch, head, query block).  Per item the CTA runs a chain of 128x128 tiles:
-//   sparse:  for each selected key block   S = Q K^T -> online softmax -> O += P V
-//   linear:  for each 128 compressed slots  S = Q Kc^T -> online softmax -> O += P Vc
+//   sparse:  for each selected key block   S = Q K^T -> softmax numerators -> O += P V
+//   linear:  for each 128 compressed slots  S = Q Kc^T -> the same -> O += P Vc
 //   gate:    S = Q Wg^T ; out = O_sparse/l_s + sigmoid(S + b) * O_linear/l_l
 // Data path: TMA (cp.async.bulk.tensor, 128-byte swizzle, one consumer CTA per copy) -> shared memory ->
 // tcgen05.mma with the S and O accumulators in tensor memory; P goes back to tensor memory as
 // bf16 and is the A operand of the PV product.  One persistent CTA of 12 warps per SM owns all 512
-// tensor-memory columns (three S buffers + O) and ~227 KB of shared memory (Q x2, K x3, V x2 tiles):
-// warps 0-7 do the softmax and the epilogue (a query row is shared by four lanes of one warp, a tile's
-// columns by two warps), warp 8 issues TMA loads, warp 9 the QK products, warp 11 the PV products and
+// tensor-memory columns (three S buffers + O) and ~227 KB of shared memory (seven tiles of Q, K and V):
+// warps 0-7 do the softmax and the epilogue (a query row is shared by four lanes of one warp), warp 8 issues TMA loads, warp 9 the QK products, warp 11 the PV products and
 // warp 10 the TMA store of the finished tile.  Items are taken heaviest first from a global counter.
 //
 // Every mbarrier wait is bounded (about two seconds); on expiry the kernel raises a flag in
@@ -29,7 +28,7 @@
 namespace wa {
 namespace sm100 {
 
-constexpr int THREADS = 384;         // warps 0..7 softmax (two threads per query row), warp 8 TMA, warp 9 QK products, warp 10 output store, warp 11 PV products
+constexpr int THREADS = 384;         // warps 0..7 softmax (four threads per query row), warp 8 TMA, warp 9 QK products, warp 10 output store, warp 11 PV products
 constexpr int REGS_SOFTMAX = 224;    // register budget per thread after the roles split (two warpgroups of softmax warps)
 constexpr int REGS_OTHER = 56;       // ... and of the warpgroup that holds the four single-purpose warps; 256*224 + 128*56 = 384*168
 constexpr int TMEM_COLS = 512;       // three S buffers: columns [0,128), [128,256), [256,384); O: [384,512)
@@ -123,15 +122,20 @@ static_assert(SMEM_BYTES <= 227 * 1024, "shared memory budget exceeded");
 //
 // PAIR (64-token blocks, more items than SMs): a work item is TWO neighbouring query blocks of a head, so all 128 rows of
 // its tile are real.  Blocks that both query blocks selected (pair_lists_kernel puts them first in both lists) are taken
-// two per tile, for all rows: a key block is then loaded once for the two, and the loads are what sparse tiles are bound by
-// (64 KB of keys and values per tile from L2).  A tile of the others holds one block of each: keys 0..63 for rows 0..63,
+// two per tile, for all rows: a key block is then loaded and scored once for the two.  A tile of the others holds one block of each: keys 0..63 for rows 0..63,
 // keys 64..127 for rows 64..127.  There the score product covers all four quadrants, the softmax only reads the two that
 // count, and the P V product is two K = 64 products, each of which writes the accumulator rows of its query block only
 // (the instruction's lane mask): a block that a row did not select never enters its sums, whatever it holds (a zero
 // probability would turn its infinities into NaN).  The linear branch and the gate run on full tiles, half as many as
 // with an item per 64-row block.
-// 12 heads, 4680 queries, the whole call: 930 -> 710 us over 21 frames with counts from the mass, 1850 -> 1560 us over 480 frames
-// with 32 blocks a row and 12 000 compressed slots.
+// 12 heads, 4680 queries, the whole call, when pairs came: 930 -> 710 us over 21 frames with counts from the mass, 1850 -> 1560 us over
+// 480 frames with 32 blocks a row and 12 000 compressed slots (549 and 1079 by now).
+//
+// What bounds it: the instructions of the softmax warps.  A 128-key tile is about 900 instructions of each of the eight, and with one
+// CTA per SM and eight copies of every branch they waited for instruction fetches as much as for their pipes (three frames of
+// 1560 tokens, cold L2: instruction cache hits 81 %, 1.33 of the cycles between issues without an instruction, special-function unit 30 %).
+// Softmax without a row maximum per tile, straight-line exponentials for full tiles and rolled epilogues made that 91 %, 0.45 and
+// 38 %, and the launch 72 -> 65 us.  The copies of K and V are not the bound: L2 hands tiles out at 18 TB/s, twice what the kernel asks for.
 template <int BLK, bool PAIR>   // routing block size: 128, or 64 (see Params::blk)
 __global__ void __launch_bounds__(THREADS, 1)
 hsa_fwd_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
@@ -1081,6 +1085,7 @@ pair_lists_kernel(const int32_t *__restrict__ index, const int32_t *__restrict__
         }
         if (lane == 0) both[item] = n_both | ((max(n[0], n[1]) - (n_both >> 1)) << 16);
     }
+    if (job.by_counts) return;
     __threadfence();
     __syncthreads();
     if (threadIdx.x == 0) last_cta = atomicAdd(job.pairs_done, 1) == (int)gridDim.x - 1;
@@ -1103,7 +1108,7 @@ schedule_kernel(const int32_t *__restrict__ num, int rows, int Nkv, SchedJob job
         return;
     }
     if (!job.gate_w) convert_gate_slice(job, 0, 0);
-    schedule_items(num, rows, Nkv, job);
+    schedule_items(num, rows, 1, Nkv, job);      // (pairs: pair_lists_kernel)
 }
 
 // ---- host side -----------------------------------------------------------------------------------
@@ -1251,6 +1256,10 @@ SchedJob hsa_sm100_sched_job(const wa_hsa_params *p, void *workspace) {
     // items of the last head are a worse end than the lightest of all (three frames, 28 MB: 107.5 against 104.9 us).  128-token
     // calls over the same window gain nothing by it (126 us either way) and their routing loses 1 us.
     job.by_head = job.paired && 4ll * p->B * p->H * p->Lkv * p->D > (64ll << 20);
+    // The order by tiles costs pair_lists_kernel 3 us at its end.  The routing's own order by counts costs nothing where the call's keys
+    // and values are compressed beside it for longer than it takes (2 items of 24 heads, 6 query blocks over 22, whole calls: 77.9
+    // against 75.0 us; 10 x 20 of 12 heads 40.3 and 39.2).
+    job.by_counts = job.paired && !job.by_head && !p->index_in && p->Lc == 0;
     return job;
 }
 

@@ -17,6 +17,7 @@ struct SchedJob {
     float *b_out;           // [128] float32
     bool paired;            // a work item is two neighbouring query blocks (rows of `num`) of one head: pair_lists_kernel makes the order
     bool by_head;           // paired: work order head by head (see sort_items_by_head)
+    bool by_counts;         // paired: the routing makes the work order, by the larger count of a pair, not pair_lists_kernel by the tiles
     int *pairs_done;        // paired: CTAs of pair_lists_kernel that are done; zero before it runs
     bool release_at_start;  // the next launch does not wait for the routing (it compresses K and V meanwhile)
     int release_dependents_after_rows;   // timing experiment (WA_B200_PDL=2), see route_row
@@ -143,8 +144,20 @@ __device__ __forceinline__ void schedule_rows(Count count_of, int rows, int Nkv,
 }
 
 // The same after a routing kernel, whose counts were written by other CTAs of this launch: they are read past L1.
-__device__ inline void schedule_items(const int32_t *num, int rows, int Nkv, const SchedJob &job) {
-    if (!job.paired) schedule_rows([&](int row) { return __ldcg(num + row); }, rows, Nkv, job);
+__device__ inline void schedule_items(const int32_t *num, int rows, int Nq, int Nkv, const SchedJob &job) {
+    __shared__ int hist[SCHED_BINS];
+    __shared__ int warp_tot[32];
+    if (!job.paired) {
+        sort_items([&](int row) { return __ldcg(num + row); }, rows, Nkv, hist, warp_tot, job.order, job.work_counter, job.error_flag);
+    } else if (job.by_counts) {
+        const int each = (Nq + 1) >> 1;
+        auto count_of = [&](int i) {      // no branches: a thread's look-ups are all on their way at once
+            const int head = i / each, q = 2 * (i - head * each);
+            const int32_t *at = num + (long long)head * Nq + q;
+            return max(__ldcg(at), __ldcg(at + (q + 1 < Nq ? 1 : 0)));
+        };
+        sort_items(count_of, rows / Nq * each, Nkv, hist, warp_tot, job.order, job.work_counter, job.error_flag);
+    }
 }
 
 // Elements [first, first + count) of the gate weight -> bf16 (it is an MMA operand) and of the bias -> float32.

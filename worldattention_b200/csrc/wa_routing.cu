@@ -985,7 +985,7 @@ __device__ __forceinline__ void route_row(const long long row, const float *__re
     __syncthreads();
     if (!last_flag || !job.order) return;
     __threadfence();
-    schedule_items(num, B * H * Nq, Nkv, job);
+    schedule_items(num, B * H * Nq, Nq, Nkv, job);
     ROUTE_STAMP(7);
 }
 
@@ -1178,7 +1178,7 @@ route_head_kernel(const float *__restrict__ qp, const float *__restrict__ kp, in
     __syncthreads();
     if (!last_flag || !job.order) return;
     __threadfence();
-    schedule_items(num, B * H * Nq, Nkv, job);
+    schedule_items(num, B * H * Nq, Nq, Nkv, job);
 }
 
 // ------------------------------------------------------------------------------------------------
@@ -1214,7 +1214,9 @@ route_topk_kernel(const float *__restrict__ qp, const float *__restrict__ kp, in
     pdl_wait();                 // pooled means, or logits, come from the launch before
     if (job.release_at_start) pdl_release_dependents();
     if (blockIdx.x == 0) {
-        if (job.order && !job.paired) schedule_rows([&](int row) { return __ldg(fixed_num + (row / Nq) % H); }, rows, Nkv, job);
+        const int each = job.paired ? (Nq + 1) >> 1 : Nq;      // items of a head
+        if (job.order && (!job.paired || job.by_counts))
+            schedule_rows([&](int item) { return __ldg(fixed_num + (item / each) % H); }, rows / Nq * each, Nkv, job);
         return;
     }
     // neighbouring rows (same head, same pooled keys) on one SM, as in route_fused_kernel
@@ -1667,23 +1669,29 @@ int route_fused_launch(const float *q_pooled, const float *k_pooled, int B, int 
                 if (e != cudaSuccess) return e;
                 attr_set.mark();
             }
-            // A warp per row: up to eight rows per CTA.  While K and V are compressed beside it, half the CTAs: see above (4 rows over 79, whole
-            // calls: 62.4 us with a cluster of eight and eight warps, 58.5 with one CTA of sixteen).
+            // A warp per row, up to eight rows per CTA; while K and V are compressed beside it, two CTAs at most, of sixteen warps (17 rows over 34
+            // of 16 heads, whole calls: 90.5 us with four of eight warps, 92.5 with one of 32, 85.9).
             int parts = 1;
-            while (WARPS < RH_WARPS && parts * 8 < Nq && parts < (job_in.release_at_start ? 4 : 8)) parts <<= 1;
+            while (WARPS < RH_WARPS && parts * 8 < Nq && parts < (job_in.release_at_start ? 2 : 8)) parts <<= 1;
             cudaLaunchConfig_t cfg{};
             cfg.gridDim = dim3(H * parts);
             cfg.blockDim = dim3(WARPS * 32);
             cfg.dynamicSmemBytes = (size_t)B * ((Nq + parts - 1) / parts) * K * 32 * sizeof(float);
             cfg.stream = stream;
             cudaLaunchAttribute attr[2];
-            attr[0].id = cudaLaunchAttributeClusterDimension;
-            attr[0].val.clusterDim.x = parts;
-            attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
-            attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-            attr[1].val.programmaticStreamSerializationAllowed = 1;
             cfg.attrs = attr;
-            cfg.numAttrs = pdl_enabled() ? 2 : 1;
+            cfg.numAttrs = 0;
+            if (parts > 1) {      // a cluster of one costs the launches around it (8 rows over 8, whole call: 30.1 us with, 27.4 without)
+                attr[cfg.numAttrs].id = cudaLaunchAttributeClusterDimension;
+                attr[cfg.numAttrs].val.clusterDim.x = parts;
+                attr[cfg.numAttrs].val.clusterDim.y = attr[cfg.numAttrs].val.clusterDim.z = 1;
+                ++cfg.numAttrs;
+            }
+            if (pdl_enabled()) {
+                attr[cfg.numAttrs].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+                attr[cfg.numAttrs].val.programmaticStreamSerializationAllowed = 1;
+                ++cfg.numAttrs;
+            }
             return cudaLaunchKernelEx(&cfg, kernel, q_pooled, k_pooled, B, H, Nq, Nkv, scale, (float)tau_min, span, fixed_num_per_head, index, num,
                                       thresholds, counters, job_in, (128 * 128 / 4 + H * parts - 1) / (H * parts) * 4);
         };
@@ -1695,7 +1703,7 @@ int route_fused_launch(const float *q_pooled, const float *k_pooled, int B, int 
         const std::integral_constant<int, 8> w8;
         const std::integral_constant<int, 16> w16;
         const std::integral_constant<int, RH_WARPS> w32;
-        const cudaError_t e = B == 1 ? launch_width(w8, w16) : launch_width(w32, w32);
+        const cudaError_t e = B > 1 ? launch_width(w32, w32) : job_in.release_at_start && Nq > 8 ? launch_width(w16, w16) : launch_width(w8, w16);
         if (e != cudaSuccess) return fail((int)e, "wa_hsa_forward(routing of short rows): %s", cudaGetErrorString(e));
         return check_launch("wa_hsa_forward(routing of short rows)");
     }
