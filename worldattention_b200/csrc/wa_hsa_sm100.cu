@@ -641,14 +641,21 @@ hsa_fwd_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
                             float xa = -INFINITY, xb = -INFINITY;
                             tmem_wait_ld16(lo);
 #pragma unroll 1
-                            for (int c = 0; c < 2 * halves; ++c) {
-                                TMEM_LDQ16(s_addr + 32 * c, lo);
+                            for (int c = 0; c < halves; ++c) {      // (32 at a time: four waits instead of two, 0.3 us of a short item's launch)
+                                TMEM_LDQ16(s_addr + 64 * c, lo);
+                                TMEM_LDQ16(s_addr + 64 * c + 32, hi);
                                 tmem_wait_ld16(lo);
-                                if (!full) mask(lo, 32 * c);
+                                tmem_wait_ld16(hi);
+                                if (!full) {
+                                    mask(lo, 64 * c);
+                                    mask(hi, 64 * c + 32);
+                                }
 #pragma unroll
                                 for (int j = 0; j < 4; ++j) {
-                                    xa = fmaxf(xa, fmaxf(__uint_as_float(lo[4 * j]), __uint_as_float(lo[4 * j + 1])));
-                                    xb = fmaxf(xb, fmaxf(__uint_as_float(lo[4 * j + 2]), __uint_as_float(lo[4 * j + 3])));
+                                    xa = fmaxf(fmaxf(xa, fmaxf(__uint_as_float(lo[4 * j]), __uint_as_float(lo[4 * j + 1]))),
+                                               fmaxf(__uint_as_float(hi[4 * j]), __uint_as_float(hi[4 * j + 1])));
+                                    xb = fmaxf(fmaxf(xb, fmaxf(__uint_as_float(lo[4 * j + 2]), __uint_as_float(lo[4 * j + 3]))),
+                                               fmaxf(__uint_as_float(hi[4 * j + 2]), __uint_as_float(hi[4 * j + 3])));
                                 }
                             }
                             const float mxA = quad_max(xa) * p.scale_log2, mxB = quad_max(xb) * p.scale_log2;
