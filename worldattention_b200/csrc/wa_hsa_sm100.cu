@@ -1020,8 +1020,8 @@ hsa_fwd_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
 // A warp per item.  Ascending, so that the CTAs that work on a head sweep its keys side by side and find in L2 what the
 // first of them fetched.  A list that names a block twice (only a caller's own routing can) stays as it is.
 // `both` receives the number of common blocks (lower half) and the item's sparse tiles (upper half).  The CTA that finishes
-// last makes the work order from the latter: what an item costs is its tiles, and two query blocks that share their blocks have
-// far fewer of them than their counts say.
+// last makes the work order from the latter (unless SchedJob::by_counts): what an item costs is its tiles, and two query blocks that
+// share their blocks have far fewer of them than their counts say.
 constexpr int PL_WARPS = 8;
 __global__ void __launch_bounds__(PL_WARPS * 32)
 pair_lists_kernel(const int32_t *__restrict__ index, const int32_t *__restrict__ num, int Nq, int Nkv, int q_items, int n_items,

@@ -1024,8 +1024,8 @@ route_fused_kernel(const float *__restrict__ qp, const float *__restrict__ kp, i
 
 // ------------------------------------------------------------------------------------------------
 // The whole routing of short rows (head_dim 128, up to 64 query blocks of a head over the batch and 128 key blocks; with a batch 64, or
-// 128 where one round of the CTA's warps does): a cluster, or a CTA, per head.  There the kernel above is a chain of waits: some twenty barriers of a row, a counter per head, the last CTA's walk
-// over all rows of the head, a second counter.  Here the logits come from the float64 matrix instruction, a 16 x 8 tile per
+// 128 where one round of the CTA's warps does): a cluster, or a CTA, per head.  There the kernel above is a chain of waits: some twenty
+// barriers of a row, a counter per head, the last CTA's walk over all rows of the head, a second counter.  Here the logits come from the float64 matrix instruction, a 16 x 8 tile per
 // warp, a row's softmax, sort and sums stay inside a warp (K keys per lane, exchanges by shuffles), and the head's threshold
 // and counts need two barriers.  Same sums (float64, rounded where the reference rounds) and the same order.
 // 12 heads, the whole call: 7 query blocks over 19 key blocks 40.5 -> 37.0 us, 37 over 37 100.1 -> 96.2 (the routing itself 20.6 -> 11.5 and
