@@ -594,7 +594,8 @@ hsa_fwd_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
                 bool started = false;      // every row of the warp has its reference point
                 // The reference point m of a row (the exponentials are 2^(s - m)) is the maximum of the row's first real tile; later
                 // tiles are computed against it WITHOUT looking for their own maximum: any m gives the same quotients as long as
-                // nothing overflows, and the sums, which are needed anyway, show when a row has outgrown its m.  Only then is the
+                // nothing overflows, and the sums, which are needed anyway, show when a row has outgrown its m: a score above it by more than 8
+                // adds more than 2^8 in any column (both exponentials end in +inf, not in a wrapped exponent).  Only then is the
                 // tile's maximum found, the accumulator rescaled and the tile computed again (its scores are still in tensor
                 // memory).  So a tile needs no pass over its scores before the exponentials, the next 32 columns are fetched
                 // while 32 are at work (fetching the next tile's first ones before this one's probabilities are handed over delays that: 421 ->
