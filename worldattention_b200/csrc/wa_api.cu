@@ -81,9 +81,10 @@ int inline_coarse_len(const wa_hsa_params *p) {
 
 // Keys and values of a float32 call are rounded once for all query blocks: a pass over memory that pays where a key block is
 // selected several times and the chip is full (12 heads over 4680 keys, 64-token blocks, the whole call without and with it: 4 query
-// blocks 210 and 219 us, 12 245 and 242, 14 286 and 278, 25 323 and 317; over 9360 keys 25 blocks 576 and 551).
-bool keeps_rounded_kv(const wa_hsa_params *p) {
-    return p->k.dtype == WA_F32 && p->v.dtype == WA_F32 && p->D == 128 &&
+// blocks 210 and 219 us, 12 245 and 242, 14 286 and 278, 25 323 and 317; over 9360 keys 25 blocks 576 and 551).  The workspace holds
+// them where this says so, and nowhere else (pointers and strides that are still zero when the size is asked for count as aligned).
+bool rounds_kv_once(const wa_hsa_params *p) {
+    return !p->part_sparse && round_kv_supported(&p->k, &p->v, p->D) &&
            (long long)p->B * p->H * ceil_div(p->Lq, p->block_size) >= sm_count();
 }
 
@@ -109,7 +110,7 @@ Workspace plan(const wa_hsa_params *p) {
     w.sparse = take(c, tokens * sizeof(__nv_bfloat16));
     w.linear = take(c, tokens * sizeof(float));
     w.tuned = take(c, hsa_sm100_workspace_bytes(p));
-    w.kv16 = take(c, keeps_rounded_kv(p) ? 2 * (size_t)p->B * p->Lkv * p->H * p->D * sizeof(__nv_bfloat16) : 0);
+    w.kv16 = take(c, rounds_kv_once(p) ? 2 * (size_t)p->B * p->Lkv * p->H * p->D * sizeof(__nv_bfloat16) : 0);
     w.total = c;
     return w;
 }
@@ -238,7 +239,7 @@ extern "C" int wa_hsa_forward(const wa_hsa_params *p, int *used_tuned, void *str
         prepared = tuned;
     }
 
-    const bool rounded = !tuned && !partial && keeps_rounded_kv(p) && round_kv_supported(&p->k, &p->v, p->D);
+    const bool rounded = rounds_kv_once(p);      // (float32: never the tcgen05 kernel)
     if (compress_inline) {
         if ((rc = compress_kv_launch(&p->k, &p->v, &kc, &vc, p->B, p->Lkv, p->H, p->D, p->proj_segment_len, p->block_size, p->k_proj,
                                      p->v_proj, p->proj_dtype, p->proj_rank, p->proj_cols, /*beside_routing=*/!p->index_in, stream,
