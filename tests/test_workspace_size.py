@@ -26,3 +26,12 @@ def test_room_for_rounded_keys_where_they_are_rounded(q_len, kv_len, block):
     assert _bytes(q_len, kv_len, block) == plain + rounded
     assert _bytes(q_len, kv_len, block, part_sparse=1 << 20) == plain              # nor are those of a call with partial outputs
     assert _bytes(q_len, kv_len, block, k_stride=0, k_ptr=0) == plain + rounded    # not known yet: enough for either
+
+
+# fixed counts and a caller's own routing select no more of a longer cache; the room for the copy is bounded by 512 MB
+@pytest.mark.parametrize("kv_len,fields,expected", [
+    (16384, dict(topk_per_head=1 << 20), True), (16385, dict(topk_per_head=1 << 20), False), (748800, dict(topk_per_head=1 << 20), False),
+    (16384, dict(index_in=1 << 20, num_in=1 << 20), True), (16385, dict(index_in=1 << 20, num_in=1 << 20), False),
+    (16385, {}, True), ((512 << 20) // (4 * H * D), {}, True), ((512 << 20) // (4 * H * D) + 1, {}, False), (748800, {}, False)])
+def test_long_caches_are_rounded_where_that_pays(kv_len, fields, expected):
+    assert _bytes(4680, kv_len, **fields) - _bytes(4680, kv_len, k_stride=H * D + 2, **fields) == (4 * B * kv_len * H * D + 255) // 256 * 256 * expected

@@ -79,12 +79,22 @@ int inline_coarse_len(const wa_hsa_params *p) {
     return total;
 }
 
+size_t rounded_kv_bytes(const wa_hsa_params *p) { return 2 * (size_t)p->B * p->Lkv * p->H * p->D * sizeof(__nv_bfloat16); }
+
 // Keys and values of a float32 call are rounded once for all query blocks: a pass over memory that pays where a key block is
 // selected several times and the chip is full (12 heads over 4680 keys, 64-token blocks, the whole call without and with it: 4 query
 // blocks 210 and 219 us, 12 245 and 242, 14 286 and 278, 25 323 and 317; over 9360 keys 25 blocks 576 and 551).  The workspace holds
 // them where this says so, and nowhere else (pointers and strides that are still zero when the size is asked for count as aligned).
+// The pass costs as much as there are keys, 3.3 us per frame of 1560 tokens.  With counts from the mass a row selects the more blocks
+// the more there are (25 query blocks over 24 frames 1963 -> 1727 us, 74 over 24 4280 -> 3801); with fixed counts, or a caller's own
+// routing, it does not, and neither is known here: with the 15 blocks of 128 a row of the repository's configurations 25 query blocks
+// over 6 frames take 430 without and 413 with, over 12 506 and 504, over 24 635 and 674, 74 over 8 810 and 793, over 24 1248 and 1284.
+// The room is bounded too, so that a call over a long cache does not need half as much again as its keys and values take.
+constexpr int ROUND_FIXED_KEYS = 16384;
+constexpr size_t ROUND_BYTES = (size_t)512 << 20;
 bool rounds_kv_once(const wa_hsa_params *p) {
-    return !p->part_sparse && round_kv_supported(&p->k, &p->v, p->D) &&
+    const bool by_mass = !p->topk_per_head && !p->index_in;
+    return !p->part_sparse && (by_mass || p->Lkv <= ROUND_FIXED_KEYS) && rounded_kv_bytes(p) <= ROUND_BYTES && round_kv_supported(&p->k, &p->v, p->D) &&
            (long long)p->B * p->H * ceil_div(p->Lq, p->block_size) >= sm_count();
 }
 
@@ -110,7 +120,7 @@ Workspace plan(const wa_hsa_params *p) {
     w.sparse = take(c, tokens * sizeof(__nv_bfloat16));
     w.linear = take(c, tokens * sizeof(float));
     w.tuned = take(c, hsa_sm100_workspace_bytes(p));
-    w.kv16 = take(c, rounds_kv_once(p) ? 2 * (size_t)p->B * p->Lkv * p->H * p->D * sizeof(__nv_bfloat16) : 0);
+    w.kv16 = take(c, rounds_kv_once(p) ? rounded_kv_bytes(p) : 0);
     w.total = c;
     return w;
 }
