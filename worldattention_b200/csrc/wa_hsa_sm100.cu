@@ -591,7 +591,7 @@ hsa_fwd_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
             for (int phase = 0; phase < 2 && ok; ++phase) {
                 const int t0 = phase == 0 ? 0 : n_sel, t1 = phase == 0 ? n_sel : n_kv;
                 float mA = -INFINITY, mB = -INFINITY, lA = 0.f, lB = 0.f;   // l: this thread's columns only
-                bool started = false;      // every row of the warp has a reference point that should do for the next tile
+                bool started = false;      // every row of the warp has its reference point
                 // The reference point m of a row (the exponentials are 2^(s - m)) is the maximum of the row's first real tile; later
                 // tiles are computed against it WITHOUT looking for their own maximum: any m gives the same quotients as long as
                 // nothing overflows, and the sums, which are needed anyway, show when a row has outgrown its m: a score above it by more than 8
@@ -605,14 +605,6 @@ hsa_fwd_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
                 // fetching of instructions, not a pipe: the special-function unit is 30 % busy, so only every eighth pair of columns takes the
                 // polynomial (with every fourth, counts from the mass: 510 against 496 us; none: the same, 3 frames 67.8 against 66.4).
                 constexpr float OUTGROWN = 256.0f;       // sum over a thread's columns, a quarter of a row's: no probability exceeds it
-                // A row that has outgrown its reference point gets one 2^ROOM above the tile's maximum: the probabilities keep their bits
-                // at any power of two, what lies 2^62 below the row's maximum becomes zero, and a row that goes on growing pays
-                // the second pass once in 72 powers of two and not with every tile.  Where one tile brings more than that, the next one looks
-                // for its maximum first, as a first tile does.  Whole calls, scores that grow by 0.1 powers of two per 64 keys over 480 frames:
-                // 1309 us without, 1113 with a room of 32, 1072 (1161 with a maximum for every tile); by 1 over 21 frames of 64-token
-                // blocks 171, 157, 153 (189); by 20, where the next tile's maximum helps, 200 -> 189 (188); four times the usual
-                // queries and keys 208, 195, 188 (215).
-                constexpr float ROOM = 64.0f;
                 constexpr uint32_t MASKED = 0xff800000u; // -inf
                 for (int t = t0; t < t1 && ok; ++t) {
                     const int buf = (sg + t) % S_BUFS;
@@ -670,9 +662,7 @@ hsa_fwd_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
                             const float mxA = quad_max(xa) * p.scale_log2, mxB = quad_max(xb) * p.scale_log2;
                             WA_TRACE(8);
                             const bool growA = mxA > mA, growB = mxB > mB;
-                            const float room = later ? ROOM : 0.0f;
-                            const float mA_new = growA ? mxA + room : mA, mB_new = growB ? mxB + room : mB;
-                            const bool steep = later && (mxA > mA + (ROOM + 8.0f) || mxB > mB + (ROOM + 8.0f));
+                            const float mA_new = growA ? mxA : mA, mB_new = growB ? mxB : mB;
                             if (__any_sync(0xffffffffu, (growA || growB) && later)) {
                                 // every PV requested so far must have landed before the accumulator is touched
                                 ok = __all_sync(0xffffffffu, mbar_wait(&bar->v_empty[(pv_count - 1u) % V_STAGES],
@@ -699,7 +689,7 @@ hsa_fwd_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
                             }
                             mA = mA_new;
                             mB = mB_new;
-                            started = __all_sync(0xffffffffu, mA > -INFINITY && mB > -INFINITY && !steep);   // (a row without a real key yet: look again)
+                            started = __all_sync(0xffffffffu, mA > -INFINITY && mB > -INFINITY);   // (a row without a real key yet: look again)
                             TMEM_LDQ16(s_addr, lo);
                         }
                         // p = 2^(s*c - m), row sums, pack to bf16
