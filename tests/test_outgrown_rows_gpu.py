@@ -55,6 +55,36 @@ def _lists(heads, nq, nkv, own):
 SHAPES = [(128, 3, 2, False), (64, 3, 2, False), (64, 24, 8, False), (64, 24, 8, True)]
 
 
+# Powers of two that each tile's keys lie above the ones before.  A reference point moves where the growth since then exceeds about 8;
+# more than 12 in one tile make the next tile look for its maximum first, whether it grows or not.
+STEPS = {"once in a while": [9, 0, 0, 60, 3, 11, 0, 13, 0, 0, 0, 9], "steep, then flat": [100, 0, 100, 100, 0, 0, 73, 71, 0, 200, 0, 0],
+         "up and down": [80, -80, 160, -100, 30, -200, 300, -5, 10, 64, 8, 1], "down": [-90, -3, -200, 0, 0, -10, 0, 0, 0, 0, 0, 0]}
+
+
+@pytest.mark.parametrize("block,heads,nq,own", SHAPES)
+@pytest.mark.parametrize("steps", list(STEPS))
+def test_growth_that_comes_and_goes(block, heads, nq, own, steps):
+    from worldattention_b200.hsa.branches import hsa_partials
+    g = torch.Generator(device=dev()).manual_seed(block + heads + own)
+    draw = lambda n: torch.randn(1, n, heads, D, generator=g, device=dev())
+    level = torch.cumsum(torch.tensor([0] + STEPS[steps], device=dev(), dtype=torch.float32), 0)
+    tile = max(128 // block, 1)               # blocks of a tile
+    nkv, slots = 13 * tile, 13 * 128
+    q, k, v, kc, vc = draw(nq * block - 5) * 0.3, draw(nkv * block - 17) * 0.3, draw(nkv * block - 17), draw(slots - 17) * 0.3, draw(slots - 17)
+    q[..., 0] = 8.0
+    unit = 1 / (8.0 * D ** -0.5 * 1.4426950408889634)
+    k[..., 0] = (level[torch.arange(k.shape[1], device=dev()) // 128] * unit)[None, :, None]
+    kc[..., 0] = (level[torch.arange(kc.shape[1], device=dev()) // 128] * unit)[None, :, None]
+    args = [t.bfloat16() for t in (q, k, v, kc, vc)]
+    index, num = _lists(heads, nq, nkv, own)
+    got, want = (hsa_partials(*args, index, num, block, force_generic=generic) for generic in (False, True))
+    assert got[4] and not want[4]
+    for a, b in zip(got[:4], want[:4]):
+        a, b = to_np(a), to_np(b)
+        max_abs, mean_rel = attention_error(a, b)
+        assert max_abs < max(MAX_ABS, 1e-5 * abs(b).max()) and mean_rel < MEAN_REL
+
+
 # ONE key of the second tile lies `nats` above all others, for every row alike: nothing but the exponential of its own column can tell.
 # Columns 0..7 of every 64 are computed by a polynomial, the others by the special-function unit; 88 nats are 127 powers of two, from
 # 90 on float32 overflows, and 177, 266 and 355 are 256, 384 and 512 powers of two.

@@ -591,7 +591,7 @@ hsa_fwd_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
             for (int phase = 0; phase < 2 && ok; ++phase) {
                 const int t0 = phase == 0 ? 0 : n_sel, t1 = phase == 0 ? n_sel : n_kv;
                 float mA = -INFINITY, mB = -INFINITY, lA = 0.f, lB = 0.f;   // l: this thread's columns only
-                bool started = false;      // every row of the warp has its reference point
+                bool started = false;      // every row of the warp has a reference point that should do for the next tile
                 // The reference point m of a row (the exponentials are 2^(s - m)) is the maximum of the row's first real tile; later
                 // tiles are computed against it WITHOUT looking for their own maximum: any m gives the same quotients as long as
                 // nothing overflows, and the sums, which are needed anyway, show when a row has outgrown its m: a score above it by more than 8
@@ -605,6 +605,14 @@ hsa_fwd_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
                 // fetching of instructions, not a pipe: the special-function unit is 30 % busy, so only every eighth pair of columns takes the
                 // polynomial (with every fourth, counts from the mass: 510 against 496 us; none: the same, 3 frames 67.8 against 66.4).
                 constexpr float OUTGROWN = 256.0f;       // sum over a thread's columns, a quarter of a row's: no probability exceeds it
+                // Where a tile raises a maximum by more than this, the next one looks for its maximum first, as a first tile does: scores that grow
+                // along the keys would otherwise be read for exponentials, for their maximum and for exponentials again, tile after tile.
+                // Whole calls, growth of 0.1 powers of two per 64 keys over 480 frames 1306 -> 1154 us (1156 with a maximum for every tile), of 3 and 20
+                // per 64-token block over 21 frames 198 -> 192 and 200 -> 189 (191 and 187).  At 20 the first is 1249; at 8, which single rows of
+                // random keys reach, three frames lose 1.0 of 80 us.  Reference points 2^64 above the maximum would make growth cheaper still, but the
+                // largest probability of a row is then rounded instead of being exactly one (queries and keys three times as large: error 0.00241 against
+                // 0.00224).
+                constexpr float STEEP = 12.0f;
                 constexpr uint32_t MASKED = 0xff800000u; // -inf
                 for (int t = t0; t < t1 && ok; ++t) {
                     const int buf = (sg + t) % S_BUFS;
@@ -663,6 +671,7 @@ hsa_fwd_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
                             WA_TRACE(8);
                             const bool growA = mxA > mA, growB = mxB > mB;
                             const float mA_new = growA ? mxA : mA, mB_new = growB ? mxB : mB;
+                            const bool steep = later && (mxA > mA + STEEP || mxB > mB + STEEP);
                             if (__any_sync(0xffffffffu, (growA || growB) && later)) {
                                 // every PV requested so far must have landed before the accumulator is touched
                                 ok = __all_sync(0xffffffffu, mbar_wait(&bar->v_empty[(pv_count - 1u) % V_STAGES],
@@ -689,7 +698,7 @@ hsa_fwd_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
                             }
                             mA = mA_new;
                             mB = mB_new;
-                            started = __all_sync(0xffffffffu, mA > -INFINITY && mB > -INFINITY);   // (a row without a real key yet: look again)
+                            started = __all_sync(0xffffffffu, mA > -INFINITY && mB > -INFINITY && !steep);   // (a row without a real key yet: look again)
                             TMEM_LDQ16(s_addr, lo);
                         }
                         // p = 2^(s*c - m), row sums, pack to bf16
