@@ -1151,7 +1151,7 @@ route_head_kernel(const float *__restrict__ qp, const float *__restrict__ kp, in
         spread = warp_sum_d(spread);
         if (lane < parts) *cluster.map_shared_rank(&gini[r], lane) = __fdiv_rn((float)spread, (float)Nkv);
     }
-    cluster.sync();
+    if (parts > 1) cluster.sync(); else __syncthreads();
     if (warp == 0) {
         double total = 0.0;
         for (int r = lane; r < rows; r += 32) total += (double)gini[r];
@@ -1628,6 +1628,20 @@ int route_select_launch(const float *block_attn, int B, int H, int Nq, int Nkv, 
 }  // namespace wa
 
 namespace wa {
+// With a batch a CTA takes 32 rows and 32 tiles of logits at a time.  Two rounds of rows pay up to 64 keys (37 rows over 37: 16.5 us against 22.6);
+// beyond, one round of rows or of tiles does (25 rows over 74: 14.7 against 20; whole calls: 37 over 74 144.9 against 147.8,
+// but 37 over 110, two rounds of both, 108.7 against 101.6).
+// Without, a warp per row, up to eight rows per CTA; while K and V are compressed beside it, two CTAs at most, of sixteen warps (17 rows over
+// 34 of 16 heads, whole calls: 90.5 us with four of eight warps, 92.5 with one of 32, 85.9), and one where that is a row per warp of few
+// keys (10 rows over 20 of 8 heads 51.6 us with two, 49.3 with one; 11 over 33 of 12 44.2 and 42.9; but 14 over 56 79.7 and 80.8).
+static int route_short_parts(int B, int Nq, int Nkv, int D, bool beside) {
+    const bool one_round = (long long)B * Nq <= RH_WARPS || (long long)B * ((Nq + 15) / 16) * ((Nkv + 7) / 8) <= RH_WARPS;
+    if (D != 128 || Nkv > RH_MAX_KEYS || (long long)B * Nq > RH_MAX_ROWS || (B > 1 && Nkv > 64 && !one_round)) return 0;
+    int parts = 1;
+    while (B == 1 && parts * (beside && Nkv <= 48 && Nq > 8 ? 16 : 8) < Nq && parts < (beside ? 2 : 8)) parts <<= 1;
+    return parts;
+}
+
 int route_fused_launch(const float *q_pooled, const float *k_pooled, int B, int H, int Nq, int Nkv, int D, double tau_min,
                        double tau_max, const int32_t *fixed_num_per_head, float *sorted, int32_t *index, int32_t *num,
                        float *thresholds, float *gini, int *counters, const SchedJob &job_in, cudaStream_t stream, bool whole_order) {
@@ -1649,12 +1663,8 @@ int route_fused_launch(const float *q_pooled, const float *k_pooled, int B, int 
     const float scale = (float)pow((double)D, -0.5), span = (float)(tau_max - tau_min);
     const long long bh = (long long)B * H;
 
-    // With a batch a CTA takes 32 rows and 32 tiles of logits at a time.  Two rounds of rows pay up to 64 keys (37 rows over 37: 16.5 us against 22.6);
-    // beyond, one round of rows or of tiles does (25 rows over 74: 14.7 against 20; whole calls: 37 over 74 144.9 against 147.8,
-    // but 37 over 110, two rounds of both, 108.7 against 101.6).
-    const bool one_round = (long long)B * Nq <= RH_WARPS || (long long)B * ((Nq + 15) / 16) * ((Nkv + 7) / 8) <= RH_WARPS;
-    const bool short_rows = D == 128 && Nkv <= RH_MAX_KEYS && (long long)B * Nq <= RH_MAX_ROWS && (B == 1 || Nkv <= 64 || one_round) &&
-                            ((uintptr_t)q_pooled % 16 == 0) && ((uintptr_t)k_pooled % 16 == 0);
+    const int parts = ((uintptr_t)q_pooled % 16 == 0) && ((uintptr_t)k_pooled % 16 == 0) ? route_short_parts(B, Nq, Nkv, D, job_in.release_at_start) : 0;
+    const bool short_rows = parts > 0;
     // route_topk_kernel, whatever the size -- unless the call's keys and values are compressed meanwhile, which is the longer of the two for
     // short rows: a CTA per row takes room on most SMs from its clusters (2 items of 24 heads, 6 query blocks over 22, whole calls:
     // 79.0 us, with a CTA per head 76.6)
@@ -1669,10 +1679,6 @@ int route_fused_launch(const float *q_pooled, const float *k_pooled, int B, int 
                 if (e != cudaSuccess) return e;
                 attr_set.mark();
             }
-            // A warp per row, up to eight rows per CTA; while K and V are compressed beside it, two CTAs at most, of sixteen warps (17 rows over 34
-            // of 16 heads, whole calls: 90.5 us with four of eight warps, 92.5 with one of 32, 85.9).
-            int parts = 1;
-            while (WARPS < RH_WARPS && parts * 8 < Nq && parts < (job_in.release_at_start ? 2 : 8)) parts <<= 1;
             cudaLaunchConfig_t cfg{};
             cfg.gridDim = dim3(H * parts);
             cfg.blockDim = dim3(WARPS * 32);
