@@ -85,3 +85,28 @@ def test_routing_beside_the_compression(b, h, nq, nkv, block, fixed):
     given = hsa_attention(*qkv, **kwargs)
     kwargs.update(k_coarse=None, v_coarse=None)
     assert torch.equal(hsa_attention(*qkv, **kwargs), given)
+
+
+# the same with float32 projections, which a kernel of fewer CTAs multiplies: its shares per segment (of 64 tokens and more) are cut to
+# fit beside the routing's CTAs, which keep their SMs to themselves where all fit; 16 rows and 48 keys are the most of one routing CTA
+@pytest.mark.parametrize("b,h,q_len,segments,seg,block", [(1, 8, 600, 3, 635, 64), (1, 12, 1000, 4, 760, 64), (1, 12, 1024, 4, 768, 64), (1, 12, 1025, 4, 769, 64),
+                                                          (1, 24, 700, 3, 300, 64), (1, 16, 128, 2, 100, 128), (1, 3, 513, 5, 640, 64), (2, 12, 200, 2, 130, 64),
+                                                          (1, 24, 1100, 12, 70, 64), (1, 74, 64, 1, 600, 64)])
+@pytest.mark.parametrize("zeros", [True, False])
+def test_compression_that_fits_beside_the_routing(b, h, q_len, segments, seg, block, zeros):
+    from tests.helpers import attention_error, to_np
+    from worldattention_b200.hsa import HSAAttention
+    g = torch.Generator(device=dev()).manual_seed(seg)
+    draw = lambda n: torch.randn(b, n, h, D, generator=g, device=dev()).bfloat16()
+    q, k, v = draw(q_len), draw(segments * seg - 3), draw(segments * seg - 3)
+    hsa = HSAAttention(h, D, block_size=block, proj_segment_len=seg).to(dev())
+    with torch.no_grad():
+        for p in (hsa.k_proj_mat, hsa.v_proj_mat):
+            p.copy_(torch.randn(p.shape, generator=g, device=dev()) * (0 if zeros else 0.1))
+        kc, vc = hsa.compress_kv_cache(k, v)
+        out, given = hsa(q, k, v), hsa(q, k, v, k_coarse=kc, v_coarse=vc)
+    if zeros:
+        assert torch.equal(out, given)
+    else:       # float32 sums of another order: a slot may round to the bf16 number next to it
+        max_abs, mean_rel = attention_error(to_np(out), to_np(given))
+        assert max_abs < 2e-2 and mean_rel < 1e-3

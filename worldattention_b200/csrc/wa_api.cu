@@ -223,6 +223,7 @@ extern "C" int wa_hsa_forward(const wa_hsa_params *p, int *used_tuned, void *str
 
     bool prepared = false;
     const int32_t *order = nullptr;
+    int routing_ctas = 0;      // that the compression has beside it, one to an SM, where their number is known
     if (p->index_in) {
         index = const_cast<int32_t *>(p->index_in);
         num = const_cast<int32_t *>(p->num_in);
@@ -242,6 +243,7 @@ extern "C" int wa_hsa_forward(const wa_hsa_params *p, int *used_tuned, void *str
             order = job.order;
         }
         job.release_at_start = compress_inline;
+        if (compress_inline) routing_ctas = p->H * route_short_parts(p->B, w.Nq, w.Nkv, p->D, true);
         if ((rc = route_fused_launch(q_pooled, k_pooled, p->B, p->H, w.Nq, w.Nkv, p->D, p->tau_min, p->tau_max,
                                      p->topk_per_head, block_attn, index, num, thresholds, gini, counters, job, stream,
                                      /*whole_order=*/p->index_out != nullptr || p->thresholds_out != nullptr)))
@@ -253,7 +255,7 @@ extern "C" int wa_hsa_forward(const wa_hsa_params *p, int *used_tuned, void *str
     if (compress_inline) {
         if ((rc = compress_kv_launch(&p->k, &p->v, &kc, &vc, p->B, p->Lkv, p->H, p->D, p->proj_segment_len, p->block_size, p->k_proj,
                                      p->v_proj, p->proj_dtype, p->proj_rank, p->proj_cols, /*beside_routing=*/!p->index_in, stream,
-                                     /*ahead=*/rounded && !p->index_in)))
+                                     /*ahead=*/rounded && !p->index_in, routing_ctas)))
             return rc;
     }
 

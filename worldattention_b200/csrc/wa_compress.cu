@@ -195,18 +195,24 @@ compress_cluster_kernel(const T *__restrict__ k, const T *__restrict__ v, long l
     pdl_wait();       // beside the routing (see compress_kv_launch): done only when that is
 }
 
-// CTAs per group: as many as are resident at once (`ctas`: one or two per SM) where the call has few groups, no share
-// shorter than 64 tokens
-inline int compress_split(long long groups, int longest, int ctas) {
-    int split = groups >= ctas ? 1 : (int)(ctas / groups);
-    if (split > ceil_div(longest, 64)) split = ceil_div(longest, 64);
-    return split > CF_MAX_SPLIT ? CF_MAX_SPLIT : split;
+// CTAs per group: as many as are resident at once (`per_sm`: one or two) where the call has few groups, no share shorter than
+// 64 tokens.  `others`: SMs that the routing beside it keeps busy.  CTAs that find no room wait for a whole round of the others, so that fewer
+// and longer shares are done sooner if all of them fit (8 heads of 3 segments of 635 tokens beside 8 routing CTAs: 6 shares 18.8 us, 5
+// 11); a share twice as long is not (24 heads of 3 segments of 1275 tokens, the whole call: 2 shares 85.7 us, 1 107.7).
+inline int compress_split(long long groups, int longest, int per_sm, int others) {
+    const auto shares = [&](int sms) {
+        const long long ctas = (long long)per_sm * sms;
+        const int split = groups >= ctas ? 1 : (int)(ctas / groups), most = longest < 64 * CF_MAX_SPLIT ? ceil_div(longest, 64) : CF_MAX_SPLIT;
+        return split < most ? split : most;
+    };
+    const int whole = shares(sm_count()), rest = others < sm_count() ? shares(sm_count() - others) : 1;
+    return 2 * rest > whole ? rest : whole;
 }
 
 template <int R, typename T>
 int compress_cluster_launch(const wa_tensor4 *k, const wa_tensor4 *v, const wa_tensor4 *ok, const wa_tensor4 *ov, int B, int L, int HD,
                             int segment_len, int block_size, const void *k_proj, const void *v_proj, int proj_dtype, int proj_rank,
-                            int proj_cols, int rank_full, bool beside, bool ahead, cudaStream_t stream, const char *what) {
+                            int proj_cols, int rank_full, bool beside, int others, bool ahead, cudaStream_t stream, const char *what) {
     const auto kernel = compress_cluster_kernel<R, T>;
     constexpr size_t smem = compress_cluster_smem<R, T>();
     static PerDeviceOnce attr_set;
@@ -216,7 +222,7 @@ int compress_cluster_launch(const wa_tensor4 *k, const wa_tensor4 *v, const wa_t
         attr_set.mark();
     }
     const int n_seg = ceil_div(L, segment_len), longest = L < segment_len ? L : segment_len;
-    const int split = compress_split((long long)(HD / 128) * n_seg * 2 * B, longest, R == 32 ? sm_count() : 2 * sm_count());
+    const int split = compress_split((long long)(HD / 128) * n_seg * 2 * B, longest, R == 32 ? 1 : 2, others);
     const int tokens = ceil_div(ceil_div(longest, split), CF_WARPS) * CF_WARPS;
     cudaLaunchConfig_t cfg{};
     cfg.gridDim = dim3(HD / 128, n_seg * split, 2 * B);
@@ -360,9 +366,17 @@ extern "C" int wa_compress_kv(const wa_tensor4 *k, const wa_tensor4 *v, const wa
                                   proj_cols, /*beside_routing=*/false, (cudaStream_t)stream);
 }
 
+// The calls of compress_cluster_kernel
+static bool cluster_covers(const wa_tensor4 *k, const wa_tensor4 *v, const wa_tensor4 *out_k, int H, int D, int rank_full, int n_seg) {
+    const size_t row4 = 4 * dtype_size(k->dtype);   // bytes of the four columns a lane loads
+    return k->dtype == out_k->dtype && k->stride_h == D && v->stride_h == D && out_k->stride_h == D && (H * D) % 128 == 0 &&
+           rank_full <= 32 && k->stride_b == v->stride_b && k->stride_l == v->stride_l && k->stride_l % 4 == 0 && k->stride_b % 4 == 0 &&
+           (uintptr_t)k->ptr % row4 == 0 && (uintptr_t)v->ptr % row4 == 0 && (long long)n_seg * CF_MAX_SPLIT <= 65535;
+}
+
 int wa::compress_kv_launch(const wa_tensor4 *k, const wa_tensor4 *v, const wa_tensor4 *out_k, const wa_tensor4 *out_v, int B, int L, int H,
                            int D, int segment_len, int block_size, const void *k_proj, const void *v_proj, int proj_dtype, int proj_rank,
-                           int proj_cols, bool beside_routing, cudaStream_t stream, bool ahead) {
+                           int proj_cols, bool beside_routing, cudaStream_t stream, bool ahead, int others) {
     const char *what = "wa_compress_kv";
     WA_REQUIRE(k && v && out_k && out_v && k->ptr && v->ptr && out_k->ptr && out_v->ptr && k_proj && v_proj,
                WA_ERR_ARG, "%s: null pointer", what);
@@ -385,16 +399,11 @@ int wa::compress_kv_launch(const wa_tensor4 *k, const wa_tensor4 *v, const wa_te
     if (compress_sm100_supported(k, v, out_k, out_v, nullptr, nullptr, H, D, proj_dtype, proj_cols, rank_full, k_proj, v_proj))
         return compress_sm100_launch(k, v, out_k, out_v, nullptr, nullptr, 0, B, L, H, D, segment_len, block_size, k_proj, v_proj,
                                      proj_rank, proj_cols, 0, rank_full, stream, beside_routing);
-    const size_t row4 = 4 * dtype_size(k->dtype);   // bytes of the four columns a lane loads
-    const bool fast = k->dtype == out_k->dtype && k->stride_h == D && v->stride_h == D && out_k->stride_h == D && (H * D) % 128 == 0 &&
-                      rank_full <= 32 && k->stride_b == v->stride_b && k->stride_l == v->stride_l && k->stride_l % 4 == 0 &&
-                      k->stride_b % 4 == 0 && (uintptr_t)k->ptr % row4 == 0 && (uintptr_t)v->ptr % row4 == 0 &&
-                      (long long)n_seg * CF_MAX_SPLIT <= 65535;
-    if (fast) {
+    if (cluster_covers(k, v, out_k, H, D, rank_full, n_seg)) {
         const auto launch = k->dtype == WA_BF16 ? (rank_full <= 16 ? compress_cluster_launch<16, __nv_bfloat16> : compress_cluster_launch<32, __nv_bfloat16>)
                                                 : (rank_full <= 16 ? compress_cluster_launch<16, float> : compress_cluster_launch<32, float>);
         return launch(k, v, out_k, out_v, B, L, H * D, segment_len, block_size, k_proj, v_proj, proj_dtype, proj_rank, proj_cols, rank_full,
-                      beside_routing, ahead, stream, what);
+                      beside_routing, others, ahead, stream, what);
     }
     dim3 grid(ceil_div(H * D, CK_THREADS), n_seg, 2 * B);
     compress_kernel<<<grid, CK_THREADS, 0, stream>>>(

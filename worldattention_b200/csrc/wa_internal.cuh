@@ -243,13 +243,17 @@ bool round_kv_supported(const wa_tensor4 *k, const wa_tensor4 *v, int D);
 // `beside`: it starts on what the launch before it leaves free, and completes only after that one.
 int round_kv_launch(const wa_tensor4 *k, const wa_tensor4 *v, int B, int L, int H, int D, void *dst, bool beside, cudaStream_t stream);
 
+// CTAs per head of the routing of short rows (route_head_kernel), 0 where another kernel routes
+int route_short_parts(int B, int Nq, int Nkv, int D, bool beside);
+
 // compress_kv by whichever kernel covers the call (wa_compress.cu).  `beside_routing`: the launch before this one on the
 // stream is a routing kernel that released its dependents at its start (SchedJob::release_at_start).  The two share nothing, so
 // the compression runs on what the routing leaves free of the chip; it completes only after the routing has, so that
 // whatever waits for it may read both.  (One latent frame of 390 tokens over three: the call 49.5 -> 43.1 us.)  `ahead`: the launch
-// after this one reads nothing of it and may start while it runs (where the kernel that covers the call does so).
+// after this one reads nothing of it and may start while it runs (where the kernel that covers the call does so).  `others`: SMs that the launch before it
+// keeps busy.
 int compress_kv_launch(const wa_tensor4 *k, const wa_tensor4 *v, const wa_tensor4 *out_k, const wa_tensor4 *out_v, int B, int L, int H, int D,
                        int segment_len, int block_size, const void *k_proj, const void *v_proj, int proj_dtype, int proj_rank, int proj_cols,
-                       bool beside_routing, cudaStream_t stream, bool ahead = false);
+                       bool beside_routing, cudaStream_t stream, bool ahead = false, int others = 0);
 
 }  // namespace wa

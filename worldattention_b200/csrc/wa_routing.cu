@@ -1634,7 +1634,7 @@ namespace wa {
 // Without, a warp per row, up to eight rows per CTA; while K and V are compressed beside it, two CTAs at most, of sixteen warps (17 rows over
 // 34 of 16 heads, whole calls: 90.5 us with four of eight warps, 92.5 with one of 32, 85.9), and one where that is a row per warp of few
 // keys (10 rows over 20 of 8 heads 51.6 us with two, 49.3 with one; 11 over 33 of 12 44.2 and 42.9; but 14 over 56 79.7 and 80.8).
-static int route_short_parts(int B, int Nq, int Nkv, int D, bool beside) {
+int route_short_parts(int B, int Nq, int Nkv, int D, bool beside) {
     const bool one_round = (long long)B * Nq <= RH_WARPS || (long long)B * ((Nq + 15) / 16) * ((Nkv + 7) / 8) <= RH_WARPS;
     if (D != 128 || Nkv > RH_MAX_KEYS || (long long)B * Nq > RH_MAX_ROWS || (B > 1 && Nkv > 64 && !one_round)) return 0;
     int parts = 1;
