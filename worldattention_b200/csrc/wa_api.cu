@@ -243,7 +243,11 @@ extern "C" int wa_hsa_forward(const wa_hsa_params *p, int *used_tuned, void *str
             order = job.order;
         }
         job.release_at_start = compress_inline;
-        if (compress_inline) routing_ctas = p->H * route_short_parts(p->B, w.Nq, w.Nkv, p->D, true);
+        if (compress_inline) {
+            routing_ctas = p->H * route_short_parts(p->B, w.Nq, w.Nkv, p->D, true);
+            job.beside_sms = compress_cluster_sms(&p->k, &p->v, &kc, &vc, p->B, p->Lkv, p->H, p->D, p->proj_segment_len, p->block_size, p->k_proj,
+                                                  p->v_proj, p->proj_dtype, p->proj_rank, p->proj_cols, routing_ctas);
+        }
         if ((rc = route_fused_launch(q_pooled, k_pooled, p->B, p->H, w.Nq, w.Nkv, p->D, p->tau_min, p->tau_max,
                                      p->topk_per_head, block_attn, index, num, thresholds, gini, counters, job, stream,
                                      /*whole_order=*/p->index_out != nullptr || p->thresholds_out != nullptr)))

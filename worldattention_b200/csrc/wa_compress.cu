@@ -374,6 +374,20 @@ static bool cluster_covers(const wa_tensor4 *k, const wa_tensor4 *v, const wa_te
            (uintptr_t)k->ptr % row4 == 0 && (uintptr_t)v->ptr % row4 == 0 && (long long)n_seg * CF_MAX_SPLIT <= 65535;
 }
 
+int wa::compress_cluster_sms(const wa_tensor4 *k, const wa_tensor4 *v, const wa_tensor4 *out_k, const wa_tensor4 *out_v, int B, int L, int H,
+                             int D, int segment_len, int block_size, const void *k_proj, const void *v_proj, int proj_dtype, int proj_rank,
+                             int proj_cols, int others) {
+    if (segment_len <= 0) segment_len = L;
+    const int n_seg = ceil_div(L, segment_len), longest = L < segment_len ? L : segment_len;
+    const int rank_full = proj_rank < ceil_div(longest, block_size) ? proj_rank : ceil_div(longest, block_size);
+    if (!cluster_covers(k, v, out_k, H, D, rank_full, n_seg) ||
+        compress_sm100_supported(k, v, out_k, out_v, nullptr, nullptr, H, D, proj_dtype, proj_cols, rank_full, k_proj, v_proj))
+        return 0;
+    const int per_sm = rank_full <= 16 ? 2 : 1;
+    const long long groups = (long long)(H * D / 128) * n_seg * 2 * B, ctas = groups * compress_split(groups, longest, per_sm, others);
+    return (int)((ctas < (1ll << 30) ? ctas + per_sm - 1 : (1ll << 30)) / per_sm);
+}
+
 int wa::compress_kv_launch(const wa_tensor4 *k, const wa_tensor4 *v, const wa_tensor4 *out_k, const wa_tensor4 *out_v, int B, int L, int H,
                            int D, int segment_len, int block_size, const void *k_proj, const void *v_proj, int proj_dtype, int proj_rank,
                            int proj_cols, bool beside_routing, cudaStream_t stream, bool ahead, int others) {

@@ -20,6 +20,7 @@ struct SchedJob {
     bool by_counts;         // paired: the routing makes the work order, by the larger count of a pair, not pair_lists_kernel by the tiles
     int *pairs_done;        // paired: CTAs of pair_lists_kernel that are done; zero before it runs
     bool release_at_start;  // the next launch does not wait for the routing (it compresses K and V meanwhile)
+    int beside_sms;         // ... and takes up so many SMs, where that is known (0: it is not)
     int release_dependents_after_rows;   // timing experiment (WA_B200_PDL=2), see route_row
 };
 
@@ -245,6 +246,11 @@ int round_kv_launch(const wa_tensor4 *k, const wa_tensor4 *v, int B, int L, int 
 
 // CTAs per head of the routing of short rows (route_head_kernel), 0 where another kernel routes
 int route_short_parts(int B, int Nq, int Nkv, int D, bool beside);
+
+// SMs that compress_kv_launch takes up if compress_cluster_kernel covers the call, otherwise 0.
+int compress_cluster_sms(const wa_tensor4 *k, const wa_tensor4 *v, const wa_tensor4 *out_k, const wa_tensor4 *out_v, int B, int L, int H,
+                         int D, int segment_len, int block_size, const void *k_proj, const void *v_proj, int proj_dtype, int proj_rank,
+                         int proj_cols, int others);
 
 // compress_kv by whichever kernel covers the call (wa_compress.cu).  `beside_routing`: the launch before this one on the
 // stream is a routing kernel that released its dependents at its start (SchedJob::release_at_start).  The two share nothing, so
