@@ -200,7 +200,7 @@ hsa_fwd_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_cons
     WA_TRACE(0);
     const int lin_tiles = (p.Lc + TILE - 1) / TILE;
 
-    // The softmax threads keep 64 scores, the packed probabilities and the parked sparse result in registers; the
+    // The softmax threads keep 32 scores of two rows, the packed probabilities, the parked sparse result and the gate values in registers; the
     // other four warps need few.  Shift the register file accordingly (whole warpgroups, as the instruction requires).
     if (warp >= 8) {
     asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(REGS_OTHER));
@@ -1418,7 +1418,7 @@ int hsa_sm100_launch_linear(const wa_hsa_params *p, int Lc, const wa_tensor4 *kc
     pl.part_sparse = nullptr; pl.lse_sparse = nullptr; pl.lse_linear = nullptr;
     pl.part_linear = linear_out;
     profile_pause(true);   // the timing bracket of this forward belongs to the sparse-branch kernel
-    const int rc = hsa_sm100_launch(&pl, Lc, kc, vc, zeros /*never read: no item selects a block*/, zeros, nq, 1, workspace, false,
+    const int rc = hsa_sm100_launch(&pl, Lc, kc, vc, zeros /*no item selects a block, but the first id of every row is read*/, zeros, nq, 1, workspace, false,
                                     nullptr, nullptr, stream);
     profile_pause(false);
     return rc;

@@ -1191,7 +1191,7 @@ route_head_kernel(const float *__restrict__ qp, const float *__restrict__ kp, in
 // made by a CTA of its own (the first) beside the rows instead of by the last one after them.
 // Bound by latency (a row is a chain of four block-wide exchanges) and, over thousands of blocks, by the float64 exponentials.
 // 128 threads a row up to 512 blocks; 256 where the row makes its own logits (a warp per eight dot products) or has up to
-// 2048; beyond, 512 threads with three CTAs per SM.
+// 2048; beyond, 512 threads with three CTAs per SM (two from some 12 500 blocks on, by their shared memory).
 // Before, a row was sorted (or, beyond 1024 blocks, selected by radix passes) with its Gini term, and two counters led to the last CTA.
 // 12 heads, 37 rows over 256 blocks: 16.7 -> 7.8 us, the call 134.0 -> 128.6; 74 rows over 11 700: 117 -> 78 with the values in registers (two
 // CTAs per SM and spills), 56 in shared memory.

@@ -309,7 +309,7 @@ struct Params {
                    // neighbouring query blocks, or one in a 128-row tile whose upper rows are computed and dropped)
     int n_items;
     int q_items;   // work items per (batch, head): Nq, or (Nq + 1) / 2 where two query blocks share one
-    const int32_t *index;   // [B,H,Nq,Nkv]
+    const int32_t *index;   // [B,H,Nq,Nkv]; the first id or two of a row are read before its count is known, and not used if it is zero
     const int32_t *num;     // [B,H,Nq]
     const int32_t *order;   // [n_items] work order (heaviest first)
     const int32_t *both;    // PAIR [n_items]: blocks that both query blocks selected; they come first in both lists of `index`
