@@ -91,7 +91,9 @@ def test_routing_beside_the_compression(b, h, nq, nkv, block, fixed):
 # fit beside the routing's CTAs, which keep their SMs to themselves where all fit; 16 rows and 48 keys are the most of one routing CTA
 @pytest.mark.parametrize("b,h,q_len,segments,seg,block", [(1, 8, 600, 3, 635, 64), (1, 12, 1000, 4, 760, 64), (1, 12, 1024, 4, 768, 64), (1, 12, 1025, 4, 769, 64),
                                                           (1, 24, 700, 3, 300, 64), (1, 16, 128, 2, 100, 128), (1, 3, 513, 5, 640, 64), (2, 12, 200, 2, 130, 64),
-                                                          (1, 24, 1100, 12, 70, 64), (1, 74, 64, 1, 600, 64)])
+                                                          (1, 24, 1100, 12, 70, 64), (1, 74, 64, 1, 600, 64),
+                                                          # ... and one of 32 warps beside which more of the compression fits
+                                                          (1, 16, 1071, 2, 1071, 64), (1, 16, 1100, 1, 1100, 64)])
 @pytest.mark.parametrize("zeros", [True, False])
 def test_compression_that_fits_beside_the_routing(b, h, q_len, segments, seg, block, zeros):
     from tests.helpers import attention_error, to_np

@@ -244,9 +244,19 @@ extern "C" int wa_hsa_forward(const wa_hsa_params *p, int *used_tuned, void *str
         }
         job.release_at_start = compress_inline;
         if (compress_inline) {
-            routing_ctas = p->H * route_short_parts(p->B, w.Nq, w.Nkv, p->D, true);
-            job.beside_sms = compress_cluster_sms(&p->k, &p->v, &kc, &vc, p->B, p->Lkv, p->H, p->D, p->proj_segment_len, p->block_size, p->k_proj,
-                                                  p->v_proj, p->proj_dtype, p->proj_rank, p->proj_cols, routing_ctas);
+            const auto sms_beside = [&](int others) {
+                return compress_cluster_sms(&p->k, &p->v, &kc, &vc, p->B, p->Lkv, p->H, p->D, p->proj_segment_len, p->block_size, p->k_proj,
+                                            p->v_proj, p->proj_dtype, p->proj_rank, p->proj_cols, others);
+            };
+            const int parts = route_short_parts(p->B, w.Nq, w.Nkv, p->D, true);
+            job.beside_sms = sms_beside(p->H * parts);
+            if (parts == 2) {
+                const int beside_one = sms_beside(p->H);
+                job.one_part = beside_one > job.beside_sms ||       // more shares, or all of them at once
+                               (beside_one + p->H <= sm_count() && job.beside_sms + 2 * p->H > sm_count());
+                if (job.one_part) job.beside_sms = beside_one;
+            }
+            routing_ctas = job.one_part ? p->H : p->H * parts;
         }
         if ((rc = route_fused_launch(q_pooled, k_pooled, p->B, p->H, w.Nq, w.Nkv, p->D, p->tau_min, p->tau_max,
                                      p->topk_per_head, block_attn, index, num, thresholds, gini, counters, job, stream,

@@ -1274,8 +1274,8 @@ SchedJob hsa_sm100_sched_job(const wa_hsa_params *p, void *workspace) {
     // calls over the same window gain nothing by it (126 us either way) and their routing loses 1 us.
     job.by_head = job.paired && 4ll * p->B * p->H * p->Lkv * p->D > (64ll << 20);
     // The order by tiles costs pair_lists_kernel 3 us at its end.  The routing's own order by counts costs nothing where the call's keys
-    // and values are compressed beside it for longer than it takes (2 items of 24 heads, 6 query blocks over 22, whole calls: 77.9
-    // against 75.0 us; 10 x 20 of 12 heads 40.3 and 39.2).
+    // and values are compressed beside it for longer than it takes (2 items of 24 heads, 6 query blocks over 22, whole calls: 70.1
+    // against 67.6 us; 10 x 20 of 16 heads 39.8 and 36.9).
     job.by_counts = job.paired && !job.by_head && !p->index_in && p->Lc == 0;
     return job;
 }

@@ -21,6 +21,7 @@ struct SchedJob {
     int *pairs_done;        // paired: CTAs of pair_lists_kernel that are done; zero before it runs
     bool release_at_start;  // the next launch does not wait for the routing (it compresses K and V meanwhile)
     int beside_sms;         // ... and takes up so many SMs, where that is known (0: it is not)
+    bool one_part;          // ... and is done sooner beside one routing CTA per head than beside two (see route_short_parts)
     int release_dependents_after_rows;   // timing experiment (WA_B200_PDL=2), see route_row
 };
 

@@ -1631,9 +1631,11 @@ namespace wa {
 // With a batch a CTA takes 32 rows and 32 tiles of logits at a time.  Two rounds of rows pay up to 64 keys (37 rows over 37: 16.5 us against 22.6);
 // beyond, one round of rows or of tiles does (25 rows over 74: 14.7 against 20; whole calls: 37 over 74 144.9 against 147.8,
 // but 37 over 110, two rounds of both, 108.7 against 101.6).
-// Without, a warp per row, up to eight rows per CTA; while K and V are compressed beside it, two CTAs at most, of sixteen warps (17 rows over
-// 34 of 16 heads, whole calls: 90.5 us with four of eight warps, 92.5 with one of 32, 85.9), and one where that is a row per warp of few
-// keys (10 rows over 20 of 8 heads 51.6 us with two, 49.3 with one; 11 over 33 of 12 44.2 and 42.9; but 14 over 56 79.7 and 80.8).
+// Without, a warp per row, up to eight rows per CTA.  While K and V are compressed beside it, two CTAs at most, of sixteen warps (36 rows over
+// 36 of 12 heads, whole calls: 70.1 us with four of eight warps, 62.3 with one of 32, 61.6), but one of 32 where the compression
+// is cut into more shares beside that, or fits beside that only (SchedJob::one_part; of 16 heads 18 rows over 18 46.9 -> 44.0, 17 over 34
+// 68.4 -> 62.7), and one of sixteen where that is a row per warp
+// of few keys (10 rows over 20 of 8 heads 51.6 us with two, 49.3 with one; 11 over 33 of 12 44.2 and 42.9; but 14 over 56 79.7 and 80.8).
 int route_short_parts(int B, int Nq, int Nkv, int D, bool beside) {
     const bool one_round = (long long)B * Nq <= RH_WARPS || (long long)B * ((Nq + 15) / 16) * ((Nkv + 7) / 8) <= RH_WARPS;
     if (D != 128 || Nkv > RH_MAX_KEYS || (long long)B * Nq > RH_MAX_ROWS || (B > 1 && Nkv > 64 && !one_round)) return 0;
@@ -1663,11 +1665,12 @@ int route_fused_launch(const float *q_pooled, const float *k_pooled, int B, int 
     const float scale = (float)pow((double)D, -0.5), span = (float)(tau_max - tau_min);
     const long long bh = (long long)B * H;
 
-    const int parts = ((uintptr_t)q_pooled % 16 == 0) && ((uintptr_t)k_pooled % 16 == 0) ? route_short_parts(B, Nq, Nkv, D, job_in.release_at_start) : 0;
+    const int two_parts = ((uintptr_t)q_pooled % 16 == 0) && ((uintptr_t)k_pooled % 16 == 0) ? route_short_parts(B, Nq, Nkv, D, job_in.release_at_start) : 0;
+    const int parts = job_in.one_part && two_parts > 0 ? 1 : two_parts;
     const bool short_rows = parts > 0;
     // route_topk_kernel, whatever the size -- unless the call's keys and values are compressed meanwhile, which is the longer of the two for
-    // short rows: a CTA per row takes room on most SMs from its clusters (2 items of 24 heads, 6 query blocks over 22, whole calls:
-    // 79.0 us, with a CTA per head 76.6)
+    // short rows: a CTA per row takes room on most SMs from its clusters (8 heads, 10 query blocks over 30, whole calls: 42.0 us, with a
+    // CTA per head 39.4; 12 heads, 7 over 19 38.3 and 35.4; 2 items of 24 heads, 6 over 22 68.8 and 67.4)
     const bool by_count = fixed_num_per_head && !whole_order && !(short_rows && job_in.release_at_start);
     if (!by_count && short_rows) {
         const auto launch = [&](auto width, auto warps) -> cudaError_t {
@@ -1712,7 +1715,7 @@ int route_fused_launch(const float *q_pooled, const float *k_pooled, int B, int 
         const std::integral_constant<int, 8> w8;
         const std::integral_constant<int, 16> w16;
         const std::integral_constant<int, RH_WARPS> w32;
-        const cudaError_t e = B > 1 ? launch_width(w32, w32) : job_in.release_at_start && Nq > 8 ? launch_width(w16, w16) : launch_width(w8, w16);
+        const cudaError_t e = B > 1 || job_in.one_part ? launch_width(w32, w32) : job_in.release_at_start && Nq > 8 ? launch_width(w16, w16) : launch_width(w8, w16);
         if (e != cudaSuccess) return fail((int)e, "wa_hsa_forward(routing of short rows): %s", cudaGetErrorString(e));
         return check_launch("wa_hsa_forward(routing of short rows)");
     }
