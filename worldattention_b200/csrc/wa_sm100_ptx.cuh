@@ -263,7 +263,7 @@ __device__ __forceinline__ float2 ex2_poly2(float2 x) {
     const float2 z = make_float2(__saturatef(fmaf(x.x, -1.0f / 255.0f, 0.50196075f)), __saturatef(fmaf(x.y, -1.0f / 255.0f, 0.50196075f)));
     constexpr float MAGIC = 12582912.0f + 128.0f;                 // 1.5 * 2^23: the integer part of x lands in the low mantissa bits
     const float2 scale = make_float2(-255.0f, -255.0f);
-    const float2 t = __ffma2_rn(z, scale, make_float2(MAGIC, MAGIC));
+    const float2 t = make_float2(fmaf(z.x, -255.0f, MAGIC), fmaf(z.y, -255.0f, MAGIC));      // (packed: 0.3 to 0.6 us of 53 to 83 a call)
     const float2 f = __ffma2_rn(z, scale, __fadd2_rn(make_float2(MAGIC, MAGIC), make_float2(-t.x, -t.y)));   // x - round(x)
     float2 q = __ffma2_rn(f, make_float2(0.0555041f, 0.0555041f), make_float2(0.2402265f, 0.2402265f));
     q = __ffma2_rn(q, f, make_float2(0.6931472f, 0.6931472f));
